@@ -34,7 +34,7 @@ def _newer(target: str, deps) -> bool:
 # Source groups that link into a library of their own: what one model family needs, so that a first start from a source-only checkout
 # compiles that and nothing else.  "ragged" = the ragged-step decoders (seq_ops.py): error state, both linear kernels, norms /
 # activations, recurrent, attention and latent-attention mixers, routed experts, argmax.
-GROUPS = {"ragged": ["lib", "linear_generic", "dense_gemm", "norm_act", "gated_delta", "attention_varlen", "attention_prefill", "attention_decode", "attention_generic",
+GROUPS = {"ragged": ["lib", "linear_generic", "dense_gemm", "norm_act", "gated_delta", "attention_varlen", "attention_prefill", "attention_prefill_umma", "attention_decode", "attention_generic",
                      "attention_api", "elementwise"],
           # latent attention + routed experts: both linear kernels (the tcgen05 one also in its grouped form), norms, the latent mixers incl. the
           # split-KV latent decode kernel, the expert kernels, argmax
@@ -42,20 +42,20 @@ GROUPS = {"ragged": ["lib", "linear_generic", "dense_gemm", "norm_act", "gated_d
           # state-space / linear-attention mixers beside softmax attention, with dense or routed feed-forwards: both linear kernels (the tcgen05 one also
           # grouped), norms, the recurrences, the SIMT attention over the paged cache and the tensor-core prefill and split-KV decode kernels it hands 128-wide
           # heads to, the expert kernels
-          "hybrid": ["lib", "linear_generic", "dense_gemm", "norm_act", "linear_recurrence", "attention_varlen", "attention_prefill", "attention_decode",
+          "hybrid": ["lib", "linear_generic", "dense_gemm", "norm_act", "linear_recurrence", "attention_varlen", "attention_prefill", "attention_prefill_umma", "attention_decode",
                      "attention_generic", "attention_api", "moe_ragged", "elementwise"],
           # softmax attention with a sink, attention without softmax over a window plus pooled blocks, latent attention, ungated routed experts: both linear
           # kernels (the tcgen05 one also grouped), norms, the per-head preparation and pooled-cache kernels, the SIMT attention over the paged cache and the
           # tensor-core kernels it hands 128-wide heads to, the latent mixers incl. the split-KV latent decode kernel, the expert kernels
-          "window": ["lib", "linear_generic", "dense_gemm", "norm_act", "attention_window", "attention_varlen", "attention_prefill", "attention_decode",
+          "window": ["lib", "linear_generic", "dense_gemm", "norm_act", "attention_window", "attention_varlen", "attention_prefill", "attention_prefill_umma", "attention_decode",
                      "attention_generic", "attention_api", "latent_attention", "mla", "moe_ragged", "elementwise"],
           # linear attention with a decay per key row beside attention whose heads mix their scores: both linear kernels, norms, the recurrences, the query / key /
           # value preparation (with the paged attention it shares a file with) and the score-mixing attention, argmax
-          "talking": ["lib", "linear_generic", "dense_gemm", "norm_act", "linear_recurrence", "attention_varlen", "attention_prefill", "attention_talking", "elementwise"],
+          "talking": ["lib", "linear_generic", "dense_gemm", "norm_act", "linear_recurrence", "attention_varlen", "attention_prefill", "attention_prefill_umma", "attention_talking", "elementwise"],
           # windowed attention with kept first tokens beside token-shift linear attention or a delta rule with a decay per key row: both linear kernels (the tcgen05 one
           # also grouped), norms, the recurrences, the per-head preparation, the attention over the paged cache, argmax
           "sliding": ["lib", "linear_generic", "dense_gemm", "norm_act", "linear_recurrence", "gated_delta", "delta_chunk", "attention_window", "attention_varlen",
-                      "attention_prefill", "attention_rows", "elementwise"]}
+                      "attention_prefill", "attention_prefill_umma", "attention_rows", "elementwise"]}
 
 
 def so_path(group=None) -> str:

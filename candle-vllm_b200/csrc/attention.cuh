@@ -48,7 +48,11 @@ struct PrefillExtras {
 void paged_attention_prefill_tc(void* out, const void* q, const void* kc, const void* vc, const uint32_t* block_tables, const uint32_t* cu_q,
                                 const uint32_t* cu_k, int num_seqs, int total_q, int num_heads, int num_kv_heads, int max_blocks, int64_t num_blocks,
                                 float scale, int window, int dtype, cudaStream_t st, int chunk = 0, const PrefillExtras* extras = nullptr);
-// the same kernel with key and value sizes of their own (multiples of 8 up to 128), kept first tokens, capped scores, one gate per output entry, an output pitch; bf16
+// the softmax form on tcgen05 (attention_prefill_umma.cu): false = not covered (misaligned rows, scale <= 0), nothing launched
+bool paged_attention_prefill_umma(void* out, const void* q, const void* kc, const void* vc, const uint32_t* block_tables, const uint32_t* cu_q, const uint32_t* cu_k,
+                                  int num_seqs, int total_q, int num_heads, int num_kv_heads, int max_blocks, int64_t num_blocks, float scale, int window, int dtype,
+                                  int chunk, const float* sink, cudaStream_t st);
+// the mma.sync kernel with key and value sizes of their own (multiples of 8 up to 128), kept first tokens, capped scores, one gate per output entry, an output pitch; bf16
 bool paged_attention_prefill_sel_supported(int dk, int dv, int block_size, const void* q, const void* kc, const void* vc);
 void paged_attention_prefill_sel(void* out, int64_t ld_out, const void* q, const void* kc, const void* vc, const uint32_t* block_tables, const uint32_t* cu_q,
                                  const uint32_t* cu_k, int num_seqs, int total_q, int num_heads, int num_kv_heads, int dk, int dv, int max_blocks, float scale, int chunk,

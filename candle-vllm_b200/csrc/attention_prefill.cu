@@ -452,6 +452,10 @@ bool paged_attention_prefill_tc_supported(int head_dim, int block_size, int dtyp
 void paged_attention_prefill_tc(void* out, const void* q, const void* kc, const void* vc, const uint32_t* block_tables, const uint32_t* cu_q,
                                 const uint32_t* cu_k, int num_seqs, int total_q, int num_heads, int num_kv_heads, int max_blocks, int64_t num_blocks,
                                 float scale, int window, int dtype, cudaStream_t st, int chunk, const PrefillExtras* extras) {
+    // the softmax form runs on tcgen05; sigmoid weights and rows that do not start on 16 bytes stay here
+    if (!(extras && extras->sigmoid) && paged_attention_prefill_umma(out, q, kc, vc, block_tables, cu_q, cu_k, num_seqs, total_q, num_heads, num_kv_heads, max_blocks,
+                                                                     num_blocks, scale, window, dtype, chunk, extras ? extras->sink : nullptr, st))
+        return;
     CUtensorMap km, vm;
     if (!make_kv_map(&km, kc, num_blocks, num_kv_heads, dtype) || !make_kv_map(&vm, vc, num_blocks, num_kv_heads, dtype)) {
         set_error(kErrCuda, "paged_attention_prefill: cuTensorMapEncodeTiled failed");

@@ -1,0 +1,480 @@
+// attention_prefill_umma.cu -- prompt attention over the paged KV cache on tcgen05: the softmax form of attention_prefill.cu (128-wide heads, 64-token
+// blocks, 16-bit cache; causal, with window, chunk and sink as there) with both products on the 5th-generation tensor cores.
+//
+// One CTA = 256 query rows of one kv head: two M = 128 tiles whose rows are (token, head) pairs, 128 / hp tokens x hp heads of the group, so the heads that share
+// keys share the tile and a short portion still fills its rows.  Keys and values are walked in tiles of 128 tokens (two pages).
+//   warps 0-3, 4-7  softmax of tile 0 / 1: thread = row; the row's 128 scores come from TMEM into registers, maximum and sum stay in the thread, P goes back to
+//                   TMEM as 16 bits over the scores it was made from, and the O of the row is rescaled in TMEM only when its maximum has grown by more than
+//                   2^8 since the last time (a stale maximum scales numerator and denominator alike; P <= 2^8 keeps its relative precision in 16 bits)
+//   warp 8          TMA: Q once (64 KB), then K and V tiles of 32 KB through a ring of five
+//   warp 9          MMA issue: S_i = Q_i K^T (128 x 128 x 128, both operands in shared memory), O_i += P_i V (P from TMEM, V token rows as the MN-major operand)
+// The two tiles alternate on the tensor pipe: while one tile's softmax runs, the other tile's O += P V and next S are computed.
+// TMEM: S_0, S_1 (P_i over the first half of S_i), O_0, O_1, 128 columns each = all 512.
+// Order on the tensor pipe is the only thing that protects P_i from the next S_i (same issuing thread, in order); the barrier of S_i(j) also says that
+// O_i += P_i V of step j - 1 is complete, because a commit covers every MMA issued before it.
+//
+// Bound: exp2 (16 per clock and SM = 1024 clocks per 128 x 128 tile) and the tensor pipe (1024 clocks for the tile's two products) are level.
+// Measured against the mma.sync kernel (B200, bf16, 32 heads / 8 kv heads): see the table at paged_attention_prefill_tc.
+#include <cuda.h>
+
+#include <type_traits>
+
+#include "attention.cuh"
+#include "tc_common.cuh"
+
+namespace b200 {
+
+namespace {
+
+using namespace tc;
+
+constexpr int kHd = 128, kPg = 64, kKt = 128;           // head size, tokens per page, keys per tile
+constexpr int kThreadsU = 12 * 32;                        // two softmax warpgroups, one for TMA and MMA (two of its warps idle)
+// registers a thread after the split: 2 x 128 x 216 + 128 x 72 = 64512 = the 384 x 168 of the launch
+constexpr int kRegsSoftmax = 216, kRegsOther = 72;
+static_assert(256 * kRegsSoftmax + 128 * kRegsOther <= kThreadsU * 168, "register split");
+constexpr int kTileBytes = 128 * kHd * 2;               // a Q, K or V tile: two halves of 64 dims, 128 rows of 128 bytes each
+constexpr int kRing = 5;
+constexpr int kSmQ = 0, kSmKv = 2 * kTileBytes, kSmBar = kSmKv + kRing * kTileBytes;
+constexpr int kNumBars = 1 + 2 * kRing + 6;             // q_full, kv_full[], kv_empty[], s_full[2], p_ready[2], o_full[2]
+constexpr int kSmFlag = kSmBar + kNumBars * 8, kSmTmem = kSmFlag + 4;
+constexpr int kSmemU = kSmTmem + 12;
+static_assert(kSmemU <= 232448, "shared memory");
+
+struct UmmaPrefillParams {
+    void* out;
+    const uint32_t* block_tables; const uint32_t* cu_q; const uint32_t* cu_k;
+    int num_seqs, num_heads, num_kv_heads, max_blocks, window, chunk;
+    int hp;                          // heads per tile (power of two, divides the heads of a kv head)
+    int tiles;                       // grid.y: upper bound of the token tiles over all sequences
+    float scale_log2;                // > 0
+    const float* sink;               // [H] or null
+};
+
+// Bounded wait: a wait that does not end (it always does unless a copy or an MMA was lost) gives up, raises the CTA's flag and lets every role leave.
+__device__ __forceinline__ bool wait_or_flag(uint32_t bar, uint32_t parity, volatile uint32_t* flag) {
+    for (uint32_t i = 0; i < (1u << 22); ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n"
+            "}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+        if ((i & 255u) == 255u && *flag) return false;
+    }
+    *flag = 1u;
+    return false;
+}
+__device__ __forceinline__ void tma_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst), "l"(map), "r"(bar),
+                 "r"(c0), "r"(c1), "r"(c2)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(dst), "l"(map), "r"(bar),
+                 "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+                 : "memory");
+}
+__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// MN-major operand, 128-byte swizzle: 64 entries of a row are contiguous, the next 64 lie `lead` bytes further, 8-row groups 1024 bytes apart
+__device__ __forceinline__ uint64_t make_mn_desc(uint32_t saddr, uint32_t lead) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
+    d |= (uint64_t)(lead >> 4) << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+__device__ __forceinline__ void ld32(uint32_t taddr, uint32_t* v) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,"
+        "%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+          "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
+          "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]),
+          "=r"(v[31])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
+template <typename T> __device__ __forceinline__ uint32_t pack2(float lo, float hi);
+template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, float hi) { __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi); return *reinterpret_cast<uint32_t*>(&v); }
+template <> __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) { __half2 v = __floats2half2_rn(lo, hi); return *reinterpret_cast<uint32_t*>(&v); }
+// two f32 operations in one issue slot
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\nfma.rn.f32x2 d, a, b, c;\nmov.b64 {%0, %1}, d;\n}\n"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nadd.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}\n"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+
+constexpr float kSlack = 8.f;        // a row's O is rescaled when its maximum has grown by more than this (log2 units)
+
+template <typename T>
+__global__ void __launch_bounds__(kThreadsU, 1)
+paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
+                               const UmmaPrefillParams p) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t sb = smem_u32(smem);
+    const int tp = 128 / p.hp;                                       // tokens per M tile; a CTA has two
+
+    // which (sequence, tile of 2 tp tokens)?  Tiles are numbered sequence by sequence and dealt out from the last: the rows with most keys start first
+    int seq = -1, tile = 0;
+    {
+        const int want = p.tiles - 1 - (int)blockIdx.y;
+        int acc = 0;
+        for (int s = 0; s < p.num_seqs; ++s) {
+            const int nt = ((int)(p.cu_q[s + 1] - p.cu_q[s]) + 2 * tp - 1) / (2 * tp);
+            if (want < acc + nt) { seq = s; tile = want - acc; break; }
+            acc += nt;
+        }
+    }
+    if (seq < 0) return;
+    const int head0 = blockIdx.x * p.hp, kvh = head0 / (p.num_heads / p.num_kv_heads);
+    const int q_begin = (int)p.cu_q[seq], qlen = (int)p.cu_q[seq + 1] - q_begin, klen = (int)(p.cu_k[seq + 1] - p.cu_k[seq]);
+    const int q0 = tile * 2 * tp, pos0 = klen - qlen + q0;           // first token of the CTA and its position
+    int first_key = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
+    if (p.chunk > 0) first_key = max(first_key, (pos0 / p.chunk) * p.chunk);
+    const int kt0 = first_key & ~(kKt - 1), page_lo = first_key / kPg, page_end = (klen - 1) / kPg;
+    // key tiles of the two M tiles (none when the tile has no token)
+    int nk[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int toks = min(tp, qlen - q0 - i * tp);
+        nk[i] = toks > 0 ? (pos0 + i * tp + toks - 1 - kt0) / kKt + 1 : 0;
+    }
+    const int n = max(nk[0], nk[1]);
+
+    const uint32_t bars = sb + kSmBar;
+    const uint32_t q_full = bars;
+    auto kv_full = [&](int s) { return bars + (1 + s) * 8; };
+    auto kv_empty = [&](int s) { return bars + (1 + kRing + s) * 8; };
+    auto s_full = [&](int i) { return bars + (1 + 2 * kRing + i) * 8; };
+    auto p_ready = [&](int i) { return bars + (3 + 2 * kRing + i) * 8; };
+    auto o_full = [&](int i) { return bars + (5 + 2 * kRing + i) * 8; };
+    volatile uint32_t* flag = reinterpret_cast<volatile uint32_t*>(smem + kSmFlag);
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + kSmTmem);
+    if (threadIdx.x == 0) {
+        *flag = 0u;
+        mbar_init(q_full, 1);
+        for (int s = 0; s < kRing; ++s) { mbar_init(kv_full(s), 1); mbar_init(kv_empty(s), 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(s_full(i), 1); mbar_init(p_ready(i), 4); mbar_init(o_full(i), 1); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 9) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
+    if (warp == 8) {
+        // ============================================ TMA ===================================================================
+        const bool leader = elect_one();
+        const uint32_t* table = p.block_tables + (int64_t)seq * p.max_blocks;
+        if (leader) {
+            mbar_expect_tx(q_full, 2 * kTileBytes);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) tma_3d(sb + kSmQ + i * kTileBytes + h * (kTileBytes / 2), &qmap, q_full, h * 64, head0, q_begin + q0 + i * tp);
+        }
+        __syncwarp();
+        int it = 0;                                                  // K(0), V(0), K(1), V(1), ...
+        bool ok = true;
+        for (int j = 0; j < n && ok; ++j) {
+            const int pg = (kt0 + j * kKt) / kPg;
+            // a page outside the keys of this CTA (before the window, past the context) is replaced by a neighbour that is inside: its scores are masked, and
+            // the values past the context are zeroed below
+            const int b0 = (int)table[min(max(pg, page_lo), page_end)], b1 = (int)table[min(max(pg + 1, page_lo), page_end)];
+#pragma unroll
+            for (int kv = 0; kv < 2; ++kv, ++it) {
+                const int s = it % kRing;
+                ok = ok && wait_or_flag(kv_empty(s), ((it / kRing) & 1) ^ 1, flag);
+                if (!ok) break;
+                if (leader) {
+                    const CUtensorMap* map = kv ? &vmap : &kmap;
+                    const uint32_t dst = sb + kSmKv + s * kTileBytes;
+                    mbar_expect_tx(kv_full(s), kTileBytes);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        tma_4d(dst + h * (kTileBytes / 2), map, kv_full(s), h * 64, kvh, 0, b0);
+                        tma_4d(dst + h * (kTileBytes / 2) + kPg * 128, map, kv_full(s), h * 64, kvh, 0, b1);
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        // nothing may be in flight into this CTA's shared memory when it leaves: the copies of the last round are awaited by their readers, unless a wait was given up
+        if (!ok) {
+            for (int k = max(0, it - kRing); k < it; ++k)
+                for (uint32_t i = 0; i < (1u << 20); ++i) {
+                    uint32_t done;
+                    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                                 : "=r"(done) : "r"(kv_full(k % kRing)), "r"((uint32_t)(k / kRing) & 1u) : "memory");
+                    if (done) break;
+                }
+        }
+    } else if (warp == 9) {
+        // ============================================ MMA ===================================================================
+        const bool leader = elect_one();
+        const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+        const uint32_t idesc_s = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(kKt >> 3) << 17) | (8u << 24);        // M 128, N 128, both K-major
+        const uint32_t idesc_o = idesc_s | (1u << 16);                                                                       // B (values) MN-major
+        bool ok = wait_or_flag(q_full, 0, flag);
+        auto scores = [&](int i, int stage) {
+            if (leader) {
+                const uint64_t a = make_b_desc(sb + kSmQ + i * kTileBytes), b = make_b_desc(sb + kSmKv + stage * kTileBytes);
+#pragma unroll
+                for (int ks = 0; ks < 8; ++ks) {
+                    const uint64_t o = (uint64_t)(((ks >> 2) * (kTileBytes / 2) + (ks & 3) * 32) >> 4);
+                    mma_ss(tmem + i * 128, a + o, b + o, idesc_s, ks > 0 ? 1u : 0u);
+                }
+                tc_commit(s_full(i));
+            }
+            __syncwarp();
+        };
+        ok = ok && wait_or_flag(kv_full(0), 0, flag);
+        if (ok) {
+            tc_fence_after();
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                if (nk[i] > 0) scores(i, 0);
+            if (leader) tc_commit(kv_empty(0));
+            __syncwarp();
+        }
+        int it = 1;
+        for (int j = 0; j < n && ok; ++j) {
+            const int vs = it % kRing, vp = (it / kRing) & 1, ks = (it + 1) % kRing, kp = ((it + 1) / kRing) & 1;
+            it += 2;
+            ok = wait_or_flag(kv_full(vs), vp, flag);
+            if (ok && j + 1 < n) ok = wait_or_flag(kv_full(ks), kp, flag);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                if (!ok || j >= nk[i]) continue;
+                ok = wait_or_flag(p_ready(i), j & 1, flag);
+                if (!ok) continue;
+                tc_fence_after();
+                if (leader) {
+                    const uint64_t b = make_mn_desc(sb + kSmKv + vs * kTileBytes, kTileBytes / 2);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        tc_mma_ts(tmem + 256 + i * 128, tmem + i * 128 + k * 8, b + (uint64_t)(k * 16 * 128 >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+                    if (j + 1 == nk[i]) tc_commit(o_full(i));
+                }
+                __syncwarp();
+                if (j + 1 < nk[i]) scores(i, ks);
+            }
+            if (leader) {
+                tc_commit(kv_empty(vs));
+                if (j + 1 < n) tc_commit(kv_empty(ks));
+            }
+            __syncwarp();
+        }
+    }
+    } else {
+        // ============================================ SOFTMAX ===============================================================
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
+        const int i = warp >> 2, row = (warp & 3) * 32 + lane;
+        const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
+        const uint32_t s_t = tmem + i * 128 + lane_addr, o_t = tmem + 256 + i * 128 + lane_addr;
+        const int tok = q0 + i * tp + row / p.hp, head = head0 + row % p.hp;       // token within the sequence
+        const int pos = klen - qlen + tok;
+        int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;                     // first visible key
+        if (p.chunk > 0) lo = max(lo, (pos / p.chunk) * p.chunk);
+        const int w_first = q0 + i * tp + ((warp & 3) * 32) / p.hp, w_last = q0 + i * tp + ((warp & 3) * 32 + 31) / p.hp;     // the warp's tokens
+        const int w_min_pos = klen - qlen + w_first;
+        int w_max_lo = p.window > 0 ? max(0, klen - qlen + w_last - p.window + 1) : 0;
+        if (p.chunk > 0) w_max_lo = max(w_max_lo, ((klen - qlen + w_last) / p.chunk) * p.chunk);
+        const float sink = p.sink ? p.sink[head] * 1.4426950408889634f : -INFINITY;
+        float m = sink;                                                             // what the row's P are scaled by (log2 units)
+        float2 l2 = make_float2(sink != -INFINITY ? 1.f : 0.f, 0.f);
+        bool ok = true;
+        const int nki = nk[i];
+        for (int j = 0; j < nki; ++j) {
+            ok = wait_or_flag(s_full(i), j & 1, flag);
+            if (!ok) break;
+            tc_fence_after();
+            uint32_t s[128];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) ld32(s_t + c * 32, s + c * 32);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            const int k0 = kt0 + j * kKt;
+            if (k0 + kKt - 1 > w_min_pos || k0 < w_max_lo) {
+                const int hi_c = pos - k0, lo_c = lo - k0;
+#pragma unroll
+                for (int c = 0; c < 128; ++c)
+                    if (c > hi_c || c < lo_c) s[c] = 0xff800000u;
+            }
+            float mx[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) mx[c] = __uint_as_float(s[c]);
+#pragma unroll
+            for (int c = 4; c < 128; ++c) mx[c & 3] = fmaxf(mx[c & 3], __uint_as_float(s[c]));
+            const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
+            if (__any_sync(0xffffffffu, top > m + kSlack)) {
+                const float mn = fmaxf(m, top);
+                const float corr = mn == -INFINITY ? 1.f : ex2(m - mn);
+                m = mn;
+                l2.x *= corr; l2.y *= corr;
+                if (j > 0) {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        uint32_t o[16];
+                        tc_ld16(o_t + c * 16, o);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * corr);
+                        tc_st16(o_t + c * 16, o);
+                    }
+                }
+            }
+            // a row that has seen no visible key yet keeps m = -inf: subtract 0, so that its exp2 are 0 and never NaN
+            const float sub = m == -INFINITY ? 0.f : -m;
+            const float2 sc = make_float2(p.scale_log2, p.scale_log2), sb2 = make_float2(sub, sub);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                uint32_t pk[8];
+                float2 part = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    float2 x = fma2(make_float2(__uint_as_float(s[c * 16 + 2 * e]), __uint_as_float(s[c * 16 + 2 * e + 1])), sc, sb2);
+                    x.x = ex2(x.x); x.y = ex2(x.y);
+                    part = add2(part, x);
+                    pk[e] = pack2<T>(x.x, x.y);
+                }
+                l2 = add2(l2, part);
+                asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(s_t + c * 8), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]),
+                             "r"(pk[3]), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7])
+                             : "memory");
+            }
+            if (k0 + kKt > klen) {
+                // rows of V past the context hold whatever the block contains (0 * NaN would poison O): zero them before this tile's product
+                const int vi = 2 * j + 1, vs = vi % kRing;
+                ok = wait_or_flag(kv_full(vs), (vi / kRing) & 1, flag);
+                if (!ok) break;
+                uint8_t* v = smem + kSmKv + vs * kTileBytes;
+                const int r0 = klen - k0;                                           // >= 1: the tile holds the row's own key or an earlier one
+                for (int idx = (warp & 3) * 32 + lane; idx < (kKt - r0) * 16; idx += 128) {
+                    const int r = r0 + (idx >> 4), ch = idx & 15;
+                    *reinterpret_cast<int4*>(v + (ch >> 3) * (kTileBytes / 2) + r * 128 + ((ch & 7) << 4)) = make_int4(0, 0, 0, 0);
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_ready(i));
+        }
+        if (nki > 0 && ok && wait_or_flag(o_full(i), 0, flag)) {
+            tc_fence_after();
+            const float l = l2.x + l2.y, inv = l > 0.f ? 1.f / l : 0.f;
+            T* dst = static_cast<T*>(p.out) + ((int64_t)(q_begin + tok) * p.num_heads + head) * kHd;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                uint32_t o[32];
+                ld32(o_t + c * 32, o);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (tok < qlen) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        uint4 w;
+                        w.x = pack2<T>(__uint_as_float(o[8 * e]) * inv, __uint_as_float(o[8 * e + 1]) * inv);
+                        w.y = pack2<T>(__uint_as_float(o[8 * e + 2]) * inv, __uint_as_float(o[8 * e + 3]) * inv);
+                        w.z = pack2<T>(__uint_as_float(o[8 * e + 4]) * inv, __uint_as_float(o[8 * e + 5]) * inv);
+                        w.w = pack2<T>(__uint_as_float(o[8 * e + 6]) * inv, __uint_as_float(o[8 * e + 7]) * inv);
+                        *reinterpret_cast<uint4*>(dst + c * 32 + e * 8) = w;
+                    }
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 9) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+    }
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encode_fn() {
+    static EncodeTiledFn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess
+                   ? reinterpret_cast<EncodeTiledFn>(f) : nullptr;
+    }();
+    return fn;
+}
+bool make_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box, bool bf16) {
+    const cuuint32_t one[4] = {1, 1, 1, 1};
+    return encode_fn()(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, rank, const_cast<void*>(base), dims, strides, box, one,
+                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+}  // namespace
+
+// q, out [total_q, H, 128]; caches [*, 64, G, 128]; false: not covered (a scale of zero or below, rows that do not start on 16 bytes), nothing was launched
+bool paged_attention_prefill_umma(void* out, const void* q, const void* kc, const void* vc, const uint32_t* block_tables, const uint32_t* cu_q, const uint32_t* cu_k,
+                                  int num_seqs, int total_q, int num_heads, int num_kv_heads, int max_blocks, int64_t num_blocks, float scale, int window, int dtype,
+                                  int chunk, const float* sink, cudaStream_t st) {
+    if (!(scale > 0.f) || (((uintptr_t)q | (uintptr_t)out | (uintptr_t)kc | (uintptr_t)vc) & 15) || !encode_fn()) return false;
+    const bool bf16 = dtype == B200_BF16;
+    const int group = num_heads / num_kv_heads;
+    int hp = 1;
+    while (hp < 128 && group % (2 * hp) == 0) hp *= 2;               // heads that share a tile: the largest power of two in the group
+    const int tp = 128 / hp;
+    const int tiles = total_q / (2 * tp) + num_seqs;                 // >= sum of ceil(q_len / 2 tp)
+    if (tiles > 65535) return false;
+    CUtensorMap qm, km, vm;
+    {
+        const cuuint64_t dims[3] = {(cuuint64_t)kHd, (cuuint64_t)num_heads, (cuuint64_t)total_q}, strides[2] = {kHd * 2, (cuuint64_t)num_heads * kHd * 2};
+        const cuuint32_t box[3] = {64, (cuuint32_t)hp, (cuuint32_t)tp};
+        if (!make_map(&qm, q, 3, dims, strides, box, bf16)) return false;
+    }
+    {
+        const cuuint64_t dims[4] = {(cuuint64_t)kHd, (cuuint64_t)num_kv_heads, (cuuint64_t)kPg, (cuuint64_t)num_blocks};
+        const cuuint64_t strides[3] = {kHd * 2, (cuuint64_t)num_kv_heads * kHd * 2, (cuuint64_t)kPg * num_kv_heads * kHd * 2};
+        const cuuint32_t box[4] = {64, 1, (cuuint32_t)kPg, 1};
+        if (!make_map(&km, kc, 4, dims, strides, box, bf16) || !make_map(&vm, vc, 4, dims, strides, box, bf16)) return false;
+    }
+    const UmmaPrefillParams p{out, block_tables, cu_q, cu_k, num_seqs, num_heads, num_kv_heads, max_blocks, window, chunk, hp, tiles, scale * 1.4426950408889634f, sink};
+    const dim3 grid(num_heads / hp, tiles);
+    if (bf16) {
+        ensure_dynamic_smem(reinterpret_cast<const void*>(paged_attn_prefill_umma_kernel<__nv_bfloat16>), kSmemU);
+        paged_attn_prefill_umma_kernel<__nv_bfloat16><<<grid, kThreadsU, kSmemU, st>>>(qm, km, vm, p);
+    } else {
+        ensure_dynamic_smem(reinterpret_cast<const void*>(paged_attn_prefill_umma_kernel<__half>), kSmemU);
+        paged_attn_prefill_umma_kernel<__half><<<grid, kThreadsU, kSmemU, st>>>(qm, km, vm, p);
+    }
+    count_launch();
+    check_launch("paged_attention_prefill");
+    return true;
+}
+
+}  // namespace b200

@@ -1,0 +1,65 @@
+"""GPU parity of the tcgen05 prompt-attention kernel (csrc/attention_prefill_umma.cu) at the sizes where its tiling can go wrong, against a float64 restatement
+in torch.  Tolerance: P and the output are rounded to 16 bits, 2^-9 relative each for bf16 (2^-12 for f16), rounding errors of the terms of one output add up
+in quadrature: relative Frobenius below 2^-8 (2^-11)."""
+import numpy as np
+import pytest
+import torch
+
+import candle_vllm_b200 as pkg
+from tests.gpu_util import DEV
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(q, kc, vc, tables, qlens, klens, scale, window):
+    out, at = [], 0
+    for i, (n, k) in enumerate(zip(qlens, klens)):
+        ids = torch.as_tensor(tables[i][: -(-k // 64)], device=q.device)
+        keys, values = kc[ids].flatten(0, 1)[:k].double(), vc[ids].flatten(0, 1)[:k].double()
+        g = q.shape[1] // keys.shape[1]
+        keys, values = keys.repeat_interleave(g, 1), values.repeat_interleave(g, 1)
+        s = torch.einsum("qhd,khd->hqk", q[at:at + n].double(), keys) * scale
+        pos, key = torch.arange(k - n, k, device=q.device)[:, None], torch.arange(k, device=q.device)[None]
+        hidden = key > pos if not window else (key > pos) | (key <= pos - window)
+        out.append(torch.einsum("hqk,khd->qhd", torch.softmax(s.masked_fill(hidden, -np.inf), 2), values))
+        at += n
+    return torch.cat(out)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("H,kvh,qlens,cached,window,loud", [
+    (4, 4, [1, 127, 128, 129, 257], [0, 1, 127, 128, 200], None, 1.0),      # one head per tile: 128 / 256 token tiles and one either side
+    (8, 4, [63, 64, 65, 128], [64, 63, 0, 129], None, 1.0),                 # two heads per tile
+    (32, 8, [1, 31, 32, 33, 63, 64, 65], [0, 700, 64, 31, 65, 64, 190], None, 1.0),   # four
+    (24, 4, [70, 5], [10, 300], None, 1.0),                                 # groups of six: two heads share a tile
+    (7, 1, [150], [77], None, 1.0),                                         # an odd group
+    (32, 1, [9, 4, 3], [500, 0, 61], None, 1.0),                            # four tokens per tile
+    (8, 2, [300, 40], [100, 250], 96, 1.0),                                 # window: starts inside the second page of a key tile
+    (8, 2, [130], [400], 1, 1.0),                                           # a window of the token itself
+    (8, 2, [200], [900], None, 6.0),                                        # loud scores: the running maximum moves by more than the slack, many times
+])
+def test_tiles_heads_and_edges(dtype, H, kvh, qlens, cached, window, loud):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(H * 1000 + len(qlens))
+    klens = [a + b for a, b in zip(qlens, cached)]
+    used = [-(-k // 64) for k in klens]
+    pool = sum(used) + 1
+    perm = np.random.default_rng(H).permutation(pool)
+    tables, at = [], 0
+    for n in used:
+        tables.append([int(x) for x in perm[at:at + n]])
+        at += n
+    mk = lambda *shape: torch.randn(shape, generator=g, device=DEV).to(dtype)
+    q, k, v = mk(sum(qlens), H, 128) * loud, mk(sum(qlens), kvh, 128), mk(sum(qlens), kvh, 128)
+    kc, vc = torch.full((pool, 64, kvh, 128), float("nan"), dtype=dtype, device=DEV), torch.full((pool, 64, kvh, 128), float("nan"), dtype=dtype, device=DEV)
+    for i, c in enumerate(cached):                  # only what a context holds is written: everything else of the pool is NaN
+        for j in range(-(-c // 64)):
+            w = min(64, c - j * 64)
+            kc[tables[i][j], :w], vc[tables[i][j], :w] = mk(w, kvh, 128), mk(w, kvh, 128)
+    prep = pkg.prepare_prompt([list(range(n)) for n in klens], tables, 64, cached, chunk_size=max(qlens))
+    _, _, meta = pkg.inputs.to_device(prep)
+    out = pkg.PagedAttention(H, 128, 128 ** -0.5, kvh, sliding_window=window).forward(q, k, v, None, kc, vc, meta)
+    ref = _reference(q, kc, vc, tables, qlens, klens, 128 ** -0.5, window)
+    assert torch.isfinite(out).all()
+    err = float((out.double() - ref).norm() / ref.norm())
+    assert err < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11), err
