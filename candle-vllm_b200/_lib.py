@@ -25,7 +25,7 @@ SYMBOLS = [
     "qmatmul_workspace_bytes", "qmatmul_f32", "qmatmul_f16act", "qmatmul_slab_count", "qmatmul_f16act_slabs", "b200_llama_peer_inbox_bytes", "b200_llama_set_peer_inboxes", "b200_llama_peer_timeouts", "b200_ipc_alloc", "b200_ipc_open", "b200_ipc_close", "b200_ipc_free",
     "dequantize_f32", "linear_16bit", "fp8_matmul", "nvfp4_matmul", "mxfp4_matmul",
     "concat_and_cache_mla", "mla_paged_decode_workspace_bytes", "mla_paged_attention",
-    "topk_softmax", "sort_expert_assignments", "moe_gemm_workspace_bytes", "moe_gemm_gguf", "moe_gemm_fp8_workspace_bytes", "moe_gemm_fp8",
+    "topk_softmax", "sort_expert_assignments", "moe_gemm_workspace_bytes", "moe_gemm_gguf", "moe_block_supported", "moe_block_workspace_bytes", "moe_block_gguf", "moe_gemm_fp8_workspace_bytes", "moe_gemm_fp8",
     "rms_norm", "fused_rope_f32", "silu_mul", "add_f32", "cast", "embedding_f32", "argmax_f32", "rope_and_cache",
     "b200_llama_create", "b200_llama_destroy", "b200_llama_set_layer", "b200_llama_set_globals", "b200_llama_set_layer_ex", "b200_llama_set_globals_ex",
     "b200_llama_set_kv_cache", "b200_llama_set_comm", "b200_llama_decode", "b200_llama_decode_resident", "b200_llama_linear_chain", "b200_llama_uses_layer_kernel", "b200_llama_mega_trace",
@@ -74,7 +74,7 @@ GROUP_SYMBOLS = {
                          "qk_head_norm_rope_cache", "paged_attention_varlen_ex", "paged_attention_rows_supported", "paged_attention_rows", "linear_grouped"],
 }
 _RESTYPES = {"b200_last_error_message": C.c_char_p, "paged_attention_decode_workspace_bytes": C.c_size_t, "qmatmul_workspace_bytes": C.c_size_t,
-             "moe_gemm_workspace_bytes": C.c_size_t, "moe_gemm_fp8_workspace_bytes": C.c_size_t, "mla_paged_decode_workspace_bytes": C.c_size_t,
+             "moe_gemm_workspace_bytes": C.c_size_t, "moe_block_workspace_bytes": C.c_size_t, "moe_gemm_fp8_workspace_bytes": C.c_size_t, "mla_paged_decode_workspace_bytes": C.c_size_t,
              "b200_llama_create": C.c_void_p, "b200_llama_peer_inbox_bytes": C.c_size_t, "b200_ipc_alloc": C.c_void_p, "b200_ipc_open": C.c_void_p,
              "b200_llama_logits": C.c_void_p, "b200_llama_next_tokens": C.c_void_p, "b200_llama_kernel_launches": C.c_int64,
              "b200_total_kernel_launches": C.c_longlong, "moe_align_rows": C.c_int64, "linear_attention_chunked_scratch": C.c_int64, "gated_delta_channel_chunked_scratch": C.c_int64}

@@ -11,9 +11,10 @@
 //                           per token (gate / up), pair when it has one per pair (down).
 // Decode is a weight stream: per layer only the experts that were hit are read, each ONCE -- the routed rows of an expert are gathered
 // (fp16, K4 order) next to each other, and the tcgen05 dequant-GEMM of qmatmul_tc.cu runs in "grouped" mode over a device-side list of
-// (expert, 128-row weight tile, chunk of <= 32 rows) items: weight tile = UMMA A (dequantised straight into TMEM), the expert's rows =
-// UMMA B through one TMA box, results scattered back to their pair rows with the routing weight folded in.  Nothing on this path
-// synchronises with the host or allocates: the item list is built on the device from this step's routing (graph-capture safe).
+// (expert, chunk of <= 32, 64 or 128 rows) entries, every 128-row weight tile of an expert against each of its chunks: weight tile = UMMA A
+// (dequantised straight into TMEM), the expert's rows = UMMA B by TMA, results scattered back to their pair rows with the routing weight
+// folded in.  Nothing on this path synchronises with the host or allocates: the chunk list is built on the device from this step's routing (graph-capture safe).
+//   moe_block_gguf          the whole block in one call: router, top-k, plan (sort + chunks), gather, gate | up in one grouped launch, SiLU * up, down, sum over slots
 #include <cuda_fp8.h>
 
 #include <type_traits>
@@ -26,21 +27,29 @@ namespace b200 {
 namespace {
 
 // ---- routing ------------------------------------------------------------------------------------------------------------------
-// one warp per token; E <= 1024 experts (32 per lane), k <= 32
+// one warp per token; E <= 32 kPer experts, k <= 32.  logits: `splits` partial sums, split_stride apart (1: finished logits).  normalise: the weights are divided by
+// their sum; all are multiplied by `scaling`.  [With 32 slots per lane whatever E, 16 tokens of 128 experts took 8.0 us.]
+template <int kPer>
 __global__ void __launch_bounds__(128)
-topk_softmax_kernel(const float* __restrict__ logits, float* __restrict__ w_out, uint32_t* __restrict__ id_out, int tokens, int E, int k) {
+topk_softmax_kernel(const float* __restrict__ logits, int splits, int64_t split_stride, float* __restrict__ w_out, uint32_t* __restrict__ id_out, int tokens, int E, int k,
+                    int normalise, float scaling) {
     pdl_wait();
     pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t = blockIdx.x * 4 + warp;
     if (t >= tokens) return;
-    constexpr int kPer = 32;
     float v[kPer];
     float mx = -INFINITY;
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
         const int e = lane + 32 * i;
-        v[i] = e < E ? logits[(int64_t)t * E + e] : -INFINITY;
+        v[i] = -INFINITY;
+        if (e < E) {
+            const float* src = logits + (int64_t)t * E + e;
+            float a = src[0];
+            for (int s = 1; s < splits; ++s) a += src[s * split_stride];
+            v[i] = a;
+        }
         mx = fmaxf(mx, v[i]);
     }
     mx = warp_max(mx);
@@ -49,6 +58,7 @@ topk_softmax_kernel(const float* __restrict__ logits, float* __restrict__ w_out,
     for (int i = 0; i < kPer; ++i) { v[i] = lane + 32 * i < E ? __expf(v[i] - mx) : 0.f; sum += v[i]; }
     sum = warp_sum(sum);
     const float inv = 1.f / sum;
+    float mine = 0.f, total = 0.f;                     // lane j keeps the weight of round j
     for (int j = 0; j < k; ++j) {                      // k rounds of arg-max; ties -> the smallest expert id
         float best = -1.f;
         int bi = 0x7fffffff;
@@ -63,88 +73,231 @@ topk_softmax_kernel(const float* __restrict__ logits, float* __restrict__ w_out,
             const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
             if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
         }
-        if (lane == 0) { w_out[(int64_t)t * k + j] = best * inv; id_out[(int64_t)t * k + j] = (uint32_t)bi; }
-        if ((bi & 31) == lane) v[bi >> 5] = -1.f;      // remove the winner (probabilities are >= 0)
+        if (lane == j) { mine = best * inv; id_out[(int64_t)t * k + j] = (uint32_t)bi; }
+        total += best * inv;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i)
+            if (lane + 32 * i == bi) v[i] = -1.f;      // remove the winner (probabilities are >= 0)
     }
+    if (lane < k) w_out[(int64_t)t * k + lane] = (normalise ? mine / total : mine) * scaling;
+}
+void topk_launch(const float* logits, int splits, int64_t split_stride, float* w, uint32_t* ids, int tokens, int E, int k, int normalise, float scaling, cudaStream_t st) {
+    auto kern = E <= 32 ? topk_softmax_kernel<1> : E <= 128 ? topk_softmax_kernel<4> : E <= 256 ? topk_softmax_kernel<8> : topk_softmax_kernel<32>;
+    launch_pdl(kern, dim3(ceil_div(tokens, 4)), dim3(128), 0, st, logits, splits, split_stride, w, ids, tokens, E, k, normalise, scaling);
+    count_launch();
 }
 
-// stable counting sort of the flattened expert ids (one CTA; pairs <= 64 Ki, experts <= 1024) and the grouped-GEMM item list
+// Router: partial logits[z][T][E] = x[T, H] . gate[E, H]^T over the z-th part of H, f32 throughout.  CTA = 64 tokens x 32 experts, thread = 4 x 4, k in steps of
+// 32 through shared memory (k-major, so that both operands are 16-byte loads), the next step's tiles in registers.  Parts because 64 x 32 tiles alone leave most SMs
+// idle; the top-k kernel adds them in a fixed order.  [900 tokens, 128 experts, H 2048: the library's f32 product took 54 us, 16 tokens 12 us.]
+constexpr int kRtT = 64, kRtE = 32, kRtK = 32;
+__global__ void __launch_bounds__(128)
+moe_router_kernel(const float* __restrict__ x, const float* __restrict__ gate, float* __restrict__ part, int tokens, int E, int H, int steps_per) {
+    __shared__ float xs[kRtK][kRtT + 4], gs[kRtK][kRtE + 4];
+    const int t0 = blockIdx.x * kRtT, e0 = blockIdx.y * kRtE, k0 = blockIdx.z * steps_per * kRtK;
+    const int steps = min(steps_per, (H - k0) / kRtK);
+    const int tid = threadIdx.x, tr = tid >> 3, er = tid & 7;         // 16 x 8 threads
+    const int lr = tid >> 3, lc = (tid & 7) * 4;                       // loads: row lr + 16 i, 4 entries from lc
+    pdl_wait();
+    pdl_trigger();
+    float4 xv[4], gv[2];
+    auto fetch = [&](int k) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { const int r = t0 + lr + 16 * i; xv[i] = r < tokens ? *reinterpret_cast<const float4*>(x + (int64_t)r * H + k + lc) : make_float4(0.f, 0.f, 0.f, 0.f); }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) { const int r = e0 + lr + 16 * i; gv[i] = r < E ? *reinterpret_cast<const float4*>(gate + (int64_t)r * H + k + lc) : make_float4(0.f, 0.f, 0.f, 0.f); }
+    };
+    float acc[4][4] = {};
+    if (steps > 0) fetch(k0);
+    for (int s = 0; s < steps; ++s) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { xs[lc][lr + 16 * i] = xv[i].x; xs[lc + 1][lr + 16 * i] = xv[i].y; xs[lc + 2][lr + 16 * i] = xv[i].z; xs[lc + 3][lr + 16 * i] = xv[i].w; }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) { gs[lc][lr + 16 * i] = gv[i].x; gs[lc + 1][lr + 16 * i] = gv[i].y; gs[lc + 2][lr + 16 * i] = gv[i].z; gs[lc + 3][lr + 16 * i] = gv[i].w; }
+        __syncthreads();
+        if (s + 1 < steps) fetch(k0 + (s + 1) * kRtK);
+#pragma unroll
+        for (int k = 0; k < kRtK; ++k) {
+            const float4 a = *reinterpret_cast<const float4*>(&xs[k][tr * 4]), b = *reinterpret_cast<const float4*>(&gs[k][er * 4]);
+            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+        }
+        __syncthreads();
+    }
+    float* o = part + (int64_t)blockIdx.z * tokens * E;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (t0 + tr * 4 + i < tokens && e0 + er * 4 + j < E) o[(int64_t)(t0 + tr * 4 + i) * E + e0 + er * 4 + j] = acc[i][j];
+}
+
+// exclusive prefix sum of one value per thread over a block of 1024; `total` gets the sum.  sums: 33 ints of shared memory
+__device__ __forceinline__ int block_scan_1024(int v, int* sums, int& total) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int n = __shfl_up_sync(0xffffffffu, inc, o); if (lane >= o) inc += n; }
+    __syncthreads();
+    if (lane == 31) sums[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+        int w = sums[lane], acc = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int n = __shfl_up_sync(0xffffffffu, acc, o); if (lane >= o) acc += n; }
+        sums[lane] = acc - w;
+        if (lane == 31) sums[32] = acc;
+    }
+    __syncthreads();
+    total = sums[32];
+    return sums[warp] + inc - v;
+}
+// chunks of <= rows sorted positions, expert by expert, from the segment [first, first + count) of expert threadIdx.x (block of 1024 = the most experts)
+__device__ __forceinline__ void write_chunks(int e, int first, int count, int rows, MoeChunk* chunks, int* num_chunks, int max_chunks, int* sums) {
+    int total;
+    const int nc = (count + rows - 1) / rows;
+    int at = block_scan_1024(nc, sums, total);
+    for (int c = 0; c < nc; ++c, ++at)
+        if (at < max_chunks) chunks[at] = MoeChunk{e, first + c * rows, min(rows, count - c * rows)};
+    if (threadIdx.x == 0) *num_chunks = min(total, max_chunks);
+}
+
+// Stable counting sort of the flattened expert ids, one CTA of 32 warps (experts <= 1024): warp w owns the w-th run of pairs and a histogram of its own; prefix sums over
+// the warps of an expert, then over the experts, give every warp its first position per expert, and a second pass ranks 32 pairs at a time by match.  With chunks it
+// also writes the chunk list of the grouped GEMM.  [One thread per expert walking every pair took 124 us for 7200 pairs of 128 experts.]
+constexpr int kSortBatch = 8;                                          // ids in flight per lane
 __global__ void __launch_bounds__(1024)
-moe_sort_kernel(const uint32_t* __restrict__ ids, uint32_t* __restrict__ sorted_expert, uint32_t* __restrict__ sorted_pair, int pairs, int E) {
+moe_sort_kernel(const uint32_t* __restrict__ ids, uint32_t* __restrict__ sorted_expert, uint32_t* __restrict__ sorted_pair, int pairs, int E, MoeChunk* __restrict__ chunks,
+                int* __restrict__ num_chunks, int rows, int max_chunks) {
+    extern __shared__ int hist[];                                      // [32][E]
+    __shared__ int start[1024], sums[33];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < 32 * E; i += 1024) hist[i] = 0;
     pdl_wait();
     pdl_trigger();
-    __shared__ int count[1024], start[1025];
-    for (int e = threadIdx.x; e < E; e += blockDim.x) count[e] = 0;
     __syncthreads();
-    for (int p = threadIdx.x; p < pairs; p += blockDim.x) atomicAdd(&count[min(ids[p], (uint32_t)E - 1)], 1);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int e = 0; e < E; ++e) { start[e] = acc; acc += count[e]; }
-        start[E] = acc;
+    const int per = ((pairs + 31) / 32 + 31) & ~31, p0 = warp * per, p1 = min(pairs, p0 + per);
+    int* mine = hist + warp * E;
+    for (int b = p0; b < p1; b += 32 * kSortBatch) {
+        int e[kSortBatch];
+#pragma unroll
+        for (int i = 0; i < kSortBatch; ++i) { const int q = b + 32 * i + lane; e[i] = q < p1 ? (int)min(ids[q], (uint32_t)E - 1) : -1; }
+#pragma unroll
+        for (int i = 0; i < kSortBatch; ++i) if (e[i] >= 0) atomicAdd(mine + e[i], 1);
     }
     __syncthreads();
-    // stable placement: thread e walks the pairs in order for its expert(s) -- pairs are few (decode) or the walk is short per expert
-    for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        if (count[e] == 0) continue;
-        int pos = start[e];
-        for (int p = 0; p < pairs; ++p)
-            if (min(ids[p], (uint32_t)E - 1) == (uint32_t)e) { sorted_expert[pos] = (uint32_t)e; sorted_pair[pos] = (uint32_t)p; ++pos; }
+    const int ex = threadIdx.x;
+    int count = 0;
+    if (ex < E)
+        for (int w = 0; w < 32; ++w) { const int c = hist[w * E + ex]; hist[w * E + ex] = count; count += c; }
+    int total;
+    const int first = block_scan_1024(count, sums, total);
+    start[ex] = first;
+    __syncthreads();
+    for (int b = p0; b < p1; b += 32 * kSortBatch) {
+        int e[kSortBatch];
+#pragma unroll
+        for (int i = 0; i < kSortBatch; ++i) { const int q = b + 32 * i + lane; e[i] = q < p1 ? (int)min(ids[q], (uint32_t)E - 1) : -1; }
+#pragma unroll
+        for (int i = 0; i < kSortBatch; ++i) {
+            const unsigned same = __match_any_sync(0xffffffffu, e[i]);
+            const int rank = __popc(same & ((1u << lane) - 1u));
+            int base = 0;
+            if (e[i] >= 0) base = mine[e[i]] + start[e[i]];
+            __syncwarp();
+            if (e[i] >= 0) {
+                if (rank == 0) mine[e[i]] += __popc(same);
+                if (sorted_expert) sorted_expert[base + rank] = (uint32_t)e[i];
+                sorted_pair[base + rank] = (uint32_t)(b + 32 * i + lane);
+            }
+            __syncwarp();
+        }
     }
+    if (chunks) write_chunks(ex, first, count, rows, chunks, num_chunks, max_chunks, sums);
+}
+void sort_launch(const uint32_t* ids, uint32_t* sorted_expert, uint32_t* sorted_pair, int pairs, int E, MoeChunk* chunks, int* num_chunks, int rows, int max_chunks, cudaStream_t st) {
+    ensure_dynamic_smem(reinterpret_cast<const void*>(moe_sort_kernel), 32 * E * 4);
+    launch_pdl(moe_sort_kernel, dim3(1), dim3(1024), (size_t)32 * E * 4, st, ids, sorted_expert, sorted_pair, pairs, E, chunks, num_chunks, rows, max_chunks);
+    count_launch();
 }
 
-// items of the grouped GEMM from the SORTED expert ids: for every expert segment, every 128-row weight tile, every chunk of 32 rows
-__global__ void __launch_bounds__(256)
-moe_items_kernel(const uint32_t* __restrict__ sorted_expert, int pairs, int E, int n, MoeItem* __restrict__ items, int* __restrict__ num_items,
-                 int max_items) {
+// the chunk list from SORTED expert ids (the grouped GEMM's own entry points): segment borders by binary search
+__global__ void __launch_bounds__(1024)
+moe_chunks_kernel(const uint32_t* __restrict__ sorted_expert, int pairs, int E, MoeChunk* __restrict__ chunks, int* __restrict__ num_chunks, int rows, int max_chunks) {
+    __shared__ int sums[33];
     pdl_wait();
     pdl_trigger();
-    __shared__ int seg_start[1025], item_base[1025];
-    // segment starts by binary search (sorted input)
-    for (int e = threadIdx.x; e <= E; e += blockDim.x) {
+    auto lower = [&](uint32_t e) {
         int lo = 0, hi = pairs;                          // first position with expert >= e
-        while (lo < hi) { const int mid = (lo + hi) >> 1; if (sorted_expert[mid] < (uint32_t)e) lo = mid + 1; else hi = mid; }
-        seg_start[e] = lo;
-    }
-    __syncthreads();
-    const int tiles = (n + 127) / 128;
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int e = 0; e < E; ++e) { item_base[e] = acc; acc += ((seg_start[e + 1] - seg_start[e] + 31) / 32) * tiles; }
-        item_base[E] = acc;
-        *num_items = acc < max_items ? acc : max_items;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        const int cnt = seg_start[e + 1] - seg_start[e];
-        const int chunks = (cnt + 31) / 32;
-        int w = item_base[e];
-        for (int t = 0; t < tiles; ++t)                  // chunks of one (expert, tile) are neighbours: the weight tile stays in L2
-            for (int c = 0; c < chunks; ++c, ++w)
-                if (w < max_items) items[w] = MoeItem{e * n + t * 128, seg_start[e] + c * 32, min(32, cnt - c * 32), t * 128};
-    }
+        while (lo < hi) { const int mid = (lo + hi) >> 1; if (sorted_expert[mid] < e) lo = mid + 1; else hi = mid; }
+        return lo;
+    };
+    const int e = threadIdx.x;
+    const int first = e < E ? lower((uint32_t)e) : 0, count = e < E ? lower((uint32_t)e + 1) - first : 0;
+    write_chunks(e, first, count, rows, chunks, num_chunks, max_chunks, sums);
 }
+
+// rows per chunk: every chunk converts its expert's weights once, larger chunks convert less often and hold more shared memory for rows they may not have.  Few rows per
+// expert (decode): 32, with the deepest weight ring.
+int chunk_rows_for(int64_t pairs, int E) { return pairs <= 24 * (int64_t)E ? 32 : (pairs <= 44 * (int64_t)E ? 64 : 128); }
+int max_chunks_for(int64_t pairs, int E, int rows) { const int64_t a = pairs / rows + E; return (int)(a < pairs ? a : pairs); }
 
 // expert-sorted fp16 (K4 order) copy of the routed activation rows: xs[j] = x[row(sorted_pair[j])], row = pair / topk when x has one row
-// per token.  Rows [pairs, pairs + 32) are zero-filled (a chunk's TMA box may run past the last routed row).
+// per token.  (A chunk's TMA box may run past the last routed row: the tensor map ends there and the box is filled with zeros.)  One warp per row, 16-byte stores.
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(const float* __restrict__ x, const uint32_t* __restrict__ sorted_pair, __half* __restrict__ xs, int pairs, int k, int per_token,
                   int topk) {
     pdl_wait();
     pdl_trigger();
-    const int j = blockIdx.x;
+    const int j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (j >= pairs) return;
     __half* dst = xs + (int64_t)j * k;
-    if (j >= pairs) {
-        for (int i = threadIdx.x * 8; i < k; i += blockDim.x * 8) *reinterpret_cast<uint4*>(dst + i) = make_uint4(0, 0, 0, 0);
-        return;
-    }
     const uint32_t pr = sorted_pair[j];
     const float* src = x + (int64_t)(per_token ? pr / (uint32_t)topk : pr) * k;
-    for (int i = threadIdx.x * 4; i < k; i += blockDim.x * 4) {
-        const float4 v = *reinterpret_cast<const float4*>(src + i);
-        const __half2 p0 = __halves2half2(from_f32<__half>(v.x), from_f32<__half>(v.z)), p1 = __halves2half2(from_f32<__half>(v.y), from_f32<__half>(v.w));
-        *reinterpret_cast<uint2*>(dst + i) = make_uint2(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1));
+    for (int i = lane * 8; i < k; i += 256) {
+        const float4 v = *reinterpret_cast<const float4*>(src + i), w = *reinterpret_cast<const float4*>(src + i + 4);
+        const __half2 p[4] = {__halves2half2(from_f32<__half>(v.x), from_f32<__half>(v.z)), __halves2half2(from_f32<__half>(v.y), from_f32<__half>(v.w)),
+                              __halves2half2(from_f32<__half>(w.x), from_f32<__half>(w.z)), __halves2half2(from_f32<__half>(w.y), from_f32<__half>(w.w))};
+        *reinterpret_cast<uint4*>(dst + i) = *reinterpret_cast<const uint4*>(p);
     }
+}
+
+// act[j] = silu(g[j]) * u[j] as fp16 in K4 order, rows in sorted order; 8 entries per thread
+__global__ void __launch_bounds__(256)
+moe_silu_mul_kernel(const float* __restrict__ g, const float* __restrict__ u, __half* __restrict__ act, int64_t total) {
+    pdl_wait();
+    pdl_trigger();
+    const int64_t i = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 8;
+    if (i >= total) return;
+    float r[8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const float4 a = *reinterpret_cast<const float4*>(g + i + 4 * h), b = *reinterpret_cast<const float4*>(u + i + 4 * h);
+        const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) r[4 * h + e] = av[e] / (1.f + expf(-av[e])) * bv[e];
+    }
+    const __half2 p[4] = {__halves2half2(from_f32<__half>(r[0]), from_f32<__half>(r[2])), __halves2half2(from_f32<__half>(r[1]), from_f32<__half>(r[3])),
+                          __halves2half2(from_f32<__half>(r[4]), from_f32<__half>(r[6])), __halves2half2(from_f32<__half>(r[5]), from_f32<__half>(r[7]))};
+    *reinterpret_cast<uint4*>(act + i) = *reinterpret_cast<const uint4*>(p);
+}
+
+// out[t] = sum over the token's slots, ascending
+__global__ void __launch_bounds__(256)
+moe_sum_slots_kernel(const float* __restrict__ y, float* __restrict__ out, int64_t total4, int h4, int topk) {
+    pdl_wait();
+    pdl_trigger();
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= total4) return;
+    const int64_t t = i / h4, c = i - t * h4;
+    const float4* src = reinterpret_cast<const float4*>(y) + t * topk * h4 + c;
+    float4 a = src[0];
+#pragma unroll 4
+    for (int s = 1; s < topk; ++s) { const float4 b = src[(int64_t)s * h4]; a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
+    reinterpret_cast<float4*>(out)[i] = a;
 }
 
 // the same from 16-bit activations into fp16 in NATURAL order (moe_gemm_fp8)
@@ -154,11 +307,8 @@ moe_gather16_kernel(const T* __restrict__ x, const uint32_t* __restrict__ sorted
     pdl_wait();
     pdl_trigger();
     const int j = blockIdx.x;
+    if (j >= pairs) return;
     __half* dst = xs + (int64_t)j * k;
-    if (j >= pairs) {
-        for (int i = threadIdx.x * 8; i < k; i += blockDim.x * 8) *reinterpret_cast<uint4*>(dst + i) = make_uint4(0, 0, 0, 0);
-        return;
-    }
     const uint32_t pr = sorted_pair[j];
     const T* src = x + (int64_t)(per_token ? pr / (uint32_t)topk : pr) * k;
     for (int i = threadIdx.x * 8; i < k; i += blockDim.x * 8) {
@@ -238,9 +388,7 @@ void topk_softmax(const float* router_logits, float* topk_weights, uint32_t* top
     B200_REQUIRE(router_logits && topk_weights && topk_ids, kErrBadArg, "topk_softmax: null pointer");
     B200_REQUIRE(num_experts >= 1 && num_experts <= 1024 && topk >= 1 && topk <= num_experts && topk <= 32, kErrUnsupported,
                  "topk_softmax: %d experts (<= 1024), top-%d (<= 32)", num_experts, topk);
-    launch_pdl(topk_softmax_kernel, dim3(ceil_div(num_tokens, 4)), dim3(128), 0, as_stream(stream), router_logits, topk_weights, topk_ids, (int)num_tokens,
-               (int)num_experts, (int)topk);
-    count_launch();
+    topk_launch(router_logits, 1, 0, topk_weights, topk_ids, num_tokens, num_experts, topk, 0, 1.f, as_stream(stream));
     check_launch("topk_softmax");
 }
 
@@ -249,14 +397,15 @@ void sort_expert_assignments(const uint32_t* topk_ids, uint32_t* expert_ids, uin
     if (num_pairs == 0) return;
     B200_REQUIRE(topk_ids && expert_ids && sorted_token_ids, kErrBadArg, "sort_expert_assignments: null pointer");
     B200_REQUIRE(num_experts >= 1 && num_experts <= 1024 && num_pairs > 0, kErrUnsupported, "sort_expert_assignments: %d experts (<= 1024)", num_experts);
-    launch_pdl(moe_sort_kernel, dim3(1), dim3(1024), 0, as_stream(stream), topk_ids, expert_ids, sorted_token_ids, (int)num_pairs, (int)num_experts);
-    count_launch();
+    sort_launch(topk_ids, expert_ids, sorted_token_ids, num_pairs, num_experts, nullptr, nullptr, 0, 0, as_stream(stream));
     check_launch("sort_expert_assignments");
 }
 
+static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
+
 size_t moe_gemm_workspace_bytes(int32_t num_pairs, int32_t n, int32_t k, int32_t num_experts) {
-    const size_t max_items = ((size_t)num_pairs / 32 + (size_t)num_experts) * (size_t)((n + 127) / 128);
-    return ((size_t)(num_pairs + 32) * (size_t)k * 2 + 255) / 256 * 256 + max_items * sizeof(MoeItem) + 256;
+    (void)n;
+    return align256((size_t)num_pairs * (size_t)k * 2) + align256(((size_t)num_pairs / 32 + (size_t)num_experts) * sizeof(MoeChunk)) + 256;
 }
 
 void moe_gemm_gguf(const float* x, const void* experts, const float* topk_weights, const uint32_t* sorted_token_ids, const uint32_t* expert_ids,
@@ -275,15 +424,16 @@ void moe_gemm_gguf(const float* x, const void* experts, const float* topk_weight
     if (qmatmul_tc_moe_supported(n, k, ggml_type) && k % 8 == 0 && workspace && workspace_bytes >= moe_gemm_workspace_bytes(num_pairs, n, k, num_experts) &&
         ((uintptr_t)workspace & 255) == 0) {
         __half* xs = static_cast<__half*>(workspace);
-        const size_t xs_bytes = ((size_t)(num_pairs + 32) * (size_t)k * 2 + 255) / 256 * 256;
-        MoeItem* items = reinterpret_cast<MoeItem*>(static_cast<char*>(workspace) + xs_bytes);
-        const int max_items = (int)(((size_t)num_pairs / 32 + (size_t)num_experts) * (size_t)((n + 127) / 128));
-        int* num_items = reinterpret_cast<int*>(items + max_items);
-        launch_pdl(moe_gather_kernel, dim3(num_pairs + 32), dim3(256), 0, st, x, sorted_token_ids, xs, (int)num_pairs, (int)k, per_token, (int)topk);
-        launch_pdl(moe_items_kernel, dim3(1), dim3(256), 0, st, expert_ids, (int)num_pairs, (int)num_experts, (int)n, items, num_items, max_items);
+        MoeChunk* chunks = reinterpret_cast<MoeChunk*>(static_cast<char*>(workspace) + align256((size_t)num_pairs * k * 2));
+        int* num_chunks = reinterpret_cast<int*>(static_cast<char*>(workspace) + moe_gemm_workspace_bytes(num_pairs, n, k, num_experts) - 256);
+        const int rows = chunk_rows_for(num_pairs, num_experts), max_chunks = max_chunks_for(num_pairs, num_experts, rows);
+        launch_pdl(moe_gather_kernel, dim3(ceil_div(num_pairs, 8)), dim3(256), 0, st, x, sorted_token_ids, xs, (int)num_pairs, (int)k, per_token, (int)topk);
+        launch_pdl(moe_chunks_kernel, dim3(1), dim3(1024), 0, st, expert_ids, (int)num_pairs, (int)num_experts, chunks, num_chunks, rows, max_chunks);
         count_launch(2);
         if (!check_launch("moe_gemm_gguf")) return;
-        qmatmul_tc_moe(xs, num_pairs + 32, experts, num_experts, out, n, n, k, ggml_type, items, num_items, max_items, sorted_token_ids, topk_weights, st);
+        const void* ws[1] = {experts};
+        float* ys[1] = {out};
+        qmatmul_tc_moe(xs, num_pairs, 1, ws, num_experts, ys, n, n, k, ggml_type, chunks, num_chunks, max_chunks, rows, sorted_token_ids, topk_weights, st);
         return;
     }
     const dim3 grid(ceil_div(n, 8), num_pairs);
@@ -292,6 +442,95 @@ void moe_gemm_gguf(const float* x, const void* experts, const float* topk_weight
     else moe_gemm_generic_kernel<B200_GGML_Q8_0><<<grid, 256, 0, st>>>(x, experts, topk_weights, sorted_token_ids, expert_ids, out, num_pairs, n, k, per_token, topk);
     count_launch();
     check_launch("moe_gemm_gguf");
+}
+
+// ---- the whole block ---------------------------------------------------------------------------------------------------------------------
+namespace {
+// how the workspace of moe_block_gguf is laid out.  The down projection's result takes the place of the sorted inputs and the gate / up results, which are dead by then.
+struct MoeBlockPlan {
+    int rows, max_chunks, splits, steps_per;
+    size_t logits, weights, ids, pair, chunks, count, act, xs, gu, y, total;
+    MoeBlockPlan(int64_t T, int64_t H, int64_t I, int E, int topk) {
+        const int64_t P = T * topk;
+        rows = chunk_rows_for(P, E); max_chunks = max_chunks_for(P, E, rows);
+        // router parts: about two CTAs per SM, at least two steps each, 16 at most (the top-k kernel adds them one after another)
+        const int64_t tiles = ((T + kRtT - 1) / kRtT) * ((E + kRtE - 1) / kRtE), steps = H / kRtK;
+        int64_t s = 296 / tiles;
+        if (s > 16) s = 16;
+        if (s > steps / 2) s = steps / 2;
+        if (s < 1) s = 1;
+        steps_per = (int)((steps + s - 1) / s); splits = (int)((steps + steps_per - 1) / steps_per);
+        size_t at = 0;
+        auto take = [&](size_t b) { const size_t o = at; at += align256(b); return o; };
+        logits = take((size_t)splits * T * E * 4); weights = take((size_t)P * 4); ids = take((size_t)P * 4); pair = take((size_t)P * 4);
+        chunks = take((size_t)max_chunks * sizeof(MoeChunk)); count = take(4); act = take((size_t)P * I * 2);
+        y = at;
+        xs = take((size_t)P * H * 2); gu = take((size_t)P * I * 8);
+        const size_t end = y + align256((size_t)P * H * 4);
+        total = at > end ? at : end;
+    }
+};
+}  // namespace
+
+// 1 when moe_block_gguf runs these sizes: the grouped tcgen05 GEMM covers the three products
+int32_t moe_block_supported(int32_t num_tokens, int32_t hidden, int32_t inter, int32_t num_experts, int32_t topk, int32_t type_gate, int32_t type_up, int32_t type_down) {
+    if (num_tokens < 1 || hidden < 1 || inter < 1 || num_experts < 1 || num_experts > 1024 || topk < 1 || topk > 32 || topk > num_experts) return 0;
+    if ((int64_t)num_tokens * topk > (1 << 20)) return 0;
+    return qmatmul_tc_moe_supported(inter, hidden, type_gate) && qmatmul_tc_moe_supported(inter, hidden, type_up) && qmatmul_tc_moe_supported(hidden, inter, type_down);
+}
+
+size_t moe_block_workspace_bytes(int32_t num_tokens, int32_t hidden, int32_t inter, int32_t num_experts, int32_t topk) {
+    if (num_tokens < 1 || hidden < 1 || inter < 1 || num_experts < 1 || topk < 1) return 0;
+    return MoeBlockPlan(num_tokens, hidden, inter, num_experts, topk).total;
+}
+
+// out[t] = sum over the top-k experts e of w_e down_e(silu(gate_e x_t) * up_e x_t), w = softmax(router x_t) at the chosen experts (over their sum when normalise) * scaling
+void moe_block_gguf(const float* x, const float* router, const void* gate, const void* up, const void* down, float* out, int32_t num_tokens, int32_t hidden,
+                    int32_t inter, int32_t num_experts, int32_t topk, int32_t type_gate, int32_t type_up, int32_t type_down, int32_t normalise, float scaling,
+                    void* workspace, size_t workspace_bytes, int64_t stream) {
+    if (num_tokens == 0) return;
+    B200_REQUIRE(x && router && gate && up && down && out, kErrBadArg, "moe_block_gguf: null pointer");
+    B200_REQUIRE(moe_block_supported(num_tokens, hidden, inter, num_experts, topk, type_gate, type_up, type_down), kErrUnsupported,
+                 "moe_block_gguf: %d tokens, hidden %d, inter %d, %d experts (<= 1024), top-%d (<= 32), types %d %d %d", num_tokens, hidden, inter, num_experts, topk,
+                 type_gate, type_up, type_down);
+    B200_REQUIRE((((uintptr_t)x | (uintptr_t)router | (uintptr_t)gate | (uintptr_t)up | (uintptr_t)down | (uintptr_t)out) & 15) == 0, kErrBadArg, "moe_block_gguf: 16-byte alignment");
+    const MoeBlockPlan p(num_tokens, hidden, inter, num_experts, topk);
+    B200_REQUIRE(workspace && ((uintptr_t)workspace & 255) == 0 && workspace_bytes >= p.total, kErrBadArg,
+                 "moe_block_gguf: workspace of moe_block_workspace_bytes() bytes, 256-byte aligned, required");
+    cudaStream_t st = as_stream(stream);
+    char* ws = static_cast<char*>(workspace);
+    float* logits = reinterpret_cast<float*>(ws + p.logits);
+    float* weights = reinterpret_cast<float*>(ws + p.weights);
+    uint32_t* ids = reinterpret_cast<uint32_t*>(ws + p.ids);
+    uint32_t* pair = reinterpret_cast<uint32_t*>(ws + p.pair);
+    MoeChunk* chunks = reinterpret_cast<MoeChunk*>(ws + p.chunks);
+    int* count = reinterpret_cast<int*>(ws + p.count);
+    __half* act = reinterpret_cast<__half*>(ws + p.act);
+    __half* xs = reinterpret_cast<__half*>(ws + p.xs);
+    const int P = num_tokens * topk;
+    float* g = reinterpret_cast<float*>(ws + p.gu);
+    float* u = g + (int64_t)P * inter;
+    float* y = reinterpret_cast<float*>(ws + p.y);
+    launch_pdl(moe_router_kernel, dim3(ceil_div(num_tokens, kRtT), ceil_div(num_experts, kRtE), p.splits), dim3(128), 0, st, x, router, logits, (int)num_tokens,
+               (int)num_experts, (int)hidden, p.steps_per);
+    topk_launch(logits, p.splits, (int64_t)num_tokens * num_experts, weights, ids, num_tokens, num_experts, topk, normalise, scaling, st);
+    sort_launch(ids, nullptr, pair, P, num_experts, chunks, count, p.rows, p.max_chunks, st);
+    launch_pdl(moe_gather_kernel, dim3(ceil_div(P, 8)), dim3(256), 0, st, x, (const uint32_t*)pair, xs, P, (int)hidden, 1, (int)topk);
+    count_launch(2);
+    if (!check_launch("moe_block_gguf")) return;
+    const void* w2[2] = {gate, up};
+    float* y2[2] = {g, u};
+    if (type_gate == type_up) qmatmul_tc_moe(xs, P, 2, w2, num_experts, y2, inter, inter, hidden, type_gate, chunks, count, p.max_chunks, p.rows, nullptr, nullptr, st);
+    else
+        for (int i = 0; i < 2; ++i)
+            qmatmul_tc_moe(xs, P, 1, w2 + i, num_experts, y2 + i, inter, inter, hidden, i ? type_up : type_gate, chunks, count, p.max_chunks, p.rows, nullptr, nullptr, st);
+    const int64_t gu = (int64_t)P * inter;
+    launch_pdl(moe_silu_mul_kernel, dim3(ceil_div(gu, 2048)), dim3(256), 0, st, (const float*)g, (const float*)u, act, gu);
+    qmatmul_tc_moe(act, P, 1, &down, num_experts, &y, hidden, hidden, inter, type_down, chunks, count, p.max_chunks, p.rows, pair, weights, st);
+    const int64_t total4 = (int64_t)num_tokens * (hidden / 4);
+    launch_pdl(moe_sum_slots_kernel, dim3(ceil_div(total4, 256)), dim3(256), 0, st, (const float*)y, out, total4, hidden / 4, (int)topk);
+    count_launch(2);
+    check_launch("moe_block_gguf");
 }
 
 size_t moe_gemm_fp8_workspace_bytes(int32_t num_pairs, int32_t n, int32_t k, int32_t num_experts) {
@@ -315,21 +554,20 @@ void moe_gemm_fp8(const void* x, const void* experts, const float* scale, const 
     cudaStream_t st = as_stream(stream);
     const int per_token = size_m != num_pairs;
     char* ws = static_cast<char*>(workspace);
-    const size_t xs_bytes = ((size_t)(num_pairs + 32) * (size_t)k * 2 + 255) / 256 * 256;
-    const int max_items = (int)(((size_t)num_pairs / 32 + (size_t)num_experts) * (size_t)((n + 127) / 128));
     const size_t base = moe_gemm_workspace_bytes(num_pairs, n, k, num_experts);
     float* y32 = reinterpret_cast<float*>(ws + base);
     float* norm = reinterpret_cast<float*>(ws + base + ((size_t)num_pairs * (size_t)n * 4 + 255) / 256 * 256);
     if (qmatmul_tc_moe_fp8_supported(n, k, block_y, block_x) && k % 8 == 0 && (((uintptr_t)x | (uintptr_t)experts) & 15) == 0) {
         __half* xs = reinterpret_cast<__half*>(ws);
-        MoeItem* items = reinterpret_cast<MoeItem*>(ws + xs_bytes);
-        int* num_items = reinterpret_cast<int*>(items + max_items);
-        if (dtype == B200_BF16) launch_pdl(moe_gather16_kernel<__nv_bfloat16>, dim3(num_pairs + 32), dim3(256), 0, st, (const __nv_bfloat16*)x, sorted_token_ids, xs, (int)num_pairs, (int)k, per_token, (int)topk);
-        else launch_pdl(moe_gather16_kernel<__half>, dim3(num_pairs + 32), dim3(256), 0, st, (const __half*)x, sorted_token_ids, xs, (int)num_pairs, (int)k, per_token, (int)topk);
-        launch_pdl(moe_items_kernel, dim3(1), dim3(256), 0, st, expert_ids, (int)num_pairs, (int)num_experts, (int)n, items, num_items, max_items);
+        MoeChunk* chunks = reinterpret_cast<MoeChunk*>(ws + align256((size_t)num_pairs * k * 2));
+        int* num_chunks = reinterpret_cast<int*>(ws + base - 256);
+        const int max_chunks = max_chunks_for(num_pairs, num_experts, 32);
+        if (dtype == B200_BF16) launch_pdl(moe_gather16_kernel<__nv_bfloat16>, dim3(num_pairs), dim3(256), 0, st, (const __nv_bfloat16*)x, sorted_token_ids, xs, (int)num_pairs, (int)k, per_token, (int)topk);
+        else launch_pdl(moe_gather16_kernel<__half>, dim3(num_pairs), dim3(256), 0, st, (const __half*)x, sorted_token_ids, xs, (int)num_pairs, (int)k, per_token, (int)topk);
+        launch_pdl(moe_chunks_kernel, dim3(1), dim3(1024), 0, st, expert_ids, (int)num_pairs, (int)num_experts, chunks, num_chunks, 32, max_chunks);
         count_launch(2);
         if (!check_launch("moe_gemm_fp8")) return;
-        qmatmul_tc_moe_fp8(xs, num_pairs + 32, experts, scale, num_experts, y32, n, n, k, block_y, block_x, items, num_items, max_items, sorted_token_ids,
+        qmatmul_tc_moe_fp8(xs, num_pairs, experts, scale, num_experts, y32, n, n, k, block_y, block_x, chunks, num_chunks, max_chunks, sorted_token_ids,
                            topk_weights, norm, st);
     } else {
         const dim3 grid(ceil_div(n, 8), num_pairs);

@@ -8,12 +8,12 @@ namespace b200 {
 void qmatmul_generic(const void* x, bool x_is_f16, const void* w, float* y, int64_t ldy, int m, int n, int k,
                      int ggml_type, int accumulate, cudaStream_t st);
 
-// tcgen05 path (qmatmul_tc.cu): fp16 activations [m,k], m <= 32 * n_mtiles; returns false when the shape is not covered
+// tcgen05 path (qmatmul_tc.cu): fp16 activations [m,k]; false when the shape is not covered (as one row tile: m <= 64)
 bool qmatmul_tc_supported(int m, int n, int k, int ggml_type);
-// same, with m > 64 served 64 rows per pass (qmatmul_dispatch)
+// same, with m > 64 served in row tiles of 128 (qmatmul_dispatch)
 bool qmatmul_tc_usable(int m, int n, int k, int ggml_type);
 // true when some output tile is split across CTAs: y must hold the addend (zeros for a plain product)
-bool qmatmul_tc_needs_zeroed_output(int n, int k);
+bool qmatmul_tc_needs_zeroed_output(int m, int n, int k);
 
 // elementwise.cu internals used by the engine
 void rope_and_cache_impl(float* qkv, void* q_out, void* key_cache, void* value_cache, const float* cos_t, const float* sin_t,

@@ -130,15 +130,18 @@ void qmatmul_generic(const void* x, bool x_is_f16, const void* w, float* y, int6
     check_launch("qmatmul_generic");
 }
 
-// rows beyond the tensor-core kernel's 64 (prefill chunks) go through it 64 at a time: every pass re-streams the weights, which at
-// >= 64 rows per pass is within ~3x of a dense GEMM and two orders faster than the SIMT fallback
+// rows beyond one tile of 64 (prompt portions) go through the tensor-core kernel in row tiles of 128, kMaxRows at a time (its unit arithmetic is 32-bit)
+static constexpr int kMaxRows = 1024;
 bool qmatmul_tc_usable(int m, int n, int k, int ggml_type) { return m >= 1 && qmatmul_tc_supported(m > 64 ? 64 : m, n, k, ggml_type); }
+static bool dispatch_needs_zeroed_output(int m, int n, int k) {
+    return (m >= kMaxRows && qmatmul_tc_needs_zeroed_output(kMaxRows, n, k)) || (m % kMaxRows && qmatmul_tc_needs_zeroed_output(m % kMaxRows, n, k));
+}
 
 void qmatmul_dispatch(const void* x_f16, const void* w, float* y, int64_t ldy, int m, int n, int k,
                       int ggml_type, int accumulate, cudaStream_t st) {
     if (qmatmul_tc_usable(m, n, k, ggml_type)) {
-        for (int m0 = 0; m0 < m; m0 += 64)
-            qmatmul_tc(static_cast<const __half*>(x_f16) + (int64_t)m0 * k, w, y + (int64_t)m0 * ldy, ldy, m - m0 < 64 ? m - m0 : 64, n, k, ggml_type,
+        for (int m0 = 0; m0 < m; m0 += kMaxRows)
+            qmatmul_tc(static_cast<const __half*>(x_f16) + (int64_t)m0 * k, w, y + (int64_t)m0 * ldy, ldy, m - m0 < kMaxRows ? m - m0 : kMaxRows, n, k, ggml_type,
                        accumulate, st);
     } else {
         qmatmul_generic(x_f16, true, w, y, ldy, m, n, k, ggml_type, accumulate, st);
@@ -200,7 +203,7 @@ void qmatmul_f16act(const void* x_f16, const void* w, float* y, int32_t m, int32
                     int32_t ggml_type, int32_t accumulate, int64_t stream) {
     if (m == 0 || n == 0) return;
     if (!qmm_check("qmatmul_f16act", x_f16, w, y, m, n, k, ggml_type)) return;
-    if (!accumulate && qmatmul_tc_usable(m, n, k, ggml_type) && qmatmul_tc_needs_zeroed_output(n, k))
+    if (!accumulate && qmatmul_tc_usable(m, n, k, ggml_type) && dispatch_needs_zeroed_output(m, n, k))
         cudaMemsetAsync(y, 0, (size_t)m * n * sizeof(float), as_stream(stream));
     qmatmul_dispatch(x_f16, w, y, n, m, n, k, ggml_type, accumulate, as_stream(stream));
 }
@@ -236,8 +239,8 @@ void qmatmul_f32(const float* x, const void* w, float* y, int32_t m, int32_t n, 
         B200_REQUIRE(workspace && workspace_bytes >= qmatmul_workspace_bytes(m, n, k), kErrBadArg,
                      "qmatmul_f32: workspace too small (%zu < %zu)", workspace_bytes, qmatmul_workspace_bytes(m, n, k));
         cast(x, workspace, (int64_t)m * k, B200_F32, B200_F16_K4, stream);
-        if (!accumulate && qmatmul_tc_needs_zeroed_output(n, k)) cudaMemsetAsync(y, 0, (size_t)m * n * sizeof(float), as_stream(stream));
-        qmatmul_dispatch(workspace, w, y, n, m, n, k, ggml_type, accumulate, as_stream(stream));      // 64 rows per tensor-core pass
+        if (!accumulate && dispatch_needs_zeroed_output(m, n, k)) cudaMemsetAsync(y, 0, (size_t)m * n * sizeof(float), as_stream(stream));
+        qmatmul_dispatch(workspace, w, y, n, m, n, k, ggml_type, accumulate, as_stream(stream));
     } else {
         qmatmul_generic(x, false, w, y, n, m, n, k, ggml_type, accumulate, as_stream(stream));
     }

@@ -38,14 +38,14 @@ namespace {
 
 using namespace tc;
 
-template <int kMB, int kType>   // batch rows padded to kMB (32 or 64) = UMMA N; GGML type of W
+template <int kMB, int kType>   // activation rows of a tile, padded to kMB (32, 64 or 128) = UMMA N; GGML type of W
 struct Cfg {
     // bytes of one super-block as staged in shared memory: Q4_K 144; Q6_K a 240-byte window that starts at the
     // 210-byte block's address rounded down to 16 (TMA box starts must be 16-byte aligned)
     // Independent accumulators: back-to-back tcgen05.mma into ONE accumulator serialise on the accumulate
     // dependency; k-step ks goes to D[ks % kAcc] and the epilogue adds them up.  Two suffice (the dequant side sets the
     // pace) and keep the epilogue's TMEM reads (64 B/clk) short: kAcc * kMB <= 128 TMEM columns.
-    static constexpr int kAcc = 2;
+    static constexpr int kAcc = kMB == 128 ? 1 : 2;                // (at N = 128 one product fills the pipe longer than the dependency)
     static constexpr int kBlk = kType == B200_GGML_Q4_K ? 144 : (is_4bit_rows(kType) ? 128 : (kType == kTypeF8 ? 256 : 240));
     static constexpr int kWBytes = kTileN * kBlk;                  // raw weights of one unit (18 KB / 30 KB)
     static constexpr int kXBytes = 4 * kMB * kXSubBytes;           // 4 sub-tiles of [kMB][64] fp16 (16 KB / 32 KB)
@@ -89,12 +89,14 @@ struct GemmParams {
     int scale_bf16, scale_by, scale_sk;
     const float* norm;             // fp8: {2^p, 2^-p} range shift of the tile scales (device)
     const uint32_t* zp;            // AWQ: packed zero points [K/g, N/8] in the marlin layout (null: symmetric, zero point 8)
-    // grouped (mixture-of-experts) mode: the tile list lives in device memory -- built from the routing of this step (moe.cu) --
-    // and every "tile" is one (expert, 128-row weight tile, chunk of <= kMB routed rows): weights at row w_row0 of the stacked
-    // [E * N, K] tensor, activations at row x_row0 of the expert-sorted fp16 copy, results scattered to row_map[x_row0 + i]
-    const MoeItem* items;          // null: dense mode
-    const int* num_items;          // device: number of items of this step
-    const uint32_t* row_map;       // sorted position -> output row
+    int m_tiles;                   // dense mode: tiles of kMB activation rows; tile id = weight tile * m_tiles + row tile (the row tiles of a weight
+                                   // tile run side by side, so its bytes come from memory once)
+    // grouped (mixture-of-experts) mode: the chunk list lives in device memory -- built from the routing of this step (moe.cu): chunk = (expert, <= kMB routed
+    // rows); tile id = chunk * n_tiles + weight tile, the weight tiles of every segment of one expert in a row.  Weights at row expert * n + n0 of a segment's
+    // stacked [E * n, K] tensor, activations at row x_row0 of the expert-sorted fp16 copy, results scattered to row_map[x_row0 + i]
+    const MoeChunk* chunks;        // null: dense mode
+    const int* num_chunks;         // device: number of chunks of this step
+    const uint32_t* row_map;       // sorted position -> output row; null: the sorted position itself
     const float* row_scale;        // per OUTPUT row multiplier (top-k routing weight) or null
     // L2 prefetch of the NEXT GEMM's weights (decode engine): once this CTA's own loads are all issued, its W producer asks the L2 to
     // fetch its 1 / grid share of up to three tensors -- HBM is idle during the drain / epilogue / next prologue (~3 us per boundary)
@@ -106,6 +108,31 @@ struct GemmParams {
 __device__ __forceinline__ int seg_of_tile(const GemmParams& p, int tile) { return (tile >= p.tile_end[0]) + (tile >= p.tile_end[1]); }
 // first tile of segment sg (constant indices only: dynamic indexing would spill the parameter struct to local memory)
 __device__ __forceinline__ int seg_first_tile(const GemmParams& p, int sg) { return sg == 0 ? 0 : (sg == 1 ? p.tile_end[0] : p.tile_end[1]); }
+__device__ __forceinline__ int seg_rows(const GemmParams& p, int sg) { return sg == 0 ? p.n[0] : (sg == 1 ? p.n[1] : p.n[2]); }
+// what a tile id means
+struct Tile {
+    int sg, n0;          // segment, first weight row within the segment's matrix
+    int wrow;            // first row of the tile in the segment's tensor (grouped: the stack of all experts)
+    int xrow, count;     // first activation row, rows
+};
+template <int kMB>
+__device__ __forceinline__ Tile tile_of(const GemmParams& p, int tile) {
+    Tile t;
+    if (p.chunks) {
+        const int c = tile / p.n_tiles, w = tile - c * p.n_tiles;
+        const MoeChunk ch = p.chunks[c];
+        t.sg = seg_of_tile(p, w);
+        t.n0 = (w - seg_first_tile(p, t.sg)) * kTileN;
+        t.wrow = ch.expert * seg_rows(p, t.sg) + t.n0;
+        t.xrow = ch.x_row0; t.count = ch.count;
+    } else {
+        const int w = p.m_tiles == 1 ? tile : tile / p.m_tiles, mt = tile - w * p.m_tiles;
+        t.sg = seg_of_tile(p, w);
+        t.n0 = t.wrow = (w - seg_first_tile(p, t.sg)) * kTileN;
+        t.xrow = mt * kMB; t.count = min(kMB, p.m - t.xrow);
+    }
+    return t;
+}
 
 // Symmetric int4 (GPTQ) in the repacked layout written by gptq_repack(): per row, per 64-k chunk, 32 bytes whose low
 // nibbles are k = 0..31 and high nibbles k = 32..63 of the chunk -- the same nibble geometry as a Q4_K chunk, so the
@@ -463,9 +490,9 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
     // ---- stream-K range of this CTA over the flattened (tile, super-block) space -----------------
     // (32-bit on purpose: 64-bit integer division costs ~500 cycles each on the SM and sat on the critical path of every
     // launch; the host guarantees total * gridDim.x < 2^31)
-    const bool moe = p.items != nullptr;
-    if (moe) pdl_wait();               // the tile list is produced by the previous kernel (routing of this step)
-    const uint32_t n_tiles_rt = moe ? (uint32_t)*reinterpret_cast<const volatile int*>(p.num_items) : (uint32_t)p.n_tiles;
+    const bool moe = p.chunks != nullptr;
+    if (moe) pdl_wait();               // the chunk list is produced by an earlier kernel (routing of this step)
+    const uint32_t n_tiles_rt = moe ? (uint32_t)*reinterpret_cast<const volatile int*>(p.num_chunks) * (uint32_t)p.n_tiles : (uint32_t)p.n_tiles * (uint32_t)p.m_tiles;
     const uint32_t total = n_tiles_rt * (uint32_t)p.nsb, nsb = (uint32_t)p.nsb;
     const uint32_t u0 = p.whole_tiles ? (n_tiles_rt * blockIdx.x / gridDim.x) * nsb : total * blockIdx.x / gridDim.x;
     const uint32_t u1 = p.whole_tiles ? (n_tiles_rt * (blockIdx.x + 1) / gridDim.x) * nsb : total * (blockIdx.x + 1) / gridDim.x;
@@ -479,13 +506,13 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_w));
         int it = 0;
         int tile = (int)tile0, sb = (int)sb0;
+        Tile ti = u0 < u1 ? tile_of<kMB>(p, tile) : Tile{};
         for (uint32_t u = u0; u < u1; ++u, ++it) {
             const int s = it % kW;
             mbar_wait(w_empty(s), ((it / kW) & 1) ^ 1);
             if (p.trace && blockIdx.x == 0 && leader && it < 32) p.trace[it * 8 + 0] = clock64();
-            const int sg = moe ? 0 : seg_of_tile(p, tile);
-            const CUtensorMap* wm = sg == 0 ? &wmap0 : (sg == 1 ? &wmap1 : &wmap2);
-            const int wrow = moe ? p.items[tile].w_row0 : (tile - seg_first_tile(p, sg)) * kTileN;      // first weight row of this tile
+            const CUtensorMap* wm = ti.sg == 0 ? &wmap0 : (ti.sg == 1 ? &wmap1 : &wmap2);
+            const int wrow = ti.wrow;
             if (leader) {
                 // W box start (bytes): Q4_K blocks are 144 B (16-aligned); Q6_K blocks (210 B) start at the block address
                 // rounded down to 16 -- TMA box starts must be 16-byte aligned
@@ -498,7 +525,7 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                             wrow, pol_w);
             }
             __syncwarp();
-            if (++sb == (int)nsb) { sb = 0; ++tile; }
+            if (++sb == (int)nsb) { sb = 0; ++tile; if (u + 1 < u1) ti = tile_of<kMB>(p, tile); }
         }
         if (leader) {
 #pragma unroll
@@ -521,10 +548,10 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_x));
         int it = 0;
         int sb = (int)sb0, xtile = (int)tile0;
+        int xrow = u0 < u1 ? tile_of<kMB>(p, xtile).xrow : 0;
         for (uint32_t u = u0; u < u1; ++u, ++it) {
             const int s = it % kX;
             mbar_wait(x_empty(s), ((it / kX) & 1) ^ 1);
-            const int xrow = moe ? p.items[xtile].x_row0 : 0;          // grouped mode: this tile's rows of the expert-sorted activations
             if (leader) {
                 mbar_expect_tx(x_full(s), C::kXBytes);
                 const uint32_t dst = smem_base + C::kXOff + s * C::kXBytes;
@@ -532,7 +559,7 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                 for (int q = 0; q < 4; ++q) tma_load_2d(dst + q * kMB * kXSubBytes, &xmap, x_full(s), sb * kSB + q * 64, xrow, pol_x);
             }
             __syncwarp();
-            if (++sb == (int)nsb) { sb = 0; ++xtile; }
+            if (++sb == (int)nsb) { sb = 0; ++xtile; if (u + 1 < u1) xrow = tile_of<kMB>(p, xtile).xrow; }
         }
     } else if (warp == kDequantWarps + 2) {
         // ======================================= MMA ISSUER ======================================
@@ -592,8 +619,8 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         // if loaded on demand -- they are fetched ONE UNIT AHEAD instead (weights: no dependency on the previous kernel)
         float m4_next[4] = {0.f, 0.f, 0.f, 0.f};
         auto m4_fetch = [&](int tl, int sbx) {
-            const int sgx = seg_of_tile(p, tl);
-            const int rw = (tl - seg_first_tile(p, sgx)) * kTileN + row, nn = sgx == 0 ? p.n[0] : (sgx == 1 ? p.n[1] : p.n[2]);
+            const int wt = p.m_tiles == 1 ? tl : tl / p.m_tiles, sgx = seg_of_tile(p, wt);      // (int4 / FP4 weights have no grouped form)
+            const int rw = (wt - seg_first_tile(p, sgx)) * kTileN + row, nn = seg_rows(p, sgx);
             const M4Ctx c{sgx == 0 ? p.scales_seg[0] : (sgx == 1 ? p.scales_seg[1] : p.scales_seg[2]), nn, p.group_size, sbx * kSB, rw < nn ? rw : 0,
                           p.scale_bf16, 0, 1, 0, nullptr, sgx == 0 ? p.zp_seg[0] : (sgx == 1 ? p.zp_seg[1] : p.zp_seg[2]), {0.f, 0.f, 0.f, 0.f}, 0};
             const int kq = sbx * kSB + qt * 64;
@@ -623,6 +650,7 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         for (uint32_t u = u0; u < u1; ++tile) {
             const uint32_t tile_begin = (uint32_t)tile * nsb, tile_end = tile_begin + nsb;
             const uint32_t seg_begin = u, seg_end = tile_end < u1 ? tile_end : u1;
+            const Tile ti = tile_of<kMB>(p, tile);
             for (; u < seg_end; ++u, ++it) {
                 float m4_cur[4] = {m4_next[0], m4_next[1], m4_next[2], m4_next[3]};
                 if constexpr (kPrefetchScales) {
@@ -637,13 +665,9 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                 const uint32_t afp = aph ^ 1;
                 const bool skip = (p.debug & 2) != 0;
                 // marlin: the scales / zero points of the weight matrix this tile belongs to (constant indices only, see seg_first_tile)
-                const int msg = kType == kTypeM4 ? seg_of_tile(p, tile) : 0;
-                int mrow = (tile - seg_first_tile(p, msg)) * kTileN + row;
-                const int mn = msg == 0 ? p.n[0] : (msg == 1 ? p.n[1] : p.n[2]);
-                if (moe) {                                 // grouped FP8: the scale row is the row of the STACKED [E * n, k] tensor
-                    const MoeItem mi = p.items[tile];
-                    mrow = mi.n0 + row < mn ? mi.w_row0 + row : 0;
-                } else if (mrow >= mn) mrow = 0;
+                const int msg = kType == kTypeM4 ? ti.sg : 0;
+                const int mn = seg_rows(p, msg);
+                const int mrow = ti.n0 + row < mn ? ti.wrow + row : 0;       // grouped FP8: the scale row is the row of the STACKED [E * n, k] tensor
                 const M4Ctx mc{msg == 0 ? p.scales_seg[0] : (msg == 1 ? p.scales_seg[1] : p.scales_seg[2]), mn, p.group_size, (int)(u - tile_begin) * kSB,
                                mrow, p.scale_bf16, p.debug, p.scale_by, p.scale_sk, p.norm,
                                msg == 0 ? p.zp_seg[0] : (msg == 1 ? p.zp_seg[1] : p.zp_seg[2]), {m4_cur[0], m4_cur[1], m4_cur[2], m4_cur[3]},
@@ -668,24 +692,27 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
             if (moe) {
                 // grouped mode: whole item per CTA; column i of the accumulator = routed row x_row0 + i of this expert's chunk, scattered
                 // to its output row (pair index) with the routing weight folded in
-                const MoeItem item = p.items[tile];
-                const int n_loc = item.n0 + row;
+                const int n_loc = ti.n0 + row, n_rows = seg_rows(p, ti.sg);
+                float* const ymoe = ti.sg == 0 ? p.y[0] : (ti.sg == 1 ? p.y[1] : p.y[2]);
                 constexpr int kColsPerWarpM = kMB / 4;
                 const float post = (kType == kTypeF8 && p.norm) ? __ldg(p.norm + 1) : 1.f;      // FP8: undo the range shift of the tile scales
 #pragma unroll
                 for (int c0 = 0; c0 < kColsPerWarpM; c0 += 8) {
+                    if (qt * kColsPerWarpM + c0 >= ti.count) break;
                     uint32_t acc[8], more[8];
                     tc_ld8(tmem + kColD + lane_addr + qt * kColsPerWarpM + c0, acc);
-                    tc_ld8(tmem + kColD + kMB + lane_addr + qt * kColsPerWarpM + c0, more);
+                    if constexpr (C::kAcc == 2) tc_ld8(tmem + kColD + kMB + lane_addr + qt * kColsPerWarpM + c0, more);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (n_loc < p.n[0]) {
+                    if (n_loc < n_rows) {
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
                             const int mi = qt * kColsPerWarpM + c0 + i;
-                            if (mi < item.count) {
-                                const uint32_t orow = __ldg(p.row_map + item.x_row0 + mi);
+                            if (mi < ti.count) {
+                                const uint32_t orow = p.row_map ? __ldg(p.row_map + ti.xrow + mi) : (uint32_t)(ti.xrow + mi);
                                 const float sc = p.row_scale ? __ldg(p.row_scale + orow) : 1.f;
-                                p.y[0][(int64_t)orow * p.ldy + n_loc] = (__uint_as_float(acc[i]) + __uint_as_float(more[i])) * (sc * post);
+                                float v = __uint_as_float(acc[i]);
+                                if constexpr (C::kAcc == 2) v += __uint_as_float(more[i]);
+                                ymoe[(int64_t)orow * p.ldy + n_loc] = v * (sc * post);
                             }
                         }
                     }
@@ -696,8 +723,8 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                 ++seg;
                 continue;
             }
-            const int sg = seg_of_tile(p, tile);
-            const int n_idx = (tile - seg_first_tile(p, sg)) * kTileN + row;
+            const int sg = ti.sg;
+            const int n_idx = ti.n0 + row;
             float* ybase = sg == 0 ? p.y[0] : (sg == 1 ? p.y[1] : p.y[2]);
             // slab mode: the k-th CTA that works on a tile writes slab k.  CTA b owns units [total*b/grid, total*(b+1)/grid),
             // so the owner of unit u is ((u+1)*grid - 1) / total and only a CTA's first segment can start inside a tile.
@@ -706,9 +733,10 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
             if (p.slabs > 0) ybase += (int64_t)ordinal * p.slab_stride;
             const int zero_slabs = (p.slabs > 0 && seg_end == tile_end) ? p.slabs - 1 - ordinal : 0;   // slabs nobody else writes
             const int n_rows = sg == 0 ? p.n[0] : (sg == 1 ? p.n[1] : p.n[2]);
-            constexpr int kColsPerWarp = kMB / 4;                 // this warp's share of the batch columns (8 or 16)
+            constexpr int kColsPerWarp = kMB / 4;                 // this warp's share of the batch columns (8, 16 or 32)
 #pragma unroll
             for (int c0 = 0; c0 < kColsPerWarp; c0 += 8) {
+                if (qt * kColsPerWarp + c0 >= ti.count) break;
                 uint32_t acc[8];
                 tc_ld8(tmem + kColD + lane_addr + qt * kColsPerWarp + c0, acc);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -724,8 +752,8 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         const int mi = qt * kColsPerWarp + c0 + i;
-                        if (mi < p.m) {
-                            float* o = ybase + (int64_t)mi * p.ldy + n_idx;
+                        if (mi < ti.count) {
+                            float* o = ybase + (int64_t)(ti.xrow + mi) * p.ldy + n_idx;
                             const float val = __uint_as_float(acc[i]);
                             if (p.slabs > 0) {
                                 *o = val;
@@ -782,9 +810,17 @@ template <int kMB, int kType>
 void launch(const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, cudaStream_t st) {
     auto kern = qmatmul_tc_kernel<kMB, kType>;
     ensure_dynamic_smem(reinterpret_cast<const void*>(kern), Cfg<kMB, kType>::kTotal);
-    const int grid = gemm_grid(p.n_tiles, p.nsb, p.whole_tiles != 0, p.slabs > 0);
+    const int grid = p.chunks ? sm_count() : gemm_grid((int64_t)p.n_tiles * p.m_tiles, p.nsb, p.whole_tiles != 0, p.slabs > 0);
     launch_pdl(kern, dim3(grid), dim3(kThreads), Cfg<kMB, kType>::kTotal, st, wm[0], wm[1], wm[2], xm, p);
     count_launch();
+}
+
+void launch_rows(int mb, int ggml_type, const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, cudaStream_t st) {
+    if (ggml_type == B200_GGML_Q4_K) {
+        if (mb == 32) launch<32, B200_GGML_Q4_K>(wm, xm, p, st); else if (mb == 64) launch<64, B200_GGML_Q4_K>(wm, xm, p, st); else launch<128, B200_GGML_Q4_K>(wm, xm, p, st);
+    } else {
+        if (mb == 32) launch<32, B200_GGML_Q6_K>(wm, xm, p, st); else if (mb == 64) launch<64, B200_GGML_Q6_K>(wm, xm, p, st); else launch<128, B200_GGML_Q6_K>(wm, xm, p, st);
+    }
 }
 
 bool make_w_map(CUtensorMap* wm, const void* w, int n, int nsb, int ggml_type) {
@@ -874,10 +910,15 @@ bool qmatmul_tc_supported(int m, int n, int k, int ggml_type) {
 // Decomposition: with many tiles per SM every CTA gets whole tiles (no split); otherwise stream-K over (tile, super-block).
 static bool use_whole_tiles(int64_t n_tiles) { return n_tiles >= 4 * (int64_t)sm_count(); }
 
+// activation rows per tile, and tiles: up to 64 rows are one tile of 32 or 64; more rows come in tiles of 128 (the weights are converted once per row tile;
+// 64-row tiles would convert twice as often)
+static int rows_per_tile(int m) { return m <= 32 ? 32 : (m <= 64 ? 64 : 128); }
+static int row_tiles(int m) { return m <= 64 ? 1 : (m + 127) / 128; }
+
 // true when some output tile is produced by more than one CTA (or accumulate): y must then hold the
 // addend (zeros for a plain product) before the launch
-bool qmatmul_tc_needs_zeroed_output(int n, int k) {
-    const int64_t n_tiles = (n + kTileN - 1) / kTileN, nsb = k / 256, total = n_tiles * nsb;
+bool qmatmul_tc_needs_zeroed_output(int m, int n, int k) {
+    const int64_t n_tiles = (int64_t)((n + kTileN - 1) / kTileN) * row_tiles(m), nsb = k / 256, total = n_tiles * nsb;
     if (use_whole_tiles(n_tiles)) return false;
     const int64_t grid = total < sm_count() ? total : sm_count();
     for (int64_t c = 1; c < grid; ++c)
@@ -924,7 +965,7 @@ int qmatmul_tc_multi(const void* x_f16, int nseg, const void* const* w, float* c
     if (nseg < 1 || nseg > kMaxSeg) { set_error(kErrBadArg, "qmatmul: %d segments (max %d)", nseg, kMaxSeg); return 0; }
     if ((uintptr_t)x_f16 & 15) { set_error(kErrBadArg, "qmatmul: x must be 16-byte aligned"); return 0; }
     const int nsb = k / 256;
-    const int mb = m <= 32 ? 32 : 64;
+    const int mb = rows_per_tile(m), mt = row_tiles(m);
     CUtensorMap wm[kMaxSeg], xm;
     GemmParams p{};
     int tiles = 0;
@@ -945,20 +986,19 @@ int qmatmul_tc_multi(const void* x_f16, int nseg, const void* const* w, float* c
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) { set_error(kErrCuda, "qmatmul: activation tensor map failed (%d)", (int)r); return 0; }
     }
-    if ((int64_t)tiles * nsb * sm_count() >= (int64_t)1 << 31) { set_error(kErrUnsupported, "qmatmul: %d tiles x %d super-blocks exceed the 32-bit unit range", tiles, nsb); return 0; }
-    p.ldy = ldy; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.accumulate = accumulate;
-    p.whole_tiles = use_whole_tiles(tiles) ? 1 : 0;
+    if ((int64_t)tiles * mt * nsb * sm_count() >= (int64_t)1 << 31) { set_error(kErrUnsupported, "qmatmul: %d tiles x %d super-blocks exceed the 32-bit unit range", tiles, nsb); return 0; }
+    p.ldy = ldy; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = mt; p.accumulate = accumulate;
+    p.whole_tiles = use_whole_tiles((int64_t)tiles * mt) ? 1 : 0;
     take_prefetch(p);
     if (slabs_avail > 0) {
-        p.slabs = qmatmul_tc_slab_count(tiles, nsb);
+        p.slabs = qmatmul_tc_slab_count((int64_t)tiles * mt, nsb);
         p.slab_stride = slab_stride;
         p.accumulate = 0;
         if (p.slabs > slabs_avail) { set_error(kErrBadArg, "qmatmul: %d slabs needed, %d provided", p.slabs, slabs_avail); return 0; }
     }
     { static const char* dbg = getenv("B200_GEMM_DEBUG"); p.debug = dbg ? atoi(dbg) : 0; }
     { static const char* tr = getenv("B200_GEMM_TRACE"); p.trace = tr ? reinterpret_cast<long long*>(strtoull(tr, nullptr, 0)) : nullptr; }
-    if (ggml_type == B200_GGML_Q4_K) { if (mb == 32) launch<32, B200_GGML_Q4_K>(wm, xm, p, st); else launch<64, B200_GGML_Q4_K>(wm, xm, p, st); }
-    else { if (mb == 32) launch<32, B200_GGML_Q6_K>(wm, xm, p, st); else launch<64, B200_GGML_Q6_K>(wm, xm, p, st); }
+    launch_rows(mb, ggml_type, wm, xm, p, st);
     check_launch("qmatmul_tc");
     return p.slabs;
 }
@@ -991,7 +1031,7 @@ static void wq16_launch(int kind, const void* x_f16, const void* w, const void* 
     GemmParams p{};
     const int tiles = (n + kTileN - 1) / kTileN;
     for (int i = 0; i < kMaxSeg; ++i) { p.y[i] = slabs; p.n[i] = n; p.tile_end[i] = i == 0 ? tiles : 0x7fffffff; }
-    p.ldy = n; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.accumulate = 0;
+    p.ldy = n; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = 1; p.accumulate = 0;
     p.whole_tiles = use_whole_tiles(tiles) ? 1 : 0;
     p.slabs = qmatmul_tc_slab_count(tiles, nsb);
     p.slab_stride = (int64_t)m * n;
@@ -1056,7 +1096,7 @@ void marlin_tc_f32_multi(const void* x_f16_k4, int nseg, const void* const* w, c
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) { set_error(kErrCuda, "marlin_4bit(f32): activation tensor map failed (%d)", (int)r); return; }
     }
-    p.ldy = ldy; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.accumulate = accumulate;
+    p.ldy = ldy; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = 1; p.accumulate = accumulate;
     p.whole_tiles = use_whole_tiles(tiles) ? 1 : 0;
     p.scales = p.scales_seg[0]; p.zp = p.zp_seg[0]; p.group_size = group_size; p.k = k; p.scale_bf16 = scale_bf16; p.scale_by = 1;
     take_prefetch(p);
@@ -1105,64 +1145,59 @@ bool qmatmul_tc_moe_supported(int n, int k, int ggml_type) {
     return false;
 }
 
+static bool moe_x_map(CUtensorMap* xm, const void* xs, int rows, int k, int box_rows, const char* who) {
+    const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
+    const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
+    const cuuint32_t es[2] = {1, 1};
+    const CUresult r = encode_fn()(xm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(xs), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { set_error(kErrCuda, "%s: activation tensor map failed (%d)", who, (int)r); return false; }
+    return true;
+}
+
 // block-scaled FP8 experts (moe_gemm_fp8): w = e4m3 [E * n, k], scale f32 [E * n / by, ceil(k / bx)] (n % by == 0), activations fp16 in
-// NATURAL order; norm = 2 device floats (scratch): the range shift of the scales, computed here
+// NATURAL order, chunks of <= 32 rows; norm = 2 device floats (scratch): the range shift of the scales, computed here
 bool qmatmul_tc_moe_fp8_supported(int n, int k, int by, int bx) { return n >= 1 && k >= 256 && k % 256 == 0 && by >= 1 && n % by == 0 && bx >= 64 && bx % 64 == 0; }
 void qmatmul_tc_moe_fp8(const void* xs_f16, int xs_rows, const void* w, const float* scale, int num_experts, float* y, int64_t ldy, int n, int k, int by, int bx,
-                        const MoeItem* items, const int* num_items, int max_items, const uint32_t* row_map, const float* row_scale, float* norm,
+                        const MoeChunk* chunks, const int* num_chunks, int max_chunks, const uint32_t* row_map, const float* row_scale, float* norm,
                         cudaStream_t st) {
-    EncodeTiledFn enc = encode_fn();
-    if (!enc) { set_error(kErrCuda, "moe_gemm_fp8: cuTensorMapEncodeTiled unavailable"); return; }
+    if (!encode_fn()) { set_error(kErrCuda, "moe_gemm_fp8: cuTensorMapEncodeTiled unavailable"); return; }
     if (((uintptr_t)xs_f16 | (uintptr_t)w) & 15) { set_error(kErrBadArg, "moe_gemm_fp8: x and w must be 16-byte aligned"); return; }
-    const int nsb = k / 256, sk = (k + bx - 1) / bx;
+    const int nsb = k / 256, sk = (k + bx - 1) / bx, tiles = (n + kTileN - 1) / kTileN;
     launch_pdl(fp8_scale_norm_kernel, dim3(1), dim3(256), 0, st, scale, (int64_t)num_experts * (n / by) * sk, norm);
     count_launch();
     CUtensorMap wm[kMaxSeg], xm;
     for (int i = 0; i < kMaxSeg; ++i) if (!make_w_map(&wm[i], w, num_experts * n, nsb, kTypeF8)) return;
-    {
-        const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)xs_rows};
-        const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-        const cuuint32_t box[2] = {64, 32};
-        const cuuint32_t es[2] = {1, 1};
-        CUresult r = enc(&xm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(xs_f16), dims, strides, box, es,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) { set_error(kErrCuda, "moe_gemm_fp8: activation tensor map failed (%d)", (int)r); return; }
-    }
-    if ((int64_t)max_items * nsb * sm_count() >= (int64_t)1 << 31) { set_error(kErrUnsupported, "moe_gemm_fp8: %d items x %d super-blocks exceed the 32-bit unit range", max_items, nsb); return; }
+    if (!moe_x_map(&xm, xs_f16, xs_rows, k, 32, "moe_gemm_fp8")) return;
+    if ((int64_t)max_chunks * tiles * nsb * sm_count() >= (int64_t)1 << 31) { set_error(kErrUnsupported, "moe_gemm_fp8: %d items x %d super-blocks exceed the 32-bit unit range", max_chunks * tiles, nsb); return; }
     GemmParams p{};
     for (int i = 0; i < kMaxSeg; ++i) { p.y[i] = y; p.n[i] = n; p.tile_end[i] = 0x7fffffff; p.scales_seg[i] = scale; p.zp_seg[i] = nullptr; }
-    p.ldy = ldy; p.m = 32; p.nsb = nsb; p.n_tiles = max_items; p.accumulate = 0; p.whole_tiles = 1;
-    p.items = items; p.num_items = num_items; p.row_map = row_map; p.row_scale = row_scale;
+    p.ldy = ldy; p.m = 32; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = 1; p.accumulate = 0; p.whole_tiles = 1;
+    p.chunks = chunks; p.num_chunks = num_chunks; p.row_map = row_map; p.row_scale = row_scale;
     p.scales = scale; p.group_size = bx; p.k = k; p.scale_by = by; p.scale_sk = sk; p.norm = norm;
     launch<32, kTypeF8>(wm, xm, p, st);
     check_launch("moe_gemm_fp8");
 }
 
-void qmatmul_tc_moe(const void* xs_f16_k4, int xs_rows, const void* w, int num_experts, float* y, int64_t ldy, int n, int k, int ggml_type,
-                    const MoeItem* items, const int* num_items, int max_items, const uint32_t* row_map, const float* row_scale, cudaStream_t st) {
-    EncodeTiledFn enc = encode_fn();
-    if (!enc) { set_error(kErrCuda, "moe_gemm: cuTensorMapEncodeTiled unavailable"); return; }
-    if (((uintptr_t)xs_f16_k4 | (uintptr_t)w) & 15) { set_error(kErrBadArg, "moe_gemm: x and w must be 16-byte aligned"); return; }
-    const int nsb = k / 256;
+// up to two stacks of GGML experts (gate and up) applied to the same sorted rows in one launch; chunk_rows = the rows per chunk the list was built with
+void qmatmul_tc_moe(const void* xs_f16_k4, int xs_rows, int nseg, const void* const* w, int num_experts, float* const* y, int64_t ldy, int n, int k, int ggml_type,
+                    const MoeChunk* chunks, const int* num_chunks, int max_chunks, int chunk_rows, const uint32_t* row_map, const float* row_scale, cudaStream_t st) {
+    if (!encode_fn()) { set_error(kErrCuda, "moe_gemm: cuTensorMapEncodeTiled unavailable"); return; }
+    const int nsb = k / 256, tiles = (n + kTileN - 1) / kTileN;
     CUtensorMap wm[kMaxSeg], xm;
-    for (int i = 0; i < kMaxSeg; ++i) if (!make_w_map(&wm[i], w, num_experts * n, nsb, ggml_type)) return;      // experts stacked along the rows
-    {
-        const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)xs_rows};
-        const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-        const cuuint32_t box[2] = {64, 32};
-        const cuuint32_t es[2] = {1, 1};
-        CUresult r = enc(&xm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(xs_f16_k4), dims, strides, box, es,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) { set_error(kErrCuda, "moe_gemm: activation tensor map failed (%d)", (int)r); return; }
-    }
-    if ((int64_t)max_items * nsb * sm_count() >= (int64_t)1 << 31) { set_error(kErrUnsupported, "moe_gemm: %d items x %d super-blocks exceed the 32-bit unit range", max_items, nsb); return; }
     GemmParams p{};
-    for (int i = 0; i < kMaxSeg; ++i) { p.y[i] = y; p.n[i] = n; p.tile_end[i] = 0x7fffffff; }
-    p.ldy = ldy; p.m = 32; p.nsb = nsb; p.n_tiles = max_items; p.accumulate = 0; p.whole_tiles = 1;
-    p.items = items; p.num_items = num_items; p.row_map = row_map; p.row_scale = row_scale;
-    if (ggml_type == B200_GGML_Q4_K) launch<32, B200_GGML_Q4_K>(wm, xm, p, st); else launch<32, B200_GGML_Q6_K>(wm, xm, p, st);
+    for (int i = 0; i < kMaxSeg; ++i) {
+        const int j = i < nseg ? i : nseg - 1;
+        if (((uintptr_t)xs_f16_k4 | (uintptr_t)w[j]) & 15) { set_error(kErrBadArg, "moe_gemm: x and w must be 16-byte aligned"); return; }
+        if (!make_w_map(&wm[i], w[j], num_experts * n, nsb, ggml_type)) return;      // experts stacked along the rows
+        p.y[i] = y[j]; p.n[i] = n; p.tile_end[i] = i < nseg ? (i + 1) * tiles : 0x7fffffff;
+    }
+    if (!moe_x_map(&xm, xs_f16_k4, xs_rows, k, chunk_rows, "moe_gemm")) return;
+    if ((int64_t)max_chunks * nseg * tiles * nsb * sm_count() >= (int64_t)1 << 31) { set_error(kErrUnsupported, "moe_gemm: %d items x %d super-blocks exceed the 32-bit unit range", max_chunks * nseg * tiles, nsb); return; }
+    p.ldy = ldy; p.m = chunk_rows; p.nsb = nsb; p.n_tiles = nseg * tiles; p.m_tiles = 1; p.accumulate = 0; p.whole_tiles = 1;
+    p.chunks = chunks; p.num_chunks = num_chunks; p.row_map = row_map; p.row_scale = row_scale;
+    launch_rows(chunk_rows, ggml_type, wm, xm, p, st);
     check_launch("moe_gemm");
 }
 

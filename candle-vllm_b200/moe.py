@@ -105,8 +105,39 @@ class FusedMoe:
         self.E, self.H, self.I, self.k = num_experts, hidden, inter, num_experts_per_tok
         self.norm_topk_prob, self.routed_scaling_factor = norm_topk_prob, routed_scaling_factor
 
+    def _block_covers(self, xs: torch.Tensor, T: int) -> bool:
+        """``moe_block_gguf`` takes the step: the grouped GEMM covers the three products and every tensor starts on 16 bytes"""
+        if xs.dtype != torch.float32 or xs.dim() != 2 or xs.shape[1] != self.H or not xs.is_cuda or tuple(self.gate.shape) != (self.E, self.H):
+            return False
+        t = self.types
+        if any(ty not in (GgmlType.Q4_K, GgmlType.Q6_K) or w.dtype != torch.uint8 or not w.is_contiguous()
+               or w.numel() != self.E * self.I * self.H // 256 * GgmlType.BLOCK[ty][1] for w, ty in zip((self.ge, self.ue, self.de), t)):
+            return False
+        require_device()
+        if not lib().moe_block_supported(C.c_int32(T), C.c_int32(self.H), C.c_int32(self.I), C.c_int32(self.E), C.c_int32(self.k), C.c_int32(t[0]), C.c_int32(t[1]),
+                                         C.c_int32(t[2])):
+            return False
+        x_at = xs.data_ptr() if xs.is_contiguous() else 0           # (a copy is made of the others)
+        return (x_at | self.gate.data_ptr() | self.ge.data_ptr() | self.ue.data_ptr() | self.de.data_ptr()) % 16 == 0
+
+    def _block(self, xs: torch.Tensor, T: int) -> torch.Tensor:
+        out = torch.empty((T, self.H), dtype=torch.float32, device=xs.device)
+        L = lib()
+        dims = [C.c_int32(v) for v in (T, self.H, self.I, self.E, self.k)]
+        need = L.moe_block_workspace_bytes(*dims)
+        ws = torch.empty(need + 256, dtype=torch.uint8, device=xs.device)
+        off = -ws.data_ptr() % 256
+        with torch.cuda.device(xs.device):
+            L.moe_block_gguf(_ptr(xs), _ptr(self.gate), _ptr(self.ge), _ptr(self.ue), _ptr(self.de), _ptr(out), *dims, *[C.c_int32(v) for v in self.types],
+                             C.c_int32(1 if self.norm_topk_prob else 0), C.c_float(1.0 if self.routed_scaling_factor is None else self.routed_scaling_factor),
+                             C.c_void_p(ws.data_ptr() + off), C.c_size_t(need), _stream(xs.device))
+        check("FusedMoe.forward")
+        return out
+
     def forward(self, xs: torch.Tensor, is_prefill: bool = False) -> torch.Tensor:
         T = xs.shape[0]
+        if self._block_covers(xs, T):
+            return self._block(xs.contiguous(), T)
         # router: a [T, H] x [H, E] f32 product on the plumbing library (the reference's `gate` Linear, moe.rs:1435); every expert
         # GEMM below runs on this backend's kernels
         router_logits = xs.float() @ self.gate.t()

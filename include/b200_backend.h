@@ -252,6 +252,15 @@ size_t moe_gemm_workspace_bytes(int32_t num_pairs, int32_t n, int32_t k, int32_t
 void moe_gemm_gguf(const float* x, const void* experts, const float* topk_weights, const uint32_t* sorted_token_ids, const uint32_t* expert_ids,
                    float* out, int32_t num_experts, int32_t topk, int32_t size_m, int32_t num_pairs, int32_t n, int32_t k, int32_t ggml_type,
                    int32_t is_prefill, void* workspace, size_t workspace_bytes, int64_t stream);
+/*   moe_block_gguf: the whole block in one call (FusedMoe::forward, moe.rs:1429-1482): x f32 [T, hidden]; router f32 [E, hidden]; gate / up stacked GGML blocks
+ *     [E, inter, hidden], down [E, hidden, inter]; out f32 [T, hidden] = sum over the top-k experts of w * down(silu(gate x) * up x), w the softmax weights of
+ *     topk_softmax (divided by their sum when normalise) times scaling.  Sizes for which moe_block_supported returns 1 (the grouped GEMM covers the three products);
+ *     16-byte aligned pointers, a 256-byte aligned workspace of moe_block_workspace_bytes(). */
+int32_t moe_block_supported(int32_t num_tokens, int32_t hidden, int32_t inter, int32_t num_experts, int32_t topk, int32_t type_gate, int32_t type_up, int32_t type_down);
+size_t moe_block_workspace_bytes(int32_t num_tokens, int32_t hidden, int32_t inter, int32_t num_experts, int32_t topk);
+void moe_block_gguf(const float* x, const float* router, const void* gate, const void* up, const void* down, float* out, int32_t num_tokens, int32_t hidden,
+                    int32_t inter, int32_t num_experts, int32_t topk, int32_t type_gate, int32_t type_up, int32_t type_down, int32_t normalise, float scaling,
+                    void* workspace, size_t workspace_bytes, int64_t stream);
 
 /* moe_gemm_fp8 -- replaces attention_rs::moe::moe_gemm_fp8 (call sites src/openai/models/layers/moe.rs:1447-1473, block-FP8
  * experts as in DeepSeek-V3 / Qwen3 FP8 checkpoints): x [size_m, k] and out [num_pairs, n] of `dtype` (B200_F16 / B200_BF16); experts e4m3
