@@ -117,6 +117,18 @@ def ensure_built(group: str) -> C.CDLL:
     return lib()
 
 
+_typed = {}
+
+
+def typed(name: str, restype, *argtypes):
+    """The library function with its argument types declared: plain ints, floats and pointers go in as they are, without a ctypes object for each (0.2 us apiece).  A
+    prototype of its own, so that the loader's untyped functions keep taking what their callers pass."""
+    f = _typed.get(name)
+    if f is None:
+        f = _typed[name] = C.CFUNCTYPE(restype, *argtypes)((name, lib()))
+    return f
+
+
 def check(what: str = "") -> None:
     """Raise BackendError if the last call on this thread recorded an error."""
     L = lib()

@@ -22,7 +22,7 @@ from typing import Dict, List, Optional, Sequence, Union
 import numpy as np
 import torch
 
-from ._lib import BackendError, check, lib, require_device
+from ._lib import BackendError, check, lib, require_device, typed
 
 
 class DType:
@@ -55,6 +55,36 @@ def _ptr(t: Optional[torch.Tensor]):
 
 def _stream(dev=None) -> C.c_int64:
     return C.c_int64(torch.cuda.current_stream(dev).cuda_stream)
+
+
+# The calls of a decode step are short against what Python spends around them, so the operators below hand the library plain ints through typed prototypes, ask for
+# the raw stream and enter a device context only when another device is current.
+_I, _P, _L, _F, _Z = C.c_int32, C.c_void_p, C.c_int64, C.c_float, C.c_size_t
+
+
+class _Here:
+    """the device is current already"""
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        return False
+
+
+_HERE = _Here()
+
+
+def _guard(dev: torch.device):
+    return _HERE if dev.index == torch._C._cuda_getDevice() else torch.cuda.device(dev)
+
+
+def _raw_stream(dev: torch.device) -> int:
+    return torch._C._cuda_getCurrentRawStream(dev.index)
+
+
+def _at(t: Optional[torch.Tensor]):
+    return None if t is None else t.data_ptr()
 
 
 def _cuda(t: torch.Tensor, name: str) -> torch.Tensor:
@@ -151,11 +181,11 @@ def reshape_and_cache(key: torch.Tensor, value: torch.Tensor, k_cache: torch.Ten
         key, value = key.contiguous(), value.contiguous()
     cache_dt = DType.FP8_E4M3 if (fp8 or k_cache.dtype == torch.uint8) else _dt(k_cache)
     require_device()
-    with torch.cuda.device(key.device):
-        lib().reshape_and_cache(_ptr(key), _ptr(value), _ptr(k_cache), _ptr(v_cache), _ptr(slot_mapping),
-                                C.c_int32(T), C.c_int32(kvh), C.c_int32(hd), C.c_int32(bs),
-                                C.c_int64(key.stride(0)), C.c_int64(value.stride(0)), C.c_int32(_dt(key)),
-                                C.c_int32(cache_dt), C.c_int32(layout), _stream(key.device))
+    dev = key.device
+    with _guard(dev):
+        typed("reshape_and_cache", None, _P, _P, _P, _P, _P, _I, _I, _I, _I, _L, _L, _I, _I, _I, _L)(
+            key.data_ptr(), value.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), slot_mapping.data_ptr(), T, kvh, hd, bs,
+            key.stride(0), value.stride(0), _dt(key), cache_dt, layout, _raw_stream(dev))
     check("reshape_and_cache")
 
 
@@ -228,8 +258,7 @@ class PagedAttention:
         self._ws = None
 
     def _workspace(self, B: int, max_blocks: int, bs: int, dev) -> torch.Tensor:
-        need = lib().paged_attention_decode_workspace_bytes(C.c_int32(B), C.c_int32(self.num_attention_heads),
-                                                            C.c_int32(self.head_dim), C.c_int32(max_blocks), C.c_int32(bs))
+        need = typed("paged_attention_decode_workspace_bytes", _Z, _I, _I, _I, _I, _I)(B, self.num_attention_heads, self.head_dim, max_blocks, bs)
         if self._ws is None or self._ws.numel() < need or self._ws.device != dev:
             self._ws = torch.zeros(int(need), dtype=torch.uint8, device=dev)
         return self._ws
@@ -273,29 +302,24 @@ class PagedAttention:
         cache_dt = DType.FP8_E4M3 if fp8 else _dt(key_cache)
         win = int(self.sliding_window or 0)
         cap = float(softcapping or 0.0)
-        L = lib()
-        with torch.cuda.device(query.device):
+        dev = query.device
+        with _guard(dev):
             if meta.is_prefill:
                 cq, ck = meta.cu_seqlens_q, meta.cu_seqlens_k
                 if cq is None or ck is None:
                     raise BackendError("prefill requires cu_seqlens_q / cu_seqlens_k")
                 n = cq.numel() - 1
-                L.paged_attention_prefill(_ptr(out), _ptr(q), _ptr(key_cache), _ptr(value_cache), _ptr(bt), _ptr(cq), _ptr(ck),
-                                          C.c_int32(n), C.c_int32(T), C.c_int32(meta.max_seqlen_q), C.c_int32(H),
-                                          C.c_int32(self.num_key_value_heads), C.c_int32(hd), C.c_int32(bs),
-                                          C.c_int32(bt.shape[1]), C.c_float(self.scale), C.c_float(cap), C.c_int32(win),
-                                          C.c_int32(_dt(q)), C.c_int32(cache_dt), C.c_int32(layout), _stream(query.device))
+                typed("paged_attention_prefill", None, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _F, _F, _I, _I, _I, _I, _L)(
+                    out.data_ptr(), q.data_ptr(), key_cache.data_ptr(), value_cache.data_ptr(), bt.data_ptr(), cq.data_ptr(), ck.data_ptr(), n, T,
+                    meta.max_seqlen_q, H, self.num_key_value_heads, hd, bs, bt.shape[1], self.scale, cap, win, _dt(q), cache_dt, layout, _raw_stream(dev))
             else:
                 cl = meta.context_lens
                 if cl is None:
                     raise BackendError("decode requires context_lens")
-                ws = self._workspace(T, bt.shape[1], bs, query.device)
-                L.paged_attention_decode(_ptr(out), _ptr(q), _ptr(key_cache), _ptr(value_cache), _ptr(bt), _ptr(cl),
-                                         C.c_int32(T), C.c_int32(H), C.c_int32(self.num_key_value_heads), C.c_int32(hd),
-                                         C.c_int32(bs), C.c_int32(bt.shape[1]), C.c_int64(nb), C.c_float(self.scale),
-                                         C.c_float(cap), C.c_int32(win), C.c_int32(_dt(q)), C.c_int32(cache_dt),
-                                         C.c_int32(layout), C.c_int32(_TORCH2B200[odt]), _ptr(ws), C.c_size_t(ws.numel()),
-                                         _stream(query.device))
+                ws = self._workspace(T, bt.shape[1], bs, dev)
+                typed("paged_attention_decode", None, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _L, _F, _F, _I, _I, _I, _I, _I, _P, _Z, _L)(
+                    out.data_ptr(), q.data_ptr(), key_cache.data_ptr(), value_cache.data_ptr(), bt.data_ptr(), cl.data_ptr(), T, H, self.num_key_value_heads, hd,
+                    bs, bt.shape[1], nb, self.scale, cap, win, _dt(q), cache_dt, layout, _TORCH2B200[odt], ws.data_ptr(), ws.numel(), _raw_stream(dev))
         check("PagedAttention.forward")
         return out
 
@@ -362,20 +386,19 @@ class QMatMul:
         x2 = x.reshape(-1, k).contiguous()
         m = x2.shape[0]
         y = torch.empty((m, n), dtype=torch.float32, device=x.device)
-        L = lib()
-        with torch.cuda.device(x.device):
+        dev, data = x.device, self.w.data.data_ptr()
+        with _guard(dev):
+            st = _raw_stream(dev)
             if x2.dtype == torch.float16:
                 xk4 = torch.empty_like(x2)          # the GEMM consumes fp16 activations in K4 order (b200_backend.h)
-                L.cast(_ptr(x2), _ptr(xk4), C.c_int64(x2.numel()), C.c_int32(DType.F16), C.c_int32(DType.F16_K4), _stream(x.device))
-                L.qmatmul_f16act(_ptr(xk4), _ptr(self.w.data), _ptr(y), C.c_int32(m), C.c_int32(n), C.c_int32(k),
-                                 C.c_int32(self.w.ggml_type), C.c_int32(0), _stream(x.device))
+                typed("cast", None, _P, _P, _L, _I, _I, _L)(x2.data_ptr(), xk4.data_ptr(), x2.numel(), DType.F16, DType.F16_K4, st)
+                typed("qmatmul_f16act", None, _P, _P, _P, _I, _I, _I, _I, _I, _L)(xk4.data_ptr(), data, y.data_ptr(), m, n, k, self.w.ggml_type, 0, st)
             else:
-                need = L.qmatmul_workspace_bytes(C.c_int32(m), C.c_int32(n), C.c_int32(k))
-                if self._ws is None or self._ws.numel() < need or self._ws.device != x.device:
-                    self._ws = torch.empty(int(need), dtype=torch.uint8, device=x.device)
-                L.qmatmul_f32(_ptr(x2), _ptr(self.w.data), _ptr(y), C.c_int32(m), C.c_int32(n), C.c_int32(k),
-                              C.c_int32(self.w.ggml_type), C.c_int32(0), _ptr(self._ws), C.c_size_t(self._ws.numel()),
-                              _stream(x.device))
+                need = typed("qmatmul_workspace_bytes", _Z, _I, _I, _I)(m, n, k)
+                if self._ws is None or self._ws.numel() < need or self._ws.device != dev:
+                    self._ws = torch.empty(int(need), dtype=torch.uint8, device=dev)
+                typed("qmatmul_f32", None, _P, _P, _P, _I, _I, _I, _I, _I, _P, _Z, _L)(
+                    x2.data_ptr(), data, y.data_ptr(), m, n, k, self.w.ggml_type, 0, self._ws.data_ptr(), self._ws.numel(), st)
         check("QMatMul.forward")
         return y.reshape(*lead, n)
 
@@ -437,9 +460,9 @@ class Linear:
         x2, out = _lin_io(x, n, k, self.bias, "Linear")
         if k % 8 or n % 8:
             raise BackendError("Linear: in / out features must be multiples of 8 (16-byte rows for TMA)")
-        with torch.cuda.device(x.device):
-            lib().linear_16bit(_ptr(x2), _ptr(self.weight), _ptr(self.bias), _ptr(out), C.c_int32(x2.shape[0]), C.c_int32(n), C.c_int32(k),
-                               C.c_int32(_dt(x2)), _stream(x.device))
+        with _guard(x.device):
+            typed("linear_16bit", None, _P, _P, _P, _P, _I, _I, _I, _I, _L)(x2.data_ptr(), self.weight.data_ptr(), _at(self.bias), out.data_ptr(), x2.shape[0], n, k,
+                                                                            _dt(x2), _raw_stream(x.device))
         check("Linear.forward")
         return out.reshape(*x.shape[:-1], n)
 
@@ -547,8 +570,8 @@ def silu_mul(gate: torch.Tensor, up: torch.Tensor, out_dtype=torch.float32) -> t
     _cuda(gate, "gate"); require_device()
     g, u = gate.contiguous().float(), up.contiguous().float()
     out = torch.empty(g.shape, dtype=out_dtype, device=g.device)
-    with torch.cuda.device(g.device):
-        lib().silu_mul(_ptr(g), _ptr(u), _ptr(out), C.c_int64(g.numel()), C.c_int32(_TORCH2B200[out_dtype]), _stream(g.device))
+    with _guard(g.device):
+        typed("silu_mul", None, _P, _P, _P, _L, _I, _L)(g.data_ptr(), u.data_ptr(), out.data_ptr(), g.numel(), _TORCH2B200[out_dtype], _raw_stream(g.device))
     check("silu_mul")
     return out
 

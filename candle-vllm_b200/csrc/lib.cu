@@ -93,12 +93,17 @@ int b200_device_sm_count(void) {
 }
 
 int b200_device_cc(void) {
+    static std::atomic<int> cached[b200::kMaxDevices];    // a device's capability does not change: 0 = not asked yet
     int dev = 0, ma = 0, mi = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&ma, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess ||
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return 0; }
+    const bool keep = dev >= 0 && dev < b200::kMaxDevices;
+    if (keep) { const int cc = cached[dev].load(std::memory_order_relaxed); if (cc) return cc; }
+    if (cudaDeviceGetAttribute(&ma, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&mi, cudaDevAttrComputeCapabilityMinor, dev) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
+    if (keep) cached[dev].store(ma * 10 + mi, std::memory_order_relaxed);
     return ma * 10 + mi;
 }
 

@@ -2,13 +2,12 @@
 (src/openai/models/layers/mla_attention.rs:479-552) over the C ABI (``concat_and_cache_mla``, ``mla_paged_attention``)."""
 from __future__ import annotations
 
-import ctypes as C
 from typing import Optional
 
 import torch
 
-from ._lib import BackendError, check, lib, require_device
-from .backend import _cuda, _dt, _ptr, _stream
+from ._lib import BackendError, check, require_device, typed
+from .backend import _F, _I, _L, _P, _Z, _at, _cuda, _dt, _guard, _raw_stream
 
 
 def concat_and_cache_mla(ckv: torch.Tensor, k_pe: torch.Tensor, ckv_cache: torch.Tensor, kpe_cache: torch.Tensor, slot_mapping: torch.Tensor) -> None:
@@ -18,9 +17,11 @@ def concat_and_cache_mla(ckv: torch.Tensor, k_pe: torch.Tensor, ckv_cache: torch
     require_device()
     if ckv.dtype != ckv_cache.dtype or k_pe.dtype != kpe_cache.dtype or ckv.dtype not in (torch.float16, torch.bfloat16):
         raise BackendError("concat_and_cache_mla: 16-bit tensors of the cache dtype expected")
-    with torch.cuda.device(ckv.device):
-        lib().concat_and_cache_mla(_ptr(ckv.contiguous()), _ptr(k_pe.contiguous()), _ptr(ckv_cache), _ptr(kpe_cache), _ptr(slot_mapping.contiguous()),
-                                   C.c_int32(ckv.shape[0]), C.c_int32(ckv.shape[-1]), C.c_int32(k_pe.shape[-1]), C.c_int32(_dt(ckv)), _stream(ckv.device))
+    c, r, slots = ckv.contiguous(), k_pe.contiguous(), slot_mapping.contiguous()
+    with _guard(ckv.device):
+        typed("concat_and_cache_mla", None, _P, _P, _P, _P, _P, _I, _I, _I, _I, _L)(
+            c.data_ptr(), r.data_ptr(), ckv_cache.data_ptr(), kpe_cache.data_ptr(), slots.data_ptr(), ckv.shape[0], ckv.shape[-1], k_pe.shape[-1], _dt(ckv),
+            _raw_stream(ckv.device))
     check("concat_and_cache_mla")
 
 
@@ -33,15 +34,16 @@ def _mla(q_absorbed, q_pe, ckv_cache, kpe_cache, block_tables, context_lens, cu_
         raise BackendError("mla attention: q and the latent cache must share a 16-bit dtype")
     out = torch.empty((rows, H, R), dtype=q_absorbed.dtype, device=q_absorbed.device)
     B, W = block_tables.shape
-    L = lib()
-    need = int(L.mla_paged_decode_workspace_bytes(C.c_int32(B), C.c_int32(H), C.c_int32(W), C.c_int32(bs)))
-    ws = torch.empty(need, dtype=torch.uint8, device=q_absorbed.device)
-    with torch.cuda.device(q_absorbed.device):
-        L.mla_paged_attention(_ptr(out), _ptr(q_absorbed.contiguous()), _ptr(q_pe.contiguous()), _ptr(ckv_cache), _ptr(kpe_cache),
-                              _ptr(block_tables.to(torch.int32).contiguous()), _ptr(context_lens.to(torch.int32).contiguous()),
-                              _ptr(None if cu_seqlens_q is None else cu_seqlens_q.to(torch.int32).contiguous()), C.c_int32(B), C.c_int32(rows), C.c_int32(H),
-                              C.c_int32(R), C.c_int32(P), C.c_int32(bs), C.c_int32(W), C.c_int64(nb), C.c_float(sm_scale), C.c_int32(_dt(q_absorbed)),
-                              _ptr(ws), C.c_size_t(need), _stream(q_absorbed.device))
+    dev = q_absorbed.device
+    need = typed("mla_paged_decode_workspace_bytes", _Z, _I, _I, _I, _I)(B, H, W, bs)
+    ws = torch.empty(need, dtype=torch.uint8, device=dev)
+    qa, qp = q_absorbed.contiguous(), q_pe.contiguous()
+    tables, lens = block_tables.to(torch.int32).contiguous(), context_lens.to(torch.int32).contiguous()
+    cu = None if cu_seqlens_q is None else cu_seqlens_q.to(torch.int32).contiguous()
+    with _guard(dev):
+        typed("mla_paged_attention", None, _P, _P, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _L, _F, _I, _P, _Z, _L)(
+            out.data_ptr(), qa.data_ptr(), qp.data_ptr(), ckv_cache.data_ptr(), kpe_cache.data_ptr(), tables.data_ptr(), lens.data_ptr(), _at(cu), B, rows, H, R, P,
+            bs, W, nb, sm_scale, _dt(q_absorbed), ws.data_ptr(), need, _raw_stream(dev))
     check("mla_paged_attention")
     return out
 

@@ -8,8 +8,8 @@ from typing import Optional, Tuple
 
 import torch
 
-from ._lib import BackendError, check, lib, require_device
-from .backend import DType, GgmlType, _cuda, _ptr, _stream
+from ._lib import BackendError, check, lib, require_device, typed
+from .backend import DType, GgmlType, _F, _I, _L, _P, _Z, _cuda, _guard, _ptr, _raw_stream, _stream
 
 
 def topk_softmax(router_logits: torch.Tensor, topk: int) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -114,23 +114,22 @@ class FusedMoe:
                or w.numel() != self.E * self.I * self.H // 256 * GgmlType.BLOCK[ty][1] for w, ty in zip((self.ge, self.ue, self.de), t)):
             return False
         require_device()
-        if not lib().moe_block_supported(C.c_int32(T), C.c_int32(self.H), C.c_int32(self.I), C.c_int32(self.E), C.c_int32(self.k), C.c_int32(t[0]), C.c_int32(t[1]),
-                                         C.c_int32(t[2])):
+        if not typed("moe_block_supported", _I, _I, _I, _I, _I, _I, _I, _I, _I)(T, self.H, self.I, self.E, self.k, t[0], t[1], t[2]):
             return False
         x_at = xs.data_ptr() if xs.is_contiguous() else 0           # (a copy is made of the others)
         return (x_at | self.gate.data_ptr() | self.ge.data_ptr() | self.ue.data_ptr() | self.de.data_ptr()) % 16 == 0
 
     def _block(self, xs: torch.Tensor, T: int) -> torch.Tensor:
         out = torch.empty((T, self.H), dtype=torch.float32, device=xs.device)
-        L = lib()
-        dims = [C.c_int32(v) for v in (T, self.H, self.I, self.E, self.k)]
-        need = L.moe_block_workspace_bytes(*dims)
+        dims = (T, self.H, self.I, self.E, self.k)
+        need = typed("moe_block_workspace_bytes", _Z, _I, _I, _I, _I, _I)(*dims)
         ws = torch.empty(need + 256, dtype=torch.uint8, device=xs.device)
-        off = -ws.data_ptr() % 256
-        with torch.cuda.device(xs.device):
-            L.moe_block_gguf(_ptr(xs), _ptr(self.gate), _ptr(self.ge), _ptr(self.ue), _ptr(self.de), _ptr(out), *dims, *[C.c_int32(v) for v in self.types],
-                             C.c_int32(1 if self.norm_topk_prob else 0), C.c_float(1.0 if self.routed_scaling_factor is None else self.routed_scaling_factor),
-                             C.c_void_p(ws.data_ptr() + off), C.c_size_t(need), _stream(xs.device))
+        at = ws.data_ptr()
+        with _guard(xs.device):
+            typed("moe_block_gguf", None, _P, _P, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _F, _P, _Z, _L)(
+                xs.data_ptr(), self.gate.data_ptr(), self.ge.data_ptr(), self.ue.data_ptr(), self.de.data_ptr(), out.data_ptr(), *dims, *self.types,
+                1 if self.norm_topk_prob else 0, 1.0 if self.routed_scaling_factor is None else self.routed_scaling_factor, at + -at % 256, need,
+                _raw_stream(xs.device))
         check("FusedMoe.forward")
         return out
 
