@@ -281,9 +281,27 @@ rope_and_cache_vec_kernel(const SlabInfo si, float* __restrict__ qkv, T16* __res
 }
 
 template <typename TOut, bool kK4 = false, bool kZeroSrc = false>
-__global__ void silu_mul_kernel(float* __restrict__ g, float* __restrict__ u, TOut* __restrict__ out, int64_t n) {
+__global__ void silu_mul_kernel(float* __restrict__ g, float* __restrict__ u, TOut* __restrict__ out, int64_t n, int vec) {
     pdl_wait();
     pdl_trigger();
+    if (vec) {                          // n a multiple of 4, 16-byte aligned: four entries per thread
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n / 4; i += (int64_t)gridDim.x * blockDim.x) {
+            const float4 a = reinterpret_cast<const float4*>(g)[i], b = reinterpret_cast<const float4*>(u)[i];
+            const float r0 = a.x / (1.f + __expf(-a.x)) * b.x, r1 = a.y / (1.f + __expf(-a.y)) * b.y;
+            const float r2 = a.z / (1.f + __expf(-a.z)) * b.z, r3 = a.w / (1.f + __expf(-a.w)) * b.w;
+            if constexpr (sizeof(TOut) == 4) {
+                reinterpret_cast<float4*>(out)[i] = make_float4(r0, r1, r2, r3);
+            } else {
+                const TOut o[4] = {from_f32<TOut>(r0), from_f32<TOut>(kK4 ? r2 : r1), from_f32<TOut>(kK4 ? r1 : r2), from_f32<TOut>(r3)};
+                reinterpret_cast<uint2*>(out)[i] = *reinterpret_cast<const uint2*>(o);
+            }
+            if (kZeroSrc) {
+                reinterpret_cast<float4*>(g)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                reinterpret_cast<float4*>(u)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+        return;
+    }
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const float a = g[i];
         out[kK4 ? k4_index(i) : i] = from_f32<TOut>(a / (1.f + __expf(-a)) * u[i]);
@@ -303,6 +321,22 @@ __global__ void cast_kernel(const TS* __restrict__ s, TD* __restrict__ d, int64_
     pdl_trigger();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         d[kK4 ? k4_index(i) : i] = from_f32<TD>(to_f32(s[i]));
+}
+
+// x -> fp16 in K4 order (8 entries per thread: n a multiple of 8, 16-byte aligned) and, in the same launch, zeros over the accumulator of the product that reads it
+__global__ void __launch_bounds__(256)
+cast_k4_zero_kernel(const float* __restrict__ x, __half* __restrict__ out, int64_t n8, float* __restrict__ zero, int64_t nz) {
+    pdl_wait();
+    pdl_trigger();
+    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = i0; i < n8; i += step) {
+        const float4 a = reinterpret_cast<const float4*>(x)[2 * i], b = reinterpret_cast<const float4*>(x)[2 * i + 1];
+        const __half h[8] = {from_f32<__half>(a.x), from_f32<__half>(a.z), from_f32<__half>(a.y), from_f32<__half>(a.w),
+                             from_f32<__half>(b.x), from_f32<__half>(b.z), from_f32<__half>(b.y), from_f32<__half>(b.w)};
+        reinterpret_cast<uint4*>(out)[i] = *reinterpret_cast<const uint4*>(h);
+    }
+    for (int64_t i = i0; i < nz / 4; i += step) reinterpret_cast<float4*>(zero)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i0 < nz % 4) zero[nz / 4 * 4 + i0] = 0.f;
 }
 
 __global__ void embedding_f32_kernel(const float* __restrict__ table, const int64_t* __restrict__ ids,
@@ -518,21 +552,37 @@ void rope_and_cache_slabs(float* qkv, const SlabInfo& si, void* q_out, void* key
                        interleaved, dtype, cache_dtype, false, stream);
 }
 
-// act = silu(gate) * up in the activation format the next linear reads (fp16 K4, or natural f16 / bf16); gate / up re-zeroed
-void silu_mul_zero_src_fmt(float* gate, float* up, void* out, int64_t numel, int fmt, int64_t stream) {
-    if (fmt == B200_F16_K4) launch_pdl(silu_mul_kernel<__half, true, true>, dim3(ew_grid(numel)), dim3(256), 0, as_stream(stream), gate, up, (__half*)out, numel);
-    else if (fmt == B200_F16) launch_pdl(silu_mul_kernel<__half, false, true>, dim3(ew_grid(numel)), dim3(256), 0, as_stream(stream), gate, up, (__half*)out, numel);
-    else if (fmt == B200_BF16) launch_pdl(silu_mul_kernel<__nv_bfloat16, false, true>, dim3(ew_grid(numel)), dim3(256), 0, as_stream(stream), gate, up, (__nv_bfloat16*)out, numel);
-    else { set_error(kErrUnsupported, "silu_mul: activation format %d", fmt); return; }
+// silu(gate) * up, four entries per thread where the sizes allow it
+template <typename TOut, bool kK4, bool kZeroSrc>
+static void silu_mul_launch(float* gate, float* up, void* out, int64_t numel, int64_t stream) {
+    const int vec = numel % 4 == 0 && (((uintptr_t)gate | (uintptr_t)up | (uintptr_t)out) & 15) == 0;
+    launch_pdl(silu_mul_kernel<TOut, kK4, kZeroSrc>, dim3(ew_grid(vec ? numel / 4 : numel)), dim3(256), 0, as_stream(stream), gate, up, (TOut*)out, numel, vec);
     count_launch();
     check_launch("silu_mul");
 }
 
-void silu_mul_zero_src(float* gate, float* up, void* out_f16_k4, int64_t numel, int64_t stream) {
-    launch_pdl(silu_mul_kernel<__half, true, true>, dim3(ew_grid(numel)), dim3(256), 0, as_stream(stream), gate, up, (__half*)out_f16_k4, numel);
-    count_launch();
-    check_launch("silu_mul");
+// x f32 -> fp16 K4, and nz floats of `zero` set to 0 (none: nz = 0), in one launch
+void cast_k4_zero(const float* x, void* out_f16_k4, int64_t n, float* zero, int64_t nz, cudaStream_t st) {
+    if (n % 8 == 0 && (((uintptr_t)x | (uintptr_t)out_f16_k4 | (uintptr_t)zero) & 15) == 0) {
+        const int64_t work = n / 8 > nz / 4 ? n / 8 : nz / 4;
+        launch_pdl(cast_k4_zero_kernel, dim3(ew_grid(work)), dim3(256), 0, st, x, (__half*)out_f16_k4, n / 8, zero, nz);
+        count_launch();
+        check_launch("cast");
+        return;
+    }
+    cast(x, out_f16_k4, n, B200_F32, B200_F16_K4, reinterpret_cast<int64_t>(st));
+    if (nz) cudaMemsetAsync(zero, 0, (size_t)nz * sizeof(float), st);
 }
+
+// act = silu(gate) * up in the activation format the next linear reads (fp16 K4, or natural f16 / bf16); gate / up re-zeroed
+void silu_mul_zero_src_fmt(float* gate, float* up, void* out, int64_t numel, int fmt, int64_t stream) {
+    if (fmt == B200_F16_K4) silu_mul_launch<__half, true, true>(gate, up, out, numel, stream);
+    else if (fmt == B200_F16) silu_mul_launch<__half, false, true>(gate, up, out, numel, stream);
+    else if (fmt == B200_BF16) silu_mul_launch<__nv_bfloat16, false, true>(gate, up, out, numel, stream);
+    else set_error(kErrUnsupported, "silu_mul: activation format %d", fmt);
+}
+
+void silu_mul_zero_src(float* gate, float* up, void* out_f16_k4, int64_t numel, int64_t stream) { silu_mul_launch<__half, true, true>(gate, up, out_f16_k4, numel, stream); }
 }  // namespace b200
 
 extern "C" {
@@ -551,12 +601,10 @@ void silu_mul(const float* gate, const float* up, void* out, int64_t numel, int3
     if (numel == 0) return;
     B200_REQUIRE(gate && up && out && numel > 0, kErrBadArg, "silu_mul: bad arguments");
     float* g = const_cast<float*>(gate); float* u = const_cast<float*>(up);
-    if (out_dtype == B200_F32) silu_mul_kernel<float><<<ew_grid(numel), 256, 0, as_stream(stream)>>>(g, u, (float*)out, numel);
-    else if (out_dtype == B200_F16) silu_mul_kernel<__half><<<ew_grid(numel), 256, 0, as_stream(stream)>>>(g, u, (__half*)out, numel);
-    else if (out_dtype == B200_F16_K4) silu_mul_kernel<__half, true><<<ew_grid(numel), 256, 0, as_stream(stream)>>>(g, u, (__half*)out, numel);
-    else { set_error(kErrUnsupported, "silu_mul: out dtype %d", out_dtype); return; }
-    count_launch();
-    check_launch("silu_mul");
+    if (out_dtype == B200_F32) silu_mul_launch<float, false, false>(g, u, out, numel, stream);
+    else if (out_dtype == B200_F16) silu_mul_launch<__half, false, false>(g, u, out, numel, stream);
+    else if (out_dtype == B200_F16_K4) silu_mul_launch<__half, true, false>(g, u, out, numel, stream);
+    else set_error(kErrUnsupported, "silu_mul: out dtype %d", out_dtype);
 }
 
 void add_f32(float* x, const float* y, int64_t numel, int64_t stream) {

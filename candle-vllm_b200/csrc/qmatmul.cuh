@@ -20,6 +20,8 @@ void rope_and_cache_impl(float* qkv, void* q_out, void* key_cache, void* value_c
                          const int64_t* positions, const int64_t* slot_mapping, int32_t num_tokens, int32_t num_heads,
                          int32_t num_kv_heads, int32_t head_dim, int32_t interleaved, int32_t dtype, int32_t cache_dtype,
                          bool zero_src, int64_t stream);
+// x f32 -> fp16 K4 and `zero` [nz] = 0 in one launch
+void cast_k4_zero(const float* x, void* out_f16_k4, int64_t n, float* zero, int64_t nz, cudaStream_t st);
 void silu_mul_zero_src(float* gate, float* up, void* out_f16_k4, int64_t numel, int64_t stream);
 void silu_mul_zero_src_fmt(float* gate, float* up, void* out, int64_t numel, int fmt, int64_t stream);
 void qmatmul_tc(const void* x_f16, const void* w, float* y, int64_t ldy, int m, int n, int k, int ggml_type,

@@ -38,26 +38,31 @@ namespace {
 
 using namespace tc;
 
-template <int kMB, int kType>   // activation rows of a tile, padded to kMB (32, 64 or 128) = UMMA N; GGML type of W
+// activation rows of a tile: at most kMB (32, 64, 128 or 256), the UMMA N is what a tile has rounded up to 32; GGML type of W
+template <int kMB, int kType>
 struct Cfg {
     // bytes of one super-block as staged in shared memory: Q4_K 144; Q6_K a 240-byte window that starts at the
     // 210-byte block's address rounded down to 16 (TMA box starts must be 16-byte aligned)
     // Independent accumulators: back-to-back tcgen05.mma into ONE accumulator serialise on the accumulate
     // dependency; k-step ks goes to D[ks % kAcc] and the epilogue adds them up.  Two suffice (the dequant side sets the
     // pace) and keep the epilogue's TMEM reads (64 B/clk) short: kAcc * kMB <= 128 TMEM columns.
-    static constexpr int kAcc = kMB == 128 ? 1 : 2;                // (at N = 128 one product fills the pipe longer than the dependency)
+    // (From N = 128 on one product fills the pipe longer than the dependency.)
+    static constexpr int kAcc = kMB >= 128 ? 1 : 2;
+    static constexpr int kACol = kMB == 256 ? 256 : 128;           // TMEM: accumulators below, then the A buffers of 128 columns
+    static constexpr int kABuf = (512 - kACol) / 128;              // 3, or 2 beside an accumulator of 256
     static constexpr int kBlk = kType == B200_GGML_Q4_K ? 144 : (is_4bit_rows(kType) ? 128 : (kType == kTypeF8 ? 256 : 240));
     static constexpr int kWBytes = kTileN * kBlk;                  // raw weights of one unit (18 KB / 30 KB)
-    static constexpr int kXBytes = 4 * kMB * kXSubBytes;           // 4 sub-tiles of [kMB][64] fp16 (16 KB / 32 KB)
+    static constexpr int kXSlices = kMB == 256 ? 1 : 4;            // 64-wide slices of the activations per stage: a whole unit, or a quarter of it at 256 rows
+    static constexpr int kXBytes = kXSlices * kMB * kXSubBytes;    // slices of [kMB][64] fp16 (16 / 32 / 64 / 32 KB)
     // Two rings.  Raw weight bytes are dead as soon as the dequant warps have pulled them into registers, so the
     // W ring is deep and recycles fast (more HBM reads in flight); the activation slices live until their MMAs
     // retire and come from L2, so the X ring is shallow.
-    static constexpr int kXStages = kMB == 32 ? 4 : 2;
+    static constexpr int kXStages = kMB == 32 || kMB == 256 ? 4 : (kMB == 64 ? 3 : 2);
     static constexpr int kWStages = (227 * 1024 - 1024 - kXStages * kXBytes) / kWBytes > 8 ? 8 : (227 * 1024 - 1024 - kXStages * kXBytes) / kWBytes;
     static constexpr int kXOff = 0;                                // 1024-aligned (128-byte swizzle)
     static constexpr int kWOff = kXStages * kXBytes;
     static constexpr int kBars = kWOff + kWStages * kWBytes;       // w_full[kW] w_empty[kW] x_full[kX] x_empty[kX] a_ready[3] a_free[3] d_full d_empty
-    static constexpr int kNumBars = 2 * kWStages + 2 * kXStages + 2 * kABufs + 2;
+    static constexpr int kNumBars = 2 * kWStages + 2 * kXStages + 2 * kABuf + 2;
     static constexpr int kTmemSlot = kBars + kNumBars * 8;
     static constexpr int kTotal = kTmemSlot + 16;
     static_assert(kWStages >= 3, "W ring too shallow");
@@ -89,7 +94,10 @@ struct GemmParams {
     int scale_bf16, scale_by, scale_sk;
     const float* norm;             // fp8: {2^p, 2^-p} range shift of the tile scales (device)
     const uint32_t* zp;            // AWQ: packed zero points [K/g, N/8] in the marlin layout (null: symmetric, zero point 8)
-    int m_tiles;                   // dense mode: tiles of kMB activation rows; tile id = weight tile * m_tiles + row tile (the row tiles of a weight
+    int mrows;                     // dense mode: activation rows per row tile (a multiple of 32 up to kMB)
+    int csplit;                    // > 1: a cluster of csplit CTAs shares every tile, each over its part of k; the partial sums meet in shared memory of the
+                                   // cluster and every CTA adds up and stores its share of the columns (plain stores in a fixed order: nothing to zero)
+    int m_tiles;                   // dense mode: row tiles; tile id = weight tile * m_tiles + row tile (the row tiles of a weight
                                    // tile run side by side, so its bytes come from memory once)
     // grouped (mixture-of-experts) mode: the chunk list lives in device memory -- built from the routing of this step (moe.cu): chunk = (expert, <= kMB routed
     // rows); tile id = chunk * n_tiles + weight tile, the weight tiles of every segment of one expert in a row.  Weights at row expert * n + n0 of a segment's
@@ -109,6 +117,15 @@ __device__ __forceinline__ int seg_of_tile(const GemmParams& p, int tile) { retu
 // first tile of segment sg (constant indices only: dynamic indexing would spill the parameter struct to local memory)
 __device__ __forceinline__ int seg_first_tile(const GemmParams& p, int sg) { return sg == 0 ? 0 : (sg == 1 ? p.tile_end[0] : p.tile_end[1]); }
 __device__ __forceinline__ int seg_rows(const GemmParams& p, int sg) { return sg == 0 ? p.n[0] : (sg == 1 ? p.n[1] : p.n[2]); }
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+    return v;
+}
+
 // what a tile id means
 struct Tile {
     int sg, n0;          // segment, first weight row within the segment's matrix
@@ -129,7 +146,7 @@ __device__ __forceinline__ Tile tile_of(const GemmParams& p, int tile) {
         const int w = p.m_tiles == 1 ? tile : tile / p.m_tiles, mt = tile - w * p.m_tiles;
         t.sg = seg_of_tile(p, w);
         t.n0 = t.wrow = (w - seg_first_tile(p, t.sg)) * kTileN;
-        t.xrow = mt * kMB; t.count = min(kMB, p.m - t.xrow);
+        t.xrow = mt * p.mrows; t.count = min(p.mrows, p.m - t.xrow);
     }
     return t;
 }
@@ -452,7 +469,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_constant__ CUtensorMap wmap1,
                   const __grid_constant__ CUtensorMap wmap2, const __grid_constant__ CUtensorMap xmap, const GemmParams p) {
     using C = Cfg<kMB, kType>;
-    constexpr int kW = C::kWStages, kX = C::kXStages;
+    constexpr int kW = C::kWStages, kX = C::kXStages, kABufs = C::kABuf, kColA = C::kACol;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t smem_base = smem_u32(smem);
@@ -494,8 +511,15 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
     if (moe) pdl_wait();               // the chunk list is produced by an earlier kernel (routing of this step)
     const uint32_t n_tiles_rt = moe ? (uint32_t)*reinterpret_cast<const volatile int*>(p.num_chunks) * (uint32_t)p.n_tiles : (uint32_t)p.n_tiles * (uint32_t)p.m_tiles;
     const uint32_t total = n_tiles_rt * (uint32_t)p.nsb, nsb = (uint32_t)p.nsb;
-    const uint32_t u0 = p.whole_tiles ? (n_tiles_rt * blockIdx.x / gridDim.x) * nsb : total * blockIdx.x / gridDim.x;
-    const uint32_t u1 = p.whole_tiles ? (n_tiles_rt * (blockIdx.x + 1) / gridDim.x) * nsb : total * (blockIdx.x + 1) / gridDim.x;
+    uint32_t u0, u1;
+    if (p.csplit > 1) {                // one tile per cluster, one part of its units per CTA
+        const uint32_t t = blockIdx.x / (uint32_t)p.csplit, r = blockIdx.x - t * (uint32_t)p.csplit;
+        u0 = t * nsb + nsb * r / (uint32_t)p.csplit;
+        u1 = t * nsb + nsb * (r + 1) / (uint32_t)p.csplit;
+    } else {
+        u0 = p.whole_tiles ? (n_tiles_rt * blockIdx.x / gridDim.x) * nsb : total * blockIdx.x / gridDim.x;
+        u1 = p.whole_tiles ? (n_tiles_rt * (blockIdx.x + 1) / gridDim.x) * nsb : total * (blockIdx.x + 1) / gridDim.x;
+    }
     const uint32_t tile0 = u0 / nsb, sb0 = u0 - tile0 * nsb;          // first unit of this CTA
 
     if (warp == kDequantWarps) {
@@ -548,55 +572,68 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_x));
         int it = 0;
         int sb = (int)sb0, xtile = (int)tile0;
-        int xrow = u0 < u1 ? tile_of<kMB>(p, xtile).xrow : 0;
+        Tile ti = u0 < u1 ? tile_of<kMB>(p, xtile) : Tile{};
         for (uint32_t u = u0; u < u1; ++u, ++it) {
-            const int s = it % kX;
-            mbar_wait(x_empty(s), ((it / kX) & 1) ^ 1);
-            if (leader) {
-                mbar_expect_tx(x_full(s), C::kXBytes);
-                const uint32_t dst = smem_base + C::kXOff + s * C::kXBytes;
+            const int nb = (ti.count + 31) >> 5;                 // only the 32-row groups that hold rows of this tile
 #pragma unroll
-                for (int q = 0; q < 4; ++q) tma_load_2d(dst + q * kMB * kXSubBytes, &xmap, x_full(s), sb * kSB + q * 64, xrow, pol_x);
+            for (int q0 = 0; q0 < 4; q0 += C::kXSlices) {
+                const int xi = it * (4 / C::kXSlices) + q0 / C::kXSlices, s = xi % kX;
+                mbar_wait(x_empty(s), ((xi / kX) & 1) ^ 1);
+                if (leader) {
+                    mbar_expect_tx(x_full(s), (uint32_t)(nb * C::kXSlices) * (32 * kXSubBytes));
+                    const uint32_t dst = smem_base + C::kXOff + s * C::kXBytes;
+#pragma unroll
+                    for (int q = 0; q < C::kXSlices; ++q)
+#pragma unroll
+                        for (int b = 0; b < kMB / 32; ++b)
+                            if (b < nb) tma_load_2d(dst + q * kMB * kXSubBytes + b * (32 * kXSubBytes), &xmap, x_full(s), sb * kSB + (q0 + q) * 64, ti.xrow + b * 32, pol_x);
+                }
+                __syncwarp();
             }
-            __syncwarp();
-            if (++sb == (int)nsb) { sb = 0; ++xtile; if (u + 1 < u1) xrow = tile_of<kMB>(p, xtile).xrow; }
+            if (++sb == (int)nsb) { sb = 0; ++xtile; if (u + 1 < u1) ti = tile_of<kMB>(p, xtile); }
         }
     } else if (warp == kDequantWarps + 2) {
         // ======================================= MMA ISSUER ======================================
         // The whole warp runs the (warp-uniform) loop so descriptors / TMEM addresses live in uniform registers;
         // one elected lane issues.  (With a single-lane loop every tcgen05.mma cost ~110 cycles of R2UR traffic.)
         const bool leader = elect_one();
-        // instruction descriptor: D = f32, A = B = f16, both K-major, N = kMB, M = 128
-        const uint32_t idesc = (1u << 4) | ((uint32_t)(kMB >> 3) << 17) | ((uint32_t)(kTileN >> 4) << 24);
         int it = 0, seg = 0;
         uint32_t tile = tile0;
         for (uint32_t u = u0; u < u1; ++tile) {
             const uint32_t tile_end = (tile + 1) * nsb;
             const uint32_t seg_end = tile_end < u1 ? tile_end : u1;
+            // instruction descriptor: D = f32, A = B = f16, both K-major, M = 128, N = the tile's rows rounded up to 32
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(((tile_of<kMB>(p, (int)tile).count + 31) >> 5) * 4) << 17) | ((uint32_t)(kTileN >> 4) << 24);
             mbar_wait(d_empty, (seg & 1) ^ 1);                 // epilogue of the previous segment has drained D
             tc_fence_after();
             bool first = true;
             for (; u < seg_end; ++u, ++it) {
-                const int xs = it % kX, ab = it % kABufs;
-                mbar_wait(x_full(xs), (it / kX) & 1);             // activations landed (TMA)
-                if (p.trace && blockIdx.x == 0 && leader && it < 32) p.trace[it * 8 + 1] = clock64();
-                mbar_wait(a_ready(ab), (it / kABufs) & 1);        // dequantised A tile is in TMEM
-                if (p.trace && blockIdx.x == 0 && leader && it < 32) p.trace[it * 8 + 2] = clock64();
-                tc_fence_after();
+                const int ab = it % kABufs;
                 const uint32_t a_t = tmem + kColA + ab * 128;
-                const uint64_t bd0 = make_b_desc(smem_base + C::kXOff + xs * C::kXBytes);
-                if (leader) {
-                    if (!(p.debug & 1)) {
 #pragma unroll
-                        for (int ks = 0; ks < 16; ++ks) {
-                            // k-step ks: 64-wide sub-tile (ks / 4), 32 bytes per k-step inside its 128-byte swizzled rows
-                            const uint64_t bd = bd0 + (uint64_t)((((ks >> 2) * kMB * kXSubBytes) + (ks & 3) * 32) >> 4);
-                            tc_mma_ts(tmem + kColD + (ks % C::kAcc) * kMB, a_t + ks * 8, bd, idesc, (first && ks < C::kAcc) ? 0u : 1u);
+                for (int q0 = 0; q0 < 4; q0 += C::kXSlices) {
+                    const int xi = it * (4 / C::kXSlices) + q0 / C::kXSlices, xs = xi % kX;
+                    mbar_wait(x_full(xs), (xi / kX) & 1);             // activations landed (TMA)
+                    if (p.trace && blockIdx.x == 0 && leader && it < 32) p.trace[it * 8 + 1] = clock64();
+                    if (q0 == 0) mbar_wait(a_ready(ab), (it / kABufs) & 1);        // dequantised A tile is in TMEM
+                    if (p.trace && blockIdx.x == 0 && leader && it < 32) p.trace[it * 8 + 2] = clock64();
+                    tc_fence_after();
+                    const uint64_t bd0 = make_b_desc(smem_base + C::kXOff + xs * C::kXBytes);
+                    if (leader) {
+                        if (!(p.debug & 1)) {
+#pragma unroll
+                            for (int kq = 0; kq < 4 * C::kXSlices; ++kq) {
+                                // k-step ks of the unit: 64-wide slice (ks / 4), 32 bytes per k-step inside its 128-byte swizzled rows
+                                const int ks = q0 * 4 + kq;
+                                const uint64_t bd = bd0 + (uint64_t)((((kq >> 2) * kMB * kXSubBytes) + (kq & 3) * 32) >> 4);
+                                tc_mma_ts(tmem + kColD + (ks % C::kAcc) * kMB, a_t + ks * 8, bd, idesc, (first && ks < C::kAcc) ? 0u : 1u);
+                            }
                         }
+                        tc_commit(x_empty(xs));           // activation slice reusable once these MMAs retire
+                        if (q0 + C::kXSlices == 4) tc_commit(a_free(ab));            // and so is the A buffer
+                        if (p.trace && blockIdx.x == 0 && it < 32) p.trace[it * 8 + 3] = clock64();
                     }
-                    tc_commit(x_empty(xs));           // activation slice reusable once these MMAs retire
-                    tc_commit(a_free(ab));            // and so is the A buffer
-                    if (p.trace && blockIdx.x == 0 && it < 32) p.trace[it * 8 + 3] = clock64();
+                    if (q0 + C::kXSlices < 4) __syncwarp();
                 }
                 __syncwarp();
                 first = false;
@@ -696,8 +733,8 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                 float* const ymoe = ti.sg == 0 ? p.y[0] : (ti.sg == 1 ? p.y[1] : p.y[2]);
                 constexpr int kColsPerWarpM = kMB / 4;
                 const float post = (kType == kTypeF8 && p.norm) ? __ldg(p.norm + 1) : 1.f;      // FP8: undo the range shift of the tile scales
-#pragma unroll
-                for (int c0 = 0; c0 < kColsPerWarpM; c0 += 8) {
+#pragma unroll 1
+                for (int c0 = 0; c0 < kColsPerWarpM; c0 += 8) {           // (rolled: see below)
                     if (qt * kColsPerWarpM + c0 >= ti.count) break;
                     uint32_t acc[8], more[8];
                     tc_ld8(tmem + kColD + lane_addr + qt * kColsPerWarpM + c0, acc);
@@ -723,6 +760,21 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                 ++seg;
                 continue;
             }
+            if (kMB == 256 && p.csplit > 1) {
+                // partial sums -> this CTA's shared memory, [column][128 rows] (the rings are drained: every load of this CTA has been consumed)
+                float* part = reinterpret_cast<float*>(smem);
+                constexpr int kCols = kMB / 4;
+#pragma unroll 1
+                for (int c0 = 0; c0 < kCols; c0 += 16) {
+                    if (qt * kCols + c0 >= ti.count) break;
+                    uint32_t acc[16];
+                    tc_ld16(tmem + kColD + lane_addr + qt * kCols + c0, acc);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) part[(qt * kCols + c0 + i) * kTileN + row] = __uint_as_float(acc[i]);
+                }
+                continue;                                             // the only tile of this CTA
+            }
             const int sg = ti.sg;
             const int n_idx = ti.n0 + row;
             float* ybase = sg == 0 ? p.y[0] : (sg == 1 ? p.y[1] : p.y[2]);
@@ -734,7 +786,9 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
             const int zero_slabs = (p.slabs > 0 && seg_end == tile_end) ? p.slabs - 1 - ordinal : 0;   // slabs nobody else writes
             const int n_rows = sg == 0 ? p.n[0] : (sg == 1 ? p.n[1] : p.n[2]);
             constexpr int kColsPerWarp = kMB / 4;                 // this warp's share of the batch columns (8, 16 or 32)
-#pragma unroll
+            // A tile's epilogue runs once or twice per CTA, out of a cold instruction cache: unrolled over the columns it took 1450 clocks per 8 columns, most of them
+            // instruction misses.  Rolled, only the first round misses.
+#pragma unroll 1
             for (int c0 = 0; c0 < kColsPerWarp; c0 += 8) {
                 if (qt * kColsPerWarp + c0 >= ti.count) break;
                 uint32_t acc[8];
@@ -769,6 +823,42 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
             if (lane == 0) mbar_arrive(d_empty);
             ++seg;
         }
+    }
+
+    if (kMB == 256 && p.csplit > 1) {
+        __syncwarp();
+        cluster_sync();                                               // every CTA's partial sums are written
+        if (warp < kDequantWarps) {
+            const int rank = (int)(blockIdx.x % (uint32_t)p.csplit), row = (int)threadIdx.x & 127;
+            const Tile ti = tile_of<kMB>(p, (int)tile0);
+            const int n_idx = ti.n0 + row, c1 = ti.count * (rank + 1) / p.csplit;
+            float* const y = (ti.sg == 0 ? p.y[0] : (ti.sg == 1 ? p.y[1] : p.y[2])) + (int64_t)ti.xrow * p.ldy + n_idx;
+            // eight columns at a time: their loads from one CTA are in flight together
+            constexpr int kStep = kDequantWarps / 4, kBatch = 8;
+            for (int c = ti.count * rank / p.csplit + ((int)threadIdx.x >> 7); c < c1; c += kStep * kBatch) {
+                float v[kBatch];
+#pragma unroll
+                for (int i = 0; i < kBatch; ++i) v[i] = 0.f;
+                for (int q = 0; q < p.csplit; ++q) {
+                    uint32_t at;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_base + (uint32_t)(c * kTileN + row) * 4), "r"((uint32_t)q));
+                    float f[kBatch];
+#pragma unroll
+                    for (int i = 0; i < kBatch; ++i) f[i] = ld_cluster_f32(at + (uint32_t)(min(c + i * kStep, c1 - 1) - c) * (kTileN * 4));
+#pragma unroll
+                    for (int i = 0; i < kBatch; ++i) v[i] += f[i];
+                }
+                if (n_idx < seg_rows(p, ti.sg)) {
+#pragma unroll
+                    for (int i = 0; i < kBatch; ++i) {
+                        if (c + i * kStep >= c1) break;
+                        float* o = y + (int64_t)(c + i * kStep) * p.ldy;
+                        *o = p.accumulate ? *o + v[i] : v[i];
+                    }
+                }
+            }
+        }
+        cluster_sync();                                               // nobody leaves while its shared memory is read
     }
 
     // ---- teardown ---------------------------------------------------------------------------------
@@ -811,16 +901,32 @@ void launch(const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, c
     auto kern = qmatmul_tc_kernel<kMB, kType>;
     ensure_dynamic_smem(reinterpret_cast<const void*>(kern), Cfg<kMB, kType>::kTotal);
     const int grid = p.chunks ? sm_count() : gemm_grid((int64_t)p.n_tiles * p.m_tiles, p.nsb, p.whole_tiles != 0, p.slabs > 0);
-    launch_pdl(kern, dim3(grid), dim3(kThreads), Cfg<kMB, kType>::kTotal, st, wm[0], wm[1], wm[2], xm, p);
+    if (p.csplit > 1) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)(p.n_tiles * p.m_tiles * p.csplit)); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = Cfg<kMB, kType>::kTotal; cfg.stream = st;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = (unsigned)p.csplit; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr; cfg.numAttrs = 2;
+        cudaLaunchKernelEx(&cfg, kern, wm[0], wm[1], wm[2], xm, p);
+    } else {
+        launch_pdl(kern, dim3(grid), dim3(kThreads), Cfg<kMB, kType>::kTotal, st, wm[0], wm[1], wm[2], xm, p);
+    }
     count_launch();
 }
 
+template <int kType>
+void launch_rows_of(int mb, const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, cudaStream_t st) {
+    if (mb == 32) launch<32, kType>(wm, xm, p, st);
+    else if (mb == 64) launch<64, kType>(wm, xm, p, st);
+    else if (mb == 128) launch<128, kType>(wm, xm, p, st);
+    else launch<256, kType>(wm, xm, p, st);
+}
 void launch_rows(int mb, int ggml_type, const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, cudaStream_t st) {
-    if (ggml_type == B200_GGML_Q4_K) {
-        if (mb == 32) launch<32, B200_GGML_Q4_K>(wm, xm, p, st); else if (mb == 64) launch<64, B200_GGML_Q4_K>(wm, xm, p, st); else launch<128, B200_GGML_Q4_K>(wm, xm, p, st);
-    } else {
-        if (mb == 32) launch<32, B200_GGML_Q6_K>(wm, xm, p, st); else if (mb == 64) launch<64, B200_GGML_Q6_K>(wm, xm, p, st); else launch<128, B200_GGML_Q6_K>(wm, xm, p, st);
-    }
+    if (ggml_type == B200_GGML_Q4_K) launch_rows_of<B200_GGML_Q4_K>(mb, wm, xm, p, st);
+    else launch_rows_of<B200_GGML_Q6_K>(mb, wm, xm, p, st);
 }
 
 bool make_w_map(CUtensorMap* wm, const void* w, int n, int nsb, int ggml_type) {
@@ -910,15 +1016,24 @@ bool qmatmul_tc_supported(int m, int n, int k, int ggml_type) {
 // Decomposition: with many tiles per SM every CTA gets whole tiles (no split); otherwise stream-K over (tile, super-block).
 static bool use_whole_tiles(int64_t n_tiles) { return n_tiles >= 4 * (int64_t)sm_count(); }
 
-// activation rows per tile, and tiles: up to 64 rows are one tile of 32 or 64; more rows come in tiles of 128 (the weights are converted once per row tile;
-// 64-row tiles would convert twice as often)
-static int rows_per_tile(int m) { return m <= 32 ? 32 : (m <= 64 ? 64 : 128); }
-static int row_tiles(int m) { return m <= 64 ? 1 : (m + 127) / 128; }
+// Up to 64 rows are one row tile and stream-K over its units, split tiles meeting in y through red.add.  More rows come in tiles of up to 256, equal and in multiples of
+// 32, and whole weight tiles: red.add of a 128 x 128 tile costs 5800 clocks (11 bytes a clock and SM), as much as four units.  With fewer tiles than SMs a cluster
+// shares each tile over k and adds up through its shared memory.
+static int rows_per_tile(int m) { return m <= 32 ? 32 : (m <= 64 ? 64 : 256); }
+static int row_tiles(int m) { return m <= 64 ? 1 : (m + 255) / 256; }
+static int tile_rows(int m) { return m <= 64 ? rows_per_tile(m) : (((m + row_tiles(m) - 1) / row_tiles(m)) + 31) / 32 * 32; }
+static int cluster_split(int64_t tiles, int nsb) {
+    int64_t s = sm_count() / tiles;
+    if (s > 8) s = 8;
+    if (s > nsb / 2) s = nsb / 2;
+    return s < 1 ? 1 : (int)s;
+}
 
 // true when some output tile is produced by more than one CTA (or accumulate): y must then hold the
 // addend (zeros for a plain product) before the launch
 bool qmatmul_tc_needs_zeroed_output(int m, int n, int k) {
-    const int64_t n_tiles = (int64_t)((n + kTileN - 1) / kTileN) * row_tiles(m), nsb = k / 256, total = n_tiles * nsb;
+    if (m > 64) return false;
+    const int64_t n_tiles = (n + kTileN - 1) / kTileN, nsb = k / 256, total = n_tiles * nsb;
     if (use_whole_tiles(n_tiles)) return false;
     const int64_t grid = total < sm_count() ? total : sm_count();
     for (int64_t c = 1; c < grid; ++c)
@@ -979,7 +1094,7 @@ int qmatmul_tc_multi(const void* x_f16, int nseg, const void* const* w, float* c
     {
         const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
         const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-        const cuuint32_t box[2] = {64, (cuuint32_t)mb};
+        const cuuint32_t box[2] = {64, 32};
         const cuuint32_t es[2] = {1, 1};
         CUresult r = enc(&xm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x_f16), dims, strides, box, es,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -987,11 +1102,13 @@ int qmatmul_tc_multi(const void* x_f16, int nseg, const void* const* w, float* c
         if (r != CUDA_SUCCESS) { set_error(kErrCuda, "qmatmul: activation tensor map failed (%d)", (int)r); return 0; }
     }
     if ((int64_t)tiles * mt * nsb * sm_count() >= (int64_t)1 << 31) { set_error(kErrUnsupported, "qmatmul: %d tiles x %d super-blocks exceed the 32-bit unit range", tiles, nsb); return 0; }
-    p.ldy = ldy; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = mt; p.accumulate = accumulate;
-    p.whole_tiles = use_whole_tiles((int64_t)tiles * mt) ? 1 : 0;
+    p.ldy = ldy; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = mt; p.mrows = tile_rows(m); p.accumulate = accumulate;
+    p.whole_tiles = m > 64 || use_whole_tiles(tiles) ? 1 : 0;
+    p.csplit = m > 64 ? cluster_split((int64_t)tiles * mt, nsb) : 1;
     take_prefetch(p);
     if (slabs_avail > 0) {
-        p.slabs = qmatmul_tc_slab_count((int64_t)tiles * mt, nsb);
+        if (m > 64) { set_error(kErrUnsupported, "qmatmul: slabs at %d rows", m); return 0; }
+        p.slabs = qmatmul_tc_slab_count(tiles, nsb);
         p.slab_stride = slab_stride;
         p.accumulate = 0;
         if (p.slabs > slabs_avail) { set_error(kErrBadArg, "qmatmul: %d slabs needed, %d provided", p.slabs, slabs_avail); return 0; }
@@ -1021,7 +1138,7 @@ static void wq16_launch(int kind, const void* x_f16, const void* w, const void* 
     {
         const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
         const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-        const cuuint32_t box[2] = {64, (cuuint32_t)mb};
+        const cuuint32_t box[2] = {64, 32};
         const cuuint32_t es[2] = {1, 1};
         CUresult r = enc(&xm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x_f16), dims, strides, box, es,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1031,7 +1148,7 @@ static void wq16_launch(int kind, const void* x_f16, const void* w, const void* 
     GemmParams p{};
     const int tiles = (n + kTileN - 1) / kTileN;
     for (int i = 0; i < kMaxSeg; ++i) { p.y[i] = slabs; p.n[i] = n; p.tile_end[i] = i == 0 ? tiles : 0x7fffffff; }
-    p.ldy = n; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = 1; p.accumulate = 0;
+    p.ldy = n; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = 1; p.mrows = mb; p.accumulate = 0;
     p.whole_tiles = use_whole_tiles(tiles) ? 1 : 0;
     p.slabs = qmatmul_tc_slab_count(tiles, nsb);
     p.slab_stride = (int64_t)m * n;
@@ -1089,14 +1206,14 @@ void marlin_tc_f32_multi(const void* x_f16_k4, int nseg, const void* const* w, c
     {
         const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
         const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-        const cuuint32_t box[2] = {64, (cuuint32_t)mb};
+        const cuuint32_t box[2] = {64, 32};
         const cuuint32_t es[2] = {1, 1};
         CUresult r = enc(&xm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x_f16_k4), dims, strides, box, es,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) { set_error(kErrCuda, "marlin_4bit(f32): activation tensor map failed (%d)", (int)r); return; }
     }
-    p.ldy = ldy; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = 1; p.accumulate = accumulate;
+    p.ldy = ldy; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = 1; p.mrows = mb; p.accumulate = accumulate;
     p.whole_tiles = use_whole_tiles(tiles) ? 1 : 0;
     p.scales = p.scales_seg[0]; p.zp = p.zp_seg[0]; p.group_size = group_size; p.k = k; p.scale_bf16 = scale_bf16; p.scale_by = 1;
     take_prefetch(p);
@@ -1145,10 +1262,10 @@ bool qmatmul_tc_moe_supported(int n, int k, int ggml_type) {
     return false;
 }
 
-static bool moe_x_map(CUtensorMap* xm, const void* xs, int rows, int k, int box_rows, const char* who) {
+static bool moe_x_map(CUtensorMap* xm, const void* xs, int rows, int k, const char* who) {
     const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-    const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
+    const cuuint32_t box[2] = {64, 32};
     const cuuint32_t es[2] = {1, 1};
     const CUresult r = encode_fn()(xm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(xs), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1169,11 +1286,11 @@ void qmatmul_tc_moe_fp8(const void* xs_f16, int xs_rows, const void* w, const fl
     count_launch();
     CUtensorMap wm[kMaxSeg], xm;
     for (int i = 0; i < kMaxSeg; ++i) if (!make_w_map(&wm[i], w, num_experts * n, nsb, kTypeF8)) return;
-    if (!moe_x_map(&xm, xs_f16, xs_rows, k, 32, "moe_gemm_fp8")) return;
+    if (!moe_x_map(&xm, xs_f16, xs_rows, k, "moe_gemm_fp8")) return;
     if ((int64_t)max_chunks * tiles * nsb * sm_count() >= (int64_t)1 << 31) { set_error(kErrUnsupported, "moe_gemm_fp8: %d items x %d super-blocks exceed the 32-bit unit range", max_chunks * tiles, nsb); return; }
     GemmParams p{};
     for (int i = 0; i < kMaxSeg; ++i) { p.y[i] = y; p.n[i] = n; p.tile_end[i] = 0x7fffffff; p.scales_seg[i] = scale; p.zp_seg[i] = nullptr; }
-    p.ldy = ldy; p.m = 32; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = 1; p.accumulate = 0; p.whole_tiles = 1;
+    p.ldy = ldy; p.m = 32; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = 1; p.mrows = 32; p.accumulate = 0; p.whole_tiles = 1;
     p.chunks = chunks; p.num_chunks = num_chunks; p.row_map = row_map; p.row_scale = row_scale;
     p.scales = scale; p.group_size = bx; p.k = k; p.scale_by = by; p.scale_sk = sk; p.norm = norm;
     launch<32, kTypeF8>(wm, xm, p, st);
@@ -1193,9 +1310,9 @@ void qmatmul_tc_moe(const void* xs_f16_k4, int xs_rows, int nseg, const void* co
         if (!make_w_map(&wm[i], w[j], num_experts * n, nsb, ggml_type)) return;      // experts stacked along the rows
         p.y[i] = y[j]; p.n[i] = n; p.tile_end[i] = i < nseg ? (i + 1) * tiles : 0x7fffffff;
     }
-    if (!moe_x_map(&xm, xs_f16_k4, xs_rows, k, chunk_rows, "moe_gemm")) return;
+    if (!moe_x_map(&xm, xs_f16_k4, xs_rows, k, "moe_gemm")) return;
     if ((int64_t)max_chunks * nseg * tiles * nsb * sm_count() >= (int64_t)1 << 31) { set_error(kErrUnsupported, "moe_gemm: %d items x %d super-blocks exceed the 32-bit unit range", max_chunks * nseg * tiles, nsb); return; }
-    p.ldy = ldy; p.m = chunk_rows; p.nsb = nsb; p.n_tiles = nseg * tiles; p.m_tiles = 1; p.accumulate = 0; p.whole_tiles = 1;
+    p.ldy = ldy; p.m = chunk_rows; p.nsb = nsb; p.n_tiles = nseg * tiles; p.m_tiles = 1; p.mrows = chunk_rows; p.accumulate = 0; p.whole_tiles = 1;
     p.chunks = chunks; p.num_chunks = num_chunks; p.row_map = row_map; p.row_scale = row_scale;
     launch_rows(chunk_rows, ggml_type, wm, xm, p, st);
     check_launch("moe_gemm");
