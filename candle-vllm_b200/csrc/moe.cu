@@ -47,7 +47,13 @@ topk_softmax_kernel(const float* __restrict__ logits, int splits, int64_t split_
         if (e < E) {
             const float* src = logits + (int64_t)t * E + e;
             float a = src[0];
-            for (int s = 1; s < splits; ++s) a += src[s * split_stride];
+            for (int s = 1; s < splits; s += 5) {            // five parts in flight (16 at most: 1 + 3 x 5), added in order
+                float b[5];
+#pragma unroll
+                for (int j = 0; j < 5; ++j) b[j] = s + j < splits ? src[(s + j) * split_stride] : 0.f;
+#pragma unroll
+                for (int j = 0; j < 5; ++j) a += b[j];
+            }
             v[i] = a;
         }
         mx = fmaxf(mx, v[i]);

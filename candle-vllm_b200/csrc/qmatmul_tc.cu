@@ -87,6 +87,7 @@ struct GemmParams {
     int whole_tiles;               // 1: CTA ranges are whole tiles (no split-K, no atomics)
     int slabs;                     // > 0: split tiles write their partial sums to DISTINCT slabs (plain stores, no atomics, no
     int64_t slab_stride;           //      pre-zeroed output): slab s of segment sg starts at y[sg] + s * slab_stride; the consumer sums
+    int one_shift;                 // int4: log2 of a group size that is a power of two >= 64 (32: one group per column); 0: other groups
     const void* scales;            // marlin: [K/g, N] in marlin-permuted order (f16 / bf16: scale_bf16); fp8: f32 [N/by, K/bx]
     const void* scales_seg[kMaxSeg];   // marlin, several weight matrices in one launch (engine: QKV, gate|up): scales / zero points of each
     const uint32_t* zp_seg[kMaxSeg];   //   segment (slot 0 = scales / zp)
@@ -464,6 +465,51 @@ __device__ __forceinline__ void dequant_unit(const uint8_t* blk, int off, uint32
     if (lane == 0) mbar_arrive(a_ready_bar);
 }
 
+// the same for int4 with ONE scale and zero point for the quarter
+template <int kQ>
+__device__ __forceinline__ void m4_unit(const uint8_t* blk, int r7, uint32_t a_col, uint32_t w_empty_bar, uint32_t a_free_bar, uint32_t a_free_parity,
+                                        uint32_t a_ready_bar, int lane, float sc, float z) {
+    uint32_t raw[M4Quarter<kQ>::kRaw];
+    M4Quarter<kQ>::load(blk, r7, raw);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) mbar_arrive(w_empty_bar);
+    const bool fast = __all_sync(0xffffffffu, fabsf(sc) * 262144.f <= 65504.f);
+    const __half2 s = __float2half2_rn(fast ? sc * 262144.f : sc), n = __float2half2_rn(-z * sc);
+    uint32_t v[32];
+    if (fast) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t x = raw[i];
+            uint32_t t0 = (x << 6) & 0x03c003c0u, t1 = (x >> 2) & 0x03c003c0u, t2 = (x << 2) & 0x03c003c0u, t3 = (x >> 6) & 0x03c003c0u;
+            const __half2 r0 = __hfma2(*reinterpret_cast<__half2*>(&t0), s, n), r1 = __hfma2(*reinterpret_cast<__half2*>(&t1), s, n);
+            const __half2 r2 = __hfma2(*reinterpret_cast<__half2*>(&t2), s, n), r3 = __hfma2(*reinterpret_cast<__half2*>(&t3), s, n);
+            v[2 * i] = *reinterpret_cast<const uint32_t*>(&r0); v[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&r1);
+            v[16 + 2 * i] = *reinterpret_cast<const uint32_t*>(&r2); v[16 + 2 * i + 1] = *reinterpret_cast<const uint32_t*>(&r3);
+        }
+    } else {
+        const uint32_t magic = 0x64006400u;
+        const __half2 k1024 = *reinterpret_cast<const __half2*>(&magic);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t x = raw[i];
+            uint32_t t[4] = {(x & 0x000f000fu) | magic, ((x >> 8) & 0x000f000fu) | magic, ((x >> 4) & 0x000f000fu) | magic, ((x >> 12) & 0x000f000fu) | magic};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const __half2 r = __hfma2(__hsub2(*reinterpret_cast<__half2*>(&t[j]), k1024), s, n);
+                v[(j >> 1) * 16 + 2 * i + (j & 1)] = *reinterpret_cast<const uint32_t*>(&r);
+            }
+        }
+    }
+    mbar_wait(a_free_bar, a_free_parity);
+    tc_fence_after();
+    tc_st32(a_col + kQ * 32, v);
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(a_ready_bar);
+}
+
 template <int kMB, int kType>
 __global__ void __launch_bounds__(kThreads, 1)
 qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_constant__ CUtensorMap wmap1,
@@ -536,6 +582,21 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
             mbar_wait(w_empty(s), ((it / kW) & 1) ^ 1);
             if (p.trace && blockIdx.x == 0 && leader && it < 32) p.trace[it * 8 + 0] = clock64();
             const CUtensorMap* wm = ti.sg == 0 ? &wmap0 : (ti.sg == 1 ? &wmap1 : &wmap2);
+            if constexpr (kType == kTypeM4) {
+                // the unit's scales (and zero points) into L2 while its weights are a ring ahead: the dequant warps load them one unit ahead, which covers an L2 hit, not HBM
+                // [without: gate|up of 4096 x 14336 at 32 rows 34.5 us; registers cannot hold them further ahead, moving a value on waits for it]
+                if (p.one_shift > 0) {
+                    const int gi = lane >> 3, c = (lane & 7) * 16, nn = seg_rows(p, ti.sg);
+                    const int groups = p.one_shift < 8 ? kSB >> p.one_shift : 1;
+                    if (gi < groups && ti.n0 + c < nn) {
+                        const size_t g = (size_t)((p.one_shift < 32 ? (uint32_t)(sb * kSB) >> p.one_shift : 0u) + (uint32_t)gi);
+                        const void* sc = ti.sg == 0 ? p.scales_seg[0] : (ti.sg == 1 ? p.scales_seg[1] : p.scales_seg[2]);
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(static_cast<const unsigned short*>(sc) + g * nn + ti.n0 + c));
+                        const uint32_t* z = ti.sg == 0 ? p.zp_seg[0] : (ti.sg == 1 ? p.zp_seg[1] : p.zp_seg[2]);
+                        if (z && (lane & 3) == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(z + g * (nn >> 3) + ((ti.n0 + c) >> 3)));
+                    }
+                }
+            }
             const int wrow = ti.wrow;
             if (leader) {
                 // W box start (bytes): Q4_K blocks are 144 B (16-aligned); Q6_K blocks (210 B) start at the block address
@@ -683,12 +744,72 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
             }
         };
         constexpr bool kPrefetchScales = kType == kTypeM4 || is_fp4(kType);
-        if constexpr (kPrefetchScales) { if (u0 < u1) m4_fetch(tile, (int)(u0 - (uint32_t)tile * nsb)); }
+        const bool kOne = kType == kTypeM4 && p.one_shift > 0;
+        if constexpr (kPrefetchScales) { if (u0 < u1 && !kOne) m4_fetch(tile, (int)(u0 - (uint32_t)tile * nsb)); }
+        // kOne (the usual groups: 64, 128, ... or one per column): one scale per quarter.  Everything about a thread's row is computed once per tile; a unit costs a shift, one
+        // multiply-add for the address and the load.  [The general form rebuilds the context per unit: 525 instructions a unit and warp against 150, gate|up of 4096 x
+        // 14336 at 32 rows 45 us.]
+        const unsigned short* sc_row = nullptr;
+        const uint32_t* zp_row = nullptr;
+        uint32_t sc_ld = 0;
+        int ft = (int)tile0, fsb = (int)sb0;               // unit whose scale is fetched next
+        auto one_tile = [&]() {
+            const int sgx = seg_of_tile(p, ft), nn = seg_rows(p, sgx), rw = (ft - seg_first_tile(p, sgx)) * kTileN + row, nx = rw < nn ? rw : 0;
+            sc_row = static_cast<const unsigned short*>(sgx == 0 ? p.scales_seg[0] : (sgx == 1 ? p.scales_seg[1] : p.scales_seg[2])) + marlin_scale_pos(nx, p.group_size > 0);
+            const uint32_t* z = sgx == 0 ? p.zp_seg[0] : (sgx == 1 ? p.zp_seg[1] : p.zp_seg[2]);
+            zp_row = z ? z + (((uint32_t)nx >> 6) << 3) + ((uint32_t)nx & 7u) : nullptr;
+            sc_ld = (uint32_t)nn;
+        };
+        auto one_fetch = [&](uint32_t& bits, uint32_t& word, uint32_t u) {
+            if (u >= u1) return;
+            const uint32_t g = p.one_shift < 32 ? (uint32_t)(fsb * kSB + qt * 64) >> p.one_shift : 0u;
+            bits = sc_row[g * sc_ld];
+            if (zp_row) word = zp_row[g * (sc_ld >> 3)];
+            if (++fsb == (int)nsb) { fsb = 0; ++ft; if (u + 1 < u1) one_tile(); }
+        };
+        uint32_t one_bits = 0u, one_word = 0u;             // of the next unit
+        const bool zp_any = p.zp_seg[0] != nullptr;                // (all segments of a launch have zero points, or none)
+        const int one_nib = 4 * ((0x73625140u >> (4 * ((row & 63) >> 3))) & 7);          // AWQ: this row's nibble in its zero-point word
+        if constexpr (kType == kTypeM4) {
+            if (kOne && u0 < u1) {
+                one_tile();
+                one_fetch(one_bits, one_word, u0);
+            }
+        }
         for (uint32_t u = u0; u < u1; ++tile) {
             const uint32_t tile_begin = (uint32_t)tile * nsb, tile_end = tile_begin + nsb;
             const uint32_t seg_begin = u, seg_end = tile_end < u1 ? tile_end : u1;
             const Tile ti = tile_of<kMB>(p, tile);
+            // grouped: lane l holds output row and multiplier of this warp's column l, fetched before the tile's units so that the epilogue does not wait for them
+            uint32_t my_row = 0;
+            float my_scale = 1.f;
+            if (moe && qt * (kMB / 4) + lane < ti.count && lane < kMB / 4) {
+                my_row = p.row_map ? __ldg(p.row_map + ti.xrow + qt * (kMB / 4) + lane) : (uint32_t)(ti.xrow + qt * (kMB / 4) + lane);
+                if (p.row_scale) my_scale = __ldg(p.row_scale + my_row);
+            }
             for (; u < seg_end; ++u, ++it) {
+                if constexpr (kType == kTypeM4) {
+                    if (kOne) {
+                        const uint32_t bits = one_bits, word = one_word;
+                        one_fetch(one_bits, one_word, u + 1);
+                        mbar_wait(w_full(ws), wph);
+                        if (p.trace && blockIdx.x == 0 && threadIdx.x == 0 && it < 32) p.trace[it * 8 + 4] = clock64();
+                        const uint8_t* blk = smem + C::kWOff + ws * C::kWBytes + row * C::kBlk;
+                        const uint32_t a_col = tmem + kColA + ab * 128 + lane_addr;
+                        const float sc = p.scale_bf16 ? __uint_as_float(bits << 16) : __half2float(__ushort_as_half((unsigned short)bits));
+                        const float z = zp_any ? (float)((word >> one_nib) & 0xFu) : 8.f;
+                        switch (qt) {
+                            case 0: m4_unit<0>(blk, row & 7, a_col, w_empty(ws), a_free(ab), aph ^ 1, a_ready(ab), lane, sc, z); break;
+                            case 1: m4_unit<1>(blk, row & 7, a_col, w_empty(ws), a_free(ab), aph ^ 1, a_ready(ab), lane, sc, z); break;
+                            case 2: m4_unit<2>(blk, row & 7, a_col, w_empty(ws), a_free(ab), aph ^ 1, a_ready(ab), lane, sc, z); break;
+                            default: m4_unit<3>(blk, row & 7, a_col, w_empty(ws), a_free(ab), aph ^ 1, a_ready(ab), lane, sc, z); break;
+                        }
+                        if (p.trace && blockIdx.x == 0 && threadIdx.x == 0 && it < 32) p.trace[it * 8 + 6] = clock64();
+                        if (++ws == kW) { ws = 0; wph ^= 1; }
+                        if (++ab == kABufs) { ab = 0; aph ^= 1; }
+                        continue;
+                    }
+                }
                 float m4_cur[4] = {m4_next[0], m4_next[1], m4_next[2], m4_next[3]};
                 if constexpr (kPrefetchScales) {
                     if (u + 1 < u1) { if (u + 1 < tile_end) m4_fetch(tile, (int)(u + 1 - tile_begin)); else m4_fetch(tile + 1, 0); }
@@ -740,17 +861,14 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                     tc_ld8(tmem + kColD + lane_addr + qt * kColsPerWarpM + c0, acc);
                     if constexpr (C::kAcc == 2) tc_ld8(tmem + kColD + kMB + lane_addr + qt * kColsPerWarpM + c0, more);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (n_loc < n_rows) {
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const int mi = qt * kColsPerWarpM + c0 + i;
-                            if (mi < ti.count) {
-                                const uint32_t orow = p.row_map ? __ldg(p.row_map + ti.xrow + mi) : (uint32_t)(ti.xrow + mi);
-                                const float sc = p.row_scale ? __ldg(p.row_scale + orow) : 1.f;
-                                float v = __uint_as_float(acc[i]);
-                                if constexpr (C::kAcc == 2) v += __uint_as_float(more[i]);
-                                ymoe[(int64_t)orow * p.ldy + n_loc] = v * (sc * post);
-                            }
+                    for (int i = 0; i < 8; ++i) {
+                        const uint32_t orow = __shfl_sync(0xffffffffu, my_row, c0 + i);
+                        const float sc = __shfl_sync(0xffffffffu, my_scale, c0 + i);
+                        if (n_loc < n_rows && qt * kColsPerWarpM + c0 + i < ti.count) {
+                            float v = __uint_as_float(acc[i]);
+                            if constexpr (C::kAcc == 2) v += __uint_as_float(more[i]);
+                            ymoe[(int64_t)orow * p.ldy + n_loc] = v * (sc * post);
                         }
                     }
                 }
@@ -1125,6 +1243,13 @@ int qmatmul_tc_multi(const void* x_f16, int nseg, const void* const* w, float* c
 // slabs (and the bias) and rounds once to f16 / bf16.  scratch = [S][m][n] f32, S = wq16_slabs(n, k).
 int wq16_slabs(int n, int k) { return qmatmul_tc_slab_count((n + kTileN - 1) / kTileN, k / 256); }
 
+// int4 groups in which a quarter of a unit (64 weights) has one scale: their log2, 32 for one group per column; 0 for all others
+static int one_shift_of(int group_size) {
+    if (group_size <= 0) return 32;
+    if (group_size < 64 || (group_size & (group_size - 1))) return 0;
+    return 31 - __builtin_clz((unsigned)group_size);
+}
+
 static void wq16_launch(int kind, const void* x_f16, const void* w, const void* scales, int scale_bf16, int group_or_bx, int by, int sk,
                         const float* norm, const uint32_t* zp, const void* bias, void* out, int out_dtype, int m, int n, int k, float* slabs, cudaStream_t st,
                         const char* who, int64_t ldy_f32 = 0, int accumulate_f32 = 0) {
@@ -1152,6 +1277,7 @@ static void wq16_launch(int kind, const void* x_f16, const void* w, const void* 
     p.whole_tiles = use_whole_tiles(tiles) ? 1 : 0;
     p.slabs = qmatmul_tc_slab_count(tiles, nsb);
     p.slab_stride = (int64_t)m * n;
+    p.one_shift = kind == kTypeM4 ? one_shift_of(group_or_bx) : 0;
     p.scales = scales; p.group_size = group_or_bx; p.k = k; p.scale_bf16 = scale_bf16; p.scale_by = by; p.scale_sk = sk; p.norm = norm; p.zp = zp;
     for (int i = 0; i < kMaxSeg; ++i) { p.scales_seg[i] = scales; p.zp_seg[i] = zp; }
     { static const char* dbg = getenv("B200_GEMM_DEBUG"); p.debug = dbg ? atoi(dbg) : 0; }
@@ -1215,9 +1341,11 @@ void marlin_tc_f32_multi(const void* x_f16_k4, int nseg, const void* const* w, c
     }
     p.ldy = ldy; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = 1; p.mrows = mb; p.accumulate = accumulate;
     p.whole_tiles = use_whole_tiles(tiles) ? 1 : 0;
+    p.one_shift = one_shift_of(group_size);
     p.scales = p.scales_seg[0]; p.zp = p.zp_seg[0]; p.group_size = group_size; p.k = k; p.scale_bf16 = scale_bf16; p.scale_by = 1;
     take_prefetch(p);
     { static const char* dbg = getenv("B200_GEMM_DEBUG"); p.debug = dbg ? atoi(dbg) : 0; }
+    { static const char* tr = getenv("B200_GEMM_TRACE"); p.trace = tr ? reinterpret_cast<long long*>(strtoull(tr, nullptr, 0)) : nullptr; }
     if (mb == 32) launch<32, kTypeM4>(wm, xm, p, st); else launch<64, kTypeM4>(wm, xm, p, st);
     check_launch("marlin_4bit(f32)");
 }
