@@ -51,22 +51,6 @@ struct UmmaPrefillParams {
     const float* sink;               // [H] or null
 };
 
-// Bounded wait: a wait that does not end (it always does unless a copy or an MMA was lost) gives up, raises the CTA's flag and lets every role leave.
-__device__ __forceinline__ bool wait_or_flag(uint32_t bar, uint32_t parity, volatile uint32_t* flag) {
-    for (uint32_t i = 0; i < (1u << 22); ++i) {
-        uint32_t ok;
-        asm volatile(
-            "{\n"
-            ".reg .pred p;\n"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n"
-            "}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
-        if ((i & 255u) == 255u && *flag) return false;
-    }
-    *flag = 1u;
-    return false;
-}
 __device__ __forceinline__ void tma_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst), "l"(map), "r"(bar),
                  "r"(c0), "r"(c1), "r"(c2)
@@ -217,7 +201,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
 #pragma unroll
             for (int kv = 0; kv < 2; ++kv, ++it) {
                 const int s = it % kRing;
-                ok = ok && wait_or_flag(kv_empty(s), ((it / kRing) & 1) ^ 1, flag);
+                ok = ok && mbar_wait_or_flag(kv_empty(s), ((it / kRing) & 1) ^ 1, flag);
                 if (!ok) break;
                 if (leader) {
                     const CUtensorMap* map = kv ? &vmap : &kmap;
@@ -248,7 +232,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
         const uint32_t idesc_s = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(kKt >> 3) << 17) | (8u << 24);        // M 128, N 128, both K-major
         const uint32_t idesc_o = idesc_s | (1u << 16);                                                                       // B (values) MN-major
-        bool ok = wait_or_flag(q_full, 0, flag);
+        bool ok = mbar_wait_or_flag(q_full, 0, flag);
         auto scores = [&](int i, int stage) {
             if (leader) {
                 const uint64_t a = make_b_desc(sb + kSmQ + i * kTileBytes), b = make_b_desc(sb + kSmKv + stage * kTileBytes);
@@ -261,7 +245,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
             }
             __syncwarp();
         };
-        ok = ok && wait_or_flag(kv_full(0), 0, flag);
+        ok = ok && mbar_wait_or_flag(kv_full(0), 0, flag);
         if (ok) {
             tc_fence_after();
 #pragma unroll
@@ -274,12 +258,12 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         for (int j = 0; j < n && ok; ++j) {
             const int vs = it % kRing, vp = (it / kRing) & 1, ks = (it + 1) % kRing, kp = ((it + 1) / kRing) & 1;
             it += 2;
-            ok = wait_or_flag(kv_full(vs), vp, flag);
-            if (ok && j + 1 < n) ok = wait_or_flag(kv_full(ks), kp, flag);
+            ok = mbar_wait_or_flag(kv_full(vs), vp, flag);
+            if (ok && j + 1 < n) ok = mbar_wait_or_flag(kv_full(ks), kp, flag);
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 if (!ok || j >= nk[i]) continue;
-                ok = wait_or_flag(p_ready(i), j & 1, flag);
+                ok = mbar_wait_or_flag(p_ready(i), j & 1, flag);
                 if (!ok) continue;
                 tc_fence_after();
                 if (leader) {
@@ -319,7 +303,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         bool ok = true;
         const int nki = nk[i];
         for (int j = 0; j < nki; ++j) {
-            ok = wait_or_flag(s_full(i), j & 1, flag);
+            ok = mbar_wait_or_flag(s_full(i), j & 1, flag);
             if (!ok) break;
             tc_fence_after();
             uint32_t s[128];
@@ -378,7 +362,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
             if (k0 + kKt > klen) {
                 // rows of V past the context hold whatever the block contains (0 * NaN would poison O): zero them before this tile's product
                 const int vi = 2 * j + 1, vs = vi % kRing;
-                ok = wait_or_flag(kv_full(vs), (vi / kRing) & 1, flag);
+                ok = mbar_wait_or_flag(kv_full(vs), (vi / kRing) & 1, flag);
                 if (!ok) break;
                 uint8_t* v = smem + kSmKv + vs * kTileBytes;
                 const int r0 = klen - k0;                                           // >= 1: the tile holds the row's own key or an earlier one
@@ -393,7 +377,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
             __syncwarp();
             if (lane == 0) mbar_arrive(p_ready(i));
         }
-        if (nki > 0 && ok && wait_or_flag(o_full(i), 0, flag)) {
+        if (nki > 0 && ok && mbar_wait_or_flag(o_full(i), 0, flag)) {
             tc_fence_after();
             const float l = l2.x + l2.y, inv = l > 0.f ? 1.f / l : 0.f;
             T* dst = static_cast<T*>(p.out) + ((int64_t)(q_begin + tok) * p.num_heads + head) * kHd;

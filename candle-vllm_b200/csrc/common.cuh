@@ -20,6 +20,9 @@ int  sm_count();                        // SM count of the CURRENT device (cache
 // depends on its arguments asks again with more).  The attribute is per device, so a per-process `static bool` would leave every
 // device but the first without it (one thread per rank in one process: src/openai/pipelines/threaded.rs:33-134 of the reference).
 void ensure_dynamic_smem(const void* kernel, int bytes);
+// clusters of `size` CTAs of a kernel that fills an SM by itself (shared memory) which the current device runs at the same time: fewer than SMs / size, a cluster lies
+// within one GPC.  Asked once per (device, size), of the first such kernel.
+int max_active_clusters(const void* kernel, int threads, int smem, int size);
 
 #define B200_REQUIRE(cond, code, ...)                  \
     do {                                               \

@@ -72,6 +72,8 @@ struct DenseParams {
     int out_dtype, bf16;
     int ksplit;                    // swap mode, f32 output: the k range is cut into ksplit parts per tile (more CTAs than weight tiles); partial
     int accumulate;                // sums meet in y through fp32 atomics.  accumulate: y += result (f32 output)
+    int csplit;                    // > 1: a cluster of csplit CTAs shares one tile, each over its part of k; the sums meet in shared memory of the cluster and every CTA
+                                   // adds up and stores its share of the columns, in a fixed order
     // grouped form: the weight operand is a stack of `groups` matrices of group_rows rows each, and tile_group[i] (device, written by an
     // earlier kernel) names the one that activation tile i multiplies; a negative entry marks a tile without rows.  Not swapped: activation
     // tiles are the 128-row tiles ta.  Swapped (few rows per group): activation tiles are the BN-row tiles tb, the weight tile ta is counted
@@ -134,9 +136,11 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
     // tile order: bands of 8 A-tiles; inside a band the B-tile index is the slow one, so the CTAs running together (consecutive tile
     // ids) work on the same B tile (weights, or activations when swapped) and neighbouring A tiles -> both stay in L2
     // split-K (swap mode only): tile id = (weight tile, k part); part z owns k blocks [nkb_all * z / ksplit, nkb_all * (z + 1) / ksplit)
+    const int crank = p.csplit > 1 ? (int)blockIdx.x % p.csplit : 0;
+    const int t_first = p.csplit > 1 ? (int)blockIdx.x / p.csplit : (int)blockIdx.x, t_step = p.csplit > 1 ? n_tiles : (int)gridDim.x;
     auto k_range = [&](int t, int& kb0, int& kb1) {
-        const int z = p.ksplit > 1 ? t % p.ksplit : 0;
-        kb0 = nkb_all * z / p.ksplit; kb1 = nkb_all * (z + 1) / p.ksplit;
+        const int z = p.csplit > 1 ? crank : p.ksplit > 1 ? t % p.ksplit : 0, parts = p.csplit > 1 ? p.csplit : p.ksplit;
+        kb0 = nkb_all * z / parts; kb1 = nkb_all * (z + 1) / parts;
     };
     auto tile_coords = [&](int t, int& ta, int& tb) {
         if (p.ksplit > 1) { ta = t / p.ksplit; tb = 0; return; }
@@ -156,7 +160,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
         uint64_t pol;
         asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
         int it = 0;
-        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+        for (int t = t_first; t < n_tiles; t += t_step) {
             int ta, tb, kb0, kb1;
             tile_coords(t, ta, tb);
             k_range(t, kb0, kb1);
@@ -185,7 +189,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
         const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
         int it = 0, tcount = 0;                                          // tcount: tiles done (skipped tiles of the grouped form do not count)
         if (p.tile_group) pdl_wait();
-        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+        for (int t = t_first; t < n_tiles; t += t_step) {
             if (p.tile_group) {
                 int ta, tb;
                 tile_coords(t, ta, tb);
@@ -224,7 +228,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
         int tcount = 0;
         bool waited = false;
         if (p.tile_group) { pdl_wait(); waited = true; }
-        for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
+        for (int t = t_first; t < n_tiles; t += t_step) {
             int ta, tb;
             tile_coords(t, ta, tb);
             if (p.tile_group && p.tile_group[p.swap ? tb : ta] < 0) continue;
@@ -232,6 +236,20 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
             mbar_wait(tmem_full(ab), (tcount >> 1) & 1);
             tc_fence_after();
             if (!waited) { pdl_wait(); waited = true; }
+            if (p.csplit > 1) {
+                // partial sums -> [4 columns][128 rows][4] over the drained ring (every load of this CTA has been consumed)
+                float4* part = reinterpret_cast<float4*>(smem);
+#pragma unroll 1
+                for (int c0 = 0; c0 < kBN; c0 += 32) {
+                    uint32_t acc[32];
+                    tc_ld32(tmem + ab * kBN + lane_addr + c0, acc);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        part[(c0 / 4 + i) * kBM + r] = make_float4(__uint_as_float(acc[4 * i]), __uint_as_float(acc[4 * i + 1]), __uint_as_float(acc[4 * i + 2]), __uint_as_float(acc[4 * i + 3]));
+                }
+                continue;                                       // the only tile of this CTA
+            }
             const int ia = ta * kBM + r;                        // index along the 128-row operand
 #pragma unroll 1
             for (int c0 = 0; c0 < kBN; c0 += 32) {
@@ -283,11 +301,218 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
         }
     }
 
+    if (p.csplit > 1) {
+        __syncwarp();
+        cluster_sync();                                                   // every CTA's sums are written
+        if (warp >= 2) {
+            int ta, tb;
+            tile_coords(t_first, ta, tb);
+            const int r = (warp & 3) * 32 + lane, ia = ta * kBM + r;
+            const TOut* bias = static_cast<const TOut*>(p.bias);
+            // eight columns at a time, two CTAs' loads in flight together
+            for (int b = kBN / 8 * crank / p.csplit; b < kBN / 8 * (crank + 1) / p.csplit; ++b) {
+                float v[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[i] = 0.f;
+#pragma unroll 4
+                for (int q = 0; q < p.csplit; ++q) {
+                    const uint32_t at = cluster_map(smem_base + (uint32_t)(b * 2 * kBM + r) * 16, (uint32_t)q);
+                    const float4 f = ld_cluster_f32x4(at), g = ld_cluster_f32x4(at + kBM * 16);
+                    v[0] += f.x; v[1] += f.y; v[2] += f.z; v[3] += f.w; v[4] += g.x; v[5] += g.y; v[6] += g.z; v[7] += g.w;
+                }
+                const int jb = tb * kBN + b * 8;
+                if (!p.swap) {
+                    if (ia >= p.m) continue;
+                    TOut* dst = static_cast<TOut*>(p.y) + (int64_t)ia * p.ldy + jb;
+                    TOut o[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        if (bias && jb + i < p.n) v[i] += to_f32(bias[jb + i]);
+                        o[i] = from_f32<TOut>(v[i]);
+                    }
+                    if (sizeof(TOut) == 2 && jb + 8 <= p.n && (((uintptr_t)dst) & 15) == 0) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(o);
+                    else
+                        for (int i = 0; i < 8; ++i)
+                            if (jb + i < p.n) dst[i] = o[i];
+                } else if (ia < p.n) {
+                    const float bv = bias ? to_f32(bias[ia]) : 0.f;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (jb + i < p.m) static_cast<TOut*>(p.y)[(int64_t)(jb + i) * p.ldy + ia] = from_f32<TOut>(v[i] + bv);
+                }
+            }
+        }
+        __syncwarp();
+        cluster_sync();                                                   // nobody leaves while its shared memory is read
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::kTmemCols));
+    }
+}
+
+// ---- two SMs on one tile --------------------------------------------------------------------------------------------------------------------------
+// y tile of 256 x 256 by a cluster of two CTAs (cta_group::2): each holds 128 rows of x, 128 rows of w and, in its TMEM, the accumulator of its own 128 rows; the leader's
+// thread issues the MMAs of both, which read the other CTA's half of w in place.  Per product of 128 x 256 an SM reads 32 KB of operands where the one-CTA kernel reads
+// 48: less shared-memory traffic and L2 traffic, which under the power cap is also clock.  Roles as above, per CTA; barriers:
+//   full[s]        the leader's, expects the bytes of both CTAs (each CTA's loads signal it)
+//   empty[s], tmem_full[b]   in both CTAs, by a commit that arrives at the pair
+//   tmem_empty[b]  the leader's, 8 arrivals: the epilogue warps of both
+struct PairCfg {
+    static constexpr int kStageBytes = 2 * kBM * kBK * 2, kStages = 6;
+    static constexpr int kBars = kStages * kStageBytes;               // full, empty [kStages], tmem_full[2], tmem_empty[2]
+    static constexpr int kFlag = kBars + (2 * kStages + 4) * 8, kTmemSlot = kFlag + 4;
+    static constexpr int kTotal = kTmemSlot + 12;
+    static_assert(kTotal <= 232448, "shared memory");
+};
+constexpr int kBand2 = 8;                                               // bands of 8 row tiles (2048 rows)
+
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t leader_bar, int c0, int c1) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst), "l"(map), "r"(leader_bar),
+                 "r"(c0), "r"(c1)
+                 : "memory");
+}
+__device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((unsigned short)3) : "memory");
+}
+
+template <typename TOut>
+__global__ void __launch_bounds__(kGemmThreads, 1)
+dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap, const DenseParams p) {
+    using C = PairCfg;
+    constexpr int kS = C::kStages, kBN = 256;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)(blockIdx.x & 1);
+    const uint32_t smem_base = smem_u32(smem), bars = smem_base + C::kBars;
+    auto full = [&](int s) { return bars + s * 8; };
+    auto empty = [&](int s) { return bars + (kS + s) * 8; };
+    auto tmem_full = [&](int b) { return bars + (2 * kS + b) * 8; };
+    auto tmem_empty = [&](int b) { return bars + (2 * kS + 2 + b) * 8; };
+    volatile uint32_t* flag = reinterpret_cast<volatile uint32_t*>(smem + C::kFlag);
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + C::kTmemSlot);
+    if (threadIdx.x == 0) {
+        *flag = 0u;
+        for (int s = 0; s < kS; ++s) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(tmem_full(b), 1); mbar_init(tmem_empty(b), 8); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();                                                       // the other CTA's barriers and TMEM exist
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    pdl_trigger();
+
+    const int n_tiles = p.tiles_a * p.tiles_b, nkb = (p.k + kBK - 1) / kBK, step = (int)(gridDim.x >> 1);
+    auto tile_coords = [&](int t, int& ta, int& tb) {                     // as above: bands of row tiles, the column tile is the slow index
+        const int per_band = kBand2 * p.tiles_b, band = t / per_band, r = t - band * per_band, rows = min(kBand2, p.tiles_a - band * kBand2);
+        tb = r / rows;
+        ta = band * kBand2 + (r - tb * rows);
+    };
+    bool ok = true;
+    if (warp == 0) {
+        pdl_wait();
+        const bool leader = elect_one();
+        int it = 0;
+        for (int t = (int)(blockIdx.x >> 1); t < n_tiles && ok; t += step) {
+            int ta, tb;
+            tile_coords(t, ta, tb);
+            for (int kb = 0; kb < nkb && ok; ++kb, ++it) {
+                const int s = it % kS;
+                ok = mbar_wait_or_flag(empty(s), ((it / kS) & 1) ^ 1, flag);
+                if (ok && leader) {
+                    if (rank == 0) mbar_expect_tx(full(s), 2 * C::kStageBytes);
+                    const uint32_t dst = smem_base + s * C::kStageBytes, bar = cluster_map(full(s), 0);
+                    tma_load_2d_pair(dst, &amap, bar, kb * kBK, ta * 256 + rank * kBM);
+                    tma_load_2d_pair(dst + C::kStageBytes / 2, &bmap, bar, kb * kBK, tb * 256 + rank * kBM);
+                }
+                __syncwarp();
+            }
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            const bool leader = elect_one();
+            const uint32_t fmt = p.bf16 ? 1u : 0u;
+            const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+            int it = 0, tcount = 0;
+            for (int t = (int)(blockIdx.x >> 1); t < n_tiles && ok; t += step, ++tcount) {
+                const int ab = tcount & 1;
+                ok = mbar_wait_or_flag(tmem_empty(ab), ((tcount >> 1) & 1) ^ 1, flag);
+                tc_fence_after();
+                for (int kb = 0; kb < nkb && ok; ++kb, ++it) {
+                    const int s = it % kS;
+                    ok = mbar_wait_or_flag(full(s), (it / kS) & 1, flag);
+                    tc_fence_after();
+                    if (ok && leader) {
+                        const uint64_t ad = make_b_desc(smem_base + s * C::kStageBytes), bd = make_b_desc(smem_base + s * C::kStageBytes + C::kStageBytes / 2);
+#pragma unroll
+                        for (int ks = 0; ks < kBK / 16; ++ks)
+                            tc_mma_pair(tmem + ab * kBN, ad + (uint64_t)(ks * 2), bd + (uint64_t)(ks * 2), idesc, (kb > 0 || ks > 0) ? 1u : 0u);
+                        tc_commit_pair(empty(s));
+                    }
+                    __syncwarp();
+                }
+                if (ok && leader) tc_commit_pair(tmem_full(ab));
+                __syncwarp();
+            }
+        }
+    } else {
+        const int qd = warp & 3, r = qd * 32 + lane;
+        const uint32_t lane_addr = (uint32_t)(qd * 32) << 16;
+        const TOut* bias = static_cast<const TOut*>(p.bias);
+        int tcount = 0;
+        pdl_wait();
+        for (int t = (int)(blockIdx.x >> 1); t < n_tiles && ok; t += step, ++tcount) {
+            int ta, tb;
+            tile_coords(t, ta, tb);
+            const int ab = tcount & 1;
+            ok = mbar_wait_or_flag(tmem_full(ab), (tcount >> 1) & 1, flag);
+            if (!ok) break;
+            tc_fence_after();
+            const int ia = ta * 256 + rank * kBM + r;
+#pragma unroll 1
+            for (int c0 = 0; c0 < kBN; c0 += 32) {
+                uint32_t acc[32];
+                tc_ld32(tmem + ab * kBN + lane_addr + c0, acc);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                const int jb = tb * kBN + c0;
+                if (ia >= p.m) continue;
+                TOut* dst = static_cast<TOut*>(p.y) + (int64_t)ia * p.ldy + jb;
+                if (jb + 32 <= p.n && (((uintptr_t)dst) & 15) == 0) {
+                    store_row16<TOut>(dst, acc, bias ? bias + jb : nullptr, bias != nullptr);
+                    store_row16<TOut>(dst + 16, acc + 16, bias ? bias + jb + 16 : nullptr, bias != nullptr);
+                } else {
+                    for (int i = 0; i < 32; ++i)
+                        if (jb + i < p.n) dst[i] = from_f32<TOut>(__uint_as_float(acc[i]) + (bias ? to_f32(bias[jb + i]) : 0.f));
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_map(tmem_empty(ab), 0)) : "memory");
+        }
+    }
+    tc_fence_before();
+    __syncwarp();
+    cluster_sync();                                                       // the pair's MMAs, arrivals and reads of the other CTA's shared memory are over
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
     }
 }
 
@@ -320,13 +545,36 @@ bool make_map(CUtensorMap* map, const void* base, int rows, int k, int64_t ld, i
     return true;
 }
 
+template <typename K>
+void launch_cluster(K kern, int grid, int cluster, size_t smem, cudaStream_t st, const CUtensorMap& am, const CUtensorMap& bm, const DenseParams& p) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(kGemmThreads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
+    cudaLaunchKernelEx(&cfg, kern, am, bm, p);
+}
+
 template <int kBN, typename TOut>
 void launch_dense(const CUtensorMap& am, const CUtensorMap& bm, const DenseParams& p, cudaStream_t st) {
     auto kern = dense_gemm_kernel<kBN, TOut>;
     ensure_dynamic_smem(reinterpret_cast<const void*>(kern), DCfg<kBN>::kTotal);
     const int tiles = p.tiles_a * p.tiles_b * p.ksplit;
     const int grid = tiles < sm_count() ? tiles : sm_count();
-    launch_pdl(kern, dim3(grid), dim3(kGemmThreads), DCfg<kBN>::kTotal, st, am, bm, p);
+    if (p.csplit > 1) launch_cluster(kern, tiles * p.csplit, p.csplit, DCfg<kBN>::kTotal, st, am, bm, p);
+    else launch_pdl(kern, dim3(grid), dim3(kGemmThreads), DCfg<kBN>::kTotal, st, am, bm, p);
+    count_launch();
+}
+
+template <typename TOut>
+void launch_pair(const CUtensorMap& am, const CUtensorMap& bm, const DenseParams& p, cudaStream_t st) {
+    auto kern = dense_gemm_pair_kernel<TOut>;
+    ensure_dynamic_smem(reinterpret_cast<const void*>(kern), PairCfg::kTotal);
+    const int tiles = p.tiles_a * p.tiles_b, pairs = sm_count() / 2;
+    launch_cluster(kern, 2 * (tiles < pairs ? tiles : pairs), 2, PairCfg::kTotal, st, am, bm, p);
     count_launch();
 }
 
@@ -335,6 +583,15 @@ void launch_out(const CUtensorMap& am, const CUtensorMap& bm, const DenseParams&
     if (p.out_dtype == B200_F32) launch_dense<kBN, float>(am, bm, p, st);
     else if (p.out_dtype == B200_BF16) launch_dense<kBN, __nv_bfloat16>(am, bm, p, st);
     else launch_dense<kBN, __half>(am, bm, p, st);
+}
+
+// CTAs that share a tile over k while there are fewer tiles than SMs: as many as keep every tile's cluster in the first round, at least four k blocks each.  [100 x 4096 x
+// 4096 as 16 clusters of 8: 26 us, a second round for the last one; as 64 single tiles 15.]
+int cluster_split(int64_t tiles, int nkb) {
+    for (int s = 8; s > 1; --s)
+        if (tiles * s <= sm_count() && s <= nkb / 4 &&
+            tiles <= max_active_clusters(reinterpret_cast<const void*>(dense_gemm_kernel<128, __nv_bfloat16>), kGemmThreads, DCfg<128>::kTotal, s)) return s;
+    return 1;
 }
 
 }  // namespace
@@ -367,14 +624,33 @@ bool dense_gemm_16(const void* x, const void* w, const void* bias, void* y, int 
             if (ks > nkb / 4) ks = nkb / 4;
             if (ks > 1) p.ksplit = ks;
         }
+        // without the caller's zeroed f32 output a cluster shares each tile over k
+        if (p.ksplit == 1 && !accumulate) p.csplit = cluster_split(p.tiles_a, (k + kBK - 1) / kBK);
         if (!make_map(&am, w, n, k, ldw, kBM, bf16) || !make_map(&bm, x, m, k, ldx, bn, bf16)) return false;
         if (bn == 32) launch_out<32>(am, bm, p, st); else launch_out<64>(am, bm, p, st);
     } else {
-        // 128 x 256 tiles when they fill the machine; mid-size m (a few hundred rows) gets narrower tiles so that every SM has one
-        int bn = 256;
-        auto tiles = [&](int b) { return (int64_t)((m + kBM - 1) / kBM) * ((n + b - 1) / b); };
-        if (tiles(256) < sm_count()) bn = 128;
-        if (bn == 128 && tiles(128) < sm_count()) bn = 64;
+        // The tile and the split that are done first by this count (clocks): rounds of CTAs (pairs) times (k blocks times the longer of the MMA, 2 BN a block, and
+        // the operands at 64 bytes a clock, plus fixed cost); a shared tile also pays for the sums' way through shared memory.
+        const int64_t nkb = (k + kBK - 1) / kBK;
+        int bn = 256, split = 1;
+        int64_t best = INT64_MAX;
+        for (int b : {256, 128, 64}) {
+            const int64_t tiles = (int64_t)((m + kBM - 1) / kBM) * ((n + b - 1) / b);
+            const int s = accumulate ? 1 : cluster_split(tiles, (int)nkb);
+            const int64_t rounds = (tiles * s + sm_count() - 1) / sm_count(), block = 2 * b > (128 + b) * 2 ? 2 * b : (128 + b) * 2;
+            const int64_t clocks = rounds * ((nkb + s - 1) / s * block + 1500) + (s > 1 ? 2000 + 16 * b : 0);
+            if (clocks < best) { best = clocks; bn = b; split = s; }
+        }
+        const int64_t pair_tiles = (int64_t)((m + 255) / 256) * ((n + 255) / 256), pairs = sm_count() / 2;
+        if (!accumulate && (pair_tiles + pairs - 1) / pairs * (nkb * 512 + 2000) <= best) {
+            p.swap = 0; p.tiles_a = (m + 255) / 256; p.tiles_b = (n + 255) / 256;
+            if (!make_map(&am, x, m, k, ldx, kBM, bf16) || !make_map(&bm, w, n, k, ldw, kBM, bf16)) return false;
+            if (out_dtype == B200_F32) launch_pair<float>(am, bm, p, st);
+            else if (out_dtype == B200_BF16) launch_pair<__nv_bfloat16>(am, bm, p, st);
+            else launch_pair<__half>(am, bm, p, st);
+            return check_launch("dense_gemm");
+        }
+        p.csplit = split;
         p.swap = 0; p.tiles_a = (m + kBM - 1) / kBM; p.tiles_b = (n + bn - 1) / bn;
         if (!make_map(&am, x, m, k, ldx, kBM, bf16) || !make_map(&bm, w, n, k, ldw, bn, bf16)) return false;
         if (bn == 256) launch_out<256>(am, bm, p, st); else if (bn == 128) launch_out<128>(am, bm, p, st); else launch_out<64>(am, bm, p, st);

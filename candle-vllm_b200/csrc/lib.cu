@@ -69,6 +69,26 @@ void ensure_dynamic_smem(const void* kernel, int bytes) {
     else cudaGetLastError();
 }
 
+int max_active_clusters(const void* kernel, int threads, int smem, int size) {
+    static std::atomic<int> cached[kMaxDevices][9];
+    int dev = 0;
+    if (size < 1 || size > 8) return 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) { cudaGetLastError(); return 0; }
+    int n = cached[dev][size].load(std::memory_order_relaxed);
+    if (n == 0) {
+        ensure_dynamic_smem(kernel, smem);
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)(size * 64)); cfg.blockDim = dim3((unsigned)threads); cfg.dynamicSmemBytes = (size_t)smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)size; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr; cfg.numAttrs = 1;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) { cudaGetLastError(); n = -1; }
+        cached[dev][size].store(n, std::memory_order_relaxed);
+    }
+    return n < 0 ? 0 : n;
+}
+
 }  // namespace b200
 
 extern "C" {

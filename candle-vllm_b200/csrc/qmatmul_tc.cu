@@ -118,15 +118,6 @@ __device__ __forceinline__ int seg_of_tile(const GemmParams& p, int tile) { retu
 // first tile of segment sg (constant indices only: dynamic indexing would spill the parameter struct to local memory)
 __device__ __forceinline__ int seg_first_tile(const GemmParams& p, int sg) { return sg == 0 ? 0 : (sg == 1 ? p.tile_end[0] : p.tile_end[1]); }
 __device__ __forceinline__ int seg_rows(const GemmParams& p, int sg) { return sg == 0 ? p.n[0] : (sg == 1 ? p.n[1] : p.n[2]); }
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-    return v;
-}
-
 // what a tile id means
 struct Tile {
     int sg, n0;          // segment, first weight row within the segment's matrix
@@ -879,8 +870,8 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                 continue;
             }
             if (kMB == 256 && p.csplit > 1) {
-                // partial sums -> this CTA's shared memory, [column][128 rows] (the rings are drained: every load of this CTA has been consumed)
-                float* part = reinterpret_cast<float*>(smem);
+                // partial sums -> this CTA's shared memory, [4 columns][128 rows][4] (the rings are drained: every load of this CTA has been consumed)
+                float4* part = reinterpret_cast<float4*>(smem);
                 constexpr int kCols = kMB / 4;
 #pragma unroll 1
                 for (int c0 = 0; c0 < kCols; c0 += 16) {
@@ -889,7 +880,9 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                     tc_ld16(tmem + kColD + lane_addr + qt * kCols + c0, acc);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) part[(qt * kCols + c0 + i) * kTileN + row] = __uint_as_float(acc[i]);
+                    for (int i = 0; i < 4; ++i)
+                        part[((qt * kCols + c0) / 4 + i) * kTileN + row] =
+                            make_float4(__uint_as_float(acc[4 * i]), __uint_as_float(acc[4 * i + 1]), __uint_as_float(acc[4 * i + 2]), __uint_as_float(acc[4 * i + 3]));
                 }
                 continue;                                             // the only tile of this CTA
             }
@@ -949,28 +942,20 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         if (warp < kDequantWarps) {
             const int rank = (int)(blockIdx.x % (uint32_t)p.csplit), row = (int)threadIdx.x & 127;
             const Tile ti = tile_of<kMB>(p, (int)tile0);
-            const int n_idx = ti.n0 + row, c1 = ti.count * (rank + 1) / p.csplit;
+            const int n_idx = ti.n0 + row, groups = (ti.count + 3) / 4, g1 = groups * (rank + 1) / p.csplit;
             float* const y = (ti.sg == 0 ? p.y[0] : (ti.sg == 1 ? p.y[1] : p.y[2])) + (int64_t)ti.xrow * p.ldy + n_idx;
-            // eight columns at a time: their loads from one CTA are in flight together
-            constexpr int kStep = kDequantWarps / 4, kBatch = 8;
-            for (int c = ti.count * rank / p.csplit + ((int)threadIdx.x >> 7); c < c1; c += kStep * kBatch) {
-                float v[kBatch];
-#pragma unroll
-                for (int i = 0; i < kBatch; ++i) v[i] = 0.f;
-                for (int q = 0; q < p.csplit; ++q) {
-                    uint32_t at;
-                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_base + (uint32_t)(c * kTileN + row) * 4), "r"((uint32_t)q));
-                    float f[kBatch];
-#pragma unroll
-                    for (int i = 0; i < kBatch; ++i) f[i] = ld_cluster_f32(at + (uint32_t)(min(c + i * kStep, c1 - 1) - c) * (kTileN * 4));
-#pragma unroll
-                    for (int i = 0; i < kBatch; ++i) v[i] += f[i];
+            for (int g = groups * rank / p.csplit + ((int)threadIdx.x >> 7); g < g1; g += kDequantWarps / 4) {
+                float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+                for (int q = 0; q < p.csplit; ++q) {                  // four columns of a CTA in one load, four CTAs in flight
+                    const float4 f = ld_cluster_f32x4(cluster_map(smem_base + (uint32_t)(g * kTileN + row) * 16, (uint32_t)q));
+                    v[0] += f.x; v[1] += f.y; v[2] += f.z; v[3] += f.w;
                 }
                 if (n_idx < seg_rows(p, ti.sg)) {
 #pragma unroll
-                    for (int i = 0; i < kBatch; ++i) {
-                        if (c + i * kStep >= c1) break;
-                        float* o = y + (int64_t)(c + i * kStep) * p.ldy;
+                    for (int i = 0; i < 4; ++i) {
+                        if (4 * g + i >= ti.count) break;
+                        float* o = y + (int64_t)(4 * g + i) * p.ldy;
                         *o = p.accumulate ? *o + v[i] : v[i];
                     }
                 }
@@ -1141,10 +1126,10 @@ static int rows_per_tile(int m) { return m <= 32 ? 32 : (m <= 64 ? 64 : 256); }
 static int row_tiles(int m) { return m <= 64 ? 1 : (m + 255) / 256; }
 static int tile_rows(int m) { return m <= 64 ? rows_per_tile(m) : (((m + row_tiles(m) - 1) / row_tiles(m)) + 31) / 32 * 32; }
 static int cluster_split(int64_t tiles, int nsb) {
-    int64_t s = sm_count() / tiles;
-    if (s > 8) s = 8;
-    if (s > nsb / 2) s = nsb / 2;
-    return s < 1 ? 1 : (int)s;
+    for (int s = 8; s > 1; --s)
+        if (tiles * s <= sm_count() && s <= nsb / 2 &&
+            tiles <= max_active_clusters(reinterpret_cast<const void*>(qmatmul_tc_kernel<256, B200_GGML_Q4_K>), kThreads, Cfg<256, B200_GGML_Q4_K>::kTotal, s)) return s;
+    return 1;
 }
 
 // true when some output tile is produced by more than one CTA (or accumulate): y must then hold the

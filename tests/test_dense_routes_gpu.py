@@ -1,0 +1,32 @@
+"""GPU parity of the dense GEMM at the sizes where its routes change or can go wrong -- tiles shared over k by a cluster, two-SM tiles, ragged rows, columns and k --
+against float64.  Tolerance: one rounding of the output to 16 bits, at most half a unit in the last place (2^-9 of the value for bf16, 2^-12 for f16), so a relative
+Frobenius error below that; the f32 sums are orders below."""
+import pytest
+import torch
+
+import candle_vllm_b200 as pkg
+from tests.gpu_util import DEV
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype,bias", [(torch.bfloat16, True), (torch.float16, False)])
+@pytest.mark.parametrize("m,n,k", [
+    (1, 4096, 4096), (31, 1024, 4096), (33, 6144, 512), (64, 2048, 2056), (5, 136, 72), (17, 14336, 1024),       # weights on the 128-row side, clusters of 8, 3, 2, 1
+    (65, 4096, 4096), (100, 4096, 4096), (127, 264, 520), (129, 1024, 4096), (200, 2048, 2048), (300, 136, 1000),     # shared tiles of 256, 128, 64 columns
+    (512, 4096, 256), (700, 4104, 328), (1000, 6144, 512),
+    (2048, 4096, 512), (2049, 4352, 264), (8192, 4096, 320), (8000, 2312, 64), (4000, 14336, 128),             # two-SM tiles: whole, ragged, fewer k blocks than stages
+])
+def test_routes(dtype, bias, m, n, k):
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(m + n + k)
+    x = torch.randn((m, k), device=DEV, generator=gen).to(dtype)
+    w = (torch.randn((n, k), device=DEV, generator=gen) * 0.05).to(dtype)
+    b = torch.randn(n, device=DEV, generator=gen).to(dtype) if bias else None
+    y = pkg.Linear(w, b).forward(x)
+    ref = x.double() @ w.double().T
+    if bias:
+        ref += b.double()
+    err = float((y.double() - ref).norm() / ref.norm())
+    assert err < (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12), err
+    assert torch.equal(y, pkg.Linear(w, b).forward(x))          # sums meet in a fixed order
