@@ -8,9 +8,9 @@
 // Every head of a sequence reads the SAME 1152 bytes per token: the op is MQA with a 576-wide key and a 512-wide value.
 //
 // Decode kernel (tensor cores, flash-decoding split over the context): a CTA of 4 warps owns (sequence, chunk of <= 256 tokens,
-// group of 16 heads).  32-token latent tiles land by TMA (nine {64 dims, 32 tokens} boxes, 128-byte swizzle, 2 stages of 36 KB); the
-// 16 heads are the M rows of mma.sync m16n8k16.  Per tile: warp w computes S for tokens [8w, 8w+8) over all 576 dims (Q fragments by
-// ldmatrix from shared memory), the warps agree on the running row maxima through shared memory, P goes to shared memory as 16-bit,
+// group of 16 heads).  32-token latent tiles land by TMA (nine {64 dims, 32 tokens} boxes, 128-byte swizzle, 3 stages of 36 KB); the
+// 16 heads are the M rows of mma.sync m16n8k16.  Per tile: warp w computes S for tokens [8w, 8w+8) over all 576 dims (Q fragments in
+// registers), the warps agree on the running row maxima through shared memory, P goes to shared memory as 16-bit,
 // and warp w accumulates O for latent dims [128w, 128w+128) over all 32 tokens.  Partials (m, l, O) per chunk are folded by a merge
 // kernel.  Bytes dominate at 16 heads per rank (TP 8): 30 flop / byte; with all 128 heads on one GPU the same tiles serve 8 head groups
 // from L2.
@@ -31,8 +31,9 @@ constexpr int kHg = 16;                                         // heads per CTA
 constexpr int kSubB = kTl * 64 * 2;                             // one {64 dims, 32 tokens} box: 4 KB
 constexpr int kStageB = 9 * kSubB;                              // 36 KB
 constexpr int kChunkTok = 256;
-constexpr int kQB = kHg * kKd * 2;                              // Q tile 16 x 576 x 2 B = 18 KB (row pitch 1152 B)
-constexpr int kSmQ = 0, kSmStage = 18432, kSmP = kSmStage + 2 * kStageB, kSmMax = kSmP + kHg * kTl * 2, kSmBar = kSmMax + 4 * kHg * 4;
+constexpr int kMlaStages = 3;                                   // three tiles per CTA, two CTAs per SM: 216 KB
+constexpr int kSmStage = 0, kSmP = kSmStage + kMlaStages * kStageB, kSmMax = kSmP + kHg * kTl * 2, kSmBar = kSmMax + 4 * kHg * 4;
+static_assert(2 * (kSmBar + 64 + 1024) <= 233472, "two CTAs per SM");
 constexpr int kMlaSmem = kSmBar + 64;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -102,7 +103,26 @@ struct MlaParams {
     int num_heads, max_blocks, max_chunks;
     float scale_log2;
     int window;                                // > 0: a row sees only the last `window` keys of its context
+    int num_seqs, places;                      // places: CTAs that run at the same time
 };
+
+// Tokens per chunk of this launch, the same for every CTA and for the merge: whole tiles, at least kChunkTok (what the workspace is sized for), and for few sequences as
+// many as let all chunks run at once, two CTAs per SM -- 32 sequences of 3000 to 4096 tokens are 460 chunks of 256 on 296 places, a second round for half of them.
+__device__ __forceinline__ int mla_chunk_tokens(const uint32_t* context_lens, int num_seqs, int head_groups, int window, int places) {
+    if (num_seqs > 128) return kChunkTok;
+    const int lane = threadIdx.x & 31;
+    int tokens = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (lane + 32 * i < num_seqs) { const int c = (int)context_lens[lane + 32 * i]; tokens += window > 0 && c > window ? window + kTl : c; }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) tokens += __shfl_xor_sync(0xffffffffu, tokens, o);
+    // on average half a chunk per sequence is padding: places - seqs * groups / 2 whole chunks
+    const int whole = places - num_seqs * head_groups / 2;
+    if (whole <= 0 || (int64_t)tokens * head_groups > (int64_t)4 * places * kChunkTok) return kChunkTok;
+    const int want = (int)(((int64_t)tokens * head_groups + whole - 1) / whole);
+    return want <= kChunkTok ? kChunkTok : (want + kTl - 1) / kTl * kTl;
+}
 
 // first key a row sees, rounded down to a whole tile: the chunks of a windowed row are counted from there (tiles never straddle a page)
 __device__ __forceinline__ int mla_first_key(int ctx, int window) { return window > 0 && ctx > window ? ctx - window : 0; }
@@ -113,32 +133,36 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap cmap, const __grid_constan
     extern __shared__ __align__(1024) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int chunk = blockIdx.x, seq = blockIdx.y, hg = blockIdx.z;
+    pdl_wait();
+    pdl_trigger();
     const int ctx = (int)p.context_lens[seq];
     const int first = mla_first_key(ctx, p.window);
-    const int tok_begin = (first & ~(kTl - 1)) + chunk * kChunkTok;
+    const int chunk_tok = mla_chunk_tokens(p.context_lens, p.num_seqs, (int)gridDim.z, p.window, p.places);
+    const int tok_begin = (first & ~(kTl - 1)) + chunk * chunk_tok;
     if (tok_begin >= ctx) return;                                     // uniform per CTA
-    const int ntok = min(kChunkTok, ctx - tok_begin), ntiles = (ntok + kTl - 1) / kTl;
+    const int ntok = min(chunk_tok, ctx - tok_begin), ntiles = (ntok + kTl - 1) / kTl;
     const uint32_t sb = smem_u32(smem);
     const uint32_t bars = sb + kSmBar;
     float* wmax = reinterpret_cast<float*>(smem + kSmMax);            // [4 warps][16 heads]
     const int heads = min(kHg, p.num_heads - hg * kHg);
 
     if (threadIdx.x == 0) {
-        mbar_init(bars, 1); mbar_init(bars + 8, 1);
+        for (int i = 0; i < kMlaStages; ++i) mbar_init(bars + 8 * i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    // Q tile -> shared memory: row h = [q_abs (512) | q_pe (64)], 1152-byte rows, 16-byte chunks XOR-swizzled by the row (ldmatrix reads 8 rows
-    // of one 16-byte column at a time: without the swizzle all 8 would hit the same banks)
+    // Q fragments (16 heads x 576, the M rows of every product) live in registers: read from shared memory per tile they were two thirds of its traffic
+    uint32_t qf[kKd / 16][4];
     {
         const T* qa = static_cast<const T*>(p.q_abs) + ((int64_t)seq * p.num_heads + hg * kHg) * kLat;
         const T* qp = static_cast<const T*>(p.q_pe) + ((int64_t)seq * p.num_heads + hg * kHg) * kRope;
-        for (int i = threadIdx.x; i < kHg * (kKd / 8); i += blockDim.x) {
-            const int h = i / (kKd / 8), c = i % (kKd / 8);           // 72 chunks of 8 elements per row
-            int4 v = make_int4(0, 0, 0, 0);
-            if (h < heads) v = c < kLat / 8 ? *reinterpret_cast<const int4*>(qa + (int64_t)h * kLat + c * 8) : *reinterpret_cast<const int4*>(qp + (int64_t)h * kRope + (c - kLat / 8) * 8);
-            *reinterpret_cast<int4*>(smem + kSmQ + h * (kKd * 2) + (((c & ~7) | ((c & 7) ^ (h & 7))) << 4)) = v;
-        }
+#pragma unroll
+        for (int ks = 0; ks < kKd / 16; ++ks)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {                             // rows g, g + 8; columns 2 t and 2 t + 8 of the k-step
+                const int h = g + (e & 1) * 8, c = ks * 16 + 2 * t + (e >> 1) * 8;
+                qf[ks][e] = h < heads ? (c < kLat ? *reinterpret_cast<const uint32_t*>(qa + (int64_t)h * kLat + c) : *reinterpret_cast<const uint32_t*>(qp + (int64_t)h * kRope + c - kLat)) : 0u;
+            }
     }
     __syncthreads();
     const uint32_t* table = p.block_tables + (int64_t)seq * p.max_blocks;
@@ -151,7 +175,8 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap cmap, const __grid_constan
         for (int j = 0; j < 8; ++j) tma_load_3d(dst + j * kSubB, &cmap, bar, j * 64, off, blk);
         tma_load_3d(dst + 8 * kSubB, &pmap, bar, 0, off, blk);
     };
-    if (threadIdx.x == 0) issue(0, 0);
+    if (threadIdx.x == 0)
+        for (int i = 0; i < kMlaStages - 1 && i < ntiles; ++i) issue(i, i);
 
     float o[16][4];
 #pragma unroll
@@ -159,13 +184,13 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap cmap, const __grid_constan
     float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;       // rows g and g + 8; l = this warp's tokens only
 
     for (int tl = 0; tl < ntiles; ++tl) {
-        const int stage = tl & 1;
-        if (threadIdx.x == 0 && tl + 1 < ntiles) issue(tl + 1, stage ^ 1);
-        mbar_wait(bars + stage * 8, (tl >> 1) & 1);
+        const int stage = tl % kMlaStages;
+        if (threadIdx.x == 0 && tl + kMlaStages - 1 < ntiles) issue(tl + kMlaStages - 1, (tl + kMlaStages - 1) % kMlaStages);     // drained before the last barrier
+        mbar_wait(bars + stage * 8, (tl / kMlaStages) & 1);
         const uint32_t kt = sb + kSmStage + stage * kStageB;
         const int valid = min(kTl, ntok - tl * kTl);
         // ---- S for this warp's 8 tokens: 36 k-steps over [ckv | kpe] -------------------------------------------------------------
-        float s[4] = {0.f, 0.f, 0.f, 0.f};
+        float s[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};       // two chains of dependent products
         {
             const int row = warp * 8 + (lane & 7);                   // token row of the tile
 #pragma unroll
@@ -173,17 +198,11 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap cmap, const __grid_constan
                 const int chunk16 = kp * 4 + (lane >> 3);            // 16-byte chunk 0..71 along the 576 dims
                 uint32_t kb[4];
                 ldmatrix_x4(kb, kt + (chunk16 >> 3) * kSubB + row * 128 + (((chunk16 & 7) ^ (row & 7)) << 4));
-                // Q fragments (A, row-major 16 x 16): ldmatrix x4 = {rows 0-7 | k lo, rows 8-15 | k lo, rows 0-7 | k hi, rows 8-15 | k hi}
-                uint32_t a0[4], a1[4];
-                {
-                    const int qr = (lane & 7) + ((lane >> 3) & 1) * 8, qc = kp * 4 + (lane >> 4);           // k-step 2 kp: chunks 4 kp + {0, 1}
-                    ldmatrix_x4(a0, sb + kSmQ + qr * (kKd * 2) + (((qc & ~7) | ((qc & 7) ^ (qr & 7))) << 4));
-                    const int qc1 = qc + 2;                                                                  // k-step 2 kp + 1: chunks 4 kp + {2, 3}
-                    ldmatrix_x4(a1, sb + kSmQ + qr * (kKd * 2) + (((qc1 & ~7) | ((qc1 & 7) ^ (qr & 7))) << 4));
-                }
-                mma_16816<T>(s, a0, kb[0], kb[1]);
-                mma_16816<T>(s, a1, kb[2], kb[3]);
+                mma_16816<T>(s, qf[2 * kp], kb[0], kb[1]);
+                mma_16816<T>(s1, qf[2 * kp + 1], kb[2], kb[3]);
             }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[e] += s1[e];
         }
         // ---- mask, row maxima agreed across the four warps --------------------------------------------------------------------------
         const int tok = warp * 8 + 2 * t;
@@ -209,8 +228,10 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap cmap, const __grid_constan
             *reinterpret_cast<uint32_t*>(ps + g * kTl + tok) = pack2<T>(p0, p1);
             *reinterpret_cast<uint32_t*>(ps + (g + 8) * kTl + tok) = pack2<T>(p2, p3);
         }
+        if (__any_sync(0xffffffffu, c_lo != 1.f || c_hi != 1.f)) {        // (the maxima move in the first tiles, hardly later)
 #pragma unroll
-        for (int i = 0; i < 16; ++i) { o[i][0] *= c_lo; o[i][1] *= c_lo; o[i][2] *= c_hi; o[i][3] *= c_hi; }
+            for (int i = 0; i < 16; ++i) { o[i][0] *= c_lo; o[i][1] *= c_lo; o[i][2] *= c_hi; o[i][3] *= c_hi; }
+        }
         // latent rows past the context may hold anything: zero them (their P is 0, but 0 * NaN would poison O); each warp cleans the
         // 128 dims it is about to read
         if (valid < kTl) {
@@ -265,22 +286,43 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap cmap, const __grid_constan
 template <typename T>
 __global__ void __launch_bounds__(128)
 mla_merge_kernel(T* __restrict__ out, const float* __restrict__ part_o, const float* __restrict__ part_ml, const uint32_t* __restrict__ context_lens,
-                 int num_heads, int max_chunks, const float* __restrict__ sink, int window) {
+                 int num_heads, int max_chunks, const float* __restrict__ sink, int window, int num_seqs, int places) {
     const int head = blockIdx.x, seq = blockIdx.y;
+    pdl_wait();
+    pdl_trigger();
     const int ctx = (int)context_lens[seq];
-    const int nchunks = (ctx - (mla_first_key(ctx, window) & ~(kTl - 1)) + kChunkTok - 1) / kChunkTok;
+    const int chunk_tok = mla_chunk_tokens(context_lens, num_seqs, (num_heads + kHg - 1) / kHg, window, places);
+    const int nchunks = (ctx - (mla_first_key(ctx, window) & ~(kTl - 1)) + chunk_tok - 1) / chunk_tok;
     const int64_t base = ((int64_t)seq * num_heads + head) * max_chunks;
     // a softmax sink (one learned score per head, no key, no value) joins the maximum and the denominator here; the partial maxima are in
     // log2 units (scores were scaled by log2 e), the sink comes in natural units
     const float sink2 = sink ? sink[head] * 1.4426950408889634f : -INFINITY;
     float M = sink2;
-    for (int c = 0; c < nchunks; ++c) M = fmaxf(M, part_ml[(base + c) * 2]);
+    // the loads of eight chunks are in flight together: the kernel is their latency
+    for (int c0 = 0; c0 < nchunks; c0 += 8) {
+        float m[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) m[i] = c0 + i < nchunks ? part_ml[(base + c0 + i) * 2] : -INFINITY;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) M = fmaxf(M, m[i]);
+    }
     float L = sink ? exp2f(sink2 - M) : 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int c = 0; c < nchunks; ++c) {
-        const float w = exp2f(part_ml[(base + c) * 2] - M);
-        L += w * part_ml[(base + c) * 2 + 1];
-        const float4 v = *reinterpret_cast<const float4*>(part_o + (base + c) * kLat + threadIdx.x * 4);
-        acc[0] += w * v.x; acc[1] += w * v.y; acc[2] += w * v.z; acc[3] += w * v.w;
+    for (int c0 = 0; c0 < nchunks; c0 += 8) {
+        float2 ml[8];
+        float4 v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const bool in = c0 + i < nchunks;
+            ml[i] = in ? *reinterpret_cast<const float2*>(part_ml + (base + c0 + i) * 2) : make_float2(-INFINITY, 0.f);
+            v[i] = in ? *reinterpret_cast<const float4*>(part_o + (base + c0 + i) * kLat + threadIdx.x * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (c0 + i >= nchunks) break;
+            const float w = exp2f(ml[i].x - M);
+            L += w * ml[i].y;
+            acc[0] += w * v[i].x; acc[1] += w * v[i].y; acc[2] += w * v[i].z; acc[3] += w * v[i].w;
+        }
     }
     const float inv = nchunks > 0 && L > 0.f ? 1.f / L : 0.f;
     T* o = out + ((int64_t)seq * num_heads + head) * kLat + threadIdx.x * 4;
@@ -434,16 +476,16 @@ void mla_paged_attention_window(void* out, const void* q_absorbed, const void* q
             const int max_chunks = (int)(((size_t)max_blocks_per_seq * block_size + kChunkTok - 1) / kChunkTok);
             MlaParams p{q_absorbed, q_pe, block_tables, context_lens, static_cast<float*>(workspace),
                         static_cast<float*>(workspace) + (size_t)num_seqs * num_heads * max_chunks * kLat, num_heads, max_blocks_per_seq, max_chunks,
-                        sm_scale * 1.4426950408889634f, window > 0 ? window : 0};
+                        sm_scale * 1.4426950408889634f, window > 0 ? window : 0, num_seqs, 2 * sm_count()};
             const dim3 grid(max_chunks, num_seqs, ceil_div(num_heads, kHg));
             if (dtype == B200_BF16) {
                 ensure_dynamic_smem(reinterpret_cast<const void*>(mla_decode_kernel<__nv_bfloat16>), kMlaSmem);
-                mla_decode_kernel<__nv_bfloat16><<<grid, 128, kMlaSmem, st>>>(cm, pm, p);
-                mla_merge_kernel<__nv_bfloat16><<<dim3(num_heads, num_seqs), 128, 0, st>>>((__nv_bfloat16*)out, p.part_o, p.part_ml, context_lens, num_heads, max_chunks, sink, p.window);
+                launch_pdl(mla_decode_kernel<__nv_bfloat16>, grid, dim3(128), kMlaSmem, st, cm, pm, p);
+                launch_pdl(mla_merge_kernel<__nv_bfloat16>, dim3(num_heads, num_seqs), dim3(128), 0, st, (__nv_bfloat16*)out, p.part_o, p.part_ml, context_lens, num_heads, max_chunks, sink, p.window, num_seqs, p.places);
             } else {
                 ensure_dynamic_smem(reinterpret_cast<const void*>(mla_decode_kernel<__half>), kMlaSmem);
-                mla_decode_kernel<__half><<<grid, 128, kMlaSmem, st>>>(cm, pm, p);
-                mla_merge_kernel<__half><<<dim3(num_heads, num_seqs), 128, 0, st>>>((__half*)out, p.part_o, p.part_ml, context_lens, num_heads, max_chunks, sink, p.window);
+                launch_pdl(mla_decode_kernel<__half>, grid, dim3(128), kMlaSmem, st, cm, pm, p);
+                launch_pdl(mla_merge_kernel<__half>, dim3(num_heads, num_seqs), dim3(128), 0, st, (__half*)out, p.part_o, p.part_ml, context_lens, num_heads, max_chunks, sink, p.window, num_seqs, p.places);
             }
             count_launch(2);
             check_launch("mla_paged_attention");

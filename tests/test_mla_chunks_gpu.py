@@ -1,0 +1,48 @@
+"""GPU parity of latent decode where the chunk length of the split-KV kernel changes: the 256-token minimum, longer chunks for few long sequences, many sequences,
+ragged contexts at chunk and tile edges -- against float64.  Tolerance: probabilities and output are rounded to 16 bits (2^-9 relative each for bf16, 2^-12 for f16),
+errors in quadrature: relative Frobenius below 2^-8 (2^-11)."""
+import numpy as np
+import pytest
+import torch
+
+from candle_vllm_b200 import mla
+from tests.gpu_util import DEV
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("heads,lens", [
+    (16, [1, 31, 32, 33, 255, 256, 257]),
+    (16, [4096 - 61 * i for i in range(32)]),                  # chunks longer than 256: one round of CTAs
+    (20, [2500, 3, 2999, 64]),                                 # a second, partly filled head group
+    (128, [900, 1500, 70]),
+    (16, [100 + 3 * i for i in range(130)]),                   # more sequences than the kernel adds up: 256
+])
+def test_decode(dtype, heads, lens):
+    gen = torch.Generator(device=DEV)
+    gen.manual_seed(heads + len(lens))
+    used = [-(-n // 64) for n in lens]
+    pool = sum(used) + 1
+    perm = np.random.default_rng(1).permutation(pool)
+    tables, at = np.zeros((len(lens), max(used)), np.int32), 0
+    for i, n in enumerate(used):
+        tables[i, :n] = perm[at:at + n]
+        at += n
+    mk = lambda *s, std=1.0: (torch.randn(s, device=DEV, generator=gen) * std).to(dtype)
+    ckv, kpe, q, qp = mk(pool, 64, 1, 512), mk(pool, 64, 1, 64), mk(len(lens), heads, 512, std=0.3), mk(len(lens), heads, 64, std=0.3)
+    scale = 192 ** -0.5
+    for i, n in enumerate(lens):                               # what lies past a context must not matter
+        if n % 64:
+            ckv[tables[i, used[i] - 1], n % 64:] = float("nan")
+            kpe[tables[i, used[i] - 1], n % 64:] = float("nan")
+    out = mla.mla_paged_decode(q, qp, ckv, kpe, torch.from_numpy(tables).to(DEV), torch.tensor(lens, dtype=torch.int32, device=DEV), scale)
+    ref = []
+    for i, n in enumerate(lens):
+        ids = torch.from_numpy(tables[i, :used[i]]).to(DEV).long()
+        c, r = ckv[ids].flatten(0, 1)[:n, 0].double(), kpe[ids].flatten(0, 1)[:n, 0].double()
+        ref.append(torch.softmax((q[i].double() @ c.T + qp[i].double() @ r.T) * scale, 1) @ c)
+    ref = torch.stack(ref)
+    assert torch.isfinite(out).all()
+    err = float((out.double() - ref).norm() / ref.norm())
+    assert err < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11), err
