@@ -30,32 +30,28 @@ namespace {
 // one warp per token; E <= 32 kPer experts, k <= 32.  logits: `splits` partial sums, split_stride apart (1: finished logits).  normalise: the weights are divided by
 // their sum; all are multiplied by `scaling`.  [With 32 slots per lane whatever E, 16 tokens of 128 experts took 8.0 us.]
 template <int kPer>
-__global__ void __launch_bounds__(128)
-topk_softmax_kernel(const float* __restrict__ logits, int splits, int64_t split_stride, float* __restrict__ w_out, uint32_t* __restrict__ id_out, int tokens, int E, int k,
-                    int normalise, float scaling) {
-    pdl_wait();
-    pdl_trigger();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t = blockIdx.x * 4 + warp;
-    if (t >= tokens) return;
+__device__ __forceinline__ void topk_token(const float* __restrict__ logits, int splits, int64_t split_stride, float* __restrict__ w_out, uint32_t* __restrict__ id_out,
+                                           int t, int E, int k, int normalise, float scaling) {
+    const int lane = threadIdx.x & 31;
     float v[kPer];
     float mx = -INFINITY;
+    constexpr int kBatch = kPer <= 8 ? 4 : 1;          // parts of all slots in flight together, added in order
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) v[i] = 0.f;
+    for (int s = 0; s < splits; s += kBatch) {
+        float b[kPer][kBatch];
+#pragma unroll
+        for (int i = 0; i < kPer; ++i)
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) b[i][j] = lane + 32 * i < E && s + j < splits ? logits[(s + j) * split_stride + (int64_t)t * E + lane + 32 * i] : 0.f;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i)
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) v[i] = s + j == 0 ? b[i][j] : v[i] + b[i][j];
+    }
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-        const int e = lane + 32 * i;
-        v[i] = -INFINITY;
-        if (e < E) {
-            const float* src = logits + (int64_t)t * E + e;
-            float a = src[0];
-            for (int s = 1; s < splits; s += 5) {            // five parts in flight (16 at most: 1 + 3 x 5), added in order
-                float b[5];
-#pragma unroll
-                for (int j = 0; j < 5; ++j) b[j] = s + j < splits ? src[(s + j) * split_stride] : 0.f;
-#pragma unroll
-                for (int j = 0; j < 5; ++j) a += b[j];
-            }
-            v[i] = a;
-        }
+        if (lane + 32 * i >= E) v[i] = -INFINITY;
         mx = fmaxf(mx, v[i]);
     }
     mx = warp_max(mx);
@@ -86,6 +82,15 @@ topk_softmax_kernel(const float* __restrict__ logits, int splits, int64_t split_
             if (lane + 32 * i == bi) v[i] = -1.f;      // remove the winner (probabilities are >= 0)
     }
     if (lane < k) w_out[(int64_t)t * k + lane] = (normalise ? mine / total : mine) * scaling;
+}
+template <int kPer>
+__global__ void __launch_bounds__(128)
+topk_softmax_kernel(const float* __restrict__ logits, int splits, int64_t split_stride, float* __restrict__ w_out, uint32_t* __restrict__ id_out, int tokens, int E, int k,
+                    int normalise, float scaling) {
+    pdl_wait();
+    pdl_trigger();
+    const int t = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (t < tokens) topk_token<kPer>(logits, splits, split_stride, w_out, id_out, t, E, k, normalise, scaling);
 }
 void topk_launch(const float* logits, int splits, int64_t split_stride, float* w, uint32_t* ids, int tokens, int E, int k, int normalise, float scaling, cudaStream_t st) {
     auto kern = E <= 32 ? topk_softmax_kernel<1> : E <= 128 ? topk_softmax_kernel<4> : E <= 256 ? topk_softmax_kernel<8> : topk_softmax_kernel<32>;
@@ -174,9 +179,12 @@ __device__ __forceinline__ void write_chunks(int e, int first, int count, int ro
 // Stable counting sort of the flattened expert ids, one CTA of 32 warps (experts <= 1024): warp w owns the w-th run of pairs and a histogram of its own; prefix sums over
 // the warps of an expert, then over the experts, give every warp its first position per expert, and a second pass ranks 32 pairs at a time by match.  With chunks it
 // also writes the chunk list of the grouped GEMM.  [One thread per expert walking every pair took 124 us for 7200 pairs of 128 experts.]
+// kPer > 0 (few tokens): the top-k of each token comes first, one warp per token, and the ids never leave the SM's caches.
 constexpr int kSortBatch = 8;                                          // ids in flight per lane
+struct TopkArgs { const float* logits; int splits; int64_t split_stride; float* weights; int tokens, k, normalise; float scaling; };
+template <int kPer>
 __global__ void __launch_bounds__(1024)
-moe_sort_kernel(const uint32_t* __restrict__ ids, uint32_t* __restrict__ sorted_expert, uint32_t* __restrict__ sorted_pair, int pairs, int E, MoeChunk* __restrict__ chunks,
+moe_sort_kernel(const TopkArgs tk, uint32_t* ids, uint32_t* __restrict__ sorted_expert, uint32_t* __restrict__ sorted_pair, int pairs, int E, MoeChunk* __restrict__ chunks,
                 int* __restrict__ num_chunks, int rows, int max_chunks) {
     extern __shared__ int hist[];                                      // [32][E]
     __shared__ int start[1024], sums[33];
@@ -184,6 +192,8 @@ moe_sort_kernel(const uint32_t* __restrict__ ids, uint32_t* __restrict__ sorted_
     for (int i = threadIdx.x; i < 32 * E; i += 1024) hist[i] = 0;
     pdl_wait();
     pdl_trigger();
+    if constexpr (kPer > 0)
+        for (int t = warp; t < tk.tokens; t += 32) topk_token<kPer>(tk.logits, tk.splits, tk.split_stride, tk.weights, ids, t, E, tk.k, tk.normalise, tk.scaling);
     __syncthreads();
     const int per = ((pairs + 31) / 32 + 31) & ~31, p0 = warp * per, p1 = min(pairs, p0 + per);
     int* mine = hist + warp * E;
@@ -224,10 +234,23 @@ moe_sort_kernel(const uint32_t* __restrict__ ids, uint32_t* __restrict__ sorted_
     }
     if (chunks) write_chunks(ex, first, count, rows, chunks, num_chunks, max_chunks, sums);
 }
-void sort_launch(const uint32_t* ids, uint32_t* sorted_expert, uint32_t* sorted_pair, int pairs, int E, MoeChunk* chunks, int* num_chunks, int rows, int max_chunks, cudaStream_t st) {
-    ensure_dynamic_smem(reinterpret_cast<const void*>(moe_sort_kernel), 32 * E * 4);
-    launch_pdl(moe_sort_kernel, dim3(1), dim3(1024), (size_t)32 * E * 4, st, ids, sorted_expert, sorted_pair, pairs, E, chunks, num_chunks, rows, max_chunks);
+template <int kPer>
+void sort_launch(const TopkArgs& tk, uint32_t* ids, uint32_t* sorted_expert, uint32_t* sorted_pair, int pairs, int E, MoeChunk* chunks, int* num_chunks, int rows, int max_chunks, cudaStream_t st) {
+    ensure_dynamic_smem(reinterpret_cast<const void*>(moe_sort_kernel<kPer>), 32 * E * 4);
+    launch_pdl(moe_sort_kernel<kPer>, dim3(1), dim3(1024), (size_t)32 * E * 4, st, tk, ids, sorted_expert, sorted_pair, pairs, E, chunks, num_chunks, rows, max_chunks);
     count_launch();
+}
+// top-k and plan of a step: one launch for up to 32 tokens (one per warp) of up to 256 experts, else the top-k over many CTAs first.  [MoE block, 128 experts,
+// one launch against two: 36.6 against 40 us at 1 token, 102 against 105 at 16; a second round of the warps loses: 150 against 144 at 57]
+void route_launch(const TopkArgs& tk, uint32_t* ids, uint32_t* sorted_pair, int pairs, int E, MoeChunk* chunks, int* num_chunks, int rows, int max_chunks, cudaStream_t st) {
+    if (tk.tokens <= 32 && E <= 256) {
+        if (E <= 32) sort_launch<1>(tk, ids, nullptr, sorted_pair, pairs, E, chunks, num_chunks, rows, max_chunks, st);
+        else if (E <= 128) sort_launch<4>(tk, ids, nullptr, sorted_pair, pairs, E, chunks, num_chunks, rows, max_chunks, st);
+        else sort_launch<8>(tk, ids, nullptr, sorted_pair, pairs, E, chunks, num_chunks, rows, max_chunks, st);
+        return;
+    }
+    topk_launch(tk.logits, tk.splits, tk.split_stride, tk.weights, ids, tk.tokens, E, tk.k, tk.normalise, tk.scaling, st);
+    sort_launch<0>(tk, ids, nullptr, sorted_pair, pairs, E, chunks, num_chunks, rows, max_chunks, st);
 }
 
 // the chunk list from SORTED expert ids (the grouped GEMM's own entry points): segment borders by binary search
@@ -403,7 +426,7 @@ void sort_expert_assignments(const uint32_t* topk_ids, uint32_t* expert_ids, uin
     if (num_pairs == 0) return;
     B200_REQUIRE(topk_ids && expert_ids && sorted_token_ids, kErrBadArg, "sort_expert_assignments: null pointer");
     B200_REQUIRE(num_experts >= 1 && num_experts <= 1024 && num_pairs > 0, kErrUnsupported, "sort_expert_assignments: %d experts (<= 1024)", num_experts);
-    sort_launch(topk_ids, expert_ids, sorted_token_ids, num_pairs, num_experts, nullptr, nullptr, 0, 0, as_stream(stream));
+    sort_launch<0>(TopkArgs{}, const_cast<uint32_t*>(topk_ids), expert_ids, sorted_token_ids, num_pairs, num_experts, nullptr, nullptr, 0, 0, as_stream(stream));
     check_launch("sort_expert_assignments");
 }
 
@@ -519,8 +542,8 @@ void moe_block_gguf(const float* x, const float* router, const void* gate, const
     float* y = reinterpret_cast<float*>(ws + p.y);
     launch_pdl(moe_router_kernel, dim3(ceil_div(num_tokens, kRtT), ceil_div(num_experts, kRtE), p.splits), dim3(128), 0, st, x, router, logits, (int)num_tokens,
                (int)num_experts, (int)hidden, p.steps_per);
-    topk_launch(logits, p.splits, (int64_t)num_tokens * num_experts, weights, ids, num_tokens, num_experts, topk, normalise, scaling, st);
-    sort_launch(ids, nullptr, pair, P, num_experts, chunks, count, p.rows, p.max_chunks, st);
+    route_launch(TopkArgs{logits, p.splits, (int64_t)num_tokens * num_experts, weights, num_tokens, topk, normalise, scaling}, ids, pair, P, num_experts, chunks, count,
+                 p.rows, p.max_chunks, st);
     launch_pdl(moe_gather_kernel, dim3(ceil_div(P, 8)), dim3(256), 0, st, x, (const uint32_t*)pair, xs, P, (int)hidden, 1, (int)topk);
     count_launch(2);
     if (!check_launch("moe_block_gguf")) return;

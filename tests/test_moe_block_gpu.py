@@ -32,6 +32,9 @@ def _block(x, router, gate, up, down, E, topk, normalise, scaling):
 @pytest.mark.parametrize("T,E,topk,H,I,types,normalise,scaling", [
     (1, 128, 8, 512, 256, (12, 12, 12), True, None),        # one token
     (16, 128, 8, 2048, 768, (12, 12, 12), True, None),      # decode: most experts have one row or none
+    (32, 256, 8, 256, 256, (12, 12, 12), True, None),       # top-k in the plan's launch: one token per warp, every slot of a lane
+    (5, 300, 4, 256, 256, (12, 12, 12), True, None),        # too many experts for it
+    (7, 31, 3, 256, 256, (12, 12, 12), False, None),        # fewer experts than lanes
     (33, 5, 2, 256, 256, (12, 12, 12), False, 2.5),         # chunks of 32 with a remainder, experts not a multiple of the router's tile
     (63, 4, 2, 512, 512, (12, 12, 12), True, None),         # about 32 rows per expert, either side of a chunk
     (300, 4, 2, 256, 768, (12, 12, 12), True, 0.5),         # chunks of 128 with remainders
