@@ -327,10 +327,11 @@ struct F4Quarter {
 // B200).  So the box starts at the block address rounded down to 16
 // and is 240 bytes wide (15 x 16: an odd number of 16-byte units per row keeps LDS.128 conflict-free); the
 // block then sits off = (210 * sb) % 16 bytes into the row slot, off in {0, 2, .., 14}, uniform per stage.
-// Each thread loads its slot with aligned LDS.128 and realigns the words it needs in registers:
-// word select by off/4 (two SEL levels) and a 16-bit funnel shift when off % 4 == 2 -- one code path.
+// Each thread loads the 16-byte groups of its slot that hold its quarter -- eight of fourteen, whatever the offset -- and realigns its words in registers: word select by
+// off / 4 (two SEL levels) and a 16-bit funnel shift when off % 4 == 2 -- one code path.  [Four copies of the code, one per off / 4, without selects: 7000 clocks a unit
+// at 32 rows in place of 2300: sixteen hot bodies of 200 instructions do not fit the instruction cache.]
 template <int kJ0, int kN>
-__device__ __forceinline__ void realign(const uint32_t (&t)[57], int wo, int sh16, uint32_t (&out)[kN]) {
+__device__ __forceinline__ void realign(const uint32_t* t, int wo, int sh16, uint32_t (&out)[kN]) {
     uint32_t s1[kN + 3], s2[kN + 1];
 #pragma unroll
     for (int i = 0; i < kN + 3; ++i) s1[i] = (wo & 1) ? t[kJ0 + i + 1] : t[kJ0 + i];
@@ -344,19 +345,17 @@ __device__ __forceinline__ void realign(const uint32_t (&t)[57], int wo, int sh1
 // ((ql[64 kHf + 32 (g&1) + l] nibble (g>>1)) | ((qh[32 kHf + l] >> 2g) & 3) << 4) - 32, times d*scales[8 kHf + 2g + l/16].
 // The 6-bit value goes to fp16 mantissa bits 4-9 (= q * 2^-20); one HFMA2 with (s*2^20, -32 s) finishes it
 // (exact path with the 1024+q magic when s*2^20 would overflow fp16).
-template <int kGp>      // kGp = 0: groups 0 (lo nibble) and 2 (hi nibble) from ql[0..31]; kGp = 1: groups 1, 3
-__device__ __forceinline__ void dequant_q6k_pair(const uint32_t (&ql)[8], uint32_t a_col, const uint32_t (&qh)[8],
-                                                 const uint32_t (&scw)[2], float dk, bool fast) {
+// kGp = 0: groups 0 (lo nibble) and 2 (hi nibble) from ql[0..31]; kGp = 1: groups 1, 3.  The quarter is a run-time value, uniform per warp: all sixteen warps run one body.
+__device__ __forceinline__ void dequant_q6k_pair(const uint32_t (&ql)[8], uint32_t a_col, const uint32_t (&qh)[8], const uint32_t (&scw)[2], float dk, bool fast, int gp) {
     // `fast` is warp-uniform; the two paths are separate straight-line blocks (a per-word branch interleaves them in the
     // instruction stream and the kernel then stalls on instruction fetch: ncu showed stall_no_inst on every line)
 #pragma unroll
     for (int hi = 0; hi < 2; ++hi) {
-        const int g = kGp + 2 * hi;             // group index 0..3 within the half
+        const int g2 = 2 * gp + 4 * hi;         // twice the group index within the half
         __half2 sh[2], nh[2];                   // scale / offset of the two 16-weight sub-groups
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-            const int sidx = 2 * g + j;
-            const int sc = (int)(int8_t)((scw[sidx >> 2] >> (8 * (sidx & 3))) & 0xff);
+            const int sc = (int)(int8_t)((scw[hi] >> (16 * gp + 8 * j)) & 0xff);          // scale 2 g + j = byte 2 gp + j of word hi
             sh[j] = __float2half2_rn(dk * (float)sc);
             // q = 32 must give exactly 0: the offset is derived from the ROUNDED scale
             nh[j] = __float2half2_rn(-32.f * (fast ? __low2float(sh[j]) * (1.f / 1048576.f) : __low2float(sh[j])));
@@ -368,7 +367,7 @@ __device__ __forceinline__ void dequant_q6k_pair(const uint32_t (&ql)[8], uint32
                 // 6-bit value -> fp16 mantissa bits 4-9 (= q * 2^-20): low nibble at bits 4-7, the two qh bits at bits 8-9
                 const uint32_t l0 = hi ? ql[i] : (ql[i] << 4);                    // bytes (0,2)
                 const uint32_t l1 = hi ? (ql[i] >> 8) : (ql[i] >> 4);             // bytes (1,3)
-                const uint32_t h0 = qh[i] << (8 - 2 * g), h1 = qh[i] >> (2 * g);
+                const uint32_t h0 = qh[i] << (8 - g2), h1 = qh[i] >> g2;
                 uint32_t t0 = (l0 & 0x00f000f0u) | (h0 & 0x03000300u);
                 uint32_t t1 = (l1 & 0x00f000f0u) | (h1 & 0x03000300u);
                 const __half2 r0 = __hfma2(*reinterpret_cast<__half2*>(&t0), sh[i >> 2], nh[i >> 2]);
@@ -379,51 +378,68 @@ __device__ __forceinline__ void dequant_q6k_pair(const uint32_t (&ql)[8], uint32
         } else {
             const uint32_t magic = 0x64006400u;
             const __half2 k1024 = *reinterpret_cast<const __half2*>(&magic);
+#pragma unroll 1
+            for (int i4 = 0; i4 < 8; i4 += 4) {            // (rarely taken)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const uint32_t lw = hi ? (ql[i] >> 4) : ql[i];                      // nibbles now at bits 0-3 of every byte
-                const uint32_t hw = qh[i] >> (2 * g);                               // 2 high bits now at bits 0-1 of every byte
-                uint32_t t0 = (lw & 0x000f000fu) | ((hw << 4) & 0x00300030u) | magic;
-                uint32_t t1 = ((lw >> 8) & 0x000f000fu) | ((hw >> 4) & 0x00300030u) | magic;
-                const __half2 r0 = __hfma2(__hsub2(*reinterpret_cast<__half2*>(&t0), k1024), sh[i >> 2], nh[i >> 2]);
-                const __half2 r1 = __hfma2(__hsub2(*reinterpret_cast<__half2*>(&t1), k1024), sh[i >> 2], nh[i >> 2]);
-                v[2 * i] = *reinterpret_cast<const uint32_t*>(&r0);
-                v[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&r1);
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t qlw = i4 ? ql[4 + k] : ql[k], qhw = i4 ? qh[4 + k] : qh[k];
+                    const uint32_t lw = hi ? (qlw >> 4) : qlw;                          // nibbles now at bits 0-3 of every byte
+                    const uint32_t hw = qhw >> g2;                                      // 2 high bits now at bits 0-1 of every byte
+                    uint32_t t0 = (lw & 0x000f000fu) | ((hw << 4) & 0x00300030u) | magic;
+                    uint32_t t1 = ((lw >> 8) & 0x000f000fu) | ((hw >> 4) & 0x00300030u) | magic;
+                    const __half2 s2 = i4 ? sh[1] : sh[0], n2 = i4 ? nh[1] : nh[0];
+                    const __half2 r0 = __hfma2(__hsub2(*reinterpret_cast<__half2*>(&t0), k1024), s2, n2);
+                    const __half2 r1 = __hfma2(__hsub2(*reinterpret_cast<__half2*>(&t1), k1024), s2, n2);
+                    const uint32_t w0 = *reinterpret_cast<const uint32_t*>(&r0), w1 = *reinterpret_cast<const uint32_t*>(&r1);
+                    if (i4) { v[8 + 2 * k] = w0; v[9 + 2 * k] = w1; } else { v[2 * k] = w0; v[2 * k + 1] = w1; }
+                }
             }
         }
-        tc_st16(a_col + g * 16, v);
+        tc_st16(a_col + g2 * 8, v);
     }
 }
 
-template <int kQ>       // quarter kQ: half kHf = kQ / 2, groups (kGp, kGp + 2) with kGp = kQ % 2: 64 weights -> two 16-column TMEM stores
-struct Q6KQuarter {
-    static constexpr int kHf = kQ >> 1, kGp = kQ & 1;
-    static constexpr int kRaw = 57;
-    static __device__ __forceinline__ void load(const uint8_t* slot, int, uint32_t (&t)[kRaw]) {
+struct Q6KRun {                                 // quarter q: half q / 2, groups (q % 2, q % 2 + 2): 64 weights -> two 16-column TMEM stores
+    // raw: [0, 12) ql words 16 half + 8 (q % 2) .., [12, 24) qh words 32 + 8 half .., [24, 32) words 48 .. 55 (scales from 48 + 2 half, d at 52)
+    static constexpr int kRaw = 32;
+    static __device__ __forceinline__ void load(const uint8_t* slot, int q, uint32_t (&t)[kRaw]) {
+        const uint4* ql = reinterpret_cast<const uint4*>(slot) + 4 * (q >> 1) + 2 * (q & 1);
+        const uint4* qh = reinterpret_cast<const uint4*>(slot) + 8 + 2 * (q >> 1);
+        const uint4* sc = reinterpret_cast<const uint4*>(slot) + 12;
+        const uint4 v[8] = {ql[0], ql[1], ql[2], qh[0], qh[1], qh[2], sc[0], sc[1]};
 #pragma unroll
-        for (int c = 0; c < 14; ++c) {
-            const uint4 v = *reinterpret_cast<const uint4*>(slot + 16 * c);
-            t[4 * c] = v.x; t[4 * c + 1] = v.y; t[4 * c + 2] = v.z; t[4 * c + 3] = v.w;
-        }
-        t[56] = 0u;
+        for (int c = 0; c < 8; ++c) { t[4 * c] = v[c].x; t[4 * c + 1] = v[c].y; t[4 * c + 2] = v[c].z; t[4 * c + 3] = v[c].w; }
     }
-    static __device__ __forceinline__ void compute(const uint32_t (&t)[kRaw], int off, uint32_t a_col) {
+    static __device__ __forceinline__ void compute(const uint32_t (&t)[kRaw], int q, int off, uint32_t a_col) {
         const int wo = off >> 2, sh16 = (off & 2) * 8;
-        uint32_t dw[1], scw[2], qh[8], ql[8];
-        realign<52, 1>(t, wo, sh16, dw);                                              // d (f16) in the low half of dw[0]
-        const float d = __half2float(__ushort_as_half((unsigned short)(dw[0] & 0xffffu)));
-        realign<48 + 2 * kHf, 2>(t, wo, sh16, scw);                                   // 8 int8 scales of this half
-        realign<32 + 8 * kHf, 8>(t, wo, sh16, qh);
+        uint32_t sc4[4], qh[8], ql[8];
+        const uint32_t d01 = (wo & 1) ? t[29] : t[28], d23 = (wo & 1) ? t[31] : t[30];                 // d (f16) is one half of word 52 + wo
+        const float d = __half2float(__ushort_as_half((unsigned short)(((wo & 2) ? d23 : d01) >> sh16)));
+        realign<24, 4>(t, wo, sh16, sc4);                                             // 16 int8 scales: the half's 8 are two of the words
+        const uint32_t scw[2] = {(q >> 1) ? sc4[2] : sc4[0], (q >> 1) ? sc4[3] : sc4[1]};
+        realign<12, 8>(t, wo, sh16, qh);
         const bool fast = __all_sync(0xffffffffu, fabsf(d) * 128.f * 1048576.f <= 65504.f);   // warp-uniform (see Q4_K)
         const float dk = fast ? d * 1048576.f : d;
-        realign<16 * kHf + 8 * kGp, 8>(t, wo, sh16, ql);
-        dequant_q6k_pair<kGp>(ql, a_col + kHf * 64, qh, scw, dk, fast);
+        realign<0, 8>(t, wo, sh16, ql);
+        dequant_q6k_pair(ql, a_col + (q >> 1) * 64, qh, scw, dk, fast, q & 1);
+    }
+};
+
+// Q4_K with the quarter as a run-time value (uniform per warp): the same arithmetic as Q4KQuarter
+struct Q4KRun {
+    static constexpr int kRaw = 12;
+    static __device__ __forceinline__ void load(const uint8_t* blk, int q, uint32_t (&raw)[kRaw]) { Q4KQuarter<0>::load(blk + q * 32, blk, raw); }
+    static __device__ __forceinline__ void compute(const uint32_t (&raw)[kRaw], int q, int, uint32_t a_col) {
+        const uint32_t sel = (q & 1) ? 0x4342u : 0x4140u;            // bytes (2,3) or (0,1) of a word -> low bytes of the two halves
+        const uint32_t b0 = __byte_perm(raw[1], 0u, sel), b1 = __byte_perm(raw[2], 0u, sel), b2 = __byte_perm(raw[3], 0u, sel);
+        const bool high = q >= 2;                                    // scale_min_pair: j < 4, or j >= 4 with two bits of each from the words before
+        const uint32_t sc2 = high ? (b2 & 0x000f000fu) | ((b0 >> 2) & 0x00300030u) : b0 & 0x003f003fu;
+        const uint32_t mn2 = high ? ((b2 >> 4) & 0x000f000fu) | ((b1 >> 2) & 0x00300030u) : b1 & 0x003f003fu;
+        Q4KQuarter<0>::finish(raw, sc2, mn2, a_col + q * 32);
     }
 };
 
 template <int kType, int kQ> struct QuarterOf;
-template <int kQ> struct QuarterOf<B200_GGML_Q4_K, kQ> { using type = Q4KQuarter<kQ>; };
-template <int kQ> struct QuarterOf<B200_GGML_Q6_K, kQ> { using type = Q6KQuarter<kQ>; };
 template <int kQ> struct QuarterOf<kTypeM4, kQ> { using type = M4Quarter<kQ>; };
 template <int kQ> struct QuarterOf<kTypeF8, kQ> { using type = F8Quarter<kQ>; };
 template <int kQ> struct QuarterOf<kTypeNV4, kQ> { using type = F4Quarter<kQ, false>; };
@@ -456,12 +472,31 @@ __device__ __forceinline__ void dequant_unit(const uint8_t* blk, int off, uint32
     if (lane == 0) mbar_arrive(a_ready_bar);
 }
 
+// GGML blocks: the quarter at run time, so that all sixteen warps run ONE body.  As four copies, one per quarter, the hot code competed for the instruction cache.
+// [Q6_K MLP of 4096 x 14336, four copies and fourteen loads against one and eight: 168 -> 128 us at 203 rows, 106 -> 82 at 32, 471 -> 360 at 600; four copies with eight
+// loads: 170, 106, 475.  Q4_K (its copies did fit): 62 -> 62 us at 32 rows.]
+template <typename Q>
+__device__ __forceinline__ void dequant_run(const uint8_t* blk, int q, int off, uint32_t a_col, uint32_t w_empty_bar, uint32_t a_free_bar, uint32_t a_free_parity,
+                                            uint32_t a_ready_bar, int lane, bool skip) {
+    uint32_t raw[Q::kRaw];
+    Q::load(blk, q, raw);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // (see dequant_unit)
+    __syncwarp();
+    if (lane == 0) mbar_arrive(w_empty_bar);
+    mbar_wait(a_free_bar, a_free_parity);
+    tc_fence_after();
+    if (!skip) Q::compute(raw, q, off, a_col);
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(a_ready_bar);
+}
+
 // the same for int4 with ONE scale and zero point for the quarter
-template <int kQ>
-__device__ __forceinline__ void m4_unit(const uint8_t* blk, int r7, uint32_t a_col, uint32_t w_empty_bar, uint32_t a_free_bar, uint32_t a_free_parity,
+__device__ __forceinline__ void m4_unit(const uint8_t* blk, int q, int r7, uint32_t a_col, uint32_t w_empty_bar, uint32_t a_free_bar, uint32_t a_free_parity,
                                         uint32_t a_ready_bar, int lane, float sc, float z) {
-    uint32_t raw[M4Quarter<kQ>::kRaw];
-    M4Quarter<kQ>::load(blk, r7, raw);
+    const uint4 qa = *reinterpret_cast<const uint4*>(blk + (((2 * q) ^ r7) << 4)), qb = *reinterpret_cast<const uint4*>(blk + (((2 * q + 1) ^ r7) << 4));
+    const uint32_t raw[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if (lane == 0) mbar_arrive(w_empty_bar);
@@ -494,7 +529,7 @@ __device__ __forceinline__ void m4_unit(const uint8_t* blk, int r7, uint32_t a_c
     }
     mbar_wait(a_free_bar, a_free_parity);
     tc_fence_after();
-    tc_st32(a_col + kQ * 32, v);
+    tc_st32(a_col + q * 32, v);
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     tc_fence_before();
     __syncwarp();
@@ -789,12 +824,7 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                         const uint32_t a_col = tmem + kColA + ab * 128 + lane_addr;
                         const float sc = p.scale_bf16 ? __uint_as_float(bits << 16) : __half2float(__ushort_as_half((unsigned short)bits));
                         const float z = zp_any ? (float)((word >> one_nib) & 0xFu) : 8.f;
-                        switch (qt) {
-                            case 0: m4_unit<0>(blk, row & 7, a_col, w_empty(ws), a_free(ab), aph ^ 1, a_ready(ab), lane, sc, z); break;
-                            case 1: m4_unit<1>(blk, row & 7, a_col, w_empty(ws), a_free(ab), aph ^ 1, a_ready(ab), lane, sc, z); break;
-                            case 2: m4_unit<2>(blk, row & 7, a_col, w_empty(ws), a_free(ab), aph ^ 1, a_ready(ab), lane, sc, z); break;
-                            default: m4_unit<3>(blk, row & 7, a_col, w_empty(ws), a_free(ab), aph ^ 1, a_ready(ab), lane, sc, z); break;
-                        }
+                        m4_unit(blk, qt, row & 7, a_col, w_empty(ws), a_free(ab), aph ^ 1, a_ready(ab), lane, sc, z);
                         if (p.trace && blockIdx.x == 0 && threadIdx.x == 0 && it < 32) p.trace[it * 8 + 6] = clock64();
                         if (++ws == kW) { ws = 0; wph ^= 1; }
                         if (++ab == kABufs) { ab = 0; aph ^= 1; }
@@ -821,6 +851,9 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                                mrow, p.scale_bf16, p.debug, p.scale_by, p.scale_sk, p.norm,
                                msg == 0 ? p.zp_seg[0] : (msg == 1 ? p.zp_seg[1] : p.zp_seg[2]), {m4_cur[0], m4_cur[1], m4_cur[2], m4_cur[3]},
                                kPrefetchScales ? 1 : 0};
+                if constexpr (kType == B200_GGML_Q4_K) dequant_run<Q4KRun>(blk, qt, 0, a_col, w_empty(ws), a_free(ab), afp, a_ready(ab), lane, skip);
+                else if constexpr (kType == B200_GGML_Q6_K) dequant_run<Q6KRun>(blk, qt, off, a_col, w_empty(ws), a_free(ab), afp, a_ready(ab), lane, skip);
+                else
                 switch (qt) {
                     case 0: dequant_unit<kType, 0>(blk, off, a_col, w_empty(ws), a_free(ab), afp, a_ready(ab), lane, skip, mc); break;
                     case 1: dequant_unit<kType, 1>(blk, off, a_col, w_empty(ws), a_free(ab), afp, a_ready(ab), lane, skip, mc); break;

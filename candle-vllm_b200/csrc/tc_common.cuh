@@ -169,14 +169,22 @@ __device__ __forceinline__ void scale_min_pair(uint32_t s0, uint32_t s1, uint32_
 template <int kC>        // kC = 32-byte chunk of qs: sub-blocks 2 kC (lo nibbles) and 2 kC + 1 (hi nibbles) -> TMEM columns [32 kC, 32 kC + 32)
 struct Q4KQuarter {
     static constexpr int kRaw = 12;
-    static __device__ __forceinline__ void load(const uint8_t* blk, int, uint32_t (&raw)[kRaw]) {
+    static __device__ __forceinline__ void load(const uint8_t* blk, int, uint32_t (&raw)[kRaw]) { load(blk + kC * 32, blk, raw); }
+    // at = the block's address + 32 bytes per quarter before this one
+    static __device__ __forceinline__ void load(const uint8_t* at, const uint8_t* blk, uint32_t (&raw)[kRaw]) {
         const uint4 hdr = *reinterpret_cast<const uint4*>(blk);              // d | dmin | scales[12]
-        const uint4 qa = *reinterpret_cast<const uint4*>(blk + 16 + kC * 32);
-        const uint4 qb = *reinterpret_cast<const uint4*>(blk + 32 + kC * 32);
+        const uint4 qa = *reinterpret_cast<const uint4*>(at + 16);
+        const uint4 qb = *reinterpret_cast<const uint4*>(at + 32);
         raw[0] = hdr.x; raw[1] = hdr.y; raw[2] = hdr.z; raw[3] = hdr.w;
         raw[4] = qa.x; raw[5] = qa.y; raw[6] = qa.z; raw[7] = qa.w; raw[8] = qb.x; raw[9] = qb.y; raw[10] = qb.z; raw[11] = qb.w;
     }
     static __device__ __forceinline__ void compute(const uint32_t (&raw)[kRaw], int, uint32_t a_col) {
+        uint32_t sc2, mn2;
+        scale_min_pair<kC>(raw[1], raw[2], raw[3], sc2, mn2);
+        finish(raw, sc2, mn2, a_col + kC * 32);
+    }
+    // sc2, mn2: the two 6-bit scales and mins (low and high nibbles) as (lo | hi << 16); a_col: the quarter's first TMEM column
+    static __device__ __forceinline__ void finish(const uint32_t (&raw)[kRaw], uint32_t sc2, uint32_t mn2, uint32_t a_col) {
         const __half2 dd = *reinterpret_cast<const __half2*>(&raw[0]);          // (d, dmin)
         const float d = __low2float(dd);
         // warp-uniform so that the .aligned tcgen05.st below is reached convergently
@@ -185,8 +193,6 @@ struct Q4KQuarter {
         const __half2 ndmin = __hneg2(__high2half2(dd));
         // 6-bit scales / mins of sub-blocks 2kC (low half) and 2kC+1 (high half) as exact fp16 integers via the 1024+q
         // magic; one HMUL2 each then rounds d*sc and dmin*m exactly like the fp32 product followed by a cast would
-        uint32_t sc2, mn2;
-        scale_min_pair<kC>(raw[1], raw[2], raw[3], sc2, mn2);
         const uint32_t magic1024 = 0x64006400u;
         const __half2 h1024 = *reinterpret_cast<const __half2*>(&magic1024);
         sc2 |= magic1024; mn2 |= magic1024;
@@ -227,7 +233,7 @@ struct Q4KQuarter {
                 v[16 + 2 * i + 1] = *reinterpret_cast<const uint32_t*>(&r3);
             }
         }
-        tc_st32(a_col + kC * 32, v);
+        tc_st32(a_col, v);
     }
 };
 
