@@ -130,18 +130,26 @@ void qmatmul_generic(const void* x, bool x_is_f16, const void* w, float* y, int6
     check_launch("qmatmul_generic");
 }
 
-// rows beyond one tile of 64 (prompt portions) go through the tensor-core kernel in row tiles of 128, kMaxRows at a time (its unit arithmetic is 32-bit)
-static constexpr int kMaxRows = 1024;
+// rows beyond one tile of 64 (prompt portions) go through the tensor-core kernel in row tiles of up to 256, kMaxRows at a time, or fewer where the products of tiles and
+// super-blocks would leave the kernel's 32-bit unit arithmetic (weights of more than 58 G elements)
+static constexpr int kMaxRows = 2048;
+static int rows_per_call(int n, int k) {
+    int rows = kMaxRows;
+    while (rows > 256 && (int64_t)((n + 127) / 128) * (k / 256) * (rows / 256) * sm_count() >= (int64_t)1 << 31) rows /= 2;
+    return rows;
+}
 bool qmatmul_tc_usable(int m, int n, int k, int ggml_type) { return m >= 1 && qmatmul_tc_supported(m > 64 ? 64 : m, n, k, ggml_type); }
 static bool dispatch_needs_zeroed_output(int m, int n, int k) {
-    return (m >= kMaxRows && qmatmul_tc_needs_zeroed_output(kMaxRows, n, k)) || (m % kMaxRows && qmatmul_tc_needs_zeroed_output(m % kMaxRows, n, k));
+    const int rows = rows_per_call(n, k);
+    return (m >= rows && qmatmul_tc_needs_zeroed_output(rows, n, k)) || (m % rows && qmatmul_tc_needs_zeroed_output(m % rows, n, k));
 }
 
 void qmatmul_dispatch(const void* x_f16, const void* w, float* y, int64_t ldy, int m, int n, int k,
                       int ggml_type, int accumulate, cudaStream_t st) {
     if (qmatmul_tc_usable(m, n, k, ggml_type)) {
-        for (int m0 = 0; m0 < m; m0 += kMaxRows)
-            qmatmul_tc(static_cast<const __half*>(x_f16) + (int64_t)m0 * k, w, y + (int64_t)m0 * ldy, ldy, m - m0 < kMaxRows ? m - m0 : kMaxRows, n, k, ggml_type,
+        const int rows = rows_per_call(n, k);
+        for (int m0 = 0; m0 < m; m0 += rows)
+            qmatmul_tc(static_cast<const __half*>(x_f16) + (int64_t)m0 * k, w, y + (int64_t)m0 * ldy, ldy, m - m0 < rows ? m - m0 : rows, n, k, ggml_type,
                        accumulate, st);
     } else {
         qmatmul_generic(x_f16, true, w, y, ldy, m, n, k, ggml_type, accumulate, st);
@@ -190,9 +198,14 @@ static bool qmm_check(const char* who, const void* x, const void* w, const float
 extern "C" {
 
 // Rows at or above this count take the "dequantise once + dense tensor-core GEMM" path: the 16-bit copy of W costs ~4.6 bytes of traffic per weight (0.56 read, 2
-// written, 2 read back), a row tile of 256 of the dequant-GEMM its conversion.  Feed-forward of 4096 x 14336 on this path / on the other: 512 rows 517 / 265 us (Q4_K),
-// 450 / 344 (Q6_K); 800 rows 634 / 439 (Q4_K); 1024 rows 647 / 645 (Q6_K).
-static constexpr int kDenseRows = 1024;
+// written, 2 read back), a row tile of 256 of the dequant-GEMM its conversion, which for Q6_K takes half as long again.  Feed-forward of 4096 x 14336 on this path / on
+// the other, us: 1024 rows 639 / 487 (Q4_K), 580 / 523 (Q6_K); 1400 rows 823 / 698, 755 / 750; 1600 rows 896 / 789, 825 / 851; 2048 rows 998 / 937, 934 / 988; of 2048 x
+// 6144 (Q4_K) 1024 rows 200 / 139, 2048 rows 270 / 246.  Where the dequant-GEMM has no tensor-core form (Q8_0, Q6_K with k not a multiple of 2048) the line stays low.
+static constexpr int kDenseRows = 512;
+static int dense_rows(int m, int n, int k, int ggml_type) {
+    if (!qmatmul_tc_usable(m, n, k, ggml_type)) return kDenseRows;
+    return ggml_type == B200_GGML_Q4_K ? 2049 : 1408;
+}
 
 size_t qmatmul_workspace_bytes(int32_t m, int32_t n, int32_t k) {
     size_t b = (size_t)(m > 0 ? m : 0) * (size_t)(k > 0 ? k : 0) * 2 + 256;    // fp16 copy of the activations
@@ -226,7 +239,7 @@ void qmatmul_f32(const float* x, const void* w, float* y, int32_t m, int32_t n, 
                  int32_t ggml_type, int32_t accumulate, void* workspace, size_t workspace_bytes, int64_t stream) {
     if (m == 0 || n == 0) return;
     if (!qmm_check("qmatmul_f32", x, w, y, m, n, k, ggml_type)) return;
-    if (m >= kDenseRows && !accumulate && k % 8 == 0 && ((uintptr_t)workspace & 15) == 0 && workspace &&
+    if (m >= dense_rows(m, n, k, ggml_type) && !accumulate && k % 8 == 0 && ((uintptr_t)workspace & 15) == 0 && workspace &&
         workspace_bytes >= qmatmul_workspace_bytes(m, n, k)) {
         // prefill chunk: weights -> fp16 once, activations -> fp16, dense tcgen05 GEMM with fp32 output (dense_gemm.cu)
         char* xs = static_cast<char*>(workspace);

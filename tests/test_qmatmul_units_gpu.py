@@ -7,7 +7,7 @@ import torch
 
 import candle_vllm_b200 as pkg
 from oracle import ggml_quants as G
-from tests.gpu_util import DEV
+from tests.gpu_util import DEV, rel_fro
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +38,19 @@ def test_each_weight_comes_back(t, rows, scales):
         x[torch.arange(rows), k0 + torch.arange(rows)] = 1.0
         y = mm.forward(x.to(DEV)).cpu().numpy().astype(np.float64)
         assert (np.abs(y.T - ref[:, k0:k0 + rows]) <= bound[:, k0:k0 + rows]).all()
+
+
+@pytest.mark.parametrize("t,m,k", [
+    (pkg.GgmlType.Q4_K, 1025, 2048), (pkg.GgmlType.Q4_K, 2048, 2048), (pkg.GgmlType.Q4_K, 2049, 2048),      # the last rows of the dequant-GEMM, the first of the dense one
+    (pkg.GgmlType.Q6_K, 1407, 2048), (pkg.GgmlType.Q6_K, 1408, 2048), (pkg.GgmlType.Q6_K, 512, 768),        # 768: no tensor-core form of the dequant-GEMM
+    (pkg.GgmlType.Q8_0, 511, 512), (pkg.GgmlType.Q8_0, 512, 512),
+])
+def test_rows_on_either_side_of_the_dense_path(t, m, k):
+    n = 200
+    rng = np.random.default_rng(m)
+    w = G.random_weight(rng, t, n, k)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    op = pkg.QMatMul.from_arc(pkg.QTensor.from_numpy(w, t, (n, k)))
+    ref = G.qmatmul_dequant(x, w, t, n, k)
+    y = op.forward(torch.from_numpy(x).to(DEV)).cpu().numpy()
+    assert rel_fro(y, ref) < 1e-3, rel_fro(y, ref)             # both sides: weights and activations rounded to f16 once
