@@ -135,6 +135,9 @@ class FusedMoe:
 
     def forward(self, xs: torch.Tensor, is_prefill: bool = False) -> torch.Tensor:
         T = xs.shape[0]
+        for name, t in (("router", self.gate), ("gate experts", self.ge), ("up experts", self.ue), ("down experts", self.de)):
+            if t.device != xs.device:                  # kernels of xs.device get raw pointers to all of them
+                raise BackendError(f"FusedMoe: the {name} are on {t.device}, the input on {xs.device}")
         if self._block_covers(xs, T):
             return self._block(xs.contiguous(), T)
         # router: a [T, H] x [H, E] f32 product on the plumbing library (the reference's `gate` Linear, moe.rs:1435); every expert
