@@ -7,7 +7,7 @@
 // the latent space: score(t) = (q_abs . ckv_t + q_pe . kpe_t) * sm_scale, out = sum_t softmax(score)_t ckv_t  -> [T, H, 512].
 // Every head of a sequence reads the SAME 1152 bytes per token: the op is MQA with a 576-wide key and a 512-wide value.
 //
-// Decode kernel (tensor cores, flash-decoding split over the context): a CTA of 4 warps owns (sequence, chunk of <= 256 tokens,
+// Decode kernel (tensor cores, flash-decoding split over the context): a CTA of 4 warps owns (sequence, chunk of 256 tokens or more,
 // group of 16 heads).  32-token latent tiles land by TMA (nine {64 dims, 32 tokens} boxes, 128-byte swizzle, 3 stages of 36 KB); the
 // 16 heads are the M rows of mma.sync m16n8k16.  Per tile: warp w computes S for tokens [8w, 8w+8) over all 576 dims (Q fragments in
 // registers), the warps agree on the running row maxima through shared memory, P goes to shared memory as 16-bit,
@@ -106,22 +106,31 @@ struct MlaParams {
     int num_seqs, places;                      // places: CTAs that run at the same time
 };
 
-// Tokens per chunk of this launch, the same for every CTA and for the merge: whole tiles, at least kChunkTok (what the workspace is sized for), and for few sequences as
-// many as let all chunks run at once, two CTAs per SM -- 32 sequences of 3000 to 4096 tokens are 460 chunks of 256 on 296 places, a second round for half of them.
+// Tokens per chunk of a launch, from the sum and the longest of its contexts (`places` CTAs run at the same time): kChunkTok, what the workspace is sized for, or longer,
+// whole tiles, where that lets all chunks run at once -- 32 sequences of 3000 to 4096 tokens are 460 chunks of 256 on 296 places, a second round for half of them.  Not
+// where one round cannot be had (more sequences times head groups than places), and not where the longest chunk would then take 1.4 times the even share of a place: a
+// few long contexts among many short ones are better cut small.
+__host__ __device__ inline int mla_chunk_rule(int64_t tokens, int longest, int num_seqs, int head_groups, int places) {
+    const int64_t work = tokens * head_groups;
+    if ((int64_t)num_seqs * head_groups > places || work > (int64_t)4 * places * kChunkTok) return kChunkTok;
+    // on average half a chunk per sequence is padding: places - seqs * groups / 2 whole chunks
+    const int whole = places - num_seqs * head_groups / 2;
+    const int64_t want = (work + whole - 1) / whole, longest_chunk = want < longest ? want : longest;
+    if (want <= kChunkTok || 5 * longest_chunk * places > 7 * work) return kChunkTok;
+    return (int)((want + kTl - 1) / kTl * kTl);
+}
+__host__ __device__ inline int mla_visible(int context, int window) { return window > 0 && context > window ? window + kTl : context; }
+// the same for every CTA of a launch and for the merge
 __device__ __forceinline__ int mla_chunk_tokens(const uint32_t* context_lens, int num_seqs, int head_groups, int window, int places) {
     if (num_seqs > 128) return kChunkTok;
     const int lane = threadIdx.x & 31;
-    int tokens = 0;
+    int tokens = 0, longest = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
-        if (lane + 32 * i < num_seqs) { const int c = (int)context_lens[lane + 32 * i]; tokens += window > 0 && c > window ? window + kTl : c; }
+        if (lane + 32 * i < num_seqs) { const int c = mla_visible((int)context_lens[lane + 32 * i], window); tokens += c; longest = max(longest, c); }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tokens += __shfl_xor_sync(0xffffffffu, tokens, o);
-    // on average half a chunk per sequence is padding: places - seqs * groups / 2 whole chunks
-    const int whole = places - num_seqs * head_groups / 2;
-    if (whole <= 0 || (int64_t)tokens * head_groups > (int64_t)4 * places * kChunkTok) return kChunkTok;
-    const int want = (int)(((int64_t)tokens * head_groups + whole - 1) / whole);
-    return want <= kChunkTok ? kChunkTok : (want + kTl - 1) / kTl * kTl;
+    for (int o = 16; o > 0; o >>= 1) { tokens += __shfl_xor_sync(0xffffffffu, tokens, o); longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o)); }
+    return mla_chunk_rule(tokens, longest, num_seqs, head_groups, places);
 }
 
 // first key a row sees, rounded down to a whole tile: the chunks of a windowed row are counted from there (tiles never straddle a page)
@@ -433,6 +442,16 @@ void concat_and_cache_mla(const void* ckv, const void* k_pe, void* ckv_cache, vo
 size_t mla_paged_decode_workspace_bytes(int32_t num_seqs, int32_t num_heads, int32_t max_blocks_per_seq, int32_t block_size) {
     const size_t chunks = ((size_t)max_blocks_per_seq * block_size + kChunkTok - 1) / kChunkTok;
     return (size_t)num_seqs * num_heads * chunks * (kLat * 4 + 8) + 256;
+}
+
+// tokens per chunk of the split-KV decode kernel, from context lengths in host memory
+int32_t mla_decode_chunk_tokens(const uint32_t* context_lens_host, int32_t num_seqs, int32_t num_heads, int32_t window, int32_t places) {
+    if (!context_lens_host || num_seqs < 1 || num_heads < 1 || places < 1) return 0;
+    if (num_seqs > 128) return kChunkTok;
+    int64_t tokens = 0;
+    int longest = 0;
+    for (int i = 0; i < num_seqs; ++i) { const int c = mla_visible((int)context_lens_host[i], window); tokens += c; longest = c > longest ? c : longest; }
+    return mla_chunk_rule(tokens, longest, num_seqs, ceil_div(num_heads, kHg), places);
 }
 
 // 1 when mla_paged_attention_sink would run these sizes on the split-KV tensor-core decode kernel (one row per sequence)

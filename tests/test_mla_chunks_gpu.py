@@ -18,6 +18,8 @@ pytestmark = pytest.mark.gpu
     (20, [2500, 3, 2999, 64]),                                 # a second, partly filled head group
     (128, [900, 1500, 70]),
     (16, [100 + 3 * i for i in range(130)]),                   # more sequences than the kernel adds up: 256
+    (128, [5000] + [70 + i for i in range(71)]),               # more (sequence, head group) pairs than places, one long context
+    (64, [200 + 2 * i for i in range(64)]),                    # as many as there are places, nearly
 ])
 def test_decode(dtype, heads, lens):
     gen = torch.Generator(device=DEV)
