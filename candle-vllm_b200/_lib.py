@@ -19,7 +19,7 @@ def lib_path() -> str:
 
 # every symbol include/b200_backend.h declares (checked by tests/test_abi.py against the header)
 SYMBOLS = [
-    "b200_abi_version", "b200_last_error", "b200_last_error_message", "b200_device_sm_count", "b200_device_cc",
+    "b200_abi_version", "b200_last_error", "b200_last_error_message", "b200_wait_limit_check", "b200_device_sm_count", "b200_device_cc",
     "copy_blocks_bf16", "copy_blocks_f16", "copy_blocks_f32", "copy_blocks_u8", "swap_blocks", "flashinfer_csr_to_paged", "reshape_and_cache",
     "paged_attention_decode_workspace_bytes", "paged_attention_decode", "paged_attention_prefill",
     "qmatmul_workspace_bytes", "qmatmul_f32", "qmatmul_f16act", "qmatmul_slab_count", "qmatmul_f16act_slabs", "b200_llama_peer_inbox_bytes", "b200_llama_set_peer_inboxes", "b200_llama_peer_timeouts", "b200_ipc_alloc", "b200_ipc_open", "b200_ipc_close", "b200_ipc_free",
@@ -50,7 +50,7 @@ SYMBOLS = [
 
 
 # what a library built from one source group (build.GROUPS) exports
-_COMMON = ["b200_abi_version", "b200_last_error", "b200_last_error_message", "b200_device_sm_count", "b200_device_cc", "b200_total_kernel_launches", "linear_16bit",
+_COMMON = ["b200_abi_version", "b200_last_error", "b200_last_error_message", "b200_wait_limit_check", "b200_device_sm_count", "b200_device_cc", "b200_total_kernel_launches", "linear_16bit",
            "linear_f32out", "rms_norm_ex", "gelu_tanh_mul", "embedding_scaled", "argmax_f32", "rms_norm", "cast", "embedding_positional", "layer_norm_ex",
            "gated_residual_add", "gated_add_layer_norm", "glu_packed", "group_rms_norm_gate", "head_gate", "add_rms_norm", "post_norm_add_rms_norm", "xielu_rows", "softcap_inplace", "scaled_post_norm_add",
            "group_rms_norm_gate_into", "cast_rows_bf16"]

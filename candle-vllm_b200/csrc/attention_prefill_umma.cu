@@ -49,6 +49,7 @@ struct UmmaPrefillParams {
     int tiles;                       // grid.y: upper bound of the token tiles over all sequences
     float scale_log2;                // > 0
     const float* sink;               // [H] or null
+    uint32_t* report;                // where a wait that was given up is reported
 };
 
 __device__ __forceinline__ void tma_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
@@ -160,6 +161,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
     auto o_full = [&](int i) { return bars + (5 + 2 * kRing + i) * 8; };
     volatile uint32_t* flag = reinterpret_cast<volatile uint32_t*>(smem + kSmFlag);
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + kSmTmem);
+    const GiveUp give_up{flag, p.report, kWaitPromptAttention, kWaitLimitNs};
     if (threadIdx.x == 0) {
         *flag = 0u;
         mbar_init(q_full, 1);
@@ -176,6 +178,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    int issued = 0;                                                  // key and value tiles that warp 8 has sent for
 
     if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther));
@@ -201,7 +204,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
 #pragma unroll
             for (int kv = 0; kv < 2; ++kv, ++it) {
                 const int s = it % kRing;
-                ok = ok && mbar_wait_or_flag(kv_empty(s), ((it / kRing) & 1) ^ 1, flag);
+                ok = ok && mbar_wait_or_flag(kv_empty(s), ((it / kRing) & 1) ^ 1, give_up) && !given_up(give_up);
                 if (!ok) break;
                 if (leader) {
                     const CUtensorMap* map = kv ? &vmap : &kmap;
@@ -213,18 +216,9 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
                         tma_4d(dst + h * (kTileBytes / 2) + kPg * 128, map, kv_full(s), h * 64, kvh, 0, b1);
                     }
                 }
+                issued = it + 1;
                 __syncwarp();
             }
-        }
-        // nothing may be in flight into this CTA's shared memory when it leaves: the copies of the last round are awaited by their readers, unless a wait was given up
-        if (!ok) {
-            for (int k = max(0, it - kRing); k < it; ++k)
-                for (uint32_t i = 0; i < (1u << 20); ++i) {
-                    uint32_t done;
-                    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-                                 : "=r"(done) : "r"(kv_full(k % kRing)), "r"((uint32_t)(k / kRing) & 1u) : "memory");
-                    if (done) break;
-                }
         }
     } else if (warp == 9) {
         // ============================================ MMA ===================================================================
@@ -232,7 +226,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
         const uint32_t idesc_s = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(kKt >> 3) << 17) | (8u << 24);        // M 128, N 128, both K-major
         const uint32_t idesc_o = idesc_s | (1u << 16);                                                                       // B (values) MN-major
-        bool ok = mbar_wait_or_flag(q_full, 0, flag);
+        bool ok = mbar_wait_or_flag(q_full, 0, give_up);
         auto scores = [&](int i, int stage) {
             if (leader) {
                 const uint64_t a = make_b_desc(sb + kSmQ + i * kTileBytes), b = make_b_desc(sb + kSmKv + stage * kTileBytes);
@@ -245,7 +239,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
             }
             __syncwarp();
         };
-        ok = ok && mbar_wait_or_flag(kv_full(0), 0, flag);
+        ok = ok && mbar_wait_or_flag(kv_full(0), 0, give_up);
         if (ok) {
             tc_fence_after();
 #pragma unroll
@@ -258,12 +252,12 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         for (int j = 0; j < n && ok; ++j) {
             const int vs = it % kRing, vp = (it / kRing) & 1, ks = (it + 1) % kRing, kp = ((it + 1) / kRing) & 1;
             it += 2;
-            ok = mbar_wait_or_flag(kv_full(vs), vp, flag);
-            if (ok && j + 1 < n) ok = mbar_wait_or_flag(kv_full(ks), kp, flag);
+            ok = mbar_wait_or_flag(kv_full(vs), vp, give_up);
+            if (ok && j + 1 < n) ok = mbar_wait_or_flag(kv_full(ks), kp, give_up);
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 if (!ok || j >= nk[i]) continue;
-                ok = mbar_wait_or_flag(p_ready(i), j & 1, flag);
+                ok = mbar_wait_or_flag(p_ready(i), j & 1, give_up);
                 if (!ok) continue;
                 tc_fence_after();
                 if (leader) {
@@ -303,7 +297,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         bool ok = true;
         const int nki = nk[i];
         for (int j = 0; j < nki; ++j) {
-            ok = mbar_wait_or_flag(s_full(i), j & 1, flag);
+            ok = mbar_wait_or_flag(s_full(i), j & 1, give_up);
             if (!ok) break;
             tc_fence_after();
             uint32_t s[128];
@@ -362,7 +356,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
             if (k0 + kKt > klen) {
                 // rows of V past the context hold whatever the block contains (0 * NaN would poison O): zero them before this tile's product
                 const int vi = 2 * j + 1, vs = vi % kRing;
-                ok = mbar_wait_or_flag(kv_full(vs), (vi / kRing) & 1, flag);
+                ok = mbar_wait_or_flag(kv_full(vs), (vi / kRing) & 1, give_up);
                 if (!ok) break;
                 uint8_t* v = smem + kSmKv + vs * kTileBytes;
                 const int r0 = klen - k0;                                           // >= 1: the tile holds the row's own key or an earlier one
@@ -377,7 +371,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
             __syncwarp();
             if (lane == 0) mbar_arrive(p_ready(i));
         }
-        if (nki > 0 && ok && mbar_wait_or_flag(o_full(i), 0, flag)) {
+        if (nki > 0 && ok && mbar_wait_or_flag(o_full(i), 0, give_up)) {
             tc_fence_after();
             const float l = l2.x + l2.y, inv = l > 0.f ? 1.f / l : 0.f;
             T* dst = static_cast<T*>(p.out) + ((int64_t)(q_begin + tok) * p.num_heads + head) * kHd;
@@ -402,6 +396,8 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
     }
     tc_fence_before();
     __syncthreads();
+    // nothing may be in flight into this CTA's shared memory when it leaves: every copy is awaited by its reader, unless a wait was given up
+    if (warp == 8 && *flag) { drain_loads(q_full, 1, 1); drain_loads(kv_full(0), kRing, issued); }
     if (warp == 9) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
@@ -451,7 +447,7 @@ bool paged_attention_prefill_umma(void* out, const void* q, const void* kc, cons
         const cuuint32_t box[4] = {64, 1, (cuuint32_t)kPg, 1};
         if (!make_map(&km, kc, 4, dims, strides, box, bf16) || !make_map(&vm, vc, 4, dims, strides, box, bf16)) return false;
     }
-    const UmmaPrefillParams p{out, block_tables, cu_q, cu_k, num_seqs, num_heads, num_kv_heads, max_blocks, window, chunk, hp, tiles, scale * 1.4426950408889634f, sink};
+    const UmmaPrefillParams p{out, block_tables, cu_q, cu_k, num_seqs, num_heads, num_kv_heads, max_blocks, window, chunk, hp, tiles, scale * 1.4426950408889634f, sink, wait_report_word()};
     const dim3 grid(num_heads / hp, tiles);
     if (bf16) {
         ensure_dynamic_smem(reinterpret_cast<const void*>(paged_attn_prefill_umma_kernel<__nv_bfloat16>), kSmemU);

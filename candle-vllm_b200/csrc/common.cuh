@@ -24,6 +24,10 @@ void ensure_dynamic_smem(const void* kernel, int bytes);
 // within one GPC.  Asked once per (device, size), of the first such kernel.
 int max_active_clusters(const void* kernel, int threads, int smem, int size);
 
+// device address of a host-mapped word in which a kernel that gave up a wait sets its bit (null if it cannot be had); b200_last_error reads and clears it
+enum WaitReport : uint32_t { kWaitPromptAttention = 1, kWaitPairGemm = 2, kWaitCheck = 4 };
+uint32_t* wait_report_word();
+
 #define B200_REQUIRE(cond, code, ...)                  \
     do {                                               \
         if (!(cond)) {                                 \

@@ -80,6 +80,7 @@ struct DenseParams {
     // inside the group, and tiles are walked group by group.
     const int32_t* tile_group;
     int group_rows;
+    uint32_t* report;              // two-SM kernel: where a wait that was given up is reported
 };
 
 template <typename TOut>
@@ -401,6 +402,7 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
     auto tmem_empty = [&](int b) { return bars + (2 * kS + 2 + b) * 8; };
     volatile uint32_t* flag = reinterpret_cast<volatile uint32_t*>(smem + C::kFlag);
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + C::kTmemSlot);
+    const GiveUp give_up{flag, p.report, kWaitPairGemm, kWaitLimitNs};
     if (threadIdx.x == 0) {
         *flag = 0u;
         for (int s = 0; s < kS; ++s) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
@@ -426,8 +428,9 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
         ta = band * kBand2 + (r - tb * rows);
     };
     bool ok = true;
+    int issued = 0;
+    pdl_wait();                                                           // every role: a wait's time is counted from here, not while the kernel before still runs
     if (warp == 0) {
-        pdl_wait();
         const bool leader = elect_one();
         int it = 0;
         for (int t = (int)(blockIdx.x >> 1); t < n_tiles && ok; t += step) {
@@ -435,13 +438,14 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
             tile_coords(t, ta, tb);
             for (int kb = 0; kb < nkb && ok; ++kb, ++it) {
                 const int s = it % kS;
-                ok = mbar_wait_or_flag(empty(s), ((it / kS) & 1) ^ 1, flag);
+                ok = mbar_wait_or_flag(empty(s), ((it / kS) & 1) ^ 1, give_up) && !given_up(give_up);
                 if (ok && leader) {
                     if (rank == 0) mbar_expect_tx(full(s), 2 * C::kStageBytes);
                     const uint32_t dst = smem_base + s * C::kStageBytes, bar = cluster_map(full(s), 0);
                     tma_load_2d_pair(dst, &amap, bar, kb * kBK, ta * 256 + rank * kBM);
                     tma_load_2d_pair(dst + C::kStageBytes / 2, &bmap, bar, kb * kBK, tb * 256 + rank * kBM);
                 }
+                if (ok) issued = it + 1;
                 __syncwarp();
             }
         }
@@ -453,11 +457,11 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
             int it = 0, tcount = 0;
             for (int t = (int)(blockIdx.x >> 1); t < n_tiles && ok; t += step, ++tcount) {
                 const int ab = tcount & 1;
-                ok = mbar_wait_or_flag(tmem_empty(ab), ((tcount >> 1) & 1) ^ 1, flag);
+                ok = mbar_wait_or_flag(tmem_empty(ab), ((tcount >> 1) & 1) ^ 1, give_up);
                 tc_fence_after();
                 for (int kb = 0; kb < nkb && ok; ++kb, ++it) {
                     const int s = it % kS;
-                    ok = mbar_wait_or_flag(full(s), (it / kS) & 1, flag);
+                    ok = mbar_wait_or_flag(full(s), (it / kS) & 1, give_up);
                     tc_fence_after();
                     if (ok && leader) {
                         const uint64_t ad = make_b_desc(smem_base + s * C::kStageBytes), bd = make_b_desc(smem_base + s * C::kStageBytes + C::kStageBytes / 2);
@@ -477,12 +481,11 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
         const uint32_t lane_addr = (uint32_t)(qd * 32) << 16;
         const TOut* bias = static_cast<const TOut*>(p.bias);
         int tcount = 0;
-        pdl_wait();
         for (int t = (int)(blockIdx.x >> 1); t < n_tiles && ok; t += step, ++tcount) {
             int ta, tb;
             tile_coords(t, ta, tb);
             const int ab = tcount & 1;
-            ok = mbar_wait_or_flag(tmem_full(ab), (tcount >> 1) & 1, flag);
+            ok = mbar_wait_or_flag(tmem_full(ab), (tcount >> 1) & 1, give_up);
             if (!ok) break;
             tc_fence_after();
             const int ia = ta * 256 + rank * kBM + r;
@@ -508,6 +511,9 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
         }
     }
     tc_fence_before();
+    __syncthreads();
+    // a wait was given up: the leader, whose barriers the loads of both CTAs signal, waits for the loads in flight before either CTA leaves
+    if (rank == 0 && warp == 0 && *flag) drain_loads(full(0), kS, issued);
     __syncwarp();
     cluster_sync();                                                       // the pair's MMAs, arrivals and reads of the other CTA's shared memory are over
     if (warp == 1) {
@@ -643,7 +649,7 @@ bool dense_gemm_16(const void* x, const void* w, const void* bias, void* y, int 
         }
         const int64_t pair_tiles = (int64_t)((m + 255) / 256) * ((n + 255) / 256), pairs = sm_count() / 2;
         if (!accumulate && (pair_tiles + pairs - 1) / pairs * (nkb * 512 + 2000) <= best) {
-            p.swap = 0; p.tiles_a = (m + 255) / 256; p.tiles_b = (n + 255) / 256;
+            p.swap = 0; p.tiles_a = (m + 255) / 256; p.tiles_b = (n + 255) / 256; p.report = wait_report_word();
             if (!make_map(&am, x, m, k, ldx, kBM, bf16) || !make_map(&bm, w, n, k, ldw, kBM, bf16)) return false;
             if (out_dtype == B200_F32) launch_pair<float>(am, bm, p, st);
             else if (out_dtype == B200_BF16) launch_pair<__nv_bfloat16>(am, bm, p, st);

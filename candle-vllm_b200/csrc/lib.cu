@@ -9,6 +9,7 @@
 #include <utility>
 
 #include "common.cuh"
+#include "tc_common.cuh"
 
 namespace b200 {
 
@@ -89,6 +90,44 @@ int max_active_clusters(const void* kernel, int threads, int smem, int size) {
     return n < 0 ? 0 : n;
 }
 
+// One word for all devices: portable pinned memory has the same address on each.  Asked for by the first launch of a kernel with bounded waits, possibly during a stream
+// capture, where allocations are refused unless the thread says that it knows.
+static std::atomic<uint32_t*> g_wait_word{nullptr};
+uint32_t* wait_report_word() {
+    uint32_t* w = g_wait_word.load(std::memory_order_acquire);
+    if (w) return w;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    w = g_wait_word.load(std::memory_order_acquire);
+    if (w) return w;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    void *host = nullptr, *dev = nullptr;
+    if (cudaHostAlloc(&host, sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess && cudaHostGetDevicePointer(&dev, host, 0) == cudaSuccess && dev == host) {
+        *static_cast<volatile uint32_t*>(host) = 0u;
+        w = static_cast<uint32_t*>(host);
+        g_wait_word.store(w, std::memory_order_release);
+    } else {
+        cudaGetLastError();
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return w;
+}
+
+// a kernel with a bounded wait on a barrier that nothing arrives at
+__global__ void wait_limit_kernel(uint32_t* report, unsigned long long limit_ns) {
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t flag;
+    const uint32_t b = tc::smem_u32(&bar);
+    if (threadIdx.x == 0) {
+        flag = 0u;
+        tc::mbar_init(b, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    tc::mbar_wait_or_flag(b, 0, tc::GiveUp{&flag, report, kWaitCheck, limit_ns});
+}
+
 }  // namespace b200
 
 extern "C" {
@@ -97,8 +136,26 @@ int b200_abi_version(void) { return 1; }
 
 int b200_last_error(void) {
     int e = b200::t_err;
+    uint32_t* const word = e ? nullptr : b200::g_wait_word.load(std::memory_order_acquire);
+    if (word && *static_cast<volatile uint32_t*>(word)) {
+        const uint32_t w = __atomic_exchange_n(word, 0u, __ATOMIC_ACQ_REL);
+        if (w) {
+            b200::set_error(b200::kErrCuda, "a kernel of an earlier call gave up a wait and left its output unwritten:%s%s%s", w & b200::kWaitPromptAttention ? " prompt attention" : "",
+                            w & b200::kWaitPairGemm ? " two-SM GEMM" : "", w & b200::kWaitCheck ? " wait limit check" : "");
+            e = b200::t_err;
+        }
+    }
     b200::t_err = 0;
     return e;
+}
+
+void b200_wait_limit_check(int32_t limit_us, int64_t stream) {
+    B200_REQUIRE(limit_us > 0 && limit_us <= 1000000, b200::kErrBadArg, "b200_wait_limit_check: %d us", limit_us);
+    uint32_t* const word = b200::wait_report_word();
+    B200_REQUIRE(word, b200::kErrCuda, "b200_wait_limit_check: no host-mapped memory");
+    b200::wait_limit_kernel<<<1, 32, 0, b200::as_stream(stream)>>>(word, (unsigned long long)limit_us * 1000ull);
+    b200::count_launch();
+    b200::check_launch("b200_wait_limit_check");
 }
 
 const char* b200_last_error_message(void) { return b200::t_msg; }

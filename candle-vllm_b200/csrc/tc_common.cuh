@@ -45,21 +45,48 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
         "}\n" ::"r"(bar), "r"(parity)
         : "memory");
 }
-// Bounded wait: a wait that does not end (it always does unless a copy or an MMA was lost) gives up after two seconds, raises the CTA's flag and lets every role leave.
-__device__ __forceinline__ bool mbar_wait_or_flag(uint32_t bar, uint32_t parity, volatile uint32_t* flag) {
-    unsigned long long t0 = 0;
-    for (uint32_t i = 0;; ++i) {
-        uint32_t ok;
-        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-        if (ok) return true;
+// Bounded waits.  A wait that does not end (it always does unless a copy or an MMA was lost) gives up after `limit_ns` of waiting; it raises the CTA's flag, so that every role
+// leaves, and its bit of the host's word, which the library's error check reads.  Time in which the CTA did not run (another process's turn on the GPU) hardly counts: an
+// interval between two looks at the clock counts 1 ms at most.
+struct GiveUp {
+    volatile uint32_t* flag;        // shared memory, 0 at first
+    uint32_t* report;               // host-mapped word (wait_report_word), may be null
+    uint32_t what;                  // this kernel's bit in it
+    unsigned long long limit_ns;
+};
+constexpr unsigned long long kWaitLimitNs = 2000000000ull;
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// all lanes of a warp; the answer is the same for all of them
+__device__ __forceinline__ bool mbar_wait_or_flag(uint32_t bar, uint32_t parity, const GiveUp& g) {
+    unsigned long long last = 0, waited = 0;
+    bool ok = true;
+    for (uint32_t i = 0; !mbar_try(bar, parity); ++i) {
         if ((i & 63u) == 63u) {
             unsigned long long t;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-            if (t0 == 0) t0 = t;
-            if (*flag) return false;
-            if (t - t0 > 2000000000ull) { *flag = 1u; return false; }
+            if (last) waited += t - last < 1000000ull ? t - last : 1000000ull;
+            last = t;
+            if (*g.flag) { ok = false; break; }
+            if (waited > g.limit_ns) {
+                *g.flag = 1u;
+                if (g.report) { atomicOr_system(g.report, g.what); __threadfence_system(); }
+                ok = false;
+                break;
+            }
         }
     }
+    return __all_sync(0xffffffffu, ok);
+}
+__device__ __forceinline__ bool given_up(const GiveUp& g) { return __any_sync(0xffffffffu, *g.flag != 0u); }
+// Copies on their way into this CTA's shared memory are waited for before it leaves: barriers full0 + 8 (k % ring) of the last `ring` of `issued` loads, for about a second
+// in all.  (After a wait was given up only: otherwise their readers have waited.)
+__device__ __forceinline__ void drain_loads(uint32_t full0, int ring, int issued) {
+    for (int k = issued > ring ? issued - ring : 0; k < issued; ++k)
+        for (uint32_t i = 0; i < (1u << 18) && !mbar_try(full0 + (uint32_t)(k % ring) * 8, (uint32_t)(k / ring) & 1u); ++i) __nanosleep(500);
 }
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");

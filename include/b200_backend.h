@@ -31,6 +31,9 @@ int         b200_abi_version(void);
 /* 0 = ok.  Last argument/launch error recorded on THIS thread; reading clears it. */
 int         b200_last_error(void);
 const char* b200_last_error_message(void);
+/* Kernels with bounded waits (prompt attention, the two-SM GEMM) that give one up leave their output unwritten and report it through b200_last_error() of a later
+ * call, of any thread, once.  b200_wait_limit_check launches a kernel whose wait of limit_us microseconds (up to 1000000) runs out: the report, to see that it arrives. */
+void        b200_wait_limit_check(int32_t limit_us, int64_t stream);
 /* SM count / compute capability of the current device (0 if no usable device). */
 int         b200_device_sm_count(void);
 int         b200_device_cc(void);

@@ -1,0 +1,40 @@
+"""A bounded wait that runs out is reported: by the error check of a later call, once, whatever the thread."""
+import ctypes as C
+import threading
+
+import pytest
+import torch
+
+import candle_vllm_b200 as pkg
+from candle_vllm_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def test_a_wait_that_runs_out_is_reported_once():
+    L = pkg.lib()
+    L.b200_wait_limit_check(C.c_int32(2000), C.c_int64(torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    with pytest.raises(pkg.BackendError, match="gave up a wait"):
+        _lib.check("any call")
+    _lib.check("the next one")
+    x = torch.ones(4, 256, device="cuda")
+    assert torch.isfinite(pkg.silu_mul(x, x)).all()           # the context is usable
+
+
+def test_another_thread_sees_it():
+    L = pkg.lib()
+    L.b200_wait_limit_check(C.c_int32(500), C.c_int64(torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    codes = []
+    t = threading.Thread(target=lambda: codes.append(L.b200_last_error()))
+    t.start()
+    t.join()
+    assert codes[0] != 0 and L.b200_last_error() == 0
+
+
+def test_limits_are_checked():
+    L = pkg.lib()
+    for us in (0, -1, 1000001):
+        L.b200_wait_limit_check(C.c_int32(us), C.c_int64(0))
+        assert L.b200_last_error() == 1
