@@ -72,14 +72,14 @@ struct DenseParams {
     int out_dtype, bf16;
     int ksplit;                    // swap mode, f32 output: the k range is cut into ksplit parts per tile (more CTAs than weight tiles); partial
     int accumulate;                // sums meet in y through fp32 atomics.  accumulate: y += result (f32 output)
-    int csplit;                    // > 1: a cluster of csplit CTAs shares one tile, each over its part of k; the sums meet in shared memory of the cluster and every CTA
-                                   // adds up and stores its share of the columns, in a fixed order
     // grouped form: the weight operand is a stack of `groups` matrices of group_rows rows each, and tile_group[i] (device, written by an
     // earlier kernel) names the one that activation tile i multiplies; a negative entry marks a tile without rows.  Not swapped: activation
     // tiles are the 128-row tiles ta.  Swapped (few rows per group): activation tiles are the BN-row tiles tb, the weight tile ta is counted
     // inside the group, and tiles are walked group by group.
     const int32_t* tile_group;
     int group_rows;
+    int csplit;                    // cluster instances: csplit CTAs share one tile, each over its part of k; the sums meet in shared memory of the cluster and every CTA adds
+                                   // up and stores its share of the columns, in a fixed order
     uint32_t* report;              // two-SM kernel: where a wait that was given up is reported
 };
 
@@ -101,7 +101,9 @@ __device__ __forceinline__ void store_row16(TOut* dst, const uint32_t* acc, cons
     }
 }
 
-template <int kBN, typename TOut>
+// kCluster: tiles shared over k by clusters, in instances of their own: with the branch at run time, or its values in common variables, the others were slower [decode step
+// with 16-bit weights, 8 layers of 8B sizes, 2 / 9 / 32 rows, us a layer: 120.2 / 124.2 / 136.4, before the cluster split 119.4 / 123.0 / 135.4]
+template <int kBN, typename TOut, bool kCluster>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap, const DenseParams p) {
     using C = DCfg<kBN>;
@@ -137,11 +139,14 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
     // tile order: bands of 8 A-tiles; inside a band the B-tile index is the slow one, so the CTAs running together (consecutive tile
     // ids) work on the same B tile (weights, or activations when swapped) and neighbouring A tiles -> both stay in L2
     // split-K (swap mode only): tile id = (weight tile, k part); part z owns k blocks [nkb_all * z / ksplit, nkb_all * (z + 1) / ksplit)
-    const int crank = p.csplit > 1 ? (int)blockIdx.x % p.csplit : 0;
-    const int t_first = p.csplit > 1 ? (int)blockIdx.x / p.csplit : (int)blockIdx.x, t_step = p.csplit > 1 ? n_tiles : (int)gridDim.x;
     auto k_range = [&](int t, int& kb0, int& kb1) {
-        const int z = p.csplit > 1 ? crank : p.ksplit > 1 ? t % p.ksplit : 0, parts = p.csplit > 1 ? p.csplit : p.ksplit;
-        kb0 = nkb_all * z / parts; kb1 = nkb_all * (z + 1) / parts;
+        if constexpr (kCluster) {
+            const int z = (int)blockIdx.x % p.csplit;
+            kb0 = nkb_all * z / p.csplit; kb1 = nkb_all * (z + 1) / p.csplit;
+        } else {
+            const int z = p.ksplit > 1 ? t % p.ksplit : 0;
+            kb0 = nkb_all * z / p.ksplit; kb1 = nkb_all * (z + 1) / p.ksplit;
+        }
     };
     auto tile_coords = [&](int t, int& ta, int& tb) {
         if (p.ksplit > 1) { ta = t / p.ksplit; tb = 0; return; }
@@ -161,7 +166,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
         uint64_t pol;
         asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
         int it = 0;
-        for (int t = t_first; t < n_tiles; t += t_step) {
+        for (int t = kCluster ? blockIdx.x / p.csplit : blockIdx.x; t < n_tiles; t += kCluster ? n_tiles : gridDim.x) {
             int ta, tb, kb0, kb1;
             tile_coords(t, ta, tb);
             k_range(t, kb0, kb1);
@@ -190,7 +195,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
         const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(kBN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
         int it = 0, tcount = 0;                                          // tcount: tiles done (skipped tiles of the grouped form do not count)
         if (p.tile_group) pdl_wait();
-        for (int t = t_first; t < n_tiles; t += t_step) {
+        for (int t = kCluster ? blockIdx.x / p.csplit : blockIdx.x; t < n_tiles; t += kCluster ? n_tiles : gridDim.x) {
             if (p.tile_group) {
                 int ta, tb;
                 tile_coords(t, ta, tb);
@@ -229,7 +234,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
         int tcount = 0;
         bool waited = false;
         if (p.tile_group) { pdl_wait(); waited = true; }
-        for (int t = t_first; t < n_tiles; t += t_step) {
+        for (int t = kCluster ? blockIdx.x / p.csplit : blockIdx.x; t < n_tiles; t += kCluster ? n_tiles : gridDim.x) {
             int ta, tb;
             tile_coords(t, ta, tb);
             if (p.tile_group && p.tile_group[p.swap ? tb : ta] < 0) continue;
@@ -237,7 +242,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
             mbar_wait(tmem_full(ab), (tcount >> 1) & 1);
             tc_fence_after();
             if (!waited) { pdl_wait(); waited = true; }
-            if (p.csplit > 1) {
+            if constexpr (kCluster) {
                 // partial sums -> [4 columns][128 rows][4] over the drained ring (every load of this CTA has been consumed)
                 float4* part = reinterpret_cast<float4*>(smem);
 #pragma unroll 1
@@ -302,12 +307,13 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
         }
     }
 
-    if (p.csplit > 1) {
+    if constexpr (kCluster) {
         __syncwarp();
         cluster_sync();                                                   // every CTA's sums are written
         if (warp >= 2) {
+            const int crank = (int)blockIdx.x % p.csplit;
             int ta, tb;
-            tile_coords(t_first, ta, tb);
+            tile_coords((int)blockIdx.x / p.csplit, ta, tb);
             const int r = (warp & 3) * 32 + lane, ia = ta * kBM + r;
             const TOut* bias = static_cast<const TOut*>(p.bias);
             // eight columns at a time, two CTAs' loads in flight together
@@ -566,7 +572,7 @@ void launch_cluster(K kern, int grid, int cluster, size_t smem, cudaStream_t st,
 
 template <int kBN, typename TOut>
 void launch_dense(const CUtensorMap& am, const CUtensorMap& bm, const DenseParams& p, cudaStream_t st) {
-    auto kern = dense_gemm_kernel<kBN, TOut>;
+    auto kern = p.csplit > 1 ? dense_gemm_kernel<kBN, TOut, true> : dense_gemm_kernel<kBN, TOut, false>;
     ensure_dynamic_smem(reinterpret_cast<const void*>(kern), DCfg<kBN>::kTotal);
     const int tiles = p.tiles_a * p.tiles_b * p.ksplit;
     const int grid = tiles < sm_count() ? tiles : sm_count();
@@ -596,7 +602,7 @@ void launch_out(const CUtensorMap& am, const CUtensorMap& bm, const DenseParams&
 int cluster_split(int64_t tiles, int nkb) {
     for (int s = 8; s > 1; --s)
         if (tiles * s <= sm_count() && s <= nkb / 4 &&
-            tiles <= max_active_clusters(reinterpret_cast<const void*>(dense_gemm_kernel<128, __nv_bfloat16>), kGemmThreads, DCfg<128>::kTotal, s)) return s;
+            tiles <= max_active_clusters(reinterpret_cast<const void*>(dense_gemm_kernel<128, __nv_bfloat16, true>), kGemmThreads, DCfg<128>::kTotal, s)) return s;
     return 1;
 }
 
