@@ -8,6 +8,9 @@
 //                   2^8 since the last time (a stale maximum scales numerator and denominator alike; P <= 2^8 keeps its relative precision in 16 bits)
 //   warp 8          TMA: Q once (64 KB), then K and V tiles of 32 KB through a ring of five
 //   warp 9          MMA issue: S_i = Q_i K^T (128 x 128 x 128, both operands in shared memory), O_i += P_i V (P from TMEM, V token rows as the MN-major operand)
+//   warps 10, 11    value tiles in which some row of the CTA has hidden keys (the diagonal, a window's or a chunk's edge, past the context): the MMA multiplies all 128 values by
+//                   a weight, 0 where the key is hidden, and 0 * inf = NaN.  They zero what lies past the context and every infinity and NaN, and say whether there was one;
+//                   the softmax warps then add those values to the rows that do see them, one by one (add_nonfinite)
 // The two tiles alternate on the tensor pipe: while one tile's softmax runs, the other tile's O += P V and next S are computed.
 // TMEM: S_0, S_1 (P_i over the first half of S_i), O_0, O_1, 128 columns each = all 512.
 // Order on the tensor pipe is the only thing that protects P_i from the next S_i (same issuing thread, in order); the barrier of S_i(j) also says that
@@ -36,13 +39,14 @@ static_assert(256 * kRegsSoftmax + 128 * kRegsOther <= kThreadsU * 168, "registe
 constexpr int kTileBytes = 128 * kHd * 2;               // a Q, K or V tile: two halves of 64 dims, 128 rows of 128 bytes each
 constexpr int kRing = 5;
 constexpr int kSmQ = 0, kSmKv = 2 * kTileBytes, kSmBar = kSmKv + kRing * kTileBytes;
-constexpr int kNumBars = 1 + 2 * kRing + 6;             // q_full, kv_full[], kv_empty[], s_full[2], p_ready[2], o_full[2]
-constexpr int kSmFlag = kSmBar + kNumBars * 8, kSmTmem = kSmFlag + 4;
-constexpr int kSmemU = kSmTmem + 12;
+constexpr int kNumBars = 1 + 2 * kRing + 8;             // q_full, kv_full[], kv_empty[], s_full[2], p_ready[2], o_full[2], scan_go, v_clean
+constexpr int kSmFlag = kSmBar + kNumBars * 8, kSmTmem = kSmFlag + 4, kSmDirty = kSmTmem + 4, kSmOInit = kSmDirty + 8;
+constexpr int kSmemU = kSmOInit + 8;
 static_assert(kSmemU <= 232448, "shared memory");
 
 struct UmmaPrefillParams {
     void* out;
+    const void* values;              // the value cache once more, for add_nonfinite
     const uint32_t* block_tables; const uint32_t* cu_q; const uint32_t* cu_k;
     int num_seqs, num_heads, num_kv_heads, max_blocks, window, chunk;
     int hp;                          // heads per tile (power of two, divides the heads of a kv head)
@@ -110,6 +114,42 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
     return d;
 }
 
+// 16-bit values: the bits of an infinity's exponent, and whether one of the two in a word is an infinity or NaN (the addition carries out of a full exponent into bit 15)
+template <typename T> struct Exponent { static constexpr uint32_t kMask = std::is_same<T, __nv_bfloat16>::value ? 0x7f807f80u : 0x7c007c00u, kOne = std::is_same<T, __nv_bfloat16>::value ? 0x00800080u : 0x04000400u; };
+template <typename T> __device__ __forceinline__ uint32_t nonfinite(uint32_t w) { return ((w & Exponent<T>::kMask) + Exponent<T>::kOne) & 0x80008000u; }
+template <typename T> __device__ __forceinline__ float half_to_f32(uint32_t h);
+template <> __device__ __forceinline__ float half_to_f32<__nv_bfloat16>(uint32_t h) { return __uint_as_float(h << 16); }
+template <> __device__ __forceinline__ float half_to_f32<__half>(uint32_t h) { return __half2float(__ushort_as_half((unsigned short)h)); }
+__device__ __forceinline__ uint32_t ld1(uint32_t taddr) {
+    uint32_t v;
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\ntcgen05.wait::ld.sync.aligned;" : "=r"(v) : "r"(taddr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st1(uint32_t taddr, uint32_t v) { asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};\ntcgen05.wait::st.sync.aligned;" ::"r"(taddr), "r"(v) : "memory"); }
+
+// A tile's infinities and NaNs, which its value tile no longer holds: O[row][d] += P[row][key] V[key][d] for the rows that see the key.  One warp, its 32 rows; key tile
+// k0, keys [c_lo, c_hi] of it are looked at, the thread's row sees [lo_c, hi_c].  The values come from the cache again (rare: nobody is in a hurry).
+template <typename T>
+__device__ __forceinline__ void add_nonfinite(const T* values, const uint32_t* table, int kvh, int num_kv_heads, int k0, int c_lo, int c_hi, int lo_c, int hi_c, uint32_t s_t, uint32_t o_t) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (int c = c_lo; c <= c_hi; ++c) {
+        const int key = k0 + c;
+        const uint2 raw = *reinterpret_cast<const uint2*>(values + (((int64_t)table[key / kPg] * kPg + key % kPg) * num_kv_heads + kvh) * kHd + lane * 4);
+#pragma unroll 1
+        for (int e = 0; e < 4; ++e) {
+            const uint32_t h = ((e & 2 ? raw.y : raw.x) >> ((e & 1) * 16)) & 0xffffu;
+            for (uint32_t hits = __ballot_sync(0xffffffffu, nonfinite<T>(h) != 0u); hits; hits &= hits - 1u) {
+                const int l = __ffs(hits) - 1, d = 4 * l + e;
+                const float v = half_to_f32<T>(__shfl_sync(0xffffffffu, h, l));
+                const float p = half_to_f32<T>((ld1(s_t + (c >> 1)) >> ((c & 1) * 16)) & 0xffffu);
+                const float o = __uint_as_float(ld1(o_t + d));
+                st1(o_t + d, __float_as_uint(c >= lo_c && c <= hi_c ? fmaf(p, v, o) : o));
+            }
+        }
+    }
+}
+
 // A row's O is rescaled when its maximum has grown by more than kSlack (log2 units) -- in the first key tiles whenever it has grown at all: there single weights are large,
 // and the largest one, 1 when the maximum is up to date, is then the one weight that 16 bits hold exactly.  [Error of the whole result against 64 bits, 8192 tokens:
 // 2.121e-3 with the slack everywhere, 2.088e-3 so, 2.078e-3 without slack; 532, 547, 588 us.]
@@ -151,6 +191,11 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         nk[i] = toks > 0 ? (pos0 + i * tp + toks - 1 - kt0) / kKt + 1 : 0;
     }
     const int n = max(nk[0], nk[1]);
+    // tiles in which a row of the CTA has hidden keys: past the first row's position, or before the last row's first key
+    const int pos_last = pos0 + min(2 * tp, qlen - q0) - 1;
+    int last_lo = p.window > 0 ? max(0, pos_last - p.window + 1) : 0;
+    if (p.chunk > 0) last_lo = max(last_lo, (pos_last / p.chunk) * p.chunk);
+    auto hides = [&](int j) { return kt0 + j * kKt + kKt - 1 > pos0 || kt0 + j * kKt < last_lo; };
 
     const uint32_t bars = sb + kSmBar;
     const uint32_t q_full = bars;
@@ -159,6 +204,9 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
     auto s_full = [&](int i) { return bars + (1 + 2 * kRing + i) * 8; };
     auto p_ready = [&](int i) { return bars + (3 + 2 * kRing + i) * 8; };
     auto o_full = [&](int i) { return bars + (5 + 2 * kRing + i) * 8; };
+    const uint32_t scan_go = bars + (7 + 2 * kRing) * 8, v_clean = scan_go + 8;              // one phase per tile that hides keys
+    volatile uint32_t* dirty = reinterpret_cast<volatile uint32_t*>(smem + kSmDirty);         // [2]: of each scanning warp
+    volatile uint32_t* o_init = reinterpret_cast<volatile uint32_t*>(smem + kSmOInit);        // [2]: O_i holds something before its first product
     volatile uint32_t* flag = reinterpret_cast<volatile uint32_t*>(smem + kSmFlag);
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + kSmTmem);
     const GiveUp give_up{flag, p.report, kWaitPromptAttention, kWaitLimitNs};
@@ -166,7 +214,9 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         *flag = 0u;
         mbar_init(q_full, 1);
         for (int s = 0; s < kRing; ++s) { mbar_init(kv_full(s), 1); mbar_init(kv_empty(s), 1); }
-        for (int i = 0; i < 2; ++i) { mbar_init(s_full(i), 1); mbar_init(p_ready(i), 4); mbar_init(o_full(i), 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(s_full(i), 1); mbar_init(p_ready(i), 4); mbar_init(o_full(i), 1); o_init[i] = 0u; }
+        mbar_init(scan_go, 1);
+        mbar_init(v_clean, 2);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -248,23 +298,28 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
             if (leader) tc_commit(kv_empty(0));
             __syncwarp();
         }
-        int it = 1;
+        int it = 1, scans = 0;
         for (int j = 0; j < n && ok; ++j) {
             const int vs = it % kRing, vp = (it / kRing) & 1, ks = (it + 1) % kRing, kp = ((it + 1) / kRing) & 1;
+            const bool scan = hides(j);
             it += 2;
             ok = mbar_wait_or_flag(kv_full(vs), vp, give_up);
+            if (ok && scan && lane == 0) mbar_arrive(scan_go);
+            __syncwarp();
             if (ok && j + 1 < n) ok = mbar_wait_or_flag(kv_full(ks), kp, give_up);
+            if (ok && scan) { ok = mbar_wait_or_flag(v_clean, scans & 1, give_up); ++scans; }
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 if (!ok || j >= nk[i]) continue;
                 ok = mbar_wait_or_flag(p_ready(i), j & 1, give_up);
                 if (!ok) continue;
                 tc_fence_after();
+                const bool add = j > 0 || o_init[i] != 0u;
                 if (leader) {
                     const uint64_t b = make_mn_desc(sb + kSmKv + vs * kTileBytes, kTileBytes / 2);
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
-                        tc_mma_ts(tmem + 256 + i * 128, tmem + i * 128 + k * 8, b + (uint64_t)(k * 16 * 128 >> 4), idesc_o, (j > 0 || k > 0) ? 1u : 0u);
+                        tc_mma_ts(tmem + 256 + i * 128, tmem + i * 128 + k * 8, b + (uint64_t)(k * 16 * 128 >> 4), idesc_o, (add || k > 0) ? 1u : 0u);
                     if (j + 1 == nk[i]) tc_commit(o_full(i));
                 }
                 __syncwarp();
@@ -274,6 +329,51 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
                 tc_commit(kv_empty(vs));
                 if (j + 1 < n) tc_commit(kv_empty(ks));
             }
+            __syncwarp();
+        }
+    } else {
+        // ============================================ VALUES THAT MUST NOT REACH HIDDEN ROWS ======================================
+        // The MMA warp says when a tile has landed (it waits for every tile in order) and waits for the answer before its products, so neither side can be a phase ahead.
+        const int w = warp - 10;
+        int scans = 0;
+        bool ok = true;
+        for (int j = 0; j < n && ok; ++j) {
+            if (!hides(j)) continue;
+            const int vi = 2 * j + 1, vs = vi % kRing;
+            ok = mbar_wait_or_flag(scan_go, scans & 1, give_up) && mbar_wait_or_flag(kv_full(vs), (vi / kRing) & 1, give_up);      // (the second one is over)
+            ++scans;
+            if (!ok) break;
+            uint8_t* const v = smem + kSmKv + vs * kTileBytes;
+            const int k0 = kt0 + j * kKt, rows = min(max(klen - k0, 0), kKt);        // rows of the tile within the context
+            // [0, behind): before the last row's first key; [ahead, rows): past the first row's position
+            const int behind = min(max(last_lo - k0, 0), rows), ahead = max(min(max(pos0 + 1 - k0, 0), rows), behind);
+            const int count = (behind + rows - ahead) * 16;
+            auto chunk = [&](int idx) {                                             // 16 bytes of a row
+                const int r = (idx >> 4) < behind ? idx >> 4 : (idx >> 4) + ahead - behind, ch = idx & 15;
+                return reinterpret_cast<uint4*>(v + (ch >> 3) * (kTileBytes / 2) + r * 128 + ((ch & 7) << 4));
+            };
+            for (int idx = rows * 16 + w * 32 + lane; idx < kKt * 16; idx += 64)
+                *reinterpret_cast<uint4*>(v + ((idx >> 3) & 1) * (kTileBytes / 2) + (idx >> 4) * 128 + ((idx & 7) << 4)) = make_uint4(0, 0, 0, 0);
+            auto bad_bits = [](uint4 x) { return nonfinite<T>(x.x) | nonfinite<T>(x.y) | nonfinite<T>(x.z) | nonfinite<T>(x.w); };
+            uint32_t bad = 0u;
+            for (int idx0 = w * 32 + lane; idx0 < count; idx0 += 8 * 64) {          // eight loads in flight
+                uint4 x[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[e] = idx0 + e * 64 < count ? *chunk(idx0 + e * 64) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) bad |= bad_bits(x[e]);
+            }
+            bad = __any_sync(0xffffffffu, bad != 0u) ? 1u : 0u;
+            if (bad) {                                                              // rare
+                auto keep = [](uint32_t u) { return u & ~((nonfinite<T>(u) >> 15) * 0xffffu); };
+#pragma unroll 1
+                for (int idx = w * 32 + lane; idx < count; idx += 64) {
+                    const uint4 x = *chunk(idx);
+                    *chunk(idx) = make_uint4(keep(x.x), keep(x.y), keep(x.z), keep(x.w));
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            if (lane == 0) { dirty[w] = bad; mbar_arrive(v_clean); }
             __syncwarp();
         }
     }
@@ -289,6 +389,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         if (p.chunk > 0) lo = max(lo, (pos / p.chunk) * p.chunk);
         const int w_first = q0 + i * tp + ((warp & 3) * 32) / p.hp, w_last = q0 + i * tp + ((warp & 3) * 32 + 31) / p.hp;     // the warp's tokens
         const int w_min_pos = klen - qlen + w_first;
+        int scans = 0;
         int w_max_lo = p.window > 0 ? max(0, klen - qlen + w_last - p.window + 1) : 0;
         if (p.chunk > 0) w_max_lo = max(w_max_lo, ((klen - qlen + w_last) / p.chunk) * p.chunk);
         const float sink = p.sink ? p.sink[head] * 1.4426950408889634f : -INFINITY;
@@ -296,16 +397,17 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         float2 l2 = make_float2(sink != -INFINITY ? 1.f : 0.f, 0.f);
         bool ok = true;
         const int nki = nk[i];
-        for (int j = 0; j < nki; ++j) {
-            ok = mbar_wait_or_flag(s_full(i), j & 1, give_up);
-            if (!ok) break;
+        // a tile without hidden keys needs no mask and no look at its values: a body of its own, so that the rare paths stay out of the hot one
+        auto step = [&](int j, auto hiding) -> bool {
+            constexpr bool kHides = decltype(hiding)::value;
+            if (!mbar_wait_or_flag(s_full(i), j & 1, give_up)) return false;
             tc_fence_after();
             uint32_t s[128];
 #pragma unroll
             for (int c = 0; c < 4; ++c) ld32(s_t + c * 32, s + c * 32);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             const int k0 = kt0 + j * kKt;
-            if (k0 + kKt - 1 > w_min_pos || k0 < w_max_lo) {
+            if (kHides && (k0 + kKt - 1 > w_min_pos || k0 < w_max_lo)) {
                 const int hi_c = pos - k0, lo_c = lo - k0;
 #pragma unroll
                 for (int c = 0; c < 128; ++c)
@@ -353,24 +455,29 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
                              "r"(pk[3]), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7])
                              : "memory");
             }
-            if (k0 + kKt > klen) {
-                // rows of V past the context hold whatever the block contains (0 * NaN would poison O): zero them before this tile's product
-                const int vi = 2 * j + 1, vs = vi % kRing;
-                ok = mbar_wait_or_flag(kv_full(vs), (vi / kRing) & 1, give_up);
-                if (!ok) break;
-                uint8_t* v = smem + kSmKv + vs * kTileBytes;
-                const int r0 = klen - k0;                                           // >= 1: the tile holds the row's own key or an earlier one
-                for (int idx = (warp & 3) * 32 + lane; idx < (kKt - r0) * 16; idx += 128) {
-                    const int r = r0 + (idx >> 4), ch = idx & 15;
-                    *reinterpret_cast<int4*>(v + (ch >> 3) * (kTileBytes / 2) + r * 128 + ((ch & 7) << 4)) = make_int4(0, 0, 0, 0);
+            if constexpr (kHides) {
+                if (!mbar_wait_or_flag(v_clean, scans & 1, give_up)) return false;
+                ++scans;
+                if (dirty[0] | dirty[1]) {                                          // (uniform over the CTA's warps)
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    if (j == 0) {
+                        const uint32_t z[16] = {};
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) tc_st16(o_t + c * 16, z);
+                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                        if (lane == 0) o_init[i] = 1u;
+                    }
+                    const int w_lo = max(first_key - k0, 0), w_hi = min(min(klen - qlen + w_last, klen - 1) - k0, kKt - 1);
+                    add_nonfinite<T>(static_cast<const T*>(p.values), p.block_tables + (int64_t)seq * p.max_blocks, kvh, p.num_kv_heads, k0, w_lo, w_hi, lo - k0, pos - k0, s_t, o_t);
                 }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(p_ready(i));
-        }
+            return true;
+        };
+        for (int j = 0; j < nki && ok; ++j) ok = hides(j) ? step(j, std::true_type{}) : step(j, std::false_type{});
         if (nki > 0 && ok && mbar_wait_or_flag(o_full(i), 0, give_up)) {
             tc_fence_after();
             const float l = l2.x + l2.y, inv = l > 0.f ? 1.f / l : 0.f;
@@ -447,7 +554,7 @@ bool paged_attention_prefill_umma(void* out, const void* q, const void* kc, cons
         const cuuint32_t box[4] = {64, 1, (cuuint32_t)kPg, 1};
         if (!make_map(&km, kc, 4, dims, strides, box, bf16) || !make_map(&vm, vc, 4, dims, strides, box, bf16)) return false;
     }
-    const UmmaPrefillParams p{out, block_tables, cu_q, cu_k, num_seqs, num_heads, num_kv_heads, max_blocks, window, chunk, hp, tiles, scale * 1.4426950408889634f, sink, wait_report_word()};
+    const UmmaPrefillParams p{out, vc, block_tables, cu_q, cu_k, num_seqs, num_heads, num_kv_heads, max_blocks, window, chunk, hp, tiles, scale * 1.4426950408889634f, sink, wait_report_word()};
     const dim3 grid(num_heads / hp, tiles);
     if (bf16) {
         ensure_dynamic_smem(reinterpret_cast<const void*>(paged_attn_prefill_umma_kernel<__nv_bfloat16>), kSmemU);

@@ -63,3 +63,52 @@ def test_tiles_heads_and_edges(dtype, H, kvh, qlens, cached, window, loud):
     assert torch.isfinite(out).all()
     err = float((out.double() - ref).norm() / ref.norm())
     assert err < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11), err
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("H,kvh,qlens,cached,window,bad", [
+    (4, 4, [200], [0], None, [(0, 1, "inf"), (0, 30, "nan"), (0, 127, "-inf"), (0, 128, "inf"), (0, 199, "nan")]),      # one head per tile: rows far before the values
+    (8, 2, [130, 40], [300, 70], None, [(0, 17, "inf"), (0, 299, "nan"), (0, 301, "inf"), (0, 420, "-inf"), (1, 69, "nan"), (1, 100, "inf")]),
+    (8, 2, [300], [500], 96, [(0, 0, "nan"), (0, 410, "inf"), (0, 480, "nan"), (0, 600, "-inf"), (0, 799, "inf")]),     # and behind a window's edge
+    (32, 8, [1, 40], [700, 0], None, [(0, 700, "inf"), (1, 39, "nan")]),
+])
+def test_values_that_are_not_finite_reach_the_rows_that_see_them_alone(dtype, H, kvh, qlens, cached, window, bad):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(H + len(bad))
+    klens = [a + b for a, b in zip(qlens, cached)]
+    tables, at = [], 0
+    for n in klens:
+        tables.append(list(range(at, at - (-n // 64))))
+        at += -(-n // 64)
+    mk = lambda *shape: torch.randn(shape, generator=g, device=DEV).to(dtype)
+    q, k, v = mk(sum(qlens), H, 128), mk(sum(qlens), kvh, 128), mk(sum(qlens), kvh, 128)
+    kc, vc = mk(at, 64, kvh, 128), mk(at, 64, kvh, 128)
+    first = np.cumsum([0] + qlens)
+    clean = vc.clone()
+    for i in range(len(qlens)):                    # what the call will write, so that the reference can start from it
+        p = torch.arange(cached[i], klens[i], device=DEV)
+        clean[torch.tensor(tables[i], device=DEV)[p // 64], p % 64] = v[first[i]:first[i + 1]]
+    spoiled = clean.clone()
+    for j, (i, pos, what) in enumerate(bad):
+        group, dim = j % kvh, (37 * j + 5) % 128
+        spoiled[tables[i][pos // 64], pos % 64, group, dim] = float(what)
+        clean[tables[i][pos // 64], pos % 64, group, dim] = 0
+    for i in range(len(qlens)):
+        p = torch.arange(cached[i], klens[i], device=DEV)
+        v[first[i]:first[i + 1]] = spoiled[torch.tensor(tables[i], device=DEV)[p // 64], p % 64]
+    prep = pkg.prepare_prompt([list(range(n)) for n in klens], tables, 64, cached, chunk_size=max(qlens))
+    _, _, meta = pkg.inputs.to_device(prep)
+    vc.copy_(spoiled)
+    out = pkg.PagedAttention(H, 128, 128 ** -0.5, kvh, sliding_window=window).forward(q, k, v, None, kc, vc, meta)
+    ref = _reference(q, kc, clean, tables, qlens, klens, 128 ** -0.5, window)
+    for j, (i, pos, what) in enumerate(bad):
+        group, dim = j % kvh, (37 * j + 5) % 128
+        rows = torch.arange(cached[i], klens[i], device=DEV)
+        sees = (rows >= pos) & ((rows < pos + window) if window else torch.ones_like(rows, dtype=torch.bool))
+        heads = slice(group * (H // kvh), (group + 1) * (H // kvh))
+        ref[first[i]:first[i + 1], heads, dim] += torch.where(sees, float(what), 0.0)[:, None]
+    finite = torch.isfinite(ref)
+    assert torch.equal(torch.isfinite(out), finite)
+    assert torch.equal(torch.isnan(out), torch.isnan(ref)) and torch.equal(out[torch.isinf(ref)].double(), ref[torch.isinf(ref)])
+    err = float((out.double() - ref)[finite].norm() / ref[finite].norm())
+    assert err < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11), err
