@@ -188,7 +188,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const int toks = min(tp, qlen - q0 - i * tp);
-        nk[i] = toks > 0 ? (pos0 + i * tp + toks - 1 - kt0) / kKt + 1 : 0;
+        nk[i] = toks > 0 ? max((pos0 + i * tp + toks - 1 - kt0) / kKt + 1, 1) : 0;      // (at least one: rows before a context that is too short see nothing and are written as 0)
     }
     const int n = max(nk[0], nk[1]);
     // tiles in which a row of the CTA has hidden keys: past the first row's position, or before the last row's first key

@@ -112,3 +112,27 @@ def test_values_that_are_not_finite_reach_the_rows_that_see_them_alone(dtype, H,
     assert torch.equal(torch.isnan(out), torch.isnan(ref)) and torch.equal(out[torch.isinf(ref)].double(), ref[torch.isinf(ref)])
     err = float((out.double() - ref)[finite].norm() / ref[finite].norm())
     assert err < (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11), err
+
+
+@pytest.mark.parametrize("H,kvh,qlens,klens", [(4, 4, [600], [100]), (8, 2, [300, 40], [20, 64]), (4, 4, [300], [300])])
+def test_rows_before_a_context_that_is_too_short_are_zero(H, kvh, qlens, klens):
+    """more rows than keys: the mask is aligned at the end, so the first rows see nothing"""
+    g = torch.Generator(device=DEV)
+    g.manual_seed(sum(qlens))
+    used = [-(-k // 64) for k in klens]
+    tables = [list(range(sum(used[:i]), sum(used[:i + 1]))) for i in range(len(used))]
+    mk = lambda *shape: torch.randn(shape, generator=g, device=DEV).to(torch.bfloat16)
+    q, kc, vc = mk(sum(qlens), H, 128), mk(sum(used), 64, kvh, 128), mk(sum(used), 64, kvh, 128)
+    k, v = mk(sum(qlens), kvh, 128), mk(sum(qlens), kvh, 128)
+    meta = pkg.InputMetadata(is_prefill=True, slot_mapping=torch.full((sum(qlens),), -1, dtype=torch.int64, device=DEV),
+                             block_tables=torch.tensor([t + [0] * (max(used) - len(t)) for t in tables], dtype=torch.int32, device=DEV), max_context_len=max(klens))
+    on = lambda a: torch.tensor(np.cumsum([0] + a), dtype=torch.int32, device=DEV)
+    meta.cu_seqlens_q, meta.cu_seqlens_k, meta.max_seqlen_q, meta.max_seqlen_k = on(qlens), on(klens), max(qlens), max(klens)
+    out = pkg.PagedAttention(H, 128, 128 ** -0.5, kvh).forward(q, k, v, None, kc, vc, meta)
+    row = 0
+    for n, c, t in zip(qlens, klens, tables):
+        blind = max(n - c, 0)
+        assert not out[row:row + blind].any()
+        ref = _reference(q[row + blind:row + n], kc, vc, [t], [n - blind], [c], 128 ** -0.5, None)
+        assert float((out[row + blind:row + n].double() - ref).norm() / ref.norm()) < 2.0 ** -8
+        row += n
