@@ -4,15 +4,15 @@
 // One CTA = 256 query rows of one kv head: two M = 128 tiles whose rows are (token, head) pairs, 128 / hp tokens x hp heads of the group, so the heads that share
 // keys share the tile and a short portion still fills its rows.  Keys and values are walked in tiles of 128 tokens (two pages).
 //   warps 0-3, 4-7  softmax of tile 0 / 1: thread = row; the row's 128 scores come from TMEM into registers, maximum and sum stay in the thread, P goes back to
-//                   TMEM as 16 bits over the scores it was made from, and the O of the row is rescaled in TMEM only when its maximum has grown by more than
-//                   2^8 since the last time (a stale maximum scales numerator and denominator alike; P <= 2^8 keeps its relative precision in 16 bits)
+//                   TMEM as 16 bits over the scores it was made from (in two parts in a row's first tile), and the O of the warp's rows is rescaled in TMEM when the maximum of
+//                   one of them has grown
 //   warp 8          TMA: Q once (64 KB), then K and V tiles of 32 KB through a ring of five
 //   warp 9          MMA issue: S_i = Q_i K^T (128 x 128 x 128, both operands in shared memory), O_i += P_i V (P from TMEM, V token rows as the MN-major operand)
 //   warps 10, 11    value tiles in which some row of the CTA has hidden keys (the diagonal, a window's or a chunk's edge, past the context): the MMA multiplies all 128 values by
 //                   a weight, 0 where the key is hidden, and 0 * inf = NaN.  They zero what lies past the context and every infinity and NaN, and say whether there was one;
 //                   the softmax warps then add those values to the rows that do see them, one by one (add_nonfinite)
 // The two tiles alternate on the tensor pipe: while one tile's softmax runs, the other tile's O += P V and next S are computed.
-// TMEM: S_0, S_1 (P_i over the first half of S_i), O_0, O_1, 128 columns each = all 512.
+// TMEM: S_0, S_1 (P_i over the first half of S_i, its second part over the other), O_0, O_1, 128 columns each = all 512.
 // Order on the tensor pipe is the only thing that protects P_i from the next S_i (same issuing thread, in order); the barrier of S_i(j) also says that
 // O_i += P_i V of step j - 1 is complete, because a commit covers every MMA issued before it.
 //
@@ -96,6 +96,11 @@ __device__ __forceinline__ void ld32(uint32_t taddr, uint32_t* v) {
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void st8(uint32_t taddr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]),
+                 "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
 __device__ __forceinline__ float ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 template <typename T> __device__ __forceinline__ uint32_t pack2(float lo, float hi);
 template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, float hi) { __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi); return *reinterpret_cast<uint32_t*>(&v); }
@@ -115,11 +120,19 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
 }
 
 // 16-bit values: the bits of an infinity's exponent, and whether one of the two in a word is an infinity or NaN (the addition carries out of a full exponent into bit 15)
-template <typename T> struct Exponent { static constexpr uint32_t kMask = std::is_same<T, __nv_bfloat16>::value ? 0x7f807f80u : 0x7c007c00u, kOne = std::is_same<T, __nv_bfloat16>::value ? 0x00800080u : 0x04000400u; };
+template <typename T> struct Exponent { static constexpr uint32_t kMask = std::is_same<T, __nv_bfloat16>::value ? 0x7f807f80u : 0x7c007c00u, kOne = std::is_same<T, __nv_bfloat16>::value ? 0x00800080u : 0x04000400u;
+    static constexpr float kTiny = std::is_same<T, __nv_bfloat16>::value ? 0x1p-126f : 0x1p-24f; };        // smallest positive (normal) value
 template <typename T> __device__ __forceinline__ uint32_t nonfinite(uint32_t w) { return ((w & Exponent<T>::kMask) + Exponent<T>::kOne) & 0x80008000u; }
 template <typename T> __device__ __forceinline__ float half_to_f32(uint32_t h);
 template <> __device__ __forceinline__ float half_to_f32<__nv_bfloat16>(uint32_t h) { return __uint_as_float(h << 16); }
 template <> __device__ __forceinline__ float half_to_f32<__half>(uint32_t h) { return __half2float(__ushort_as_half((unsigned short)h)); }
+// two f32 -> 16 bits, rounded towards 0
+template <typename T> __device__ __forceinline__ uint32_t pack2_down(float lo, float hi) {
+    uint32_t r;
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    else asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
 __device__ __forceinline__ uint32_t ld1(uint32_t taddr) {
     uint32_t v;
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];\ntcgen05.wait::ld.sync.aligned;" : "=r"(v) : "r"(taddr) : "memory");
@@ -150,11 +163,13 @@ __device__ __forceinline__ void add_nonfinite(const T* values, const uint32_t* t
     }
 }
 
-// A row's O is rescaled when its maximum has grown by more than kSlack (log2 units) -- in the first key tiles whenever it has grown at all: there single weights are large,
-// and the largest one, 1 when the maximum is up to date, is then the one weight that 16 bits hold exactly.  [Error of the whole result against 64 bits, 8192 tokens:
-// 2.121e-3 with the slack everywhere, 2.088e-3 so, 2.078e-3 without slack; 532, 547, 588 us.]
-constexpr float kSlack = 8.f;
-constexpr int kExactTiles = 8;
+// P of a row's first key tile is held as two 16-bit parts (the second in the half of S that P leaves free) and multiplied twice: with few keys, single weights are large
+// and their rounding is what the result's error consists of.  In the later tiles P is one part, and the maximum is up to date in every tile, so that a row's largest weight
+// is 1, which 16 bits hold exactly.  The first part is rounded down and the second kept above 0, so that a value that is infinite stays so.
+// [Error of the result against 64 bits, relative to the mma.sync kernel's (one part, maximum up to date every 32 keys), restated for contexts of 40 to 8192 keys: with a
+// maximum that may lag by 2^8 1.3 to 2 % above it for scores of deviation 1, 13 to 26 % above for 3; up to date, one part: 0 to 2 % above; so: 22 % below to 0.1 % above.
+// It costs 7 to 10 %: three prompts of 280 to 700 tokens on cached prefixes 80 -> 86 us, 8192 tokens 562 -> 617; two tiles in two parts 2 and 8 us more.]
+constexpr int kTwoPartTiles = 1;
 
 template <typename T>
 __global__ void __launch_bounds__(kThreadsU, 1)
@@ -320,6 +335,10 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
                         tc_mma_ts(tmem + 256 + i * 128, tmem + i * 128 + k * 8, b + (uint64_t)(k * 16 * 128 >> 4), idesc_o, (add || k > 0) ? 1u : 0u);
+                    if (j < kTwoPartTiles) {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) tc_mma_ts(tmem + 256 + i * 128, tmem + i * 128 + 64 + k * 8, b + (uint64_t)(k * 16 * 128 >> 4), idesc_o, 1u);
+                    }
                     if (j + 1 == nk[i]) tc_commit(o_full(i));
                 }
                 __syncwarp();
@@ -398,8 +417,8 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         bool ok = true;
         const int nki = nk[i];
         // a tile without hidden keys needs no mask and no look at its values: a body of its own, so that the rare paths stay out of the hot one
-        auto step = [&](int j, auto hiding) -> bool {
-            constexpr bool kHides = decltype(hiding)::value;
+        auto step = [&](int j, auto hiding, auto two_parts) -> bool {
+            constexpr bool kHides = decltype(hiding)::value, kTwo = decltype(two_parts)::value;
             if (!mbar_wait_or_flag(s_full(i), j & 1, give_up)) return false;
             tc_fence_after();
             uint32_t s[128];
@@ -419,7 +438,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
 #pragma unroll
             for (int c = 4; c < 128; ++c) mx[c & 3] = fmaxf(mx[c & 3], __uint_as_float(s[c]));
             const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
-            if (__any_sync(0xffffffffu, top > m + (j < kExactTiles ? 0.f : kSlack))) {
+            if (__any_sync(0xffffffffu, top > m)) {
                 const float mn = fmaxf(m, top);
                 const float corr = mn == -INFINITY ? 1.f : ex2(m - mn);
                 m = mn;
@@ -441,21 +460,24 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
             const float2 sc = make_float2(p.scale_log2, p.scale_log2), sb2 = make_float2(sub, sub);
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
-                uint32_t pk[8];
+                uint32_t pk[8], low[8];
                 float2 part = make_float2(0.f, 0.f);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     float2 x = fma2(make_float2(__uint_as_float(s[c * 16 + 2 * e]), __uint_as_float(s[c * 16 + 2 * e + 1])), sc, sb2);
                     x.x = ex2(x.x); x.y = ex2(x.y);
                     part = add2(part, x);
-                    pk[e] = pack2<T>(x.x, x.y);
+                    pk[e] = kTwo ? pack2_down<T>(x.x, x.y) : pack2<T>(x.x, x.y);
+                    if constexpr (kTwo) {
+                        const float h0 = half_to_f32<T>(pk[e] & 0xffffu), h1 = half_to_f32<T>(pk[e] >> 16);
+                        low[e] = pack2<T>(fmaxf(x.x - h0, h0 > 0.f ? Exponent<T>::kTiny : 0.f), fmaxf(x.y - h1, h1 > 0.f ? Exponent<T>::kTiny : 0.f));
+                    }
                 }
                 l2 = add2(l2, part);
-                asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(s_t + c * 8), "r"(pk[0]), "r"(pk[1]), "r"(pk[2]),
-                             "r"(pk[3]), "r"(pk[4]), "r"(pk[5]), "r"(pk[6]), "r"(pk[7])
-                             : "memory");
+                st8(s_t + c * 8, pk);
+                if constexpr (kTwo) st8(s_t + 64 + c * 8, low);
             }
-            if constexpr (kHides) {
+            if (kHides && (!kTwo || hides(j))) {                                    // (the two-part step serves both kinds)
                 if (!mbar_wait_or_flag(v_clean, scans & 1, give_up)) return false;
                 ++scans;
                 if (dirty[0] | dirty[1]) {                                          // (uniform over the CTA's warps)
@@ -477,7 +499,9 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
             if (lane == 0) mbar_arrive(p_ready(i));
             return true;
         };
-        for (int j = 0; j < nki && ok; ++j) ok = hides(j) ? step(j, std::true_type{}) : step(j, std::false_type{});
+        static_assert(kTwoPartTiles == 1, "the first step below");
+        if (nki > 0) ok = step(0, std::true_type{}, std::true_type{});
+        for (int j = 1; j < nki && ok; ++j) ok = hides(j) ? step(j, std::true_type{}, std::false_type{}) : step(j, std::false_type{}, std::false_type{});
         if (nki > 0 && ok && mbar_wait_or_flag(o_full(i), 0, give_up)) {
             tc_fence_after();
             const float l = l2.x + l2.y, inv = l > 0.f ? 1.f / l : 0.f;

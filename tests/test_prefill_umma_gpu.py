@@ -136,3 +136,30 @@ def test_rows_before_a_context_that_is_too_short_are_zero(H, kvh, qlens, klens):
         ref = _reference(q[row + blind:row + n], kc, vc, [t], [n - blind], [c], 128 ** -0.5, None)
         assert float((out[row + blind:row + n].double() - ref).norm() / ref.norm()) < 2.0 ** -8
         row += n
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("new,cached,loud", [(700, 0, 1.0), (300, 1500, 1.0), (200, 5000, 1.0), (700, 1500, 3.0), (200, 5000, 3.0), (40, 0, 1.0)])
+def test_no_less_precise_than_the_kernel_on_mma_sync(dtype, new, cached, loud):
+    """Both round P to 16 bits once (mma.sync: against a maximum that is up to date every 32 keys).  A query that does not start on 16 bytes takes the mma.sync kernel, so
+    both run on the same values.  Margin: 0.5 %, the spread of the ratio between draws of this size."""
+    g = torch.Generator(device=DEV)
+    g.manual_seed(new + cached)
+    H, kvh, klen = 8, 2, new + cached
+    used = -(-klen // 64)
+    mk = lambda *shape: torch.randn(shape, generator=g, device=DEV).to(dtype)
+    q, k, v = mk(new, H, 128) * loud, mk(new, kvh, 128), mk(new, kvh, 128)
+    kc, vc = mk(used, 64, kvh, 128), mk(used, 64, kvh, 128)
+    prep = pkg.prepare_prompt([list(range(klen))], [list(range(used))], 64, [cached], chunk_size=new)
+    _, _, meta = pkg.inputs.to_device(prep)
+    buf = torch.empty(q.numel() + 8, dtype=dtype, device=DEV)
+    off = buf[4:4 + q.numel()].view(q.shape)
+    off.copy_(q)
+    assert q.data_ptr() % 16 == 0 and off.data_ptr() % 16 == 8
+    op = pkg.PagedAttention(H, 128, 128 ** -0.5, kvh)
+    errs = []
+    for x in (off, q):
+        out = op.forward(x, k, v, None, kc, vc, meta)
+        ref = _reference(q, kc, vc, [list(range(used))], [new], [klen], 128 ** -0.5, None)
+        errs.append(float((out.double() - ref).norm() / ref.norm()))
+    assert errs[1] <= 1.005 * errs[0], errs
