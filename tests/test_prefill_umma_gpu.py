@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import candle_vllm_b200 as pkg
+from candle_vllm_b200 import seq_ops
 from tests.gpu_util import DEV
 
 pytestmark = pytest.mark.gpu
@@ -163,3 +164,39 @@ def test_no_less_precise_than_the_kernel_on_mma_sync(dtype, new, cached, loud):
         ref = _reference(q, kc, vc, [list(range(used))], [new], [klen], 128 ** -0.5, None)
         errs.append(float((out.double() - ref).norm() / ref.norm()))
     assert errs[1] <= 1.005 * errs[0], errs
+
+
+@pytest.mark.parametrize("H,kvh,qlens,cached,chunk,sink", [
+    (8, 2, [257], [127], 128, False),              # a chunk border at the edge of a key tile, inside a query tile
+    (8, 2, [300, 33], [190, 64], 192, True),       # chunks that are no multiple of a key tile, with a sink
+    (4, 4, [129], [0], 64, True),
+    (8, 2, [200, 1], [900, 700], 0, True),         # a sink over many key tiles
+])
+def test_chunks_and_sinks_at_tile_edges(H, kvh, qlens, cached, chunk, sink):
+    g = torch.Generator(device=DEV)
+    g.manual_seed(H + chunk)
+    klens = [a + b for a, b in zip(qlens, cached)]
+    tables, at = [], 0
+    for n in klens:
+        tables.append(list(range(at, at - (-n // 64))))
+        at += -(-n // 64)
+    mk = lambda *shape: torch.randn(shape, generator=g, device=DEV).to(torch.bfloat16)
+    q, kc, vc = mk(sum(qlens), H, 128), mk(at, 64, kvh, 128), mk(at, 64, kvh, 128)
+    s = torch.randn(H, generator=g, device=DEV) * 2 if sink else None
+    prep = pkg.inputs.prepare_step([dict(tokens=[0] * n, start=c, block_table=t, slot=i) for i, (n, c, t) in enumerate(zip(qlens, cached, tables))], 64)
+    batch = seq_ops.StepBatch.from_host(prep, DEV)
+    out = seq_ops.paged_attention_varlen_sink(q.reshape(-1, H * 128), kc, vc, batch, H, kvh, 128, 128, 64, 128 ** -0.5, chunk, 0, s, torch.bfloat16).view(-1, H, 128)
+    ref, row = [], 0
+    for n, k, t in zip(qlens, klens, tables):
+        keys, values = (c[torch.tensor(t, device=DEV)].flatten(0, 1)[:k].double().repeat_interleave(H // kvh, 1) for c in (kc, vc))
+        score = torch.einsum("qhd,khd->hqk", q[row:row + n].double(), keys) * 128 ** -0.5
+        pos, key = torch.arange(k - n, k, device=DEV)[:, None], torch.arange(k, device=DEV)[None]
+        hidden = (key > pos) | (key < pos // chunk * chunk) if chunk else key > pos
+        score = score.masked_fill(hidden, -np.inf)
+        if sink:
+            score = torch.cat([score, s.double()[:, None, None].expand(-1, n, 1)], 2)
+        ref.append(torch.einsum("hqk,khd->qhd", torch.softmax(score, 2)[..., :k], values))
+        row += n
+    ref = torch.cat(ref)
+    err = float((out.double() - ref).norm() / ref.norm())
+    assert torch.isfinite(out).all() and err < 2.0 ** -8, err
