@@ -222,6 +222,8 @@ void qmatmul_f16act(const void* x_f16, const void* w, float* y, int32_t m, int32
     qmatmul_dispatch(x_f16, w, y, n, m, n, k, ggml_type, accumulate, as_stream(stream));
 }
 
+int32_t qmatmul_decode_kernel_registers(int32_t ggml_type) { return ggml_type == B200_GGML_Q4_K || ggml_type == B200_GGML_Q6_K ? qmatmul_tc_decode_registers(ggml_type) : 0; }
+
 int32_t qmatmul_slab_count(int32_t m, int32_t n, int32_t k, int32_t ggml_type) {
     if (m <= 0 || n <= 0 || k <= 0) return 0;
     return qmatmul_slabs_needed(1, &n, &ggml_type, m, k);

@@ -103,7 +103,7 @@ struct GemmParams {
     // grouped (mixture-of-experts) mode: the chunk list lives in device memory -- built from the routing of this step (moe.cu): chunk = (expert, <= kMB routed
     // rows); tile id = chunk * n_tiles + weight tile, the weight tiles of every segment of one expert in a row.  Weights at row expert * n + n0 of a segment's
     // stacked [E * n, K] tensor, activations at row x_row0 of the expert-sorted fp16 copy, results scattered to row_map[x_row0 + i]
-    const MoeChunk* chunks;        // null: dense mode
+    const MoeChunk* chunks;        // grouped instances only
     const int* num_chunks;         // device: number of chunks of this step
     const uint32_t* row_map;       // sorted position -> output row; null: the sorted position itself
     const float* row_scale;        // per OUTPUT row multiplier (top-k routing weight) or null
@@ -124,10 +124,10 @@ struct Tile {
     int wrow;            // first row of the tile in the segment's tensor (grouped: the stack of all experts)
     int xrow, count;     // first activation row, rows
 };
-template <int kMB>
+template <int kMB, bool kGrouped>
 __device__ __forceinline__ Tile tile_of(const GemmParams& p, int tile) {
     Tile t;
-    if (p.chunks) {
+    if constexpr (kGrouped) {
         const int c = tile / p.n_tiles, w = tile - c * p.n_tiles;
         const MoeChunk ch = p.chunks[c];
         t.sg = seg_of_tile(p, w);
@@ -135,7 +135,7 @@ __device__ __forceinline__ Tile tile_of(const GemmParams& p, int tile) {
         t.wrow = ch.expert * seg_rows(p, t.sg) + t.n0;
         t.xrow = ch.x_row0; t.count = ch.count;
     } else {
-        const int w = p.m_tiles == 1 ? tile : tile / p.m_tiles, mt = tile - w * p.m_tiles;
+        const int w = kMB <= 64 || p.m_tiles == 1 ? tile : tile / p.m_tiles, mt = kMB <= 64 ? 0 : tile - w * p.m_tiles;      // up to 64 rows are one row tile
         t.sg = seg_of_tile(p, w);
         t.n0 = t.wrow = (w - seg_first_tile(p, t.sg)) * kTileN;
         t.xrow = mt * p.mrows; t.count = min(p.mrows, p.m - t.xrow);
@@ -536,8 +536,13 @@ __device__ __forceinline__ void m4_unit(const uint8_t* blk, int q, int r7, uint3
     if (lane == 0) mbar_arrive(a_ready_bar);
 }
 
-template <int kMB, int kType>
-__global__ void __launch_bounds__(kThreads, 1)
+// Registers: a kernel of 608 threads at 96 registers leaves too few on the SM for a block of the small kernels between two products (256 threads of 32), so that the next
+// product's prologue and its weight stream could not begin beside them.  The Q4_K kernel of up to 32 rows fits into 80; it is bound as for 768 threads, which is 80, because
+// the compiler's own choice moved between 79 and 95 with the code around.  [Decode step of 16 layers, 8B sizes, 95 against 79 registers: 81.3 / 78.2 us a layer at 2 rows,
+// 85.8 / 80.4 at 9, 94.0 / 89.6 at 32.]
+template <int kMB, int kType> constexpr int bound_threads() { return kMB == 32 && kType == B200_GGML_Q4_K ? 768 : kThreads; }
+template <int kMB, int kType, bool kGrouped>
+__global__ void __launch_bounds__(bound_threads<kMB, kType>(), 1)
 qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_constant__ CUtensorMap wmap1,
                   const __grid_constant__ CUtensorMap wmap2, const __grid_constant__ CUtensorMap xmap, const GemmParams p) {
     using C = Cfg<kMB, kType>;
@@ -579,12 +584,13 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
     // ---- stream-K range of this CTA over the flattened (tile, super-block) space -----------------
     // (32-bit on purpose: 64-bit integer division costs ~500 cycles each on the SM and sat on the critical path of every
     // launch; the host guarantees total * gridDim.x < 2^31)
-    const bool moe = p.chunks != nullptr;
+    constexpr bool moe = kGrouped;
     if (moe) pdl_wait();               // the chunk list is produced by an earlier kernel (routing of this step)
-    const uint32_t n_tiles_rt = moe ? (uint32_t)*reinterpret_cast<const volatile int*>(p.num_chunks) * (uint32_t)p.n_tiles : (uint32_t)p.n_tiles * (uint32_t)p.m_tiles;
+    const uint32_t n_tiles_rt = moe ? (uint32_t)*reinterpret_cast<const volatile int*>(p.num_chunks) * (uint32_t)p.n_tiles : (uint32_t)p.n_tiles * (kMB <= 64 ? 1u : (uint32_t)p.m_tiles);
     const uint32_t total = n_tiles_rt * (uint32_t)p.nsb, nsb = (uint32_t)p.nsb;
     uint32_t u0, u1;
-    if (p.csplit > 1) {                // one tile per cluster, one part of its units per CTA
+    constexpr bool kClusters = kMB == 256 && !kGrouped;
+    if (kClusters && p.csplit > 1) {                // one tile per cluster, one part of its units per CTA
         const uint32_t t = blockIdx.x / (uint32_t)p.csplit, r = blockIdx.x - t * (uint32_t)p.csplit;
         u0 = t * nsb + nsb * r / (uint32_t)p.csplit;
         u1 = t * nsb + nsb * (r + 1) / (uint32_t)p.csplit;
@@ -602,7 +608,7 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_w));
         int it = 0;
         int tile = (int)tile0, sb = (int)sb0;
-        Tile ti = u0 < u1 ? tile_of<kMB>(p, tile) : Tile{};
+        Tile ti = u0 < u1 ? tile_of<kMB, kGrouped>(p, tile) : Tile{};
         for (uint32_t u = u0; u < u1; ++u, ++it) {
             const int s = it % kW;
             mbar_wait(w_empty(s), ((it / kW) & 1) ^ 1);
@@ -636,7 +642,7 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                             wrow, pol_w);
             }
             __syncwarp();
-            if (++sb == (int)nsb) { sb = 0; ++tile; if (u + 1 < u1) ti = tile_of<kMB>(p, tile); }
+            if (++sb == (int)nsb) { sb = 0; ++tile; if (u + 1 < u1) ti = tile_of<kMB, kGrouped>(p, tile); }
         }
         if (leader) {
 #pragma unroll
@@ -659,9 +665,9 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_x));
         int it = 0;
         int sb = (int)sb0, xtile = (int)tile0;
-        Tile ti = u0 < u1 ? tile_of<kMB>(p, xtile) : Tile{};
+        Tile ti = u0 < u1 ? tile_of<kMB, kGrouped>(p, xtile) : Tile{};
         for (uint32_t u = u0; u < u1; ++u, ++it) {
-            const int nb = (ti.count + 31) >> 5;                 // only the 32-row groups that hold rows of this tile
+            const int nb = kMB == 32 || (kMB == 64 && !kGrouped) ? kMB / 32 : (ti.count + 31) >> 5;                 // only the 32-row groups that hold rows of this tile
 #pragma unroll
             for (int q0 = 0; q0 < 4; q0 += C::kXSlices) {
                 const int xi = it * (4 / C::kXSlices) + q0 / C::kXSlices, s = xi % kX;
@@ -677,7 +683,7 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                 }
                 __syncwarp();
             }
-            if (++sb == (int)nsb) { sb = 0; ++xtile; if (u + 1 < u1) ti = tile_of<kMB>(p, xtile); }
+            if (++sb == (int)nsb) { sb = 0; ++xtile; if (u + 1 < u1) ti = tile_of<kMB, kGrouped>(p, xtile); }
         }
     } else if (warp == kDequantWarps + 2) {
         // ======================================= MMA ISSUER ======================================
@@ -690,7 +696,9 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
             const uint32_t tile_end = (tile + 1) * nsb;
             const uint32_t seg_end = tile_end < u1 ? tile_end : u1;
             // instruction descriptor: D = f32, A = B = f16, both K-major, M = 128, N = the tile's rows rounded up to 32
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(((tile_of<kMB>(p, (int)tile).count + 31) >> 5) * 4) << 17) | ((uint32_t)(kTileN >> 4) << 24);
+            uint32_t n8 = kMB / 8;                             // (constant where a tile's rows always round up to kMB: nothing to look up before the first wait)
+            if constexpr (kMB > 64 || (kMB == 64 && kGrouped)) n8 = (uint32_t)((tile_of<kMB, kGrouped>(p, (int)tile).count + 31) >> 5) * 4;
+            const uint32_t idesc = (1u << 4) | (n8 << 17) | ((uint32_t)(kTileN >> 4) << 24);
             mbar_wait(d_empty, (seg & 1) ^ 1);                 // epilogue of the previous segment has drained D
             tc_fence_after();
             bool first = true;
@@ -743,8 +751,8 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         // if loaded on demand -- they are fetched ONE UNIT AHEAD instead (weights: no dependency on the previous kernel)
         float m4_next[4] = {0.f, 0.f, 0.f, 0.f};
         auto m4_fetch = [&](int tl, int sbx) {
-            const int wt = p.m_tiles == 1 ? tl : tl / p.m_tiles, sgx = seg_of_tile(p, wt);      // (int4 / FP4 weights have no grouped form)
-            const int rw = (wt - seg_first_tile(p, sgx)) * kTileN + row, nn = seg_rows(p, sgx);
+            const int sgx = seg_of_tile(p, tl);                    // (int4 / FP4 weights: up to 64 rows, no grouped form)
+            const int rw = (tl - seg_first_tile(p, sgx)) * kTileN + row, nn = seg_rows(p, sgx);
             const M4Ctx c{sgx == 0 ? p.scales_seg[0] : (sgx == 1 ? p.scales_seg[1] : p.scales_seg[2]), nn, p.group_size, sbx * kSB, rw < nn ? rw : 0,
                           p.scale_bf16, 0, 1, 0, nullptr, sgx == 0 ? p.zp_seg[0] : (sgx == 1 ? p.zp_seg[1] : p.zp_seg[2]), {0.f, 0.f, 0.f, 0.f}, 0};
             const int kq = sbx * kSB + qt * 64;
@@ -805,7 +813,7 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         for (uint32_t u = u0; u < u1; ++tile) {
             const uint32_t tile_begin = (uint32_t)tile * nsb, tile_end = tile_begin + nsb;
             const uint32_t seg_begin = u, seg_end = tile_end < u1 ? tile_end : u1;
-            const Tile ti = tile_of<kMB>(p, tile);
+            const Tile ti = tile_of<kMB, kGrouped>(p, tile);
             // grouped: lane l holds output row and multiplier of this warp's column l, fetched before the tile's units so that the epilogue does not wait for them
             uint32_t my_row = 0;
             float my_scale = 1.f;
@@ -902,7 +910,7 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                 ++seg;
                 continue;
             }
-            if (kMB == 256 && p.csplit > 1) {
+            if (kClusters && p.csplit > 1) {
                 // partial sums -> this CTA's shared memory, [4 columns][128 rows][4] (the rings are drained: every load of this CTA has been consumed)
                 float4* part = reinterpret_cast<float4*>(smem);
                 constexpr int kCols = kMB / 4;
@@ -969,12 +977,12 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         }
     }
 
-    if (kMB == 256 && p.csplit > 1) {
+    if (kClusters && p.csplit > 1) {
         __syncwarp();
         cluster_sync();                                               // every CTA's partial sums are written
         if (warp < kDequantWarps) {
             const int rank = (int)(blockIdx.x % (uint32_t)p.csplit), row = (int)threadIdx.x & 127;
-            const Tile ti = tile_of<kMB>(p, (int)tile0);
+            const Tile ti = tile_of<kMB, kGrouped>(p, (int)tile0);
             const int n_idx = ti.n0 + row, groups = (ti.count + 3) / 4, g1 = groups * (rank + 1) / p.csplit;
             float* const y = (ti.sg == 0 ? p.y[0] : (ti.sg == 1 ? p.y[1] : p.y[2])) + (int64_t)ti.xrow * p.ldy + n_idx;
             for (int g = groups * rank / p.csplit + ((int)threadIdx.x >> 7); g < g1; g += kDequantWarps / 4) {
@@ -1032,11 +1040,11 @@ int gemm_grid(int64_t n_tiles, int nsb, bool whole_tiles, bool slab_mode) {
     return (int)grid;
 }
 
-template <int kMB, int kType>
-void launch(const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, cudaStream_t st) {
-    auto kern = qmatmul_tc_kernel<kMB, kType>;
+template <int kMB, int kType, bool kGrouped>
+void launch_kernel(const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, cudaStream_t st) {
+    auto kern = qmatmul_tc_kernel<kMB, kType, kGrouped>;
     ensure_dynamic_smem(reinterpret_cast<const void*>(kern), Cfg<kMB, kType>::kTotal);
-    const int grid = p.chunks ? sm_count() : gemm_grid((int64_t)p.n_tiles * p.m_tiles, p.nsb, p.whole_tiles != 0, p.slabs > 0);
+    const int grid = kGrouped ? sm_count() : gemm_grid((int64_t)p.n_tiles * p.m_tiles, p.nsb, p.whole_tiles != 0, p.slabs > 0);
     if (p.csplit > 1) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(p.n_tiles * p.m_tiles * p.csplit)); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = Cfg<kMB, kType>::kTotal; cfg.stream = st;
@@ -1053,16 +1061,23 @@ void launch(const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, c
     count_launch();
 }
 
+template <int kMB, int kType> void launch(const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, cudaStream_t st) { launch_kernel<kMB, kType, false>(wm, xm, p, st); }
+
 template <int kType>
 void launch_rows_of(int mb, const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, cudaStream_t st) {
     if (mb == 32) launch<32, kType>(wm, xm, p, st);
     else if (mb == 64) launch<64, kType>(wm, xm, p, st);
-    else if (mb == 128) launch<128, kType>(wm, xm, p, st);
     else launch<256, kType>(wm, xm, p, st);
 }
 void launch_rows(int mb, int ggml_type, const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, cudaStream_t st) {
     if (ggml_type == B200_GGML_Q4_K) launch_rows_of<B200_GGML_Q4_K>(mb, wm, xm, p, st);
     else launch_rows_of<B200_GGML_Q6_K>(mb, wm, xm, p, st);
+}
+template <int kType>
+void launch_grouped(int chunk_rows, const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, cudaStream_t st) {
+    if (chunk_rows == 32) launch_kernel<32, kType, true>(wm, xm, p, st);
+    else if (chunk_rows == 64) launch_kernel<64, kType, true>(wm, xm, p, st);
+    else launch_kernel<128, kType, true>(wm, xm, p, st);
 }
 
 bool make_w_map(CUtensorMap* wm, const void* w, int n, int nsb, int ggml_type) {
@@ -1161,7 +1176,7 @@ static int tile_rows(int m) { return m <= 64 ? rows_per_tile(m) : (((m + row_til
 static int cluster_split(int64_t tiles, int nsb) {
     for (int s = 8; s > 1; --s)
         if (tiles * s <= sm_count() && s <= nsb / 2 &&
-            tiles <= max_active_clusters(reinterpret_cast<const void*>(qmatmul_tc_kernel<256, B200_GGML_Q4_K>), kThreads, Cfg<256, B200_GGML_Q4_K>::kTotal, s)) return s;
+            tiles <= max_active_clusters(reinterpret_cast<const void*>(qmatmul_tc_kernel<256, B200_GGML_Q4_K, false>), kThreads, Cfg<256, B200_GGML_Q4_K>::kTotal, s)) return s;
     return 1;
 }
 
@@ -1254,6 +1269,14 @@ int qmatmul_tc_multi(const void* x_f16, int nseg, const void* const* w, float* c
     launch_rows(mb, ggml_type, wm, xm, p, st);
     check_launch("qmatmul_tc");
     return p.slabs;
+}
+
+int qmatmul_tc_decode_registers(int ggml_type) {
+    cudaFuncAttributes a{};
+    const void* kern = ggml_type == B200_GGML_Q4_K ? reinterpret_cast<const void*>(qmatmul_tc_kernel<32, B200_GGML_Q4_K, false>)
+                                                   : reinterpret_cast<const void*>(qmatmul_tc_kernel<32, B200_GGML_Q6_K, false>);
+    if (cudaFuncGetAttributes(&a, kern) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return a.numRegs;
 }
 
 // ---- weight-only GEMMs with 16-bit output (marlin_4bit_*, fp8_matmul) ----------------------------------------------
@@ -1439,7 +1462,7 @@ void qmatmul_tc_moe_fp8(const void* xs_f16, int xs_rows, const void* w, const fl
     p.ldy = ldy; p.m = 32; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = 1; p.mrows = 32; p.accumulate = 0; p.whole_tiles = 1;
     p.chunks = chunks; p.num_chunks = num_chunks; p.row_map = row_map; p.row_scale = row_scale;
     p.scales = scale; p.group_size = bx; p.k = k; p.scale_by = by; p.scale_sk = sk; p.norm = norm;
-    launch<32, kTypeF8>(wm, xm, p, st);
+    launch_kernel<32, kTypeF8, true>(wm, xm, p, st);
     check_launch("moe_gemm_fp8");
 }
 
@@ -1460,7 +1483,8 @@ void qmatmul_tc_moe(const void* xs_f16_k4, int xs_rows, int nseg, const void* co
     if ((int64_t)max_chunks * nseg * tiles * nsb * sm_count() >= (int64_t)1 << 31) { set_error(kErrUnsupported, "moe_gemm: %d items x %d super-blocks exceed the 32-bit unit range", max_chunks * nseg * tiles, nsb); return; }
     p.ldy = ldy; p.m = chunk_rows; p.nsb = nsb; p.n_tiles = nseg * tiles; p.m_tiles = 1; p.mrows = chunk_rows; p.accumulate = 0; p.whole_tiles = 1;
     p.chunks = chunks; p.num_chunks = num_chunks; p.row_map = row_map; p.row_scale = row_scale;
-    launch_rows(chunk_rows, ggml_type, wm, xm, p, st);
+    if (ggml_type == B200_GGML_Q4_K) launch_grouped<B200_GGML_Q4_K>(chunk_rows, wm, xm, p, st);
+    else launch_grouped<B200_GGML_Q6_K>(chunk_rows, wm, xm, p, st);
     check_launch("moe_gemm");
 }
 

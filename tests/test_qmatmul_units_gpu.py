@@ -1,6 +1,8 @@
 """Every weight of a GGML block, one by one: unit rows of activations give back the dequantised weights, so each quarter of a block, each offset of a Q6_K block
 in its 16-byte groups (210 bytes a block: eight offsets over eight blocks) and both scale paths (block scales that fit f16 after the multiplication by a power of
 two, and larger ones; the choice is made per warp of 32 rows) show in the output."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -54,3 +56,8 @@ def test_rows_on_either_side_of_the_dense_path(t, m, k):
     ref = G.qmatmul_dequant(x, w, t, n, k)
     y = op.forward(torch.from_numpy(x).to(DEV)).cpu().numpy()
     assert rel_fro(y, ref) < 1e-3, rel_fro(y, ref)             # both sides: weights and activations rounded to f16 once
+
+
+def test_the_decode_kernel_leaves_registers_for_its_neighbours():
+    """65536 registers an SM: 608 threads of 80 leave room for two blocks of 256 threads of 32 (rotation, norms, activation), of 96 for none"""
+    assert 0 < pkg.lib().qmatmul_decode_kernel_registers(C.c_int32(pkg.GgmlType.Q4_K)) <= 80
