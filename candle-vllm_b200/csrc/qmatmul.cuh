@@ -8,9 +8,13 @@ namespace b200 {
 void qmatmul_generic(const void* x, bool x_is_f16, const void* w, float* y, int64_t ldy, int m, int n, int k,
                      int ggml_type, int accumulate, cudaStream_t st);
 
+// From this many rows on a GGML weight is rounded to f16 once on its way to the tensor cores, whichever route takes the product: dequantised in f32 first, or in the
+// dequant-GEMM's instance that does the same per unit.  (Below, the dequant-GEMM rounds scale, offset and result.)
+constexpr int kSingleRoundingRows = 512;
+
 // tcgen05 path (qmatmul_tc.cu): fp16 activations [m,k]; false when the shape is not covered (as one row tile: m <= 64)
 bool qmatmul_tc_supported(int m, int n, int k, int ggml_type);
-// same, with m > 64 served in row tiles of 128 (qmatmul_dispatch)
+// same, with m > 64 served in row tiles of up to 256 (qmatmul_dispatch)
 bool qmatmul_tc_usable(int m, int n, int k, int ggml_type);
 // true when some output tile is split across CTAs: y must hold the addend (zeros for a plain product)
 bool qmatmul_tc_needs_zeroed_output(int m, int n, int k);

@@ -197,14 +197,29 @@ static bool qmm_check(const char* who, const void* x, const void* w, const float
 
 extern "C" {
 
-// Rows at or above this count take the "dequantise once + dense tensor-core GEMM" path: the 16-bit copy of W costs ~4.6 bytes of traffic per weight (0.56 read, 2
-// written, 2 read back), a row tile of 256 of the dequant-GEMM its conversion, which for Q6_K takes half as long again.  Feed-forward of 4096 x 14336 on this path / on
-// the other, us: 1024 rows 639 / 487 (Q4_K), 580 / 523 (Q6_K); 1400 rows 823 / 698, 755 / 750; 1600 rows 896 / 789, 825 / 851; 2048 rows 998 / 937, 934 / 988; of 2048 x
-// 6144 (Q4_K) 1024 rows 200 / 139, 2048 rows 270 / 246.  Where the dequant-GEMM has no tensor-core form (Q8_0, Q6_K with k not a multiple of 2048) the line stays low.
-static constexpr int kDenseRows = 512;
-static int dense_rows(int m, int n, int k, int ggml_type) {
-    if (!qmatmul_tc_usable(m, n, k, ggml_type)) return kDenseRows;
-    return ggml_type == B200_GGML_Q4_K ? 2049 : 1408;
+// Which products take the "dequantise once + dense tensor-core GEMM" path: the 16-bit copy of W costs ~4.6 bytes of traffic per weight (0.56 read, 2 written, 2 read back), a
+// row tile of 256 of the dequant-GEMM its conversion, in the instance that rounds a weight once, as the 16-bit copy does.  us, this path / dequant-GEMM:
+//                 1024 x 4096    4096 x 4096    14336 x 4096    4096 x 14336    6144 x 2048    2048 x 6144    (n x k)
+//   Q4_K  512     28.9 / 25.6    66.8 / 28.3    153 / 78        184 / 79        56.3 / 31.6    53.8 / 29.7
+//         1024    35.7 / 25.6    66.8 / 44.0    205 / 155       205 / 145       81.9 / 61.6    70.8 / 42.1
+//         1150    35.8 / 26.1    67.1 / 78.4    216 / 169       210 / 245       79.0 / 57.7    69.7 / 59.7
+//         1536    50.0 / 31.3    91.6 / 81.0    255 / 224       283 / 243       70.7 / 54.7    74.0 / 62.2
+//         2048    52.4 / 34.4    97.1 / 84.8    316 / 307       304 / 261       94.7 / 91.5    80.8 / 73.7
+//   Q6_K  512     25.0 / 21.2    58.3 / 28.6    125 / 78        168 / 86        57.1 / 34.9    58.4 / 32.3
+//         1024    33.8 / 22.7    58.5 / 43.6    186 / 160       182 / 152       79.0 / 64.3    80.1 / 48.9
+//         1150    35.8 / 27.9    58.7 / 78.6    197 / 165       185 / 248       69.4 / 61.1    64.6 / 58.7
+//         1536    49.1 / 31.2    83.5 / 80.6    227 / 244       255 / 251       66.7 / 56.8    70.0 / 62.0
+//         2048    50.3 / 34.5    88.5 / 84.9    319 / 325       316 / 296       105 / 95.8     77.0 / 75.2
+// So Q4_K stays with the dequant-GEMM as far as one call of it goes (a second would convert the weights again; 2300 rows 338 / 342 at 14336 x 4096, 100 / 101 at 4096 x 4096),
+// Q6_K to where wide matrices lose what narrow ones gain; and below that, what takes the dequant-GEMM a second round of tiles that leaves it under three fifths full, while the
+// dense GEMM's tiles of 128 x 256 fit one round, goes the dense way (1025 to 1152 rows of 4096 columns on 148 SMs).  Where the dequant-GEMM has no tensor-core form (Q8_0, Q6_K
+// with k not a multiple of 2048) the dense path starts at kDenseRows.
+static constexpr int kDenseRows = kSingleRoundingRows;
+static bool takes_dense_path(int m, int n, int k, int ggml_type) {
+    if (m < kDenseRows) return false;
+    if (!qmatmul_tc_usable(m, n, k, ggml_type) || m > (ggml_type == B200_GGML_Q4_K ? kMaxRows : 1407)) return true;
+    const int64_t sms = sm_count(), tiles = (int64_t)((n + 127) / 128) * ((m + 255) / 256), rounds = (tiles + sms - 1) / sms;
+    return rounds > 1 && 5 * tiles < 3 * rounds * sms && (int64_t)((m + 127) / 128) * ((n + 255) / 256) <= sms;
 }
 
 size_t qmatmul_workspace_bytes(int32_t m, int32_t n, int32_t k) {
@@ -241,7 +256,7 @@ void qmatmul_f32(const float* x, const void* w, float* y, int32_t m, int32_t n, 
                  int32_t ggml_type, int32_t accumulate, void* workspace, size_t workspace_bytes, int64_t stream) {
     if (m == 0 || n == 0) return;
     if (!qmm_check("qmatmul_f32", x, w, y, m, n, k, ggml_type)) return;
-    if (m >= dense_rows(m, n, k, ggml_type) && !accumulate && k % 8 == 0 && ((uintptr_t)workspace & 15) == 0 && workspace &&
+    if (takes_dense_path(m, n, k, ggml_type) && !accumulate && k % 8 == 0 && ((uintptr_t)workspace & 15) == 0 && workspace &&
         workspace_bytes >= qmatmul_workspace_bytes(m, n, k)) {
         // prefill chunk: weights -> fp16 once, activations -> fp16, dense tcgen05 GEMM with fp32 output (dense_gemm.cu)
         char* xs = static_cast<char*>(workspace);

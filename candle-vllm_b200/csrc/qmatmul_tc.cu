@@ -98,6 +98,7 @@ struct GemmParams {
     int mrows;                     // dense mode: activation rows per row tile (a multiple of 32 up to kMB)
     int csplit;                    // > 1: a cluster of csplit CTAs shares every tile, each over its part of k; the partial sums meet in shared memory of the
                                    // cluster and every CTA adds up and stores its share of the columns (plain stores in a fixed order: nothing to zero)
+    int exact;                     // host: the instance that rounds a weight once
     int m_tiles;                   // dense mode: row tiles; tile id = weight tile * m_tiles + row tile (the row tiles of a weight
                                    // tile run side by side, so its bytes come from memory once)
     // grouped (mixture-of-experts) mode: the chunk list lives in device memory -- built from the routing of this step (moe.cu): chunk = (expert, <= kMB routed
@@ -341,24 +342,40 @@ __device__ __forceinline__ void realign(const uint32_t* t, int wo, int sh16, uin
     for (int i = 0; i < kN; ++i) out[i] = __funnelshift_r(s2[i], s2[i + 1], sh16);
 }
 
+// a pair of weights: kExact (q + n) s, q + n exact, with s in two parts; else q s + n
+template <bool kExact>
+__device__ __forceinline__ __half2 q6k_weight2(__half2 q, __half2 s, __half2 n, __half2 s_low) {
+    if constexpr (!kExact) return __hfma2(q, s, n);
+    const __half2 c = __hadd2(q, n);
+    return __hfma2(c, s, __hmul2(c, s_low));
+}
+
 // This thread's row, half kHf of the super-block (128 weights = 4 groups of 32): group g weight l is
 // ((ql[64 kHf + 32 (g&1) + l] nibble (g>>1)) | ((qh[32 kHf + l] >> 2g) & 3) << 4) - 32, times d*scales[8 kHf + 2g + l/16].
 // The 6-bit value goes to fp16 mantissa bits 4-9 (= q * 2^-20); one HFMA2 with (s*2^20, -32 s) finishes it
 // (exact path with the 1024+q magic when s*2^20 would overflow fp16).
 // kGp = 0: groups 0 (lo nibble) and 2 (hi nibble) from ql[0..31]; kGp = 1: groups 1, 3.  The quarter is a run-time value, uniform per warp: all sixteen warps run one body.
+// kExact: one rounding of d * scale * (q - 32) to f16, as in dequantize_f16 -- the scale in two f16 parts, (q - 32) times the second (below the first's last place) added in the
+// HFMA2 of the first.  Otherwise scale, offset and result are rounded.
+template <bool kExact>
 __device__ __forceinline__ void dequant_q6k_pair(const uint32_t (&ql)[8], uint32_t a_col, const uint32_t (&qh)[8], const uint32_t (&scw)[2], float dk, bool fast, int gp) {
     // `fast` is warp-uniform; the two paths are separate straight-line blocks (a per-word branch interleaves them in the
     // instruction stream and the kernel then stalls on instruction fetch: ncu showed stall_no_inst on every line)
 #pragma unroll
     for (int hi = 0; hi < 2; ++hi) {
         const int g2 = 2 * gp + 4 * hi;         // twice the group index within the half
-        __half2 sh[2], nh[2];                   // scale / offset of the two 16-weight sub-groups
+        __half2 sh[2], nh[2], sl[2];            // scale / offset / second part of the scale of the two 16-weight sub-groups
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             const int sc = (int)(int8_t)((scw[hi] >> (16 * gp + 8 * j)) & 0xff);          // scale 2 g + j = byte 2 gp + j of word hi
             sh[j] = __float2half2_rn(dk * (float)sc);
             // q = 32 must give exactly 0: the offset is derived from the ROUNDED scale
-            nh[j] = __float2half2_rn(-32.f * (fast ? __low2float(sh[j]) * (1.f / 1048576.f) : __low2float(sh[j])));
+            if constexpr (kExact) {
+                sl[j] = __float2half2_rn(dk * (float)sc - __low2float(sh[j]));
+                nh[j] = __float2half2_rn(fast ? -32.f / 1048576.f : -1056.f);         // 32 in the units of the words below
+            } else {
+                nh[j] = __float2half2_rn(-32.f * (fast ? __low2float(sh[j]) * (1.f / 1048576.f) : __low2float(sh[j])));
+            }
         }
         uint32_t v[16];
         if (fast) {
@@ -370,8 +387,8 @@ __device__ __forceinline__ void dequant_q6k_pair(const uint32_t (&ql)[8], uint32
                 const uint32_t h0 = qh[i] << (8 - g2), h1 = qh[i] >> g2;
                 uint32_t t0 = (l0 & 0x00f000f0u) | (h0 & 0x03000300u);
                 uint32_t t1 = (l1 & 0x00f000f0u) | (h1 & 0x03000300u);
-                const __half2 r0 = __hfma2(*reinterpret_cast<__half2*>(&t0), sh[i >> 2], nh[i >> 2]);
-                const __half2 r1 = __hfma2(*reinterpret_cast<__half2*>(&t1), sh[i >> 2], nh[i >> 2]);
+                const __half2 r0 = q6k_weight2<kExact>(*reinterpret_cast<__half2*>(&t0), sh[i >> 2], nh[i >> 2], sl[i >> 2]);
+                const __half2 r1 = q6k_weight2<kExact>(*reinterpret_cast<__half2*>(&t1), sh[i >> 2], nh[i >> 2], sl[i >> 2]);
                 v[2 * i] = *reinterpret_cast<const uint32_t*>(&r0);
                 v[2 * i + 1] = *reinterpret_cast<const uint32_t*>(&r1);
             }
@@ -388,8 +405,9 @@ __device__ __forceinline__ void dequant_q6k_pair(const uint32_t (&ql)[8], uint32
                     uint32_t t0 = (lw & 0x000f000fu) | ((hw << 4) & 0x00300030u) | magic;
                     uint32_t t1 = ((lw >> 8) & 0x000f000fu) | ((hw >> 4) & 0x00300030u) | magic;
                     const __half2 s2 = i4 ? sh[1] : sh[0], n2 = i4 ? nh[1] : nh[0];
-                    const __half2 r0 = __hfma2(__hsub2(*reinterpret_cast<__half2*>(&t0), k1024), s2, n2);
-                    const __half2 r1 = __hfma2(__hsub2(*reinterpret_cast<__half2*>(&t1), k1024), s2, n2);
+                    const __half2 l2 = i4 ? sl[1] : sl[0];
+                    const __half2 r0 = kExact ? q6k_weight2<true>(*reinterpret_cast<__half2*>(&t0), s2, n2, l2) : __hfma2(__hsub2(*reinterpret_cast<__half2*>(&t0), k1024), s2, n2);
+                    const __half2 r1 = kExact ? q6k_weight2<true>(*reinterpret_cast<__half2*>(&t1), s2, n2, l2) : __hfma2(__hsub2(*reinterpret_cast<__half2*>(&t1), k1024), s2, n2);
                     const uint32_t w0 = *reinterpret_cast<const uint32_t*>(&r0), w1 = *reinterpret_cast<const uint32_t*>(&r1);
                     if (i4) { v[8 + 2 * k] = w0; v[9 + 2 * k] = w1; } else { v[2 * k] = w0; v[2 * k + 1] = w1; }
                 }
@@ -399,6 +417,7 @@ __device__ __forceinline__ void dequant_q6k_pair(const uint32_t (&ql)[8], uint32
     }
 }
 
+template <bool kExact>
 struct Q6KRun {                                 // quarter q: half q / 2, groups (q % 2, q % 2 + 2): 64 weights -> two 16-column TMEM stores
     // raw: [0, 12) ql words 16 half + 8 (q % 2) .., [12, 24) qh words 32 + 8 half .., [24, 32) words 48 .. 55 (scales from 48 + 2 half, d at 52)
     static constexpr int kRaw = 32;
@@ -421,11 +440,19 @@ struct Q6KRun {                                 // quarter q: half q / 2, groups
         const bool fast = __all_sync(0xffffffffu, fabsf(d) * 128.f * 1048576.f <= 65504.f);   // warp-uniform (see Q4_K)
         const float dk = fast ? d * 1048576.f : d;
         realign<0, 8>(t, wo, sh16, ql);
-        dequant_q6k_pair(ql, a_col + (q >> 1) * 64, qh, scw, dk, fast, q & 1);
+        dequant_q6k_pair<kExact>(ql, a_col + (q >> 1) * 64, qh, scw, dk, fast, q & 1);
     }
 };
 
-// Q4_K with the quarter as a run-time value (uniform per warp): the same arithmetic as Q4KQuarter
+// two f32 -> f16x2, one rounding, saturating like from_f32
+__device__ __forceinline__ uint32_t pack_f16_sat(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+// Q4_K with the quarter as a run-time value (uniform per warp): the same arithmetic as Q4KQuarter, or (kExact) that of dequantize_f16: d * scale * q - dmin * min in f32, rounded to
+// f16 once.  A nibble becomes an f32 where it lies: in the mantissa of 2^23, which is then taken off, a power of two that goes into the scale.
+template <bool kExact>
 struct Q4KRun {
     static constexpr int kRaw = 12;
     static __device__ __forceinline__ void load(const uint8_t* blk, int q, uint32_t (&raw)[kRaw]) { Q4KQuarter<0>::load(blk + q * 32, blk, raw); }
@@ -435,6 +462,26 @@ struct Q4KRun {
         const bool high = q >= 2;                                    // scale_min_pair: j < 4, or j >= 4 with two bits of each from the words before
         const uint32_t sc2 = high ? (b2 & 0x000f000fu) | ((b0 >> 2) & 0x00300030u) : b0 & 0x003f003fu;
         const uint32_t mn2 = high ? ((b2 >> 4) & 0x000f000fu) | ((b1 >> 2) & 0x00300030u) : b1 & 0x003f003fu;
+        if constexpr (kExact) {
+            const float2 dd = __half22float2(*reinterpret_cast<const __half2*>(&raw[0]));        // (d, dmin); the products with 6-bit integers are exact
+            const float s0 = dd.x * (float)(sc2 & 0xffffu), s1 = dd.x * (float)(sc2 >> 16), n0 = -dd.y * (float)(mn2 & 0xffffu), n1 = -dd.y * (float)(mn2 >> 16);
+            const float2 big = make_float2(-8388608.f, -8388608.f);
+            auto pair = [&](uint32_t x, uint32_t y, uint32_t mask, float s, float n) {            // the nibbles of x and y under the mask
+                const float2 f = add2(make_float2(__uint_as_float((x & mask) | 0x4b000000u), __uint_as_float((y & mask) | 0x4b000000u)), big);
+                const float2 w = fma2(f, make_float2(s, s), make_float2(n, n));
+                return pack_f16_sat(w.x, w.y);
+            };
+            uint32_t v[32];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t x = raw[4 + i], y = x >> 16;                                       // bytes 0, 1 and 2, 3
+                v[2 * i] = pair(x, y, 0xfu, s0, n0);
+                v[2 * i + 1] = pair(x, y, 0xf00u, s0 * (1.f / 256.f), n0);
+                v[16 + 2 * i] = pair(x, y, 0xf0u, s1 * (1.f / 16.f), n1);
+                v[16 + 2 * i + 1] = pair(x, y, 0xf000u, s1 * (1.f / 4096.f), n1);
+            }
+            tc_st32(a_col + q * 32, v);
+        } else
         Q4KQuarter<0>::finish(raw, sc2, mn2, a_col + q * 32);
     }
 };
@@ -541,7 +588,8 @@ __device__ __forceinline__ void m4_unit(const uint8_t* blk, int q, int r7, uint3
 // the compiler's own choice moved between 79 and 95 with the code around.  [Decode step of 16 layers, 8B sizes, 95 against 79 registers: 81.3 / 78.2 us a layer at 2 rows,
 // 85.8 / 80.4 at 9, 94.0 / 89.6 at 32.]
 template <int kMB, int kType> constexpr int bound_threads() { return kMB == 32 && kType == B200_GGML_Q4_K ? 768 : kThreads; }
-template <int kMB, int kType, bool kGrouped>
+// kExact: weights rounded once, for row counts that the dense route would otherwise serve, which rounds them once
+template <int kMB, int kType, bool kGrouped, bool kExact = false>
 __global__ void __launch_bounds__(bound_threads<kMB, kType>(), 1)
 qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_constant__ CUtensorMap wmap1,
                   const __grid_constant__ CUtensorMap wmap2, const __grid_constant__ CUtensorMap xmap, const GemmParams p) {
@@ -859,8 +907,8 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                                mrow, p.scale_bf16, p.debug, p.scale_by, p.scale_sk, p.norm,
                                msg == 0 ? p.zp_seg[0] : (msg == 1 ? p.zp_seg[1] : p.zp_seg[2]), {m4_cur[0], m4_cur[1], m4_cur[2], m4_cur[3]},
                                kPrefetchScales ? 1 : 0};
-                if constexpr (kType == B200_GGML_Q4_K) dequant_run<Q4KRun>(blk, qt, 0, a_col, w_empty(ws), a_free(ab), afp, a_ready(ab), lane, skip);
-                else if constexpr (kType == B200_GGML_Q6_K) dequant_run<Q6KRun>(blk, qt, off, a_col, w_empty(ws), a_free(ab), afp, a_ready(ab), lane, skip);
+                if constexpr (kType == B200_GGML_Q4_K) dequant_run<Q4KRun<kExact>>(blk, qt, 0, a_col, w_empty(ws), a_free(ab), afp, a_ready(ab), lane, skip);
+                else if constexpr (kType == B200_GGML_Q6_K) dequant_run<Q6KRun<kExact>>(blk, qt, off, a_col, w_empty(ws), a_free(ab), afp, a_ready(ab), lane, skip);
                 else
                 switch (qt) {
                     case 0: dequant_unit<kType, 0>(blk, off, a_col, w_empty(ws), a_free(ab), afp, a_ready(ab), lane, skip, mc); break;
@@ -1040,9 +1088,9 @@ int gemm_grid(int64_t n_tiles, int nsb, bool whole_tiles, bool slab_mode) {
     return (int)grid;
 }
 
-template <int kMB, int kType, bool kGrouped>
+template <int kMB, int kType, bool kGrouped, bool kExact = false>
 void launch_kernel(const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, cudaStream_t st) {
-    auto kern = qmatmul_tc_kernel<kMB, kType, kGrouped>;
+    auto kern = qmatmul_tc_kernel<kMB, kType, kGrouped, kExact>;
     ensure_dynamic_smem(reinterpret_cast<const void*>(kern), Cfg<kMB, kType>::kTotal);
     const int grid = kGrouped ? sm_count() : gemm_grid((int64_t)p.n_tiles * p.m_tiles, p.nsb, p.whole_tiles != 0, p.slabs > 0);
     if (p.csplit > 1) {
@@ -1067,6 +1115,7 @@ template <int kType>
 void launch_rows_of(int mb, const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, cudaStream_t st) {
     if (mb == 32) launch<32, kType>(wm, xm, p, st);
     else if (mb == 64) launch<64, kType>(wm, xm, p, st);
+    else if (p.exact) launch_kernel<256, kType, false, true>(wm, xm, p, st);
     else launch<256, kType>(wm, xm, p, st);
 }
 void launch_rows(int mb, int ggml_type, const CUtensorMap* wm, const CUtensorMap& xm, const GemmParams& p, cudaStream_t st) {
@@ -1256,6 +1305,7 @@ int qmatmul_tc_multi(const void* x_f16, int nseg, const void* const* w, float* c
     p.ldy = ldy; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = mt; p.mrows = tile_rows(m); p.accumulate = accumulate;
     p.whole_tiles = m > 64 || use_whole_tiles(tiles) ? 1 : 0;
     p.csplit = m > 64 ? cluster_split((int64_t)tiles * mt, nsb) : 1;
+    p.exact = m >= kSingleRoundingRows ? 1 : 0;
     take_prefetch(p);
     if (slabs_avail > 0) {
         if (m > 64) { set_error(kErrUnsupported, "qmatmul: slabs at %d rows", m); return 0; }

@@ -55,7 +55,49 @@ def test_rows_on_either_side_of_the_dense_path(t, m, k):
     op = pkg.QMatMul.from_arc(pkg.QTensor.from_numpy(w, t, (n, k)))
     ref = G.qmatmul_dequant(x, w, t, n, k)
     y = op.forward(torch.from_numpy(x).to(DEV)).cpu().numpy()
-    assert rel_fro(y, ref) < 1e-3, rel_fro(y, ref)             # both sides: weights and activations rounded to f16 once
+    assert rel_fro(y, ref) < 1e-3, rel_fro(y, ref)
+
+
+@pytest.mark.parametrize("t", [pkg.GgmlType.Q4_K, pkg.GgmlType.Q6_K])
+@pytest.mark.parametrize("rows", [512, 640, 2048])
+@pytest.mark.parametrize("scales", ["small", "large", "mixed"])
+def test_from_512_rows_a_weight_is_rounded_once(t, rows, scales):
+    """unit rows of activations again: what comes back is the f32 weight rounded to f16, half a unit in the last place, whichever route takes the product"""
+    n, k = 136, 2048
+    rng = np.random.default_rng(rows)
+    w = G.random_weight(rng, t, n, k).reshape(n * (k // 256), -1).copy()
+    d = np.full(w.shape[0], {"small": 2e-4, "large": 0.02, "mixed": 2e-4}[scales], np.float16)
+    if scales == "mixed":
+        d[rng.random(w.shape[0]) < 0.03] = 0.02
+    d = (d * rng.uniform(0.8, 1.2, d.shape)).astype(np.float16)          # scales whose products do not fit f16
+    if t == pkg.GgmlType.Q4_K:
+        w[:, 0:2] = d.view(np.uint8).reshape(-1, 2)
+        w[:, 2:4] = (d * np.float16(0.37)).astype(np.float16).view(np.uint8).reshape(-1, 2)
+    else:
+        w[:, 208:210] = d.view(np.uint8).reshape(-1, 2)
+    ref = G.dequantize_weight(w, t, n, k).astype(np.float64)
+    mm = pkg.QMatMul.from_arc(pkg.QTensor.from_numpy(w.reshape(-1), t, (n, k)))
+    # 2^-11 of the value or half of f16's smallest step; a 1/64 more for the second part of a Q6_K scale, which is rounded itself, far below
+    bound = np.abs(ref) * 2.0 ** -11 * (1 + 1 / 64) + 2.0 ** -25 * (1 + 1 / 64) + (2.0 ** -25 if t == pkg.GgmlType.Q6_K else 0.0)
+    for k0 in range(0, k, rows):
+        count = min(rows, k - k0)
+        x = torch.zeros(rows, k)
+        x[torch.arange(count), k0 + torch.arange(count)] = 1.0
+        y = mm.forward(x.to(DEV)).cpu().numpy().astype(np.float64)
+        assert (np.abs(y[:count].T - ref[:, k0:k0 + count]) <= bound[:, k0:k0 + count]).all()
+
+
+@pytest.mark.parametrize("t", [pkg.GgmlType.Q4_K, pkg.GgmlType.Q6_K])
+@pytest.mark.parametrize("m,n", [(1024, 4096), (1025, 4096), (1152, 4096), (1153, 4096), (600, 9600), (700, 14336)])
+def test_rounds_of_tiles_either_side_of_the_dense_path(t, m, n):
+    """one rounding of the weights and one of the activations to f16, 2.0e-4 of a value each in the mean square, 2.9e-4 together, on either route; 3.45e-4 leaves no room for a
+    second rounding of the weights"""
+    k = 2048
+    q = pkg.QTensor.from_numpy(G.random_weight(np.random.default_rng(m), t, n, k), t, (n, k))
+    x = torch.randn(m, k, generator=torch.Generator(device=DEV).manual_seed(m), device=DEV)
+    ref = x.double() @ pkg.dequantize(q).double().T
+    err = float((pkg.QMatMul.from_arc(q).forward(x).double() - ref).norm() / ref.norm())
+    assert err < 2.0 ** -11.5, err
 
 
 def test_the_decode_kernel_leaves_registers_for_its_neighbours():
