@@ -100,6 +100,48 @@ def test_rounds_of_tiles_either_side_of_the_dense_path(t, m, n):
     assert err < 2.0 ** -11.5, err
 
 
+@pytest.mark.parametrize("t", [pkg.GgmlType.Q4_K, pkg.GgmlType.Q6_K])
+@pytest.mark.parametrize("m,n,k", [(65, 200, 2048), (200, 136, 4096), (256, 4096, 2048), (700, 384, 2048), (100, 20000, 2048)])
+def test_accumulate_adds_to_what_is_there(t, m, n, k):
+    """row tiles with the addend: clusters read, add and write; whole tiles of a CTA add in memory"""
+    rng = np.random.default_rng(m)
+    w = G.random_weight(rng, t, n, k)
+    q = pkg.QTensor.from_numpy(w, t, (n, k))
+    x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).to(DEV)
+    start = torch.from_numpy(rng.standard_normal((m, n)).astype(np.float32)).to(DEV) * 3
+    y, L = start.clone(), pkg.lib()
+    ws = torch.empty(int(L.qmatmul_workspace_bytes(C.c_int32(m), C.c_int32(n), C.c_int32(k))), dtype=torch.uint8, device=DEV)
+    L.qmatmul_f32(C.c_void_p(x.data_ptr()), C.c_void_p(q.data.data_ptr()), C.c_void_p(y.data_ptr()), C.c_int32(m), C.c_int32(n), C.c_int32(k), C.c_int32(t), C.c_int32(1),
+                  C.c_void_p(ws.data_ptr()), C.c_size_t(ws.numel()), C.c_int64(torch.cuda.current_stream().cuda_stream))
+    assert L.b200_last_error() == 0
+    product = x.double() @ pkg.dequantize(q).double().T
+    err = float(((y.double() - start.double()) - product).norm() / product.norm())
+    assert err < 1e-3, err
+
+
+@pytest.mark.parametrize("t,m", [(pkg.GgmlType.Q4_K, 100), (pkg.GgmlType.Q6_K, 200), (pkg.GgmlType.Q4_K, 600)])
+def test_clusters_in_a_captured_graph(t, m):
+    rng = np.random.default_rng(m)
+    n, k = 640, 4096
+    op = pkg.QMatMul.from_arc(pkg.QTensor.from_numpy(G.random_weight(rng, t, n, k), t, (n, k)))
+    lin = pkg.Linear(torch.randn(1024, 640, device=DEV).bfloat16(), None)
+    x = torch.randn(m, k, device=DEV)
+    run = lambda: lin.forward(op.forward(x).bfloat16())
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        run()
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        out = run()
+    for seed in (1, 2):
+        x.copy_(torch.randn(m, k, generator=torch.Generator(device=DEV).manual_seed(seed), device=DEV))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, run())
+
+
 def test_the_decode_kernel_leaves_registers_for_its_neighbours():
     """65536 registers an SM: 608 threads of 80 leave room for two blocks of 256 threads of 32 (rotation, norms, activation), of 96 for none"""
     assert 0 < pkg.lib().qmatmul_decode_kernel_registers(C.c_int32(pkg.GgmlType.Q4_K)) <= 80
