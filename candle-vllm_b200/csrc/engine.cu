@@ -178,7 +178,7 @@ void lm_head(b200_llama* m, int B, cudaStream_t st) {
     const int H = m->cfg.hidden;
     const b200_linear& o = m->output;
     const bool ggml_tc = o.kind == B200_LIN_GGML && qmatmul_tc_usable(B, m->vocab_l, H, o.type);
-    if ((ggml_tc && qmatmul_tc_needs_zeroed_output(B, m->vocab_l, H)) || o.kind == B200_LIN_DENSE16) {      // split tiles meet in y through atomics
+    if ((ggml_tc && qmatmul_dispatch_needs_zeroed_output(B, m->vocab_l, H)) || o.kind == B200_LIN_DENSE16) {      // split tiles meet in y through atomics
         launch_pdl(zero_f32_kernel, dim3(sm_count() * 2), dim3(256), 0, st, m->logits, (int64_t)B * m->vocab_l); count_launch();
     }
     linear(m, o, m->xn, m->logits, m->vocab_l, B, m->vocab_l, H, 0, st);

@@ -18,6 +18,8 @@ bool qmatmul_tc_supported(int m, int n, int k, int ggml_type);
 bool qmatmul_tc_usable(int m, int n, int k, int ggml_type);
 // true when some output tile is split across CTAs: y must hold the addend (zeros for a plain product)
 bool qmatmul_tc_needs_zeroed_output(int m, int n, int k);
+// the same for qmatmul_dispatch, which serves many rows in several calls, the last one perhaps of few
+bool qmatmul_dispatch_needs_zeroed_output(int m, int n, int k);
 
 // elementwise.cu internals used by the engine
 void rope_and_cache_impl(float* qkv, void* q_out, void* key_cache, void* value_cache, const float* cos_t, const float* sin_t,

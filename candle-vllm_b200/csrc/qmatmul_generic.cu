@@ -139,7 +139,7 @@ static int rows_per_call(int n, int k) {
     return rows;
 }
 bool qmatmul_tc_usable(int m, int n, int k, int ggml_type) { return m >= 1 && qmatmul_tc_supported(m > 64 ? 64 : m, n, k, ggml_type); }
-static bool dispatch_needs_zeroed_output(int m, int n, int k) {
+bool qmatmul_dispatch_needs_zeroed_output(int m, int n, int k) {
     const int rows = rows_per_call(n, k);
     return (m >= rows && qmatmul_tc_needs_zeroed_output(rows, n, k)) || (m % rows && qmatmul_tc_needs_zeroed_output(m % rows, n, k));
 }
@@ -232,7 +232,7 @@ void qmatmul_f16act(const void* x_f16, const void* w, float* y, int32_t m, int32
                     int32_t ggml_type, int32_t accumulate, int64_t stream) {
     if (m == 0 || n == 0) return;
     if (!qmm_check("qmatmul_f16act", x_f16, w, y, m, n, k, ggml_type)) return;
-    if (!accumulate && qmatmul_tc_usable(m, n, k, ggml_type) && dispatch_needs_zeroed_output(m, n, k))
+    if (!accumulate && qmatmul_tc_usable(m, n, k, ggml_type) && qmatmul_dispatch_needs_zeroed_output(m, n, k))
         cudaMemsetAsync(y, 0, (size_t)m * n * sizeof(float), as_stream(stream));
     qmatmul_dispatch(x_f16, w, y, n, m, n, k, ggml_type, accumulate, as_stream(stream));
 }
@@ -269,7 +269,7 @@ void qmatmul_f32(const float* x, const void* w, float* y, int32_t m, int32_t n, 
     if (qmatmul_tc_usable(m, n, k, ggml_type)) {
         B200_REQUIRE(workspace && workspace_bytes >= qmatmul_workspace_bytes(m, n, k), kErrBadArg,
                      "qmatmul_f32: workspace too small (%zu < %zu)", workspace_bytes, qmatmul_workspace_bytes(m, n, k));
-        cast_k4_zero(x, workspace, (int64_t)m * k, y, !accumulate && dispatch_needs_zeroed_output(m, n, k) ? (int64_t)m * n : 0, as_stream(stream));
+        cast_k4_zero(x, workspace, (int64_t)m * k, y, !accumulate && qmatmul_dispatch_needs_zeroed_output(m, n, k) ? (int64_t)m * n : 0, as_stream(stream));
         qmatmul_dispatch(workspace, w, y, n, m, n, k, ggml_type, accumulate, as_stream(stream));
     } else {
         qmatmul_generic(x, false, w, y, n, m, n, k, ggml_type, accumulate, as_stream(stream));

@@ -237,3 +237,22 @@ def test_engine_argument_errors():
     prep = pkg.prepare_decode([3] * 9, [1] * 9, [[1]] * 9, cfg.block_size)
     with pytest.raises(pkg.BackendError, match="num_seqs"):
         model.decode(prep)
+
+
+def test_rows_past_the_last_whole_call_of_the_head():
+    """2050 sequences: the head's product is one call of 2048 rows and one of 2, whose tiles are split and meet in the logits by addition: the same step twice gives the same
+    logits, and those of the last two sequences are what a step of them alone gives (1e-3 of the largest: sums in another order, one rounding apart)"""
+    cfg = pkg.LlamaConfig(hidden=2048, num_layers=1, num_heads=16, num_kv_heads=2, head_dim=128, ffn=2048, vocab=1024, max_pos=128, block_size=64, max_num_seqs=2050, max_blocks_per_seq=2)
+    w = synthetic.make_weights(cfg, DEV, seed=3)
+    B, nb = 2050, 2050
+    eng = pkg.CacheEngine(cfg.num_layers, cfg.num_kv_heads, cfg.head_dim, pkg.CacheConfig(cfg.block_size, nb))
+    synthetic.fill_kv_cache(eng.gpu_cache, seed=1)
+    model = pkg.GGUFLLaMa(cfg, w, eng.gpu_cache)
+    lens, tokens, tables = [1 + i % 60 for i in range(B)], [(7 * i) % cfg.vocab for i in range(B)], [[i] for i in range(B)]
+    prep = pkg.prepare_decode(lens, tokens, tables, cfg.block_size)
+    _, first = model.decode(prep, want_logits=True)
+    _, second = model.decode(prep, want_logits=True)
+    scale = np.abs(first).max()
+    assert np.isfinite(first).all() and np.abs(second - first).max() < 1e-3 * scale
+    _, alone = model.decode(pkg.prepare_decode(lens[-2:], tokens[-2:], tables[-2:], cfg.block_size), want_logits=True)
+    assert np.abs(first[-2:] - alone).max() < 1e-3 * scale
