@@ -378,6 +378,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
                 }
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();                                                           // every lane's stores and fence, then the arrival
             if (lane == 0) { dirty[w] = bad; mbar_arrive(v_clean); }
             __syncwarp();
         }

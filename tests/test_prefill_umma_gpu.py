@@ -72,6 +72,7 @@ def test_tiles_heads_and_edges(dtype, H, kvh, qlens, cached, window, loud):
     (8, 2, [130, 40], [300, 70], None, [(0, 17, "inf"), (0, 299, "nan"), (0, 301, "inf"), (0, 420, "-inf"), (1, 69, "nan"), (1, 100, "inf")]),
     (8, 2, [300], [500], 96, [(0, 0, "nan"), (0, 410, "inf"), (0, 480, "nan"), (0, 600, "-inf"), (0, 799, "inf")]),     # and behind a window's edge
     (32, 8, [1, 40], [700, 0], None, [(0, 700, "inf"), (1, 39, "nan")]),
+    (8, 2, [200], [2900], None, [(0, 3, "inf"), (0, 100, "-inf"), (0, 2000, "nan"), (0, 3050, "inf")]),              # among the weights in two parts, seen by all
 ])
 def test_values_that_are_not_finite_reach_the_rows_that_see_them_alone(dtype, H, kvh, qlens, cached, window, bad):
     g = torch.Generator(device=DEV)
