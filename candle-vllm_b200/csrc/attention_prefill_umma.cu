@@ -352,30 +352,37 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
             const int k0 = kt0 + j * kKt, rows = min(max(klen - k0, 0), kKt);        // rows of the tile within the context
             // [0, behind): before the last row's first key; [ahead, rows): past the first row's position
             const int behind = min(max(last_lo - k0, 0), rows), ahead = max(min(max(pos0 + 1 - k0, 0), rows), behind);
-            const int count = (behind + rows - ahead) * 16;
-            auto chunk = [&](int idx) {                                             // 16 bytes of a row
-                const int r = (idx >> 4) < behind ? idx >> 4 : (idx >> 4) + ahead - behind, ch = idx & 15;
-                return reinterpret_cast<uint4*>(v + (ch >> 3) * (kTileBytes / 2) + r * 128 + ((ch & 7) << 4));
+            // a lane has one 16-byte column of every fourth row of a range
+            uint8_t* const col = v + ((lane >> 3) & 1) * (kTileBytes / 2) + ((lane & 7) << 4);
+            const int r_own = 2 * w + (lane >> 4);
+            for (int r = rows + r_own; r < kKt; r += 4) *reinterpret_cast<uint4*>(col + r * 128) = make_uint4(0, 0, 0, 0);
+            uint32_t top = 0u;                                                      // largest magnitudes, as two 16-bit integers
+            auto look = [&](int from, int to) {
+                for (int r = from + r_own; r < to; r += 32) {                       // eight loads in flight
+                    uint4 x[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) x[e] = r + 4 * e < to ? *reinterpret_cast<const uint4*>(col + (r + 4 * e) * 128) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        top = __vimax3_u16x2(top, x[e].x & 0x7fff7fffu, x[e].y & 0x7fff7fffu);
+                        top = __vimax3_u16x2(top, x[e].z & 0x7fff7fffu, x[e].w & 0x7fff7fffu);
+                    }
+                }
             };
-            for (int idx = rows * 16 + w * 32 + lane; idx < kKt * 16; idx += 64)
-                *reinterpret_cast<uint4*>(v + ((idx >> 3) & 1) * (kTileBytes / 2) + (idx >> 4) * 128 + ((idx & 7) << 4)) = make_uint4(0, 0, 0, 0);
-            auto bad_bits = [](uint4 x) { return nonfinite<T>(x.x) | nonfinite<T>(x.y) | nonfinite<T>(x.z) | nonfinite<T>(x.w); };
-            uint32_t bad = 0u;
-            for (int idx0 = w * 32 + lane; idx0 < count; idx0 += 8 * 64) {          // eight loads in flight
-                uint4 x[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) x[e] = idx0 + e * 64 < count ? *chunk(idx0 + e * 64) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) bad |= bad_bits(x[e]);
-            }
-            bad = __any_sync(0xffffffffu, bad != 0u) ? 1u : 0u;
+            look(0, behind);
+            look(ahead, rows);
+            const uint32_t bad = __any_sync(0xffffffffu, (top & 0xffffu) >= (Exponent<T>::kMask & 0xffffu) || (top >> 16) >= (Exponent<T>::kMask & 0xffffu)) ? 1u : 0u;
             if (bad) {                                                              // rare
                 auto keep = [](uint32_t u) { return u & ~((nonfinite<T>(u) >> 15) * 0xffffu); };
+                auto clean = [&](int from, int to) {                                // the rows this lane has looked at
 #pragma unroll 1
-                for (int idx = w * 32 + lane; idx < count; idx += 64) {
-                    const uint4 x = *chunk(idx);
-                    *chunk(idx) = make_uint4(keep(x.x), keep(x.y), keep(x.z), keep(x.w));
-                }
+                    for (int r = from + r_own; r < to; r += 4) {
+                        uint4* const at = reinterpret_cast<uint4*>(col + r * 128);
+                        *at = make_uint4(keep(at->x), keep(at->y), keep(at->z), keep(at->w));
+                    }
+                };
+                clean(0, behind);
+                clean(ahead, rows);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();                                                           // every lane's stores and fence, then the arrival
