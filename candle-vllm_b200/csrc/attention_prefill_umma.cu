@@ -4,7 +4,7 @@
 // One CTA = 256 query rows of one kv head: two M = 128 tiles whose rows are (token, head) pairs, 128 / hp tokens x hp heads of the group, so the heads that share
 // keys share the tile and a short portion still fills its rows.  Keys and values are walked in tiles of 128 tokens (two pages).
 //   warps 0-3, 4-7  softmax of tile 0 / 1: thread = row; the row's 128 scores come from TMEM into registers, maximum and sum stay in the thread, P goes back to
-//                   TMEM as 16 bits over the scores it was made from (in two parts in a row's first tile), and the O of the warp's rows is rescaled in TMEM when the maximum of
+//                   TMEM as 16 bits over the scores it was made from (in two parts for a row's first keys), and the O of the warp's rows is rescaled in TMEM when the maximum of
 //                   one of them has grown
 //   warp 8          TMA: Q once (64 KB), then K and V tiles of 32 KB through a ring of five
 //   warp 9          MMA issue: S_i = Q_i K^T (128 x 128 x 128, both operands in shared memory), O_i += P_i V (P from TMEM, V token rows as the MN-major operand)
@@ -106,18 +106,24 @@ template <typename T> __device__ __forceinline__ uint32_t pack2(float lo, float 
 template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, float hi) { __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi); return *reinterpret_cast<uint32_t*>(&v); }
 template <> __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi) { __half2 v = __floats2half2_rn(lo, hi); return *reinterpret_cast<uint32_t*>(&v); }
 // 16-bit values: the bits of an infinity's exponent, and whether one of the two in a word is an infinity or NaN (the addition carries out of a full exponent into bit 15)
-template <typename T> struct Exponent { static constexpr uint32_t kMask = std::is_same<T, __nv_bfloat16>::value ? 0x7f807f80u : 0x7c007c00u, kOne = std::is_same<T, __nv_bfloat16>::value ? 0x00800080u : 0x04000400u;
-    static constexpr float kTiny = std::is_same<T, __nv_bfloat16>::value ? 0x1p-126f : 0x1p-24f; };        // smallest positive (normal) value
+template <typename T> struct Exponent { static constexpr uint32_t kMask = std::is_same<T, __nv_bfloat16>::value ? 0x7f807f80u : 0x7c007c00u, kOne = std::is_same<T, __nv_bfloat16>::value ? 0x00800080u : 0x04000400u; };
 template <typename T> __device__ __forceinline__ uint32_t nonfinite(uint32_t w) { return ((w & Exponent<T>::kMask) + Exponent<T>::kOne) & 0x80008000u; }
 template <typename T> __device__ __forceinline__ float half_to_f32(uint32_t h);
 template <> __device__ __forceinline__ float half_to_f32<__nv_bfloat16>(uint32_t h) { return __uint_as_float(h << 16); }
 template <> __device__ __forceinline__ float half_to_f32<__half>(uint32_t h) { return __half2float(__ushort_as_half((unsigned short)h)); }
-// two f32 -> 16 bits, rounded towards 0
-template <typename T> __device__ __forceinline__ uint32_t pack2_down(float lo, float hi) {
-    uint32_t r;
-    if constexpr (std::is_same<T, __nv_bfloat16>::value) asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    else asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
+// two weights as two 16-bit parts each: the first rounded down from just below the weight, the second what is left, above 0 wherever the first is
+template <typename T> __device__ __forceinline__ void two_parts_of(float2 x, uint32_t& first, uint32_t& second) {
+    const float2 below = fma2(x, make_float2(-0x1p-20f, -0x1p-20f), x);
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) asm("cvt.rz.bf16x2.f32 %0, %1, %2;" : "=r"(first) : "f"(below.y), "f"(below.x));
+    else asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(first) : "f"(below.y), "f"(below.x));
+    const float2 rest = fma2(make_float2(half_to_f32<T>(first & 0xffffu), half_to_f32<T>(first >> 16)), make_float2(-1.f, -1.f), x);
+    second = pack2<T>(rest.x, rest.y);
+    if constexpr (std::is_same<T, __half>::value) {                     // (f16 may round it to 0: its smallest step then)
+        const uint32_t step = 0x00010001u;
+        const __half2 least = __hmin2(*reinterpret_cast<const __half2*>(&first), *reinterpret_cast<const __half2*>(&step));
+        const __half2 r = __hmax2(*reinterpret_cast<const __half2*>(&second), least);
+        second = *reinterpret_cast<const uint32_t*>(&r);
+    }
 }
 __device__ __forceinline__ uint32_t ld1(uint32_t taddr) {
     uint32_t v;
@@ -149,13 +155,14 @@ __device__ __forceinline__ void add_nonfinite(const T* values, const uint32_t* t
     }
 }
 
-// P of a row's first key tile is held as two 16-bit parts (the second in the half of S that P leaves free) and multiplied twice: with few keys, single weights are large
-// and their rounding is what the result's error consists of.  In the later tiles P is one part, and the maximum is up to date in every tile, so that a row's largest weight
-// is 1, which 16 bits hold exactly.  The first part is rounded down and the second kept above 0, so that a value that is infinite stays so.
+// P of a row's first keys is held as two 16-bit parts (the second in the half of S that P leaves free) and multiplied twice: with few keys, single weights are large and their
+// rounding is what the result's error consists of.  Everywhere else P is one part, and the maximum is up to date in every tile, so that a row's largest weight is 1, which
+// 16 bits hold exactly.  The first part is rounded down and the second kept above 0, so that a value that is infinite stays so.  64 keys, 128 in contexts of more than 2048.
 // [Error of the result against 64 bits, relative to the mma.sync kernel's (one part, maximum up to date every 32 keys), restated for contexts of 40 to 8192 keys: with a
-// maximum that may lag by 2^8 1.3 to 2 % above it for scores of deviation 1, 13 to 26 % above for 3; up to date, one part: 0 to 2 % above; so: 22 % below to 0.1 % above.
-// It costs 7 to 10 %: three prompts of 280 to 700 tokens on cached prefixes 80 -> 86 us, 8192 tokens 562 -> 617; two tiles in two parts 2 and 8 us more.]
-constexpr int kTwoPartTiles = 1;
+// maximum that may lag by 2^8 1.3 to 2 % above it for scores of deviation 1, 13 to 26 % above for 3; up to date, one part: 0 to 2.3 % above; so: 17 % below to 0.2 % above.
+// us, with lag / up to date / so: three prompts of 280 to 700 tokens on cached prefixes 77.4 / 80.0 / 81.2, four of 700 on prefixes of 90 37.2 / 37.2 / 39.1, 300 tokens on
+// 4000 75.8 / 83.9 / 84.1, 8192 tokens 561 / 601 / 608.]
+__device__ __forceinline__ int two_part_keys(int klen) { return klen > 2048 ? kKt : kKt / 2; }
 
 template <typename T>
 __global__ void __launch_bounds__(kThreadsU, 1)
@@ -191,7 +198,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         const int toks = min(tp, qlen - q0 - i * tp);
         nk[i] = toks > 0 ? max((pos0 + i * tp + toks - 1 - kt0) / kKt + 1, 1) : 0;      // (at least one: rows before a context that is too short see nothing and are written as 0)
     }
-    const int n = max(nk[0], nk[1]);
+    const int n = max(nk[0], nk[1]), two_keys = two_part_keys(klen);
     // tiles in which a row of the CTA has hidden keys: past the first row's position, or before the last row's first key
     const int pos_last = pos0 + min(2 * tp, qlen - q0) - 1;
     int last_lo = p.window > 0 ? max(0, pos_last - p.window + 1) : 0;
@@ -321,9 +328,10 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
                         tc_mma_ts(tmem + 256 + i * 128, tmem + i * 128 + k * 8, b + (uint64_t)(k * 16 * 128 >> 4), idesc_o, (add || k > 0) ? 1u : 0u);
-                    if (j < kTwoPartTiles) {
+                    if (j == 0) {
 #pragma unroll
-                        for (int k = 0; k < 8; ++k) tc_mma_ts(tmem + 256 + i * 128, tmem + i * 128 + 64 + k * 8, b + (uint64_t)(k * 16 * 128 >> 4), idesc_o, 1u);
+                        for (int k = 0; k < 8; ++k)
+                            if (k * 16 < two_keys) tc_mma_ts(tmem + 256 + i * 128, tmem + i * 128 + 64 + k * 8, b + (uint64_t)(k * 16 * 128 >> 4), idesc_o, 1u);
                     }
                     if (j + 1 == nk[i]) tc_commit(o_full(i));
                 }
@@ -461,15 +469,12 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
                     float2 x = fma2(make_float2(__uint_as_float(s[c * 16 + 2 * e]), __uint_as_float(s[c * 16 + 2 * e + 1])), sc, sb2);
                     x.x = ex2(x.x); x.y = ex2(x.y);
                     part = add2(part, x);
-                    pk[e] = kTwo ? pack2_down<T>(x.x, x.y) : pack2<T>(x.x, x.y);
-                    if constexpr (kTwo) {
-                        const float h0 = half_to_f32<T>(pk[e] & 0xffffu), h1 = half_to_f32<T>(pk[e] >> 16);
-                        low[e] = pack2<T>(fmaxf(x.x - h0, h0 > 0.f ? Exponent<T>::kTiny : 0.f), fmaxf(x.y - h1, h1 > 0.f ? Exponent<T>::kTiny : 0.f));
-                    }
+                    if (kTwo && c * 16 < two_keys) two_parts_of<T>(x, pk[e], low[e]);
+                    else pk[e] = pack2<T>(x.x, x.y);
                 }
                 l2 = add2(l2, part);
                 st8(s_t + c * 8, pk);
-                if constexpr (kTwo) st8(s_t + 64 + c * 8, low);
+                if (kTwo && c * 16 < two_keys) st8(s_t + 64 + c * 8, low);
             }
             if (kHides && (!kTwo || hides(j))) {                                    // (the two-part step serves both kinds)
                 if (!mbar_wait_or_flag(v_clean, scans & 1, give_up)) return false;
@@ -493,7 +498,6 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
             if (lane == 0) mbar_arrive(p_ready(i));
             return true;
         };
-        static_assert(kTwoPartTiles == 1, "the first step below");
         if (nki > 0) ok = step(0, std::true_type{}, std::true_type{});
         for (int j = 1; j < nki && ok; ++j) ok = hides(j) ? step(j, std::true_type{}, std::false_type{}) : step(j, std::false_type{}, std::false_type{});
         if (nki > 0 && ok && mbar_wait_or_flag(o_full(i), 0, give_up)) {
