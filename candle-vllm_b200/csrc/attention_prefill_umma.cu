@@ -262,7 +262,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
 #pragma unroll
             for (int kv = 0; kv < 2; ++kv, ++it) {
                 const int s = it % kRing;
-                ok = ok && mbar_wait_or_flag(kv_empty(s), ((it / kRing) & 1) ^ 1, give_up) && !given_up(give_up);
+                ok = ok && mbar_wait_or_flag(kv_empty(s), ((it / kRing) & 1) ^ 1, give_up);
                 if (!ok) break;
                 if (leader) {
                     const CUtensorMap* map = kv ? &vmap : &kmap;

@@ -444,7 +444,7 @@ dense_gemm_pair_kernel(const __grid_constant__ CUtensorMap amap, const __grid_co
             tile_coords(t, ta, tb);
             for (int kb = 0; kb < nkb && ok; ++kb, ++it) {
                 const int s = it % kS;
-                ok = mbar_wait_or_flag(empty(s), ((it / kS) & 1) ^ 1, give_up) && !given_up(give_up);
+                ok = mbar_wait_or_flag(empty(s), ((it / kS) & 1) ^ 1, give_up);
                 if (ok && leader) {
                     if (rank == 0) mbar_expect_tx(full(s), 2 * C::kStageBytes);
                     const uint32_t dst = smem_base + s * C::kStageBytes, bar = cluster_map(full(s), 0);

@@ -81,7 +81,6 @@ __device__ __forceinline__ bool mbar_wait_or_flag(uint32_t bar, uint32_t parity,
     }
     return __all_sync(0xffffffffu, ok);
 }
-__device__ __forceinline__ bool given_up(const GiveUp& g) { return __any_sync(0xffffffffu, *g.flag != 0u); }
 // Copies on their way into this CTA's shared memory are waited for before it leaves: barriers full0 + 8 (k % ring) of the last `ring` of `issued` loads, for about a second
 // in all.  (After a wait was given up only: otherwise their readers have waited.)
 __device__ __forceinline__ void drain_loads(uint32_t full0, int ring, int issued) {
