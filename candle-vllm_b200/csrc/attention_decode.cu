@@ -51,7 +51,7 @@ constexpr int kMaxSeqs = 1024;
 // (K: LDS.128 of a token row; V: the transposing 8-bit ldmatrix of sm_100a) -- there is no f16 staging tile.  [A first version
 // expanded each tile into a per-warp f16 staging tile (LDS + cvt + STS, then the 16-bit ldmatrix code): 0.45-0.59 of the HBM peak,
 // bound by the shared-memory round trip and the 24 KB per warp it cost; profiles/r02_fp8_attention.md.]
-#ifndef B200_FP8_WARPS          // tuning aids (tools/gpu_run_r02m.sh builds variants)
+#ifndef B200_FP8_WARPS          // tuning aids
 #define B200_FP8_WARPS 8
 #endif
 #ifndef B200_FP8_STAGES
@@ -480,7 +480,7 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_
             }
             // ---- O += P V : 2 k-steps (16 tokens) x 16 n-tiles (8 dims) ---------------------------
             if constexpr (kFp8) {
-                // ldmatrix.m16n16.trans.b8 (sm_100a; fragment layout probed, tools/probes/ldmatrix_b8_probe.cu): with row addresses
+                // ldmatrix.m16n16.trans.b8 (sm_100a; fragment layout probed): with row addresses
                 // r = 0..15 from lanes 0..15 (x2: a second matrix from lanes 16..31), lane (g, t) receives bytes (rows 4t..4t+3, column g)
                 // and (rows 4t..4t+3, column g + 8).  Rows are tokens, columns dims of a 16-byte chunk; matrix row r is pointed at
                 // token (r >> 2) + 4 (r & 3) of the k-step, so the low half-word of a register holds tokens (t, t + 4) = the k slots

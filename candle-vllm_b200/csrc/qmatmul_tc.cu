@@ -521,7 +521,7 @@ __device__ __forceinline__ void dequant_unit(const uint8_t* blk, int off, uint32
 
 // GGML blocks: the quarter at run time, so that all sixteen warps run ONE body.  As four copies, one per quarter, the hot code competed for the instruction cache.
 // [Q6_K MLP of 4096 x 14336, four copies and fourteen loads against one and eight: 168 -> 128 us at 203 rows, 106 -> 82 at 32, 471 -> 360 at 600; four copies with eight
-// loads: 170, 106, 475.  Q4_K (its copies did fit): 62 -> 62 us at 32 rows.]
+// loads: 170, 106, 475.  Q4_K: 62 -> 62 us at 32 rows, a captured decode step of 16 layers 95.4 -> 93.8 us a layer.]
 template <typename Q>
 __device__ __forceinline__ void dequant_run(const uint8_t* blk, int q, int off, uint32_t a_col, uint32_t w_empty_bar, uint32_t a_free_bar, uint32_t a_free_parity,
                                             uint32_t a_ready_bar, int lane, bool skip) {
