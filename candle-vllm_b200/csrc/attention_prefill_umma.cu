@@ -18,8 +18,8 @@
 //
 // Bound: exp2 (16 per clock and SM) and the tensor pipe need 1024 clocks each for a 128 x 128 tile; the counters say 42 % of either, and 32 % of the issue slots (4096 tokens).  What
 // takes the time is a tile's chain -- scores, maximum, exponentials, P, rescaled O -- with two tiles in flight per SM, and power in a loop.
-// us, mma.sync kernel / this one (B200, bf16, 32 heads / 8 kv heads): 8192 tokens 2290 / 617, three prompts of 280 to 700 tokens on cached prefixes 238 / 83, 300 tokens on 4000
-// 167 / 86, 32 single tokens on 1000 164 / 53, one on 700 26 / 18.
+// us, mma.sync kernel / this one (B200, bf16, 32 heads / 8 kv heads): 8192 tokens 2290 / 603, three prompts of 280 to 700 tokens on cached prefixes 238 / 82, 300 tokens on 4000
+// 167 / 82, 32 single tokens on 1000 164 / 53, one on 700 26 / 18.
 #include <cuda.h>
 
 #include <type_traits>
@@ -162,8 +162,8 @@ __device__ __forceinline__ void add_nonfinite(const T* values, const uint32_t* t
 // 16 bits hold exactly.  The first part is rounded down and the second kept above 0, so that a value that is infinite stays so.  64 keys, 128 in contexts of more than 2048.
 // [Error of the result against 64 bits, relative to the mma.sync kernel's (one part, maximum up to date every 32 keys), restated for contexts of 40 to 8192 keys: with a
 // maximum that may lag by 2^8 1.3 to 2 % above it for scores of deviation 1, 13 to 26 % above for 3; up to date, one part: 0 to 2.3 % above; so: 17 % below to 0.2 % above.
-// us, with lag / up to date / so: three prompts of 280 to 700 tokens on cached prefixes 77.4 / 80.0 / 81.2, four of 700 on prefixes of 90 37.2 / 37.2 / 39.1, 300 tokens on
-// 4000 75.8 / 83.9 / 84.1, 8192 tokens 561 / 601 / 608.]
+// us, with lag / so: three prompts of 280 to 700 tokens on cached prefixes 77.4 / 81.8, four of 700 on prefixes of 90 37.2 / 39.3, 300 tokens on 4000 75.8 / 82.0, 8192 tokens
+// 561 / 603.]
 __device__ __forceinline__ int two_part_keys(int klen) { return klen > 2048 ? kKt : kKt / 2; }
 
 template <typename T>
@@ -442,22 +442,13 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
 #pragma unroll
             for (int c = 4; c < 128; ++c) mx[c & 3] = fmaxf(mx[c & 3], __uint_as_float(s[c]));
             const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * p.scale_log2;
-            if (__any_sync(0xffffffffu, top > m)) {
+            const bool grown = __any_sync(0xffffffffu, top > m);
+            float corr = 1.f;
+            if (grown) {
                 const float mn = fmaxf(m, top);
-                const float corr = mn == -INFINITY ? 1.f : ex2(m - mn);
+                corr = mn == -INFINITY ? 1.f : ex2(m - mn);
                 m = mn;
                 l2.x *= corr; l2.y *= corr;
-                if (j > 0) {
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        uint32_t o[16];
-                        tc_ld16(o_t + c * 16, o);
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * corr);
-                        tc_st16(o_t + c * 16, o);
-                    }
-                }
             }
             // a row that has seen no visible key yet keeps m = -inf: subtract 0, so that its exp2 are 0 and never NaN
             const float sub = m == -INFINITY ? 0.f : -m;
@@ -478,6 +469,21 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
                 st8(s_t + c * 8, pk);
                 if (kTwo && c * 16 < two_keys) st8(s_t + 64 + c * 8, low);
             }
+            // O of the warp's rows, after the exponentials: its loads run beside what they leave in flight [before them: 8192 tokens 612 us, 300 tokens on 4000 85]
+            if (grown && j > 0) {
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        uint32_t o[16];
+                        tc_ld16(o_t + c * 16, o);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int e = 0; e < 16; e += 2) {
+                            const float2 r = fma2(make_float2(__uint_as_float(o[e]), __uint_as_float(o[e + 1])), make_float2(corr, corr), make_float2(-0.f, -0.f));
+                            o[e] = __float_as_uint(r.x); o[e + 1] = __float_as_uint(r.y);
+                        }
+                        tc_st16(o_t + c * 16, o);
+                    }
+                }
             if (kHides && (!kTwo || hides(j))) {                                    // (the two-part step serves both kinds)
                 if (!mbar_wait_or_flag(v_clean, scans & 1, give_up)) return false;
                 ++scans;
