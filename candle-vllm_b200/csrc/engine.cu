@@ -152,16 +152,6 @@ void linear(b200_llama* m, const b200_linear& l, const void* x16, float* y, int6
         default: set_error(kErrUnsupported, "engine: linear kind %d", l.kind);
     }
 }
-// weight bytes of a linear the tcgen05 dequant-GEMM streams (0: another kernel serves it) -- for the L2 prefetch hint
-size_t lin_stream_bytes(const b200_linear& l, int n, int k) {
-    if (l.kind == B200_LIN_GGML) return l.type == B200_GGML_Q4_K ? (size_t)n * (k / 256) * 144 : (l.type == B200_GGML_Q6_K ? (size_t)n * (k / 256) * 210 : 0);
-    return 0;       // int4: measured slightly slower with the hint (5.81 vs 5.74 ms per step, config 3) -- its scale loads already queue at the L2
-}
-void prefetch_next(std::initializer_list<std::pair<const b200_linear*, std::pair<int, int>>> next) {
-    const void* ptrs[3]; size_t bytes[3]; int n = 0;
-    for (const auto& e : next) { if (n == 3) break; ptrs[n] = e.first->w; bytes[n] = lin_stream_bytes(*e.first, e.second.first, e.second.second); if (bytes[n]) ++n; }
-    qmatmul_tc_prefetch_next(n, ptrs, bytes);
-}
 // several int4 linears over the same activations (QKV, gate|up) as one launch when they share group size, scale dtype and zero-point form
 bool marlin_fusable(std::initializer_list<const b200_linear*> ls) {
     const b200_linear* f = *ls.begin();
@@ -352,9 +342,7 @@ int forward(b200_llama* m, int B, cudaStream_t st, bool linear_only = false) {
     for (int l = 0; l < c.num_layers; ++l) {
         const b200_llama_layer_ex& w = m->layers[l];
         if (!fused_ar || l == 0) rms_norm(m->x, w.attn_norm, m->xn, B, H, c.rms_eps, fmt, s);
-        // QKV / gate / up accumulate (split-K) into buffers that their consumers leave zeroed.  Every GEMM of the chain tells the L2 what
-        // the NEXT one will stream (prefetch_next): fetched from the tail of the launch, while HBM is otherwise idle
-        prefetch_next({{&w.wo, {H, qd}}});
+        // QKV / gate / up accumulate (split-K) into buffers that their consumers leave zeroed.
         if (all_ggml) {   // fused QKV: three weight matrices, one launch
             const void* ws[3] = {w.wq.w, w.wk.w, w.wv.w};
             const int ts[3] = {w.wq.type, w.wk.type, w.wv.type}, ns[3] = {qd, kd, kd};
@@ -379,7 +367,6 @@ int forward(b200_llama* m, int B, cudaStream_t st, bool linear_only = false) {
                                c.block_size, c.max_blocks_per_seq, m->num_blocks, 1.0f / sqrtf((float)hd), 0.f, 0,
                                B200_BF16, c.kv_dtype, B200_KV_FLASH, fmt, m->attn_ws, m->attn_ws_bytes, s);
         }
-        prefetch_next({{&w.w1, {m->ffn_l, H}}, {&w.w3, {m->ffn_l, H}}});
         if (c.tp_world == 1) {
             linear(m, w.wo, m->attn16, m->x, H, B, H, qd, 1, st);                        // x += wo(attn)
         } else if (fused_ar) {
@@ -393,7 +380,6 @@ int forward(b200_llama* m, int B, cudaStream_t st, bool linear_only = false) {
             add_f32(m->x, m->partial, (int64_t)B * H, s);
         }
         if (!fused_ar) rms_norm(m->x, w.ffn_norm, m->xn, B, H, c.rms_eps, fmt, s);
-        prefetch_next({{&w.w2, {H, m->ffn_l}}});
         if (all_ggml) {   // fused gate | up
             const void* ws[2] = {w.w1.w, w.w3.w};
             const int ts[2] = {w.w1.type, w.w3.type}, ns[2] = {m->ffn_l, m->ffn_l};
@@ -409,10 +395,6 @@ int forward(b200_llama* m, int B, cudaStream_t st, bool linear_only = false) {
             linear(m, w.w3, m->xn, m->up, m->ffn_l, B, m->ffn_l, H, 0, st);
         }
         silu_mul_zero_src_fmt(m->gate, m->up, m->act16, (int64_t)B * m->ffn_l, fmt, s);      // act = silu(gate)*up; gate/up re-zeroed
-        if (l + 1 < c.num_layers) {
-            const b200_llama_layer_ex& nx = m->layers[l + 1];
-            prefetch_next({{&nx.wq, {qd, H}}, {&nx.wk, {kd, H}}, {&nx.wv, {kd, H}}});
-        }
         if (c.tp_world == 1) {
             linear(m, w.w2, m->act16, m->x, H, B, H, m->ffn_l, 1, st);                   // x += w2(act)
         } else if (fused_ar) {

@@ -106,6 +106,10 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
         " [%0], [%1, {%3, %4}], [%2], %5;" ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "l"(policy)
         : "memory");
 }
+// contiguous bytes: both addresses and the size are multiples of 16
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
 // one elected lane of a converged warp (warp-uniform predicate source for the single-thread tcgen05 / TMA issue)
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred;
