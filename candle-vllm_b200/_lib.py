@@ -129,6 +129,38 @@ def typed(name: str, restype, *argtypes):
     return f
 
 
+_calls_module = None
+
+
+def calls():
+    """The natively entered operators (``csrc/py_calls.cpp``), or False where they are not built: the callers then go through ctypes."""
+    global _calls_module
+    if _calls_module is None:
+        path = os.path.join(_HERE, "_calls.so")
+        if not os.path.exists(path) or not os.path.exists(_SO):
+            _calls_module = False
+            return False
+        import importlib.machinery
+        import importlib.util
+        spec = importlib.util.spec_from_loader("_calls", importlib.machinery.ExtensionFileLoader("_calls", path))
+        try:
+            m = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(m)
+            lib()
+            m.bind(_SO)
+            _calls_module = m
+        except ImportError as e:            # built against another torch or library
+            import warnings
+            warnings.warn(f"{path} cannot be used ({e}): operators are called through ctypes")
+            _calls_module = False
+    return _calls_module
+
+
+def fail(what: str, code: int) -> None:
+    """raise the error a natively entered call came back with"""
+    raise BackendError(f"{what}: {lib().b200_last_error_message().decode()} (code {code})")
+
+
 def check(what: str = "") -> None:
     """Raise BackendError if the last call on this thread recorded an error."""
     L = lib()

@@ -22,7 +22,7 @@ from typing import Dict, List, Optional, Sequence, Union
 import numpy as np
 import torch
 
-from ._lib import BackendError, check, lib, require_device, typed
+from ._lib import BackendError, calls, check, fail, lib, require_device, typed
 
 
 class DType:
@@ -270,6 +270,16 @@ class PagedAttention:
         """q [T, heads, hd], k/v [T, kvh, hd] (model dtype).  Writes k/v into the cache at
         ``slot_mapping`` first (K3), then attends over the paged cache (K1 decode / K2 prefill).
         Returns [T, heads, hd]."""
+        native = calls()
+        if native and out_dtype is None and key is not None:
+            m = input_metadata
+            r = native.paged_attention(m.is_prefill, query, key, value, key_cache, value_cache, m.slot_mapping, m.block_tables, m.context_lens, m.cu_seqlens_q, m.cu_seqlens_k, self._ws,
+                                       self.num_attention_heads, self.num_key_value_heads, self.head_dim, m.max_seqlen_q, self.sliding_window or 0, self.scale,
+                                       softcapping or 0.0, self.fp8_kvcache)
+            if r is not None:
+                if r.__class__ is int:
+                    fail("reshape_and_cache" if r < 0 else "PagedAttention.forward", abs(r))
+                return r
         _cuda(query, "query")
         if key_cache is None or value_cache is None:
             raise BackendError("PagedAttention.forward requires a KV cache on this backend")
@@ -375,6 +385,12 @@ class QMatMul:
         return cls(qtensor)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        native = calls()
+        if native:
+            n, k = self.w.shape
+            r = native.qmatmul(x, self.w.data, n, k, self.w.ggml_type, self._ws)
+            if r is not None:
+                return r if r.__class__ is not int else fail("QMatMul.forward", r)
         _cuda(x, "x")
         n, k = self.w.shape
         if x.shape[-1] != k:
@@ -454,6 +470,11 @@ class Linear:
         self.bias = None if bias is None else _cuda(bias, "bias").to(weight.dtype).contiguous()
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        native = calls()
+        if native:
+            r = native.linear(x, self.weight, self.bias)
+            if r is not None:
+                return r if r.__class__ is not int else fail("Linear.forward", r)
         n, k = self.weight.shape
         if x.dtype != self.weight.dtype:
             raise BackendError(f"Linear: activation dtype {x.dtype} != weight dtype {self.weight.dtype}")
@@ -567,6 +588,11 @@ def fused_rope(q: torch.Tensor, k: torch.Tensor, cos: torch.Tensor, sin: torch.T
 
 
 def silu_mul(gate: torch.Tensor, up: torch.Tensor, out_dtype=torch.float32) -> torch.Tensor:
+    native = calls()
+    if native and out_dtype is torch.float32:
+        r = native.silu_mul(gate, up)
+        if r is not None:
+            return r if r.__class__ is not int else fail("silu_mul", r)
     _cuda(gate, "gate"); require_device()
     g, u = gate.contiguous().float(), up.contiguous().float()
     out = torch.empty(g.shape, dtype=out_dtype, device=g.device)

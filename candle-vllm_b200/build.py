@@ -62,6 +62,33 @@ def so_path(group=None) -> str:
     return SO if group is None else os.path.join(HERE, f"libb200backend.{group}.so")
 
 
+CALLS = os.path.join(HERE, "_calls.so")
+
+
+def build_calls(force: bool = False, verbose: bool = False) -> str:
+    """``_calls.so``: the operators of ``csrc/py_calls.cpp`` as Python functions.  Needs the headers of torch and of Python; without it the package calls the library through ctypes."""
+    src = os.path.join(CSRC, "py_calls.cpp")
+    if not force and not _newer(CALLS, [src] + glob.glob(os.path.join(HERE, "..", "include", "*.h"))):
+        return CALLS
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension as ext
+    inc = [a for d in ext.include_paths() + [os.path.join(os.path.dirname(os.path.dirname(NVCC)), "include"), sysconfig.get_paths()["include"], os.path.join(HERE, "..", "include")]
+           for a in ("-I", d)]
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    tmp = f"{CALLS}.{os.getpid()}.tmp"
+    cmd = [CCBIN, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + inc + [src, "-o", tmp, "-L", libs,
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-ldl", f"-Wl,-rpath,{libs}"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode:
+        sys.stderr.write(r.stdout + r.stderr)
+    if r.returncode:
+        raise RuntimeError("py_calls.cpp failed")
+    os.replace(tmp, CALLS)
+    return CALLS
+
+
 def build(force: bool = False, verbose: bool = False, group=None) -> str:
     os.makedirs(OBJ, exist_ok=True)
     srcs = sorted(glob.glob(os.path.join(CSRC, "*.cu")))
@@ -98,6 +125,8 @@ def build(force: bool = False, verbose: bool = False, group=None) -> str:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
         os.replace(tmp, SO)              # a reader never sees a half-written library
+    if group is None:
+        build_calls(force, verbose)
     return SO
 
 
