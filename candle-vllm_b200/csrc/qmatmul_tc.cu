@@ -66,8 +66,8 @@ struct Cfg {
     static constexpr int kXOff = 0;                                // 1024-aligned (128-byte swizzle)
     static constexpr int kWOff = kXStages * kXBytes;
     static constexpr int kScOff = kWOff + kWStages * kWBytes;
-    static constexpr int kBars = kScOff + kWStages * kScBytes;     // w_full[kW] w_empty[kW] x_full[kX] x_empty[kX] a_ready[] a_free[] d_full[] d_empty[] d_last
-    static constexpr int kNumBars = 2 * kWStages + 2 * kXStages + 2 * kGroups + 2 * kDBufs + 1;
+    static constexpr int kBars = kScOff + kWStages * kScBytes;     // w_full[2 kW] w_empty[kW] x_full[kX] x_empty[kX] a_ready[] a_free[] d_full[] d_empty[] d_last
+    static constexpr int kNumBars = 3 * kWStages + 2 * kXStages + 2 * kGroups + 2 * kDBufs + 1;
     static constexpr int kTmemSlot = kBars + kNumBars * 8;
     static constexpr int kTotal = kTmemSlot + 16;
     static_assert(kWStages >= 3 && kWStages >= kGroups, "W ring too shallow");
@@ -499,15 +499,19 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t smem_base = smem_u32(smem);
     const uint32_t bars = smem_base + C::kBars;
+    // Two w_full barriers for a stage, in turn: a group of warps meets a stage only where it takes the unit, so that it does not follow the phases that other groups wait for, and a
+    // wait for a phase's parity must not find the phase before last.  Barrier it % 2 kW can: when a group comes to unit `it` it has taken it - kGroups, whose load was issued after
+    // every unit up to it - kGroups - kW had been read, it - 2 kW among them.
+    static_assert(kW >= kGroups, "barriers of the W ring");
     auto w_full = [&](int s) { return bars + s * 8; };
-    auto w_empty = [&](int s) { return bars + (kW + s) * 8; };
-    auto x_full = [&](int s) { return bars + (2 * kW + s) * 8; };
-    auto x_empty = [&](int s) { return bars + (2 * kW + kX + s) * 8; };
-    auto a_ready = [&](int b) { return bars + (2 * kW + 2 * kX + b) * 8; };
-    auto a_free = [&](int b) { return bars + (2 * kW + 2 * kX + kGroups + b) * 8; };
-    auto d_full = [&](int b) { return bars + (2 * kW + 2 * kX + 2 * kGroups + b) * 8; };
-    auto d_empty = [&](int b) { return bars + (2 * kW + 2 * kX + 2 * kGroups + kDBufs + b) * 8; };
-    const uint32_t d_last = bars + (2 * kW + 2 * kX + 2 * kGroups + 2 * kDBufs) * 8;
+    auto w_empty = [&](int s) { return bars + (2 * kW + s) * 8; };
+    auto x_full = [&](int s) { return bars + (3 * kW + s) * 8; };
+    auto x_empty = [&](int s) { return bars + (3 * kW + kX + s) * 8; };
+    auto a_ready = [&](int b) { return bars + (3 * kW + 2 * kX + b) * 8; };
+    auto a_free = [&](int b) { return bars + (3 * kW + 2 * kX + kGroups + b) * 8; };
+    auto d_full = [&](int b) { return bars + (3 * kW + 2 * kX + 2 * kGroups + b) * 8; };
+    auto d_empty = [&](int b) { return bars + (3 * kW + 2 * kX + 2 * kGroups + kDBufs + b) * 8; };
+    const uint32_t d_last = bars + (3 * kW + 2 * kX + 2 * kGroups + 2 * kDBufs) * 8;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + C::kTmemSlot);
     constexpr bool moe = kGrouped;
     constexpr bool kClusters = kMB == 256 && !kGrouped;
@@ -561,7 +565,7 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         }
     };
     auto w_load = [&]() {                               // the next unit's weights into the ring
-        const int s = w_it % kW;
+        const int s = w_it % kW, full = w_it % (2 * kW);
         mbar_wait(w_empty(s), ((w_it / kW) & 1) ^ 1);
         const CUtensorMap* wm = w_ti.sg == 0 ? &wmap0 : (w_ti.sg == 1 ? &wmap1 : &wmap2);
         if (w_leader) {
@@ -569,17 +573,17 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
             // rounded down to 16 -- TMA box starts must be 16-byte aligned
             const uint32_t dst = smem_base + C::kWOff + s * C::kWBytes;
             if constexpr (kType == kTypeM4) {
-                mbar_expect_tx(w_full(s), C::kWBytes + w_sc_bytes);
-            } else mbar_expect_tx(w_full(s), C::kWBytes);
+                mbar_expect_tx(w_full(full), C::kWBytes + w_sc_bytes);
+            } else mbar_expect_tx(w_full(full), C::kWBytes);
             if constexpr (kType == kTypeF8) {           // two 128-byte-swizzled boxes per unit
-                tma_load_2d(dst, wm, w_full(s), w_sb * 256, w_ti.wrow, pol_w);
-                tma_load_2d(dst + 16384, wm, w_full(s), w_sb * 256 + 128, w_ti.wrow, pol_w);
+                tma_load_2d(dst, wm, w_full(full), w_sb * 256, w_ti.wrow, pol_w);
+                tma_load_2d(dst + 16384, wm, w_full(full), w_sb * 256 + 128, w_ti.wrow, pol_w);
             } else
-                tma_load_2d(dst, wm, w_full(s), kType == B200_GGML_Q4_K ? w_sb * 144 : (is_4bit_rows(kType) ? w_sb * 128 : ((w_sb * 210) & ~15)), w_ti.wrow, pol_w);
+                tma_load_2d(dst, wm, w_full(full), kType == B200_GGML_Q4_K ? w_sb * 144 : (is_4bit_rows(kType) ? w_sb * 128 : ((w_sb * 210) & ~15)), w_ti.wrow, pol_w);
         }
         __syncwarp();
         if constexpr (kType == kTypeM4) {               // (after the expected bytes are known to the barrier)
-            if (w_piece) bulk_load(smem_base + C::kScOff + s * C::kScBytes + w_piece_to, w_src + (size_t)(p.one_shift < 32 ? (uint32_t)(w_sb * kSB) >> p.one_shift : 0u) * w_pitch, w_piece, w_full(s));
+            if (w_piece) bulk_load(smem_base + C::kScOff + s * C::kScBytes + w_piece_to, w_src + (size_t)(p.one_shift < 32 ? (uint32_t)(w_sb * kSB) >> p.one_shift : 0u) * w_pitch, w_piece, w_full(full));
         }
         ++w_it;
         if (++w_sb == (int)nsb) { w_sb = 0; ++w_tile; if (u0 + (uint32_t)w_it < u1) w_take_tile(); }
@@ -591,7 +595,7 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
     if (warp == kWarpW) {
         w_leader = elect_one();
         if (w_leader) {
-            for (int s = 0; s < kW; ++s) { mbar_init(w_full(s), 1); mbar_init(w_empty(s), 4); }
+            for (int s = 0; s < kW; ++s) { mbar_init(w_full(s), 1); mbar_init(w_full(kW + s), 1); mbar_init(w_empty(s), 4); }
             for (int s = 0; s < kX; ++s) { mbar_init(x_full(s), 1); mbar_init(x_empty(s), 1); }
             for (int b = 0; b < kGroups; ++b) { mbar_init(a_ready(b), 4); mbar_init(a_free(b), 1); }
             for (int b = 0; b < kDBufs; ++b) { mbar_init(d_full(b), 1); mbar_init(d_empty(b), C::kEpi * 4); }
@@ -711,7 +715,7 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         const int row = qd * 32 + lane;                    // weight row within the tile = TMEM lane
         const uint32_t a_col = tmem + kColA + g * 128 + ((uint32_t)(qd * 32) << 16);
         if (kType == kTypeF8 && !moe) pdl_wait();          // p.norm comes from the kernel before
-        int ws = g;
+        int wf = g;                                        // unit % 2 kW: its full barrier; its stage is wf % kW
         uint32_t wph = 0;
         UnitBars ub{0u, a_free(g), 1u, lane};
         int tile = (int)tile0, sb = (int)sb0;
@@ -746,7 +750,8 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
             }
             skip_units(kGroups);
             if (kAhead && u + kGroups < u1) fetch();
-            mbar_wait(w_full(ws), wph);
+            mbar_wait(w_full(wf), wph);
+            const int ws = wf >= kW ? wf - kW : wf;
             ub.w_empty = w_empty(ws);
             const uint8_t* stage = smem + C::kWOff + ws * C::kWBytes;
             const uint8_t* blk = stage + row * C::kBlk;
@@ -772,8 +777,8 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
             __syncwarp();
             if (lane == 0) mbar_arrive(a_ready(g));
             ub.a_parity ^= 1;
-            ws += kGroups;
-            if (ws >= kW) { ws -= kW; wph ^= 1; }
+            wf += kGroups;
+            if (wf >= 2 * kW) { wf -= 2 * kW; wph ^= 1; }
         }
         }
         // ======================================== EPILOGUE =======================================
