@@ -155,6 +155,8 @@ reshape_and_cache_flash_vec_kernel(const int4* __restrict__ key, const int4* __r
                                    int4* __restrict__ kc, int4* __restrict__ vc,
                                    const int64_t* __restrict__ slot_mapping, int row_vecs,
                                    int64_t key_stride_vecs, int64_t value_stride_vecs) {
+    pdl_wait();
+    pdl_trigger();               // the attention kernel behind it may set itself up meanwhile
     const int t = blockIdx.x;
     const int64_t slot = slot_mapping[t];
     if (slot < 0) return;
@@ -171,6 +173,8 @@ __global__ void __launch_bounds__(128)
 reshape_and_cache_flash_fp8_vec_kernel(const TIn* __restrict__ key, const TIn* __restrict__ value, uint8_t* __restrict__ kc,
                                        uint8_t* __restrict__ vc, const int64_t* __restrict__ slot_mapping, int n,
                                        int64_t key_stride, int64_t value_stride) {
+    pdl_wait();
+    pdl_trigger();
     const int t = blockIdx.x;
     const int64_t slot = slot_mapping[t];
     if (slot < 0) return;
@@ -292,20 +296,20 @@ void reshape_and_cache(const void* key, const void* value, void* key_cache, void
     if (layout == B200_KV_FLASH && !fp8 && cache_dtype == in_dtype && in_dtype != B200_F32 && n % 8 == 0 &&
         key_stride % 8 == 0 && value_stride % 8 == 0 && ((uintptr_t)key & 15) == 0 && ((uintptr_t)value & 15) == 0 &&
         ((uintptr_t)key_cache & 15) == 0 && ((uintptr_t)value_cache & 15) == 0) {
-        reshape_and_cache_flash_vec_kernel<<<num_tokens, 128, 0, st>>>(
-            (const int4*)key, (const int4*)value, (int4*)key_cache, (int4*)value_cache, slot_mapping, n / 8,
-            key_stride / 8, value_stride / 8);
+        launch_pdl(reshape_and_cache_flash_vec_kernel, dim3(num_tokens), dim3(128), 0, st,
+                   (const int4*)key, (const int4*)value, (int4*)key_cache, (int4*)value_cache, slot_mapping, n / 8,
+                   key_stride / 8, value_stride / 8);
     } else if (layout == B200_KV_FLASH && fp8 && n % 16 == 0 && (key_stride * (in_dtype == B200_F32 ? 4 : 2)) % 16 == 0 &&
                (value_stride * (in_dtype == B200_F32 ? 4 : 2)) % 16 == 0 &&
                ((((uintptr_t)key | (uintptr_t)value | (uintptr_t)key_cache | (uintptr_t)value_cache)) & 15) == 0 &&
                (in_dtype == B200_F32 || in_dtype == B200_BF16 || in_dtype == B200_F16)) {
         const int threads = n / 16 >= 128 ? 128 : ((n / 16 + 31) / 32) * 32;
         if (in_dtype == B200_F32)
-            reshape_and_cache_flash_fp8_vec_kernel<float><<<num_tokens, threads, 0, st>>>((const float*)key, (const float*)value, (uint8_t*)key_cache, (uint8_t*)value_cache, slot_mapping, n, key_stride, value_stride);
+            launch_pdl(reshape_and_cache_flash_fp8_vec_kernel<float>, dim3(num_tokens), dim3(threads), 0, st, (const float*)key, (const float*)value, (uint8_t*)key_cache, (uint8_t*)value_cache, slot_mapping, n, key_stride, value_stride);
         else if (in_dtype == B200_BF16)
-            reshape_and_cache_flash_fp8_vec_kernel<__nv_bfloat16><<<num_tokens, threads, 0, st>>>((const __nv_bfloat16*)key, (const __nv_bfloat16*)value, (uint8_t*)key_cache, (uint8_t*)value_cache, slot_mapping, n, key_stride, value_stride);
+            launch_pdl(reshape_and_cache_flash_fp8_vec_kernel<__nv_bfloat16>, dim3(num_tokens), dim3(threads), 0, st, (const __nv_bfloat16*)key, (const __nv_bfloat16*)value, (uint8_t*)key_cache, (uint8_t*)value_cache, slot_mapping, n, key_stride, value_stride);
         else
-            reshape_and_cache_flash_fp8_vec_kernel<__half><<<num_tokens, threads, 0, st>>>((const __half*)key, (const __half*)value, (uint8_t*)key_cache, (uint8_t*)value_cache, slot_mapping, n, key_stride, value_stride);
+            launch_pdl(reshape_and_cache_flash_fp8_vec_kernel<__half>, dim3(num_tokens), dim3(threads), 0, st, (const __half*)key, (const __half*)value, (uint8_t*)key_cache, (uint8_t*)value_cache, slot_mapping, n, key_stride, value_stride);
     } else if (in_dtype == B200_F32) {
         launch_rac<float>(key, value, key_cache, value_cache, slot_mapping, num_tokens, num_kv_heads, head_dim, block_size, key_stride, value_stride, cache_dtype, in_dtype, layout, st);
     } else if (in_dtype == B200_BF16) {

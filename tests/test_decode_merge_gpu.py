@@ -1,0 +1,46 @@
+"""The merge of the decode kernel's chunk partials: a warp per head (head counts that are no multiple of four), chunk counts on either side of what is loaded ahead (8) and of what a warp's
+lanes hold (32), chunks that the decode kernel has halved, outputs that start on an odd multiple of two bytes."""
+import ctypes as C
+
+import pytest
+import torch
+
+import candle_vllm_b200 as pkg
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(q, kc, vc, tables, lens, group):
+    out = []
+    for b, n in enumerate(lens):
+        k = kc[tables[b, :-(-n // 64)].long()].flatten(0, 1)[:n].double().repeat_interleave(group, 1)
+        v = vc[tables[b, :-(-n // 64)].long()].flatten(0, 1)[:n].double().repeat_interleave(group, 1)
+        p = torch.softmax(torch.einsum("hd,khd->hk", q[b].double(), k) * 128 ** -0.5, 1)
+        out.append(torch.einsum("hk,khd->hd", p, v))
+    return torch.stack(out)
+
+
+@pytest.mark.parametrize("heads,kv_heads", [(1, 1), (6, 3), (8, 2), (8, 1), (32, 8)])
+@pytest.mark.parametrize("lens", [[1], [64 * 8], [64 * 8 + 1], [64 * 32, 3], [64 * 32 + 1], [64 * 70 + 5, 64, 700], [4600, 4664, 4300, 17] * 8])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_merge(heads, kv_heads, lens, offset):
+    gen = torch.Generator(device="cuda").manual_seed(len(lens) + heads)
+    mk = lambda *s: torch.randn(*s, generator=gen, device="cuda").bfloat16()
+    width = max(-(-n // 64) for n in lens)
+    blocks = 300
+    kc, vc, q = mk(blocks, 64, kv_heads, 128), mk(blocks, 64, kv_heads, 128), mk(len(lens), heads, 128)
+    tables = torch.randint(0, blocks, (len(lens), width), generator=gen, device="cuda", dtype=torch.int32)
+    ctx = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    held = torch.zeros(q.numel() + 8, dtype=torch.bfloat16, device="cuda")
+    L = pkg.lib()
+    ws = torch.zeros(int(L.paged_attention_decode_workspace_bytes(*map(C.c_int32, (len(lens), heads, 128, width, 64)))), dtype=torch.uint8, device="cuda")
+    p = lambda t: C.c_void_p(t.data_ptr())
+    out = held[offset:offset + q.numel()].view_as(q)
+    for _ in range(2):                                    # the work queue is left as it was found
+        L.paged_attention_decode(p(out), p(q), p(kc), p(vc), p(tables), p(ctx), *map(C.c_int32, (len(lens), heads, kv_heads, 128, 64, width)), C.c_int64(blocks), C.c_float(128 ** -0.5),
+                                 C.c_float(0), *map(C.c_int32, (0, 2, 2, 0, 2)), p(ws), C.c_size_t(ws.numel()), C.c_int64(torch.cuda.current_stream().cuda_stream))
+        assert L.b200_last_error() == 0
+    ref = _reference(q, kc, vc, tables, lens, heads // kv_heads)
+    # weights and result rounded to bf16: 2^-9 / sqrt(3) each in the mean square
+    assert float((out.double() - ref).norm() / ref.norm()) < 2.5e-3
+    assert not held[:offset].any() and not held[offset + q.numel():].any()
