@@ -482,9 +482,11 @@ struct MoeBlockPlan {
     MoeBlockPlan(int64_t T, int64_t H, int64_t I, int E, int topk) {
         const int64_t P = T * topk;
         rows = chunk_rows_for(P, E); max_chunks = max_chunks_for(P, E, rows);
-        // router parts: about two CTAs per SM, at least two steps each, 16 at most (the top-k kernel adds them one after another)
+        // router parts: about six CTAs per SM, at least two steps each, 16 at most (the top-k kernel adds them one after another).  A CTA is four warps; with two per SM too few run
+        // to hide their loads, and half the SMs had one.  [us the block with two / four / six, 128 experts: 900 tokens 262 / 248 / 240, 600 - / 208 / 205, 300 146 / 144 / 144; up to
+        // 100 tokens level, the parts are 16 either way]
         const int64_t tiles = ((T + kRtT - 1) / kRtT) * ((E + kRtE - 1) / kRtE), steps = H / kRtK;
-        int64_t s = 296 / tiles;
+        int64_t s = 888 / tiles;
         if (s > 16) s = 16;
         if (s > steps / 2) s = steps / 2;
         if (s < 1) s = 1;
