@@ -720,9 +720,11 @@ void paged_attention_decode_tma(const DecodeArgs& a, cudaStream_t st) {
         set_error(kErrBadArg, "paged_attention_decode: workspace too small (%zu < %zu bytes)", a.workspace_bytes, need);
         return;
     }
-    // layout: [counter (256 B)] [partial O] [partial (m, l)]
+    if ((uintptr_t)a.workspace & 3) { set_error(kErrBadArg, "paged_attention_decode: workspace must start on 4 bytes"); return; }
+    // layout: [counter] [partial O] [partial (m, l)].  The merge reads partial O sixteen bytes at a time, so it starts on the last such boundary that leaves the counter's five words
+    // 244 to 256 bytes, wherever the caller's workspace starts.
     p.counter = static_cast<unsigned int*>(a.workspace);
-    p.part_o = reinterpret_cast<float*>(static_cast<char*>(a.workspace) + 256);
+    p.part_o = reinterpret_cast<float*>(((uintptr_t)a.workspace + 256) & ~(uintptr_t)15);
     p.part_ml = p.part_o + n_part * kHeadDim;
     CUtensorMap km, vm;
     if (!make_kv_map(&km, a.kc, a.num_blocks, a.num_kv_heads, a.dtype, a.fp8) || !make_kv_map(&vm, a.vc, a.num_blocks, a.num_kv_heads, a.dtype, a.fp8)) return;

@@ -44,3 +44,37 @@ def test_merge(heads, kv_heads, lens, offset):
     # weights and result rounded to bf16: 2^-9 / sqrt(3) each in the mean square
     assert float((out.double() - ref).norm() / ref.norm()) < 2.5e-3
     assert not held[:offset].any() and not held[offset + q.numel():].any()
+
+
+@pytest.mark.parametrize("shift", [4, 8, 12, 2])
+def test_workspace_may_start_on_any_word(shift):
+    """the merge's 16-byte reads are aligned inside the workspace; one that starts inside a word is refused before anything is launched"""
+    lens, heads, kv_heads, width = [700, 64 * 9 + 1], 8, 2, 11
+    gen = torch.Generator(device="cuda").manual_seed(shift)
+    mk = lambda *s: torch.randn(*s, generator=gen, device="cuda").bfloat16()
+    kc, vc, q = mk(30, 64, kv_heads, 128), mk(30, 64, kv_heads, 128), mk(2, heads, 128)
+    tables = torch.randint(0, 30, (2, width), generator=gen, device="cuda", dtype=torch.int32)
+    ctx = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    L = pkg.lib()
+    need = int(L.paged_attention_decode_workspace_bytes(*map(C.c_int32, (2, heads, 128, width, 64))))
+    held = torch.zeros(need + 64, dtype=torch.uint8, device="cuda")
+    held[shift + need:] = 7
+    p = lambda t, by=0: C.c_void_p(t.data_ptr() + by)
+
+    def call(by):
+        out = torch.zeros_like(q)
+        L.paged_attention_decode(p(out), p(q), p(kc), p(vc), p(tables), p(ctx), *map(C.c_int32, (2, heads, kv_heads, 128, 64, width)), C.c_int64(30), C.c_float(128 ** -0.5),
+                                 C.c_float(0), *map(C.c_int32, (0, 2, 2, 0, 2)), p(held, by), C.c_size_t(need), C.c_int64(torch.cuda.current_stream().cuda_stream))
+        return out, L.b200_last_error()
+
+    if shift % 4:
+        out, code = call(shift)
+        assert code != 0 and b"workspace" in L.b200_last_error_message() and not out.any() and not held[:need].any()
+        return
+    outs = [call(shift), call(shift)]
+    assert (held[shift + need:] == 7).all()
+    held[:shift + need] = 0
+    outs.append(call(0))
+    assert all(code == 0 and torch.equal(out, outs[2][0]) for out, code in outs)
+    ref = _reference(q, kc, vc, tables, lens, heads // kv_heads)
+    assert float((outs[0][0].double() - ref).norm() / ref.norm()) < 2.5e-3
