@@ -57,7 +57,14 @@ PyObject* result(at::Tensor&& out) {
 
 at::Tensor fresh(at::IntArrayRef sizes, const at::Tensor& like, at::ScalarType type) { return at::empty(sizes, at::TensorOptions().dtype(type).device(like.device())); }
 
-int64_t integer(PyObject* o) { return PyLong_AsLongLong(o); }          // (the caller's own numbers)
+// The caller's numbers.  False for what converts to none (None, a float where an integer belongs): Python's way decides what becomes of it.
+bool known(bool ok) {
+    if (!ok) PyErr_Clear();
+    return ok;
+}
+bool number(PyObject* o, int64_t& v) { v = PyLong_AsLongLong(o); return known(v != -1 || !PyErr_Occurred()); }
+bool number(PyObject* o, double& v) { v = PyFloat_AsDouble(o); return known(v != -1.0 || !PyErr_Occurred()); }
+bool number(PyObject* o, bool& v) { const int t = PyObject_IsTrue(o); v = t > 0; return known(t >= 0); }
 
 // linear(x, weight, bias or None)
 PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
@@ -88,9 +95,10 @@ PyObject* py_qmatmul(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (!L.ready || n_args != 6 || a[5] == Py_None) Py_RETURN_NONE;
     const at::Tensor *x = plain(a[0]), *w = plain(a[1]), *ws = plain(a[5]);
     if (!x || !w || !ws || x->dim() < 1 || x->scalar_type() != at::kFloat || w->scalar_type() != at::kByte || ws->scalar_type() != at::kByte) Py_RETURN_NONE;
-    const int64_t n = integer(a[2]), k = integer(a[3]), type = integer(a[4]), m = k > 0 ? x->numel() / k : 0;
+    int64_t n, k, type;
+    if (!number(a[2], n) || !number(a[3], k) || !number(a[4], type)) Py_RETURN_NONE;
+    const int64_t m = k > 0 ? x->numel() / k : 0;
     const int dev = x->get_device();
-    if (PyErr_Occurred()) return nullptr;
     if (x->size(-1) != k || !fits(m) || !fits(n) || !fits(k) || dev != c10::cuda::current_device() || !here(*w, dev) || !here(*ws, dev) || L.cc() < 100) Py_RETURN_NONE;
     if ((uint64_t)ws->numel() < L.qmatmul_bytes((int32_t)m, (int32_t)n, (int32_t)k)) Py_RETURN_NONE;
     at::DimVector sizes(x->sizes().begin(), x->sizes().end());
@@ -130,15 +138,16 @@ PyObject* py_silu_mul(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 PyObject* py_paged_attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     HANDLE_TH_ERRORS
     if (!L.ready || n_args != 20) Py_RETURN_NONE;
-    const bool prompt = PyObject_IsTrue(*a++) == 1;
+    bool prompt, e4m3;
+    if (!number(*a++, prompt)) Py_RETURN_NONE;
     const at::Tensor *q = plain(a[0]), *k = plain(a[1]), *v = plain(a[2]), *kc = plain(a[3]), *vc = plain(a[4]), *slots = plain(a[5]), *bt = plain(a[6]);
     if (!q || !k || !v || !kc || !vc || !slots || !bt) Py_RETURN_NONE;
     const at::Tensor *lens = prompt || a[7] == Py_None ? nullptr : plain(a[7]), *cu_q = prompt ? plain(a[8]) : nullptr, *cu_k = prompt ? plain(a[9]) : nullptr, *ws = prompt || a[10] == Py_None ? nullptr : plain(a[10]);
     if (prompt ? (!cu_q || !cu_k) : (!lens || !ws)) Py_RETURN_NONE;
-    const int64_t H = integer(a[11]), G = integer(a[12]), hd = integer(a[13]), longest = integer(a[14]), window = integer(a[15]);
-    const double scale = PyFloat_AsDouble(a[16]), cap = PyFloat_AsDouble(a[17]);
-    const bool e4m3 = PyObject_IsTrue(a[18]) == 1;
-    if (PyErr_Occurred()) return nullptr;
+    int64_t H, G, hd, window, longest = 0;
+    double scale, cap;
+    if (!number(a[11], H) || !number(a[12], G) || !number(a[13], hd) || (prompt && !number(a[14], longest)) || !number(a[15], window) || !number(a[16], scale) || !number(a[17], cap) ||
+        !number(a[18], e4m3)) Py_RETURN_NONE;
     const int type = type16(*q), dev = q->get_device();
     auto words = [&](const at::Tensor& t) { return t.scalar_type() == at::kInt || t.scalar_type() == at::kUInt32; };
     if (type < 0 || q->dim() != 3 || q->size(1) != H || q->size(2) != hd || k->dim() != 3 || v->dim() != 3 || k->sizes() != v->sizes() || k->size(1) != G || k->size(2) != hd) Py_RETURN_NONE;

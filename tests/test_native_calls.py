@@ -123,3 +123,23 @@ def test_paged_attention(through_python, prompt, fp8, strided):
     with pytest.raises(pkg.BackendError):                 # 80 wide heads: refused by the library, natively too
         odd = pkg.PagedAttention(H, 72, 1.0, G_)
         odd.forward(mk(T, H, 72), mk(T, G_, 72), mk(T, G_, 72), None, torch.zeros(nb, 64, G_, 72, dtype=torch.float32, device="cuda"), torch.zeros(nb, 64, G_, 72, dtype=torch.float32, device="cuda"), meta)
+
+
+@pytest.mark.gpu
+def test_numbers_that_only_python_takes(through_python):
+    """a window that is a float, a longest query that a decode step does not have: taken as they are on the way through Python, on the first call and, with the workspace there, on later ones"""
+    T, H, G_, hd = 3, 8, 2, 128
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    mk = lambda *s: torch.randn(*s, generator=gen, device="cuda").bfloat16()
+    q, k, v, kc, vc = mk(T, H, hd), mk(T, G_, hd), mk(T, G_, hd), mk(4, 64, G_, hd), mk(4, 64, G_, hd)
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    meta = pkg.InputMetadata(False, torch.arange(T, device="cuda") + 70, i32([[0, 1]] * T), context_lens=i32([71, 72, 73]), max_seqlen_q=None)
+    for window in (None, 4096.0, 20.0):
+        op = pkg.PagedAttention(H, hd, hd ** -0.5, G_, sliding_window=window)
+        ref = through_python(lambda: op.forward(q, k, v, None, kc, vc, meta))
+        for _ in range(2):
+            assert torch.equal(op.forward(q, k, v, None, kc, vc, meta), ref)
+    native = _lib.calls()
+    assert native.paged_attention(False, q, k, v, kc, vc, meta.slot_mapping, meta.block_tables, meta.context_lens, None, None, op._ws, H, G_, hd, None, 20.0, 1.0, 0.0, False) is None
+    x, w = torch.zeros(1, 256, device="cuda"), torch.zeros(144 * 8, dtype=torch.uint8, device="cuda")
+    assert native.qmatmul(x, w, 8.0, 256, 12, torch.zeros(1 << 20, dtype=torch.uint8, device="cuda")) is None
