@@ -66,10 +66,13 @@ CALLS = os.path.join(HERE, "_calls.so")
 
 
 def build_calls(force: bool = False, verbose: bool = False) -> str:
-    """``_calls.so``: the operators of ``csrc/py_calls.cpp`` as Python functions.  Needs the headers of torch and of Python; without it the package calls the library through ctypes."""
+    """``_calls.so``: the operators of ``csrc/py_calls.cpp`` as Python functions.  Needs the headers of torch and of Python; without it the package calls the library through ctypes.
+    Raises where it cannot be built, and leaves none of older sources behind."""
     src = os.path.join(CSRC, "py_calls.cpp")
     if not force and not _newer(CALLS, [src] + glob.glob(os.path.join(HERE, "..", "include", "*.h"))):
         return CALLS
+    if os.path.exists(CALLS):
+        os.remove(CALLS)
     import sysconfig
 
     import torch
@@ -126,7 +129,10 @@ def build(force: bool = False, verbose: bool = False, group=None) -> str:
             raise RuntimeError("link failed")
         os.replace(tmp, SO)              # a reader never sees a half-written library
     if group is None:
-        build_calls(force, verbose)
+        try:
+            build_calls(force, verbose)
+        except (ImportError, OSError, RuntimeError) as e:       # no torch, no headers, no compiler: the library is complete without it
+            sys.stderr.write(f"{os.path.basename(CALLS)} not built ({e}): operators will be called through ctypes\n")
     return SO
 
 

@@ -1,6 +1,9 @@
 """The natively entered operators (csrc/py_calls.cpp) against the way through Python: the same results, the same refusals, and None -- the Python way -- for arguments they are not made for.
 The buffers that logits are read back to: lent while anything made from them is alive."""
 import gc
+import importlib.util
+import os
+import sys
 
 import numpy as np
 import pytest
@@ -45,6 +48,30 @@ def test_tensors_on_the_host_are_left_to_python():
     assert native.silu_mul(1, x) is None and native.silu_mul(x) is None
     with pytest.raises(pkg.BackendError):
         pkg.Linear(torch.zeros(8, 8).half())
+
+
+@pytest.fixture
+def build_in(tmp_path):
+    """build.py over a folder of its own that has a finished library and native calls of older sources"""
+    spec = importlib.util.spec_from_file_location("b200_build_under_test", os.path.join(os.path.dirname(_lib.__file__), "build.py"))
+    b = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(b)
+    b.HERE, b.CSRC, b.OBJ, b.SO, b.CALLS = str(tmp_path), str(tmp_path), str(tmp_path / "obj"), str(tmp_path / "lib.so"), str(tmp_path / "_calls.so")
+    for name in ("lib.so", "_calls.so", "py_calls.cpp"):
+        (tmp_path / name).write_text("")
+    os.utime(tmp_path / "_calls.so", (1, 1))
+    return b
+
+
+@pytest.mark.parametrize("missing", ["torch", "compiler", "headers"])
+def test_the_library_is_built_without_native_calls(build_in, missing, monkeypatch, capfd):
+    b = build_in
+    if missing == "torch":
+        monkeypatch.setitem(sys.modules, "torch", None)
+    else:
+        b.CCBIN = "/bin/false" if missing == "headers" else "/no/compiler"
+    assert b.build() == b.SO
+    assert not os.path.exists(b.CALLS) and "ctypes" in capfd.readouterr().err
 
 
 @pytest.fixture
