@@ -132,11 +132,19 @@ def typed(name: str, restype, *argtypes):
 _calls_module = None
 
 
+def _calls_path() -> str:
+    """as ``build.calls_path``: one file per Python and build of torch"""
+    import sys
+
+    import torch
+    return os.path.join(_HERE, f"_calls.{sys.implementation.cache_tag}-torch-{torch.__version__}-{(torch.version.git_version or '')[:10]}.so")
+
+
 def calls():
-    """The natively entered operators (``csrc/py_calls.cpp``), or False where they are not built: the callers then go through ctypes."""
+    """The natively entered operators (``csrc/py_calls.cpp``), or False where they are not built for this Python and torch: the callers then go through ctypes."""
     global _calls_module
     if _calls_module is None:
-        path = os.path.join(_HERE, "_calls.so")
+        path = _calls_path()
         if not os.path.exists(path) or not os.path.exists(_SO):
             _calls_module = False
             return False
@@ -149,7 +157,7 @@ def calls():
             lib()
             m.bind(_SO)
             _calls_module = m
-        except ImportError as e:            # built against another torch or library
+        except ImportError as e:            # built against another library
             import warnings
             warnings.warn(f"{path} cannot be used ({e}): operators are called through ctypes")
             _calls_module = False

@@ -62,13 +62,18 @@ def so_path(group=None) -> str:
     return SO if group is None else os.path.join(HERE, f"libb200backend.{group}.so")
 
 
-CALLS = os.path.join(HERE, "_calls.so")
+def calls_path() -> str:
+    """Where the native operator calls of the running Python and torch are.  They have the layout of torch's tensors compiled in, so that a file is for one Python and one build of torch and
+    bears both names: after an update it is not found, and not loaded by mistake."""
+    import torch
+    return os.path.join(HERE, f"_calls.{sys.implementation.cache_tag}-torch-{torch.__version__}-{(torch.version.git_version or '')[:10]}.so")
 
 
 def build_calls(force: bool = False, verbose: bool = False) -> str:
-    """``_calls.so``: the operators of ``csrc/py_calls.cpp`` as Python functions.  Needs the headers of torch and of Python; without it the package calls the library through ctypes.
+    """``_calls.*.so``: the operators of ``csrc/py_calls.cpp`` as Python functions.  Needs the headers of torch and of Python; without it the package calls the library through ctypes.
     Raises where it cannot be built, and leaves none of older sources behind."""
     src = os.path.join(CSRC, "py_calls.cpp")
+    CALLS = calls_path()
     if not force and not _newer(CALLS, [src] + glob.glob(os.path.join(HERE, "..", "include", "*.h"))):
         return CALLS
     if os.path.exists(CALLS):
@@ -132,7 +137,7 @@ def build(force: bool = False, verbose: bool = False, group=None) -> str:
         try:
             build_calls(force, verbose)
         except (ImportError, OSError, RuntimeError) as e:       # no torch, no headers, no compiler: the library is complete without it
-            sys.stderr.write(f"{os.path.basename(CALLS)} not built ({e}): operators will be called through ctypes\n")
+            sys.stderr.write(f"the native operator calls are not built ({e}): operators will be called through ctypes\n")
     return SO
 
 

@@ -56,22 +56,39 @@ def build_in(tmp_path):
     spec = importlib.util.spec_from_file_location("b200_build_under_test", os.path.join(os.path.dirname(_lib.__file__), "build.py"))
     b = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(b)
-    b.HERE, b.CSRC, b.OBJ, b.SO, b.CALLS = str(tmp_path), str(tmp_path), str(tmp_path / "obj"), str(tmp_path / "lib.so"), str(tmp_path / "_calls.so")
-    for name in ("lib.so", "_calls.so", "py_calls.cpp"):
+    assert b.calls_path() == _lib._calls_path()
+    b.HERE, b.CSRC, b.OBJ, b.SO = str(tmp_path), str(tmp_path), str(tmp_path / "obj"), str(tmp_path / "lib.so")
+    for name in ("lib.so", b.calls_path(), "py_calls.cpp"):
         (tmp_path / name).write_text("")
-    os.utime(tmp_path / "_calls.so", (1, 1))
+    os.utime(b.calls_path(), (1, 1))
     return b
 
 
 @pytest.mark.parametrize("missing", ["torch", "compiler", "headers"])
 def test_the_library_is_built_without_native_calls(build_in, missing, monkeypatch, capfd):
     b = build_in
+    stale = b.calls_path()
     if missing == "torch":
         monkeypatch.setitem(sys.modules, "torch", None)
     else:
         b.CCBIN = "/bin/false" if missing == "headers" else "/no/compiler"
     assert b.build() == b.SO
-    assert not os.path.exists(b.CALLS) and "ctypes" in capfd.readouterr().err
+    assert os.path.exists(stale) == (missing == "torch") and "ctypes" in capfd.readouterr().err       # (whose it is cannot be known without torch)
+
+
+def test_native_calls_of_another_torch_are_not_loaded(monkeypatch, tmp_path):
+    native = _lib.calls()
+    if not native:
+        pytest.skip("not built")
+    for name in ("_calls.so", os.path.basename(_lib._calls_path()), os.path.basename(_lib._SO)):
+        (tmp_path / name).symlink_to(_lib._calls_path())
+    monkeypatch.setattr(_lib, "_HERE", str(tmp_path))
+    monkeypatch.setattr(_lib, "_SO", str(tmp_path / os.path.basename(_lib._SO)))
+    for what, value in ((torch, "__version__"), (torch.version, "git_version"), (sys.implementation, "cache_tag")):
+        with monkeypatch.context() as m:
+            m.setattr(_lib, "_calls_module", None)
+            m.setattr(what, value, "0123456789a")
+            assert _lib.calls() is False
 
 
 @pytest.fixture
