@@ -95,17 +95,22 @@ def _clinear(w) -> _CLinear:
 
 class _HostRows:
     """Where a step's logits are read back to: two pinned buffers, lent out as arrays and taken back when nothing refers to one any more (a copy into pageable memory goes through the
-    driver's staging, 180 us for 32 rows of 16384).  With both lent out, or for more than 64 MB, an array of its own."""
+    driver's staging, 180 us for 32 rows of 16384).  A buffer is made when it is first needed: an engine whose logits are never asked for pins nothing.  With both lent out, for more than
+    64 MB, or where no memory can be pinned, an array of its own."""
 
     def __init__(self, rows: int, cols: int, pinned: bool = True):
-        self.cols = cols
-        self.free = [torch.empty((rows, cols), dtype=torch.float32, pin_memory=pinned) for _ in range(2 if rows * cols * 4 <= 64 << 20 else 0)]
+        self.rows, self.cols, self.pinned = rows, cols, pinned
+        self.free, self.unmade = [], [None] * (2 if rows * cols * 4 <= 64 << 20 else 0)
 
     def take(self, rows: int) -> np.ndarray:
         try:
             buffer = self.free.pop()
         except IndexError:
-            return np.empty((rows, self.cols), np.float32)
+            try:
+                self.unmade.pop()
+                buffer = torch.empty((self.rows, self.cols), dtype=torch.float32, pin_memory=self.pinned)
+            except (IndexError, RuntimeError):
+                return np.empty((rows, self.cols), np.float32)
         out = buffer[:rows].numpy()
         weakref.finalize(out.base, self.free.append, buffer).atexit = False         # the owner of the memory, which every view of the array keeps, not the array
         return out

@@ -37,6 +37,25 @@ def test_host_rows_come_back_when_nothing_refers_to_them():
     assert not many.free and many.take(2).shape == (2, 1 << 13)
 
 
+def test_host_rows_are_pinned_when_they_are_needed(monkeypatch):
+    made = []
+    monkeypatch.setattr(llama.torch, "empty", lambda *a, pin_memory, **k: made.append(pin_memory) or torch.zeros(*a, **k))
+    rows = llama._HostRows(4, 6)
+    assert not made
+    a = rows.take(2)
+    assert made == [True]
+    del a
+    gc.collect()
+    held = rows.take(3)
+    assert made == [True] and held.shape == (3, 6)
+
+    def refused(*a, **k):
+        raise RuntimeError("out of memory")
+    monkeypatch.setattr(llama.torch, "empty", refused)
+    assert rows.take(4).shape == (4, 6)
+    assert llama._HostRows(4, 6).take(1).shape == (1, 6)
+
+
 def test_tensors_on_the_host_are_left_to_python():
     native = _lib.calls()
     if not native:
