@@ -802,18 +802,23 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
             float* ybase = sg == 0 ? p.y[0] : (sg == 1 ? p.y[1] : p.y[2]);
             const int db = seg % kDBufs;
             const uint32_t d_t = tmem + db * kMB + lane_addr;
-            // grouped, results scattered or weighted: lane l holds output row and multiplier of column l of a round, fetched before the tile's sums are waited for
+            // grouped, results scattered or weighted: lane l holds output row and multiplier of column l % 8 in this warp's rounds l / 8 and l / 8 + 4, fetched before the tile's sums are
+            // waited for  [a round at a time, ahead of the stores of the one before: 1250 clocks a round, the two reads one after the other; with these and the addresses below side by side a
+            // tile of 125 routed rows is stored in 5000 clocks instead of 10000, us the block: 900 tokens of 128 experts 237 -> 215, 2000 of 32 experts 208 -> 179, 4000 of 256 925 -> 811]
             const bool scattered = moe && (p.row_map != nullptr || p.row_scale != nullptr);
-            uint32_t my_row = 0;
-            float my_scale = 1.f;
-            auto columns = [&](int c0) {
-                const int i = c0 + (lane & 7);
-                if (i < ti.count) {
-                    my_row = p.row_map ? __ldg(p.row_map + ti.xrow + i) : (uint32_t)(ti.xrow + i);
-                    if (p.row_scale) my_scale = __ldg(p.row_scale + my_row);
-                }
-            };
-            if (scattered) columns(first_col);
+            constexpr int kHeld = kGrouped && kMB > 32 ? 2 : 1;
+            static_assert(!kGrouped || kMB <= 4 * 8 * kHeld * C::kEpi, "rounds of a warp in a tile");
+            uint32_t my_row[kHeld] = {};
+            float my_scale[kHeld];
+#pragma unroll
+            for (int b = 0; b < kHeld; ++b) {
+                const int i = first_col + ((lane >> 3) + 4 * b) * step + (lane & 7);
+                my_scale[b] = 1.f;
+                if (scattered && i < ti.count) my_row[b] = p.row_map ? __ldg(p.row_map + ti.xrow + i) : (uint32_t)(ti.xrow + i);
+            }
+#pragma unroll
+            for (int b = 0; b < kHeld; ++b)
+                if (scattered && p.row_scale && first_col + ((lane >> 3) + 4 * b) * step + (lane & 7) < ti.count) my_scale[b] = __ldg(p.row_scale + my_row[b]);
             const float post = moe && kType == kTypeF8 && p.norm ? __ldg(p.norm + 1) : 1.f;      // FP8: undo the range shift of the tile scales
             // slab mode: the k-th CTA that works on a tile writes slab k.  CTA b owns units [total*b/grid, total*(b+1)/grid),
             // so the owner of unit u is ((u+1)*grid - 1) / total and only a CTA's first segment can start inside a tile.
@@ -844,7 +849,7 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
             }
             // (rolled: a tile's epilogue runs out of a cold instruction cache, only the first round misses)
 #pragma unroll 1
-            for (int c0 = first_col; c0 < ti.count; c0 += step) {
+            for (int c0 = first_col, r = 0; c0 < ti.count; c0 += step, ++r) {
                 uint32_t acc[8];
                 tc_ld8(d_t + c0, acc);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -853,29 +858,37 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                     __syncwarp();
                     if (lane == 0) mbar_arrive(d_empty(db));
                 }
+                // Eight addresses side by side, then the stores: with one address that is moved on, or made anew for each, every store waited until the one before had read it, 130 to 150
+                // clocks apiece  [4096 x 4096 int4, us at 32 / 64 rows: 14.5 / 20.1, now 11.7 / 15.0; NVFP4 15.1 / 20.5, now 12.8 / 15.6].
+                float* o[8];
                 if (scattered) {
                     // column i of the accumulator = routed row x_row0 + i of this expert's chunk, scattered to its output row (pair index) with the routing weight folded in
-                    const uint32_t row_now = my_row;
-                    const float scale_now = my_scale;
-                    if (c0 + step < ti.count) columns(c0 + step);
+                    const uint32_t row_now = r < 4 ? my_row[0] : my_row[kHeld - 1];
+                    const float scale_now = r < 4 ? my_scale[0] : my_scale[kHeld - 1];
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
-                        const uint32_t orow = __shfl_sync(0xffffffffu, row_now, i);
-                        const float sc = __shfl_sync(0xffffffffu, scale_now, i);
-                        if (n_idx < n_rows && c0 + i < ti.count) ybase[(int64_t)orow * p.ldy + n_idx] = __uint_as_float(acc[i]) * (sc * post);
+                        const uint32_t orow = __shfl_sync(0xffffffffu, row_now, (r & 3) * 8 + i);
+                        const float sc = __shfl_sync(0xffffffffu, scale_now, (r & 3) * 8 + i);
+                        o[i] = ybase + (int64_t)orow * p.ldy + n_idx;
+                        acc[i] = __float_as_uint(__uint_as_float(acc[i]) * (sc * post));
                     }
-                } else if (n_idx < n_rows) {
-                    // Eight addresses side by side: with one that is moved on, every store waited until the one before had read it, 150 clocks apiece  [4096 x 4096 int4, us at 32 / 64
-                    // rows: 14.5 / 20.1, now 11.7 / 15.0; NVFP4 15.1 / 20.5, now 12.8 / 15.6]
+                } else {
                     int64_t ldy = p.ldy;
                     asm volatile("" : "+l"(ldy));                     // (multiples of it kept over the rounds are sixteen registers)
-                    float* o[8] = {ybase + (ti.xrow + c0) * ldy + n_idx};
+                    o[0] = ybase + (ti.xrow + c0) * ldy + n_idx;
 #pragma unroll
                     for (int i = 1; i < 8; ++i) o[i] = o[i - 1] + ldy;
+                    if (moe) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) acc[i] = __float_as_uint(__uint_as_float(acc[i]) * post);
+                    }
+                }
+                asm volatile("" : "+l"(o[0]), "+l"(o[1]), "+l"(o[2]), "+l"(o[3]), "+l"(o[4]), "+l"(o[5]), "+l"(o[6]), "+l"(o[7]));
+                if (n_idx < n_rows) {
                     if (store) {
 #pragma unroll
                         for (int i = 0; i < 8; ++i)
-                            if (c0 + i < ti.count) *o[i] = moe ? __uint_as_float(acc[i]) * post : __uint_as_float(acc[i]);
+                            if (c0 + i < ti.count) *o[i] = __uint_as_float(acc[i]);
                         for (int z = 1; z <= zero_slabs; ++z) {
 #pragma unroll
                             for (int i = 0; i < 8; ++i)
@@ -912,12 +925,15 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                     v[0] += f.x; v[1] += f.y; v[2] += f.z; v[3] += f.w;
                 }
                 if (n_idx < seg_rows(p, ti.sg)) {
+                    float* const o[4] = {y + (int64_t)(4 * g) * p.ldy, y + (int64_t)(4 * g + 1) * p.ldy, y + (int64_t)(4 * g + 2) * p.ldy, y + (int64_t)(4 * g + 3) * p.ldy};
+                    if (p.accumulate) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        if (4 * g + i >= ti.count) break;
-                        float* o = y + (int64_t)(4 * g + i) * p.ldy;
-                        *o = p.accumulate ? *o + v[i] : v[i];
+                        for (int i = 0; i < 4; ++i)
+                            if (4 * g + i < ti.count) v[i] += *o[i];
                     }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (4 * g + i < ti.count) *o[i] = v[i];
                 }
             }
         }
