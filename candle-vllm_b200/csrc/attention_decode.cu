@@ -152,7 +152,7 @@ struct DecodeParams {
     float* part_o;                    // [B*kvh*max_chunks][group][128]
     float* part_ml;                   // [B*kvh*max_chunks][group][2]  (m in log2 domain, l)
     unsigned int* counter;            // dynamic work queue head (zero on entry; the merge kernel re-zeroes it)
-    int num_seqs, num_heads, num_kv_heads, max_blocks, chunk_pages, max_chunks;
+    int num_seqs, num_heads, num_kv_heads, max_blocks, chunk_pages, min_pages, max_chunks;      // min_pages: the smaller of the two sizes a chunk may come to have
     int adaptive_chunks;           // 1: the kernel may halve chunk_pages from the device-side context lengths (B200_ATTN_ADAPTIVE=0: off)
     int static_walk;               // queue mode: 0 per-warp tickets, 1 CTA tickets (FP8 cache), 2 static walk (B200_ATTN_STATIC overrides)
     float scale_log2;                 // scale * log2(e)
@@ -536,41 +536,52 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_
     }
 }
 
-// Merges the chunk partials: a warp per (sequence, head), four dims a lane.  The kernel is latency: launched beside the decode kernel, it has the context length before that kernel
-// ends (which lets its dependents start only after it has waited for what came before), and when it has ended asks at once for the chunk size and for the partials of the
-// chunks that exist under the larger of the two sizes.  A lane holds the maximum and the sum of one chunk, so that the weights cost one exponential a lane.
-// [A thread per dim; chunk size, first eight chunks and the rest one after the other: the merge added 7.3 us to 32 sequences of about 4000 keys and 3.3 to one of 700, now 6.2 and 2.7; with
-// the cache write launched programmatically as well, whole calls 93.7 -> 90.1 and 10.6 -> 9.5 us.]
-template <typename T, typename TOut, bool kK4>
+// Merges the chunk partials of one (sequence, head), four dims a lane: by a warp, or (kSplit 4) by a CTA whose warps take every fourth chunk each, if there may be more than kSplitChunks.
+// The kernel is latency: launched beside the decode kernel, it has the context length before that kernel ends (which lets its dependents start only after it has waited for what came
+// before), and when it has ended asks at once for the chunk size and for the partials of all chunks that there are under the smaller of the two sizes; what the larger size leaves unwritten
+// is not looked at.  A lane holds the maximum and the sum of one chunk, so that the weights cost one exponential a lane.
+// [us the whole call, a thread per dim with everything after the wait / a warp for any number of chunks, asking first for the chunks of the larger size / now: 32 sequences of about 4000
+// keys 93.7 / 90.1 / 90; one of 700 9.0 / 8.8 / 8.2; four of 700 under a table of 128 blocks 10.8 / 11.3 / 10.6; one of 8000 with 4 kv heads 16.8 / 18.7 / 10.4, of 30000 23.6 / 24.2 / 17.4.]
+// kSplitChunks: a warp's lanes hold 32.  [Four warps from 16 on: 8 sequences of 4000 keys, 32 chunks each, 19.2 -> 20.2 with an 8-bit cache, one of 1400, 22 chunks, 9.1 -> 8.4; from 32 on:
+// one of 3000, 47 chunks, 11.0 -> 8.9.]
+constexpr int kSplitChunks = 32;
+template <typename T, typename TOut, bool kK4, int kSplit>
 __global__ void __launch_bounds__(128)
 paged_attn_merge_kernel(TOut* __restrict__ out, const float* __restrict__ part_o, const float* __restrict__ part_ml,
                         const uint32_t* __restrict__ context_lens, unsigned int* __restrict__ counter, int num_heads,
-                        int num_kv_heads, int group, int max_chunks, int chunk_pages) {
-    const int head = blockIdx.x * 4 + (threadIdx.x >> 5), b = blockIdx.y, lane = threadIdx.x & 31;
+                        int num_kv_heads, int group, int max_chunks, int chunk_pages, int min_pages) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, b = blockIdx.y;
+    const int head = kSplit > 1 ? (int)blockIdx.x : (int)blockIdx.x * 4 + warp;
     const int h = min(head, num_heads - 1) / group, r = min(head, num_heads - 1) - h * group;
     const int ctx = (int)context_lens[b];
-    const int at_least = (ctx + chunk_pages * kPage - 1) / (chunk_pages * kPage);       // chunks, if the decode kernel keeps the proposed size; up to twice as many if it halves it
-    const float2* const mls = reinterpret_cast<const float2*>(part_ml) + ((int64_t)b * num_kv_heads + h) * max_chunks * group + r;
-    const float4* const os = reinterpret_cast<const float4*>(part_o) + (((int64_t)b * num_kv_heads + h) * max_chunks * group + r) * (kHeadDim / 4) + lane;
-    const int64_t o_pitch = (int64_t)group * (kHeadDim / 4);
+    const int most = min((ctx + min_pages * kPage - 1) / (min_pages * kPage), max_chunks), fewest = (ctx + chunk_pages * kPage - 1) / (chunk_pages * kPage);
+    const int part = kSplit > 1 ? warp : 0, shift = kSplit > 1 && most > kSplitChunks ? 2 : 0, parts = 1 << shift;
+    static_assert(kSplit == 1 || kSplit == 4, "parts");
+    auto own = [&](int chunks) { return (chunks - part + parts - 1) >> shift; };         // of that many, this warp's: part, part + parts, ...
+    const int64_t first = (((int64_t)b * num_kv_heads + h) * max_chunks + part) * group + r, pitch = (int64_t)group * parts;
+    const float2* const mls = reinterpret_cast<const float2*>(part_ml) + first;
+    const float4* const os = reinterpret_cast<const float4*>(part_o) + first * (kHeadDim / 4) + lane;
+    const int64_t o_pitch = pitch * (kHeadDim / 4);
     pdl_wait();
     pdl_trigger();
-    if (head >= num_heads) return;
+    if (head >= num_heads || part >= parts) return;
     const int settled = (int)*reinterpret_cast<volatile unsigned int*>(counter + 4);    // the chunk size the decode kernel settled on
     constexpr int kU = 8;                                                                // partials in flight at a time
+    const int ahead = own(most);
     const float2 none = make_float2(-INFINITY, 0.f);
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float2 ml = lane < at_least ? mls[(int64_t)lane * group] : none;
+    float2 ml = lane < ahead ? mls[(int64_t)lane * pitch] : none;
     float4 o[kU];
 #pragma unroll
-    for (int i = 0; i < kU; ++i) o[i] = i < at_least ? os[i * o_pitch] : zero;
-    const int nchunks = (ctx + settled * kPage - 1) / (settled * kPage);
+    for (int i = 0; i < kU; ++i) o[i] = i < ahead ? os[i * o_pitch] : zero;
+    const int nchunks = own(settled == chunk_pages ? fewest : most);
     if (blockIdx.x == 0 && b == 0 && threadIdx.x == 0) *counter = 0u;                   // leave the work queue ready for the next launch
     float M = -INFINITY, L = 0.f;
     float4 acc = zero;
     for (int s0 = 0; s0 < nchunks; s0 += 32) {
         const int n = min(32, nchunks - s0);
-        if (s0 > 0 || lane >= at_least) ml = lane < n ? mls[(int64_t)(s0 + lane) * group] : none;
+        if (s0 > 0) ml = lane < n ? mls[(int64_t)(s0 + lane) * pitch] : none;
+        else if (lane >= n) ml = none;
         const float bm = fmaxf(M, warp_max(ml.x));
         const float corr = bm == -INFINITY ? 1.f : exp2f(M - bm);                        // (first chunks: exp2(-inf) = 0 on zero accumulators)
         const float w = bm == -INFINITY ? 0.f : exp2f(ml.x - bm);
@@ -578,9 +589,10 @@ paged_attn_merge_kernel(TOut* __restrict__ out, const float* __restrict__ part_o
         L = L * corr + warp_sum(w * ml.y);
         M = bm;
         for (int c0 = 0; c0 < n; c0 += kU) {
+            if (s0 + c0 > 0) {
 #pragma unroll
-            for (int i = 0; i < kU; ++i)
-                if (s0 + c0 > 0 || i >= at_least) o[i] = c0 + i < n ? os[(int64_t)(s0 + c0 + i) * o_pitch] : zero;
+                for (int i = 0; i < kU; ++i) o[i] = c0 + i < n ? os[(int64_t)(s0 + c0 + i) * o_pitch] : zero;
+            }
 #pragma unroll
             for (int i = 0; i < kU; ++i) {
                 const float wi = __shfl_sync(0xffffffffu, w, (c0 + i) & 31);
@@ -588,10 +600,27 @@ paged_attn_merge_kernel(TOut* __restrict__ out, const float* __restrict__ part_o
             }
         }
     }
+    if (kSplit > 1 && parts > 1) {
+        __shared__ float4 accs[kSplit][32];
+        __shared__ float2 sums[kSplit];
+        accs[warp][lane] = acc;
+        if (lane == 0) sums[warp] = make_float2(M, L);
+        __syncthreads();
+        if (warp > 0) return;
+        L = 0.f; acc = zero;
+#pragma unroll
+        for (int i = 0; i < kSplit; ++i) M = fmaxf(M, sums[i].x);
+#pragma unroll
+        for (int i = 0; i < kSplit; ++i) {
+            const float w = M == -INFINITY ? 0.f : exp2f(sums[i].x - M);
+            const float4 a = accs[i][lane];
+            L += w * sums[i].y; acc.x += w * a.x; acc.y += w * a.y; acc.z += w * a.z; acc.w += w * a.w;
+        }
+    }
     const float inv[4] = {acc.x, acc.y, acc.z, acc.w};
     TOut res[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) res[kK4 ? (int)k4_index(e) : e] = from_f32<TOut>(to_f32(from_f32<T>(nchunks > 0 && L > 0.f ? inv[e] / L : 0.f)));
+    for (int e = 0; e < 4; ++e) res[kK4 ? (int)k4_index(e) : e] = from_f32<TOut>(to_f32(from_f32<T>(ctx > 0 && L > 0.f ? inv[e] / L : 0.f)));
     TOut* const dst = out + ((int64_t)b * num_heads + head) * kHeadDim + lane * 4;
     if (reinterpret_cast<uintptr_t>(out) & (4 * sizeof(TOut) - 1)) {                     // (an output that does not start on four entries)
         for (int e = 0; e < 4; ++e) dst[e] = res[e];
@@ -658,9 +687,14 @@ void launch(const DecodeArgs& a, const CUtensorMap& kmap, const CUtensorMap& vma
     const int grid = (int)(want < sm_count() ? want : sm_count());
     launch_pdl(kern, dim3(grid), dim3(PL::kThreads), PL::kTotal, st, kmap, vmap, p);
     count_launch();
-    launch_pdl(paged_attn_merge_kernel<T, TOut, kK4>, dim3((a.num_heads + 3) / 4, a.num_seqs), dim3(128), 0, st,
-               static_cast<TOut*>(a.out), (const float*)p.part_o, (const float*)p.part_ml, a.context_lens, p.counter, (int)a.num_heads,
-               (int)a.num_kv_heads, (int)kGroup, (int)p.max_chunks, (int)p.chunk_pages);
+    auto merge = [&](auto split) {
+        constexpr int kSplit = decltype(split)::value;
+        launch_pdl(paged_attn_merge_kernel<T, TOut, kK4, kSplit>, dim3(kSplit > 1 ? a.num_heads : (a.num_heads + 3) / 4, a.num_seqs), dim3(128), 0, st,
+                   static_cast<TOut*>(a.out), (const float*)p.part_o, (const float*)p.part_ml, a.context_lens, p.counter, (int)a.num_heads,
+                   (int)a.num_kv_heads, (int)kGroup, (int)p.max_chunks, (int)p.chunk_pages, (int)p.min_pages);
+    };
+    if (p.max_chunks > kSplitChunks) merge(std::integral_constant<int, 4>{});
+    else merge(std::integral_constant<int, 1>{});
     count_launch();
 }
 
@@ -711,8 +745,8 @@ void paged_attention_decode_tma(const DecodeArgs& a, cudaStream_t st) {
     p.chunk_pages = pick_chunk_pages(a.num_seqs, a.num_kv_heads, a.max_blocks);
     { static const int sw = [] { const char* e = getenv("B200_ATTN_STATIC"); return e ? atoi(e) : 1; }(); p.static_walk = a.fp8 ? sw : 0; }     // queue mode (see the kernel): CTA tickets with FP8 KV (+7 %; -2 % with 16-bit KV, 6 warps)
     { static const int ad = [] { const char* e = getenv("B200_ATTN_ADAPTIVE"); return e ? atoi(e) : 1; }(); p.adaptive_chunks = ad; }
-    const int min_pages = p.adaptive_chunks && p.chunk_pages > 1 ? p.chunk_pages / 2 : p.chunk_pages;      // the kernel may halve the chunk
-    p.max_chunks = (a.max_blocks + min_pages - 1) / min_pages;
+    p.min_pages = p.adaptive_chunks && p.chunk_pages > 1 ? p.chunk_pages / 2 : p.chunk_pages;      // the kernel may halve the chunk
+    p.max_chunks = (a.max_blocks + p.min_pages - 1) / p.min_pages;
     p.scale_log2 = a.scale * 1.4426950408889634f;
     const size_t n_part = (size_t)a.num_seqs * a.num_kv_heads * p.max_chunks * group;
     const size_t need = n_part * (kHeadDim * 4 + 8) + 256;
