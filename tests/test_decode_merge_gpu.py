@@ -78,3 +78,25 @@ def test_workspace_may_start_on_any_word(shift):
     assert all(code == 0 and torch.equal(out, outs[2][0]) for out, code in outs)
     ref = _reference(q, kc, vc, tables, lens, heads // kv_heads)
     assert float((outs[0][0].double() - ref).norm() / ref.norm()) < 2.5e-3
+
+
+@pytest.mark.parametrize("lens,width", [([700, 100, 64], 128), ([1, 700, 2100], 128), ([3000], 47), ([4200, 64, 2048, 2049], 66)])
+def test_merge_looks_at_written_partials_only(lens, width):
+    """the partials of chunks that the larger chunk size leaves out are asked for and not looked at; tables wider than the contexts, few and many chunks in one launch"""
+    heads, kv_heads = 8, 2
+    gen = torch.Generator(device="cuda").manual_seed(width)
+    mk = lambda *s: torch.randn(*s, generator=gen, device="cuda").bfloat16()
+    kc, vc, q = mk(80, 64, kv_heads, 128), mk(80, 64, kv_heads, 128), mk(len(lens), heads, 128)
+    tables = torch.randint(0, 80, (len(lens), width), generator=gen, device="cuda", dtype=torch.int32)
+    ctx = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    L = pkg.lib()
+    need = int(L.paged_attention_decode_workspace_bytes(*map(C.c_int32, (len(lens), heads, 128, width, 64))))
+    ws = torch.full((need,), 255, dtype=torch.uint8, device="cuda")                # NaN everywhere but in the header
+    ws[:256] = 0
+    out = torch.zeros_like(q)
+    p = lambda t: C.c_void_p(t.data_ptr())
+    L.paged_attention_decode(p(out), p(q), p(kc), p(vc), p(tables), p(ctx), *map(C.c_int32, (len(lens), heads, kv_heads, 128, 64, width)), C.c_int64(80), C.c_float(128 ** -0.5), C.c_float(0),
+                             *map(C.c_int32, (0, 2, 2, 0, 2)), p(ws), C.c_size_t(need), C.c_int64(torch.cuda.current_stream().cuda_stream))
+    assert L.b200_last_error() == 0
+    ref = _reference(q, kc, vc, tables, lens, heads // kv_heads)
+    assert float((out.double() - ref).norm() / ref.norm()) < 2.5e-3                # as in test_merge
