@@ -13,7 +13,7 @@
 //
 // One warp per output row, lanes over K in 16-byte weight chunks, 8 activation rows per pass: a shape-generic SIMT kernel
 // (any m / n / k the formats allow).  The m <= 64 decode shapes of block-FP8 run on the tcgen05 pipeline instead
-// (qmatmul_tc.cu: F8Quarter, fp8_tc_run).  B200_FP8_GENERIC=1 forces the SIMT kernel (tests compare the two).
+// (qmatmul_tc.cu: f8_row, fp8_tc_run).  B200_FP8_GENERIC=1 forces the SIMT kernel (tests compare the two).
 #include <cstdlib>
 
 #include "qmatmul.cuh"
@@ -170,7 +170,7 @@ void launch(const Dec& dec, const void* x, const void* bias, void* out, int m, i
 }
 
 // x (f16 / bf16) -> fp16 in "K8" order for the FP4 GEMM on the tcgen05 pipeline: within every aligned group of 8 along k the
-// positions 0..7 hold k = 0,4,1,5,2,6,3,7 (qmatmul_tc.cu, F4Quarter)
+// positions 0..7 hold k = 0,4,1,5,2,6,3,7 (qmatmul_tc.cu, f4_row)
 template <typename T>
 __global__ void cast_f16_k8_kernel(const T* __restrict__ x, __half* __restrict__ out, int64_t groups) {
     pdl_wait();

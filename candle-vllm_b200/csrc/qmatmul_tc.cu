@@ -1,5 +1,5 @@
-// qmatmul_tc.cu -- tcgen05 dequant-GEMM for weight-only quantised linears at decode batch sizes (m <= 64):
-// GGML Q4_K / Q6_K (QMatMul), symmetric int4 (marlin_4bit_*) and block-scaled FP8 (fp8_matmul).
+// qmatmul_tc.cu -- tcgen05 dequant-GEMM for weight-only quantised linears: GGML Q4_K / Q6_K (QMatMul, up to 2048 rows, and routed
+// experts), int4 (marlin_4bit_*, marlin_awq_4bit_*), block-scaled FP8 and FP4 (fp8_matmul, nvfp4_matmul, mxfp4_matmul) in passes of up to 64 rows.
 //
 //   y[m, n] (+)= sum_k x[m, k] * dequant(W)[n, k]        W row-major over n, verbatim checkpoint bytes (GGUF blocks, ...)
 //
@@ -92,14 +92,13 @@ struct GemmParams {
     int whole_tiles;               // 1: CTA ranges are whole tiles (no split-K, no atomics)
     int slabs;                     // > 0: split tiles write their partial sums to DISTINCT slabs (plain stores, no atomics, no
     int64_t slab_stride;           //      pre-zeroed output): slab s of segment sg starts at y[sg] + s * slab_stride; the consumer sums
-    int one_shift;                 // int4: log2 of a group size that is a power of two >= 64 (32: one group per column); 0: other groups
+    int one_shift;                 // int4: log2 of the group size (64 or 128; 32: one group per column); 0: scales that the bulk copies cannot take
     const void* scales;            // marlin: [K/g, N] in marlin-permuted order (f16 / bf16: scale_bf16); fp8: f32 [N/by, K/bx]
     const void* scales_seg[kMaxSeg];   // marlin, several weight matrices in one launch (engine: QKV, gate|up): scales / zero points of each
-    const uint32_t* zp_seg[kMaxSeg];   //   segment (slot 0 = scales / zp)
+    const uint32_t* zp_seg[kMaxSeg];   //   segment; zero points: AWQ, packed [K/g, N/8] in the marlin layout (null: symmetric, zero point 8)
     int group_size, k;             // marlin group size / fp8 bx
     int scale_bf16, scale_by, scale_sk;
     const float* norm;             // fp8: {2^p, 2^-p} range shift of the tile scales (device)
-    const uint32_t* zp;            // AWQ: packed zero points [K/g, N/8] in the marlin layout (null: symmetric, zero point 8)
     int mrows;                     // dense mode: activation rows per row tile (a multiple of 32 up to kMB)
     int csplit;                    // > 1: a cluster of csplit CTAs shares every tile, each over its part of k; the partial sums meet in shared memory of the
                                    // cluster and every CTA adds up and stores its share of the columns (plain stores in a fixed order: nothing to zero)
@@ -352,7 +351,7 @@ __device__ __forceinline__ int marlin_scale_pos(int n, bool grouped) {
 __device__ __forceinline__ int awq_word(int n) { return ((n >> 6) << 3) + (n & 7); }
 __device__ __forceinline__ int awq_shift(int n) { return 4 * ((0x73625140u >> (4 * ((n & 63) >> 3))) & 7); }           // inverse of [0,2,4,6,1,3,5,7]: 0,4,1,5,2,6,3,7
 __device__ __forceinline__ float m4_scale(uint32_t bits, int bf16) { return bf16 ? __uint_as_float(bits << 16) : __half2float(__ushort_as_half((unsigned short)bits)); }
-// The usual groups (64, 128, ... or one per column): a quarter has one scale.  scales: of the unit, `groups` (1, 2 or 4) rows of 128 in the marlin order, from byte 1024 on as many of
+// A quarter has one scale (groups of 64 or 128, or one per column).  scales: of the unit, `groups` (1, 2 or 4) rows of 128 in the marlin order, from byte 1024 on as many of
 // 16 zero-point words
 __device__ __forceinline__ void m4_row(const uint8_t* blk, const uint8_t* scales, int row, uint32_t a_col, const UnitBars& ub, int groups, bool grouped, int bf16, bool zeros) {
     const int r7 = row & 7;
@@ -392,18 +391,18 @@ struct M4Row {                                   // where the scales and zero po
     __device__ __forceinline__ float scale(uint32_t g) const { return m4_scale(sc[(size_t)g * ld], bf16); }
     __device__ __forceinline__ float zero(uint32_t g) const { return zp ? (float)((zp[(size_t)g * (ld >> 3)] >> shift) & 0xFu) : 8.f; }
 };
-// groups in which a quarter may lie in two (32, or sizes that are no power of two): every scale where it is used
+// scales or zero points that do not start on 16 bytes: a quarter's where it is used (the groups are 64, 128 or one per column, so that a quarter lies in one)
 __device__ __forceinline__ void m4_row_general(const uint8_t* blk, int r7, uint32_t a_col, const UnitBars& ub, const M4Row& m, int k0, int group_size) {
 #pragma unroll 1
     for (int q = 0; q < 4; ++q) {
         if (q == 0) ub.wait_buffer();
-        const uint32_t g0 = (uint32_t)((k0 + q * 64) / group_size), g1 = (uint32_t)((k0 + q * 64 + 32) / group_size);
-        const float s0 = m.scale(g0), s1 = m.scale(g1), z0 = m.zero(g0), z1 = m.zero(g1);
+        const uint32_t g = (uint32_t)((k0 + q * 64) / group_size);
+        const float s = m.scale(g), z = m.zero(g);
         const uint4 a = *reinterpret_cast<const uint4*>(blk + (((2 * q) ^ r7) << 4)), b = *reinterpret_cast<const uint4*>(blk + (((2 * q + 1) ^ r7) << 4));
         if (q == 3) ub.release();
-        const bool fast = __all_sync(0xffffffffu, fmaxf(fabsf(s0), fabsf(s1)) * kNibbleScale <= 65504.f);
-        nibbles_to_tmem(a, b, fast, __float2half2_rn(fast ? s0 * kNibbleScale : s0), __float2half2_rn(-z0 * s0), __float2half2_rn(fast ? s1 * kNibbleScale : s1),
-                        __float2half2_rn(-z1 * s1), a_col + q * 32);
+        const bool fast = __all_sync(0xffffffffu, fabsf(s) * kNibbleScale <= 65504.f);
+        const __half2 S = __float2half2_rn(fast ? s * kNibbleScale : s), N = __float2half2_rn(-z * s);
+        nibbles_to_tmem(a, b, fast, S, N, S, N, a_col + q * 32);
     }
 }
 
@@ -1200,14 +1199,12 @@ int qmatmul_tc_decode_registers(int ggml_type) {
 // slabs (and the bias) and rounds once to f16 / bf16.  scratch = [S][m][n] f32, S = wq16_slabs(n, k).
 int wq16_slabs(int n, int k) { return qmatmul_tc_slab_count((n + kTileN - 1) / kTileN, k / 256); }
 
-// int4 groups in which a quarter of a unit (64 weights) has one scale: their log2, 32 for one group per column; 0 for all others, and where the scales cannot be copied in pieces of
-// 16 bytes (rows of 128 scales and 16 zero-point words of every tile start on such a boundary if the tensors do and n % 64 == 0)
-static int one_shift_of(int group_size, int nseg, const int* n, const void* const* scales, const void* const* qzeros) {
+// int4: log2 of the group size (64 or 128, the callers take no others; 32: one group per column), 0 where the scales cannot be copied in pieces of 16 bytes (rows of 128 scales and 16
+// zero-point words of every tile start on such a boundary if the tensors do: the callers take n % 64 == 0 only)
+static int one_shift_of(int group_size, int nseg, const void* const* scales, const void* const* qzeros) {
     for (int i = 0; i < nseg; ++i)
-        if (n[i] % 64 || ((uintptr_t)scales[i] & 15) || (qzeros && ((uintptr_t)qzeros[i] & 15))) return 0;
-    if (group_size <= 0) return 32;
-    if (group_size < 64 || (group_size & (group_size - 1))) return 0;
-    return 31 - __builtin_clz((unsigned)group_size);
+        if (((uintptr_t)scales[i] | (qzeros ? (uintptr_t)qzeros[i] : 0)) & 15) return 0;
+    return group_size <= 0 ? 32 : 31 - __builtin_clz((unsigned)group_size);
 }
 
 static void wq16_launch(int kind, const void* x_f16, const void* w, const void* scales, int scale_bf16, int group_or_bx, int by, int sk,
@@ -1238,8 +1235,8 @@ static void wq16_launch(int kind, const void* x_f16, const void* w, const void* 
     p.slabs = qmatmul_tc_slab_count(tiles, nsb);
     p.slab_stride = (int64_t)m * n;
     const void* const zps[1] = {zp};
-    p.one_shift = kind == kTypeM4 ? one_shift_of(group_or_bx, 1, &n, &scales, zps) : 0;
-    p.scales = scales; p.group_size = group_or_bx; p.k = k; p.scale_bf16 = scale_bf16; p.scale_by = by; p.scale_sk = sk; p.norm = norm; p.zp = zp;
+    p.one_shift = kind == kTypeM4 ? one_shift_of(group_or_bx, 1, &scales, zps) : 0;
+    p.scales = scales; p.group_size = group_or_bx; p.k = k; p.scale_bf16 = scale_bf16; p.scale_by = by; p.scale_sk = sk; p.norm = norm;
     for (int i = 0; i < kMaxSeg; ++i) { p.scales_seg[i] = scales; p.zp_seg[i] = zp; }
     if (kind == kTypeM4) { if (mb == 32) launch<32, kTypeM4>(wm, xm, p, st); else launch<64, kTypeM4>(wm, xm, p, st); }
     else if (kind == kTypeNV4) { if (mb == 32) launch<32, kTypeNV4>(wm, xm, p, st); else launch<64, kTypeNV4>(wm, xm, p, st); }
@@ -1301,8 +1298,8 @@ void marlin_tc_f32_multi(const void* x_f16_k4, int nseg, const void* const* w, c
     }
     p.ldy = ldy; p.m = m; p.nsb = nsb; p.n_tiles = tiles; p.m_tiles = 1; p.mrows = mb; p.accumulate = accumulate;
     p.whole_tiles = use_whole_tiles(tiles) ? 1 : 0;
-    p.one_shift = one_shift_of(group_size, nseg, n, scales, qzeros);
-    p.scales = p.scales_seg[0]; p.zp = p.zp_seg[0]; p.group_size = group_size; p.k = k; p.scale_bf16 = scale_bf16; p.scale_by = 1;
+    p.one_shift = one_shift_of(group_size, nseg, scales, qzeros);
+    p.scales = p.scales_seg[0]; p.group_size = group_size; p.k = k; p.scale_bf16 = scale_bf16; p.scale_by = 1;
     if (mb == 32) launch<32, kTypeM4>(wm, xm, p, st); else launch<64, kTypeM4>(wm, xm, p, st);
     check_launch("marlin_4bit(f32)");
 }
