@@ -40,6 +40,7 @@ int qmatmul_tc_multi(const void* x_f16, int nseg, const void* const* w, float* c
 int qmatmul_tc_slab_count(int64_t n_tiles, int nsb);
 // registers a thread of the kernel of up to 32 rows (Q4_K, Q6_K)
 int qmatmul_tc_decode_registers(int ggml_type);
+int qmatmul_tc_weight_rings(int32_t* stages_and_groups, int capacity);
 // legacy (accumulating) form; falls back to separate launches
 void qmatmul_dispatch_multi(const void* x_f16, int nseg, const void* const* w, const int* types, float* const* y, const int* n,
                             int64_t ldy, int m, int k, int accumulate, cudaStream_t st);

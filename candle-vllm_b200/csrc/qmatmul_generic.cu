@@ -239,6 +239,8 @@ void qmatmul_f16act(const void* x_f16, const void* w, float* y, int32_t m, int32
 
 int32_t qmatmul_decode_kernel_registers(int32_t ggml_type) { return ggml_type == B200_GGML_Q4_K || ggml_type == B200_GGML_Q6_K ? qmatmul_tc_decode_registers(ggml_type) : 0; }
 
+int32_t qmatmul_weight_rings(int32_t* stages_and_groups, int32_t capacity) { return qmatmul_tc_weight_rings(stages_and_groups, stages_and_groups ? capacity : 0); }
+
 int32_t qmatmul_slab_count(int32_t m, int32_t n, int32_t k, int32_t ggml_type) {
     if (m <= 0 || n <= 0 || k <= 0) return 0;
     return qmatmul_slabs_needed(1, &n, &ggml_type, m, k);

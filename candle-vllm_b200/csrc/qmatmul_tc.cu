@@ -1194,6 +1194,20 @@ int qmatmul_tc_decode_registers(int ggml_type) {
     return a.numRegs;
 }
 
+int qmatmul_tc_weight_rings(int32_t* stages_and_groups, int capacity) {
+    int n = 0;
+    auto add = [&](int stages, int groups) {
+        if (n < capacity) { stages_and_groups[2 * n] = stages; stages_and_groups[2 * n + 1] = groups; }
+        ++n;
+    };
+#define ADD(rows, type) add(Cfg<rows, type>::kWStages, Cfg<rows, type>::kGroups)
+    ADD(32, B200_GGML_Q4_K); ADD(64, B200_GGML_Q4_K); ADD(128, B200_GGML_Q4_K); ADD(256, B200_GGML_Q4_K);
+    ADD(32, B200_GGML_Q6_K); ADD(64, B200_GGML_Q6_K); ADD(128, B200_GGML_Q6_K); ADD(256, B200_GGML_Q6_K);
+    ADD(32, kTypeM4); ADD(64, kTypeM4); ADD(32, kTypeF8); ADD(64, kTypeF8); ADD(32, kTypeNV4); ADD(64, kTypeNV4); ADD(32, kTypeMX4); ADD(64, kTypeMX4);
+#undef ADD
+    return n;
+}
+
 // ---- weight-only GEMMs with 16-bit output (marlin_4bit_*, fp8_matmul) ----------------------------------------------
 // stream-K over all SMs with fp32 partial-sum slabs in the caller's scratch, then one small finishing pass that adds the
 // slabs (and the bias) and rounds once to f16 / bf16.  scratch = [S][m][n] f32, S = wq16_slabs(n, k).

@@ -154,6 +154,9 @@ int32_t qmatmul_slab_count(int32_t m, int32_t n, int32_t k, int32_t ggml_type);
 /* Registers a thread of the dequant-GEMM for up to 32 rows (Q4_K, Q6_K; 0: no such kernel or no device).  608 threads: with more than 80 the small kernels between two
  * products find no room beside it on an SM, and its weight stream cannot start under them. */
 int32_t qmatmul_decode_kernel_registers(int32_t ggml_type);
+/* Stages of the weight ring and groups of dequantising warps that take its units in turn, a pair for each instance of the dequant-GEMM (what its barriers have to
+ * hold for); up to `capacity` pairs are written, the number of instances comes back. */
+int32_t qmatmul_weight_rings(int32_t* stages_and_groups, int32_t capacity);
 int32_t qmatmul_f16act_slabs(const void* x_f16, const void* w, float* y_slabs, int32_t slabs_avail, int32_t m, int32_t n,
                              int32_t k, int32_t ggml_type, int64_t stream);
 /* QTensor::dequantize: W -> f32 [n,k] (linear.rs:808-842 forward_via_dequant) */
