@@ -483,8 +483,9 @@ struct MoeBlockPlan {
         const int64_t P = T * topk;
         rows = chunk_rows_for(P, E); max_chunks = max_chunks_for(P, E, rows);
         // router parts: about six CTAs per SM, at least two steps each, 16 at most (the top-k kernel adds them one after another).  A CTA is four warps; with two per SM too few run
-        // to hide their loads, and half the SMs had one.  [us the block with two / four / six, 128 experts: 900 tokens 262 / 248 / 240, 600 - / 208 / 205, 300 146 / 144 / 144; up to
-        // 100 tokens level, the parts are 16 either way]
+        // to hide their loads, and half the SMs had one.  [us the block with two / six.  8 experts: 4000 tokens 203 / 183, 16000 844 / 796; 32 experts: 900 101 / 101, 2000 200 / 194, 8000
+        // 777 / 770; 128 experts: 300 144 / 137, 900 240 / 218, 2000 474 / 442, 8000 1726 / 1695; 256 experts: 900 303 / 256, 2000 504 / 430, 4000 857 / 855, 8000 1483 / 1482.  Few tokens:
+        // level, the parts are 16 either way]
         const int64_t tiles = ((T + kRtT - 1) / kRtT) * ((E + kRtE - 1) / kRtE), steps = H / kRtK;
         int64_t s = 888 / tiles;
         if (s > 16) s = 16;
