@@ -1,8 +1,11 @@
 // py_calls.cpp -- the operators that a decode step calls most, as native Python functions over the C ABI.
 //
-// A call of a few microseconds on the GPU was entered through 10 to 12 us of Python: shape and type checks, views that change nothing, an allocation, a foreign-function call with a
+// A call of a few microseconds on the GPU was entered through 10 to 26 us of Python: shape and type checks, views that change nothing, an allocation, a foreign-function call with a
 // dozen arguments, the error check.  Here a call whose arguments are plain -- torch tensors of the exact class, on the current device, contiguous, of the types the kernel takes -- is
-// checked, allocated for and launched natively.  Anything else returns None and the caller goes the way through Python: nothing is accepted here that is refused there.  [B200 box, us a call, Python -> here: Linear.forward 14.8, QMatMul.forward 16.4, silu_mul 9.4, PagedAttention.forward (decode, with its cache write) 24.2.]
+// checked, allocated for and launched natively.  Anything else returns None and the caller goes the way through Python: nothing is accepted here that is refused there.  So do the calls
+// that find no workspace or too small a one, an operator's first and those that grow it.
+// [Host time, us a call, Python -> here: Linear.forward 12.8 -> 4.2, QMatMul.forward 16.6 -> 7.4, silu_mul 10.2 -> 4.2, PagedAttention.forward (decode, with its cache write) 25.2 -> 9.7; a
+// call that is left to Python 0.3 more than without the look.]
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -31,15 +34,20 @@ struct Library {
     bool ready = false;
 } L;
 
-// A contiguous tensor of torch's own class with memory on the current device, or null.  (Subclasses, fake and batched tensors, other devices: not here.)
-const at::Tensor* plain(PyObject* o) {
+// A tensor of torch's own class with memory on a device, contiguous or of rows [heads, width] a stride apart, or null.  (Subclasses, fake and batched tensors: not here.)
+const at::Tensor* rows(PyObject* o) {
     if (!THPVariable_CheckExact(o)) return nullptr;
     const at::Tensor& t = THPVariable_Unpack(o);
     if (!t.defined() || t.layout() != at::kStrided || !t.is_cuda() || !t.has_storage() || t.is_neg() || t.is_conj()) return nullptr;
     if (t.unsafeGetTensorImpl()->key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper, c10::DispatchKey::Python,
                                                                        c10::DispatchKey::Functionalize, c10::DispatchKey::Batched}))) return nullptr;
-    return t.is_contiguous() ? &t : nullptr;
+    return t.is_contiguous() || (t.dim() == 3 && t.stride(2) == 1 && t.stride(1) == t.size(2)) ? &t : nullptr;
 }
+const at::Tensor* plain(PyObject* o) {
+    const at::Tensor* t = rows(o);
+    return t && t->is_contiguous() ? t : nullptr;
+}
+int64_t row_stride(const at::Tensor& t) { return t.is_contiguous() ? t.size(1) * t.size(2) : t.stride(0); }
 bool here(const at::Tensor& t, int device) { return t.get_device() == device; }
 int type16(const at::Tensor& t) { return t.scalar_type() == at::kBFloat16 ? B200_BF16 : (t.scalar_type() == at::kHalf ? B200_F16 : -1); }
 bool fits(int64_t v) { return v > 0 && v <= INT32_MAX; }
@@ -132,7 +140,7 @@ PyObject* py_silu_mul(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     END_HANDLE_TH_ERRORS
 }
 
-// paged_attention(prompt, q [T, H, hd], k, v [T, G, hd], k_cache, v_cache [blocks, bs, G, hd], slots i64, tables i32 [B, W], lens i32 [B] or None, cu_q, cu_k i32 [B + 1] or None,
+// paged_attention(prompt, q [T, H, hd], k, v [T, G, hd] (rows any stride apart: parts of a fused projection), k_cache, v_cache [blocks, bs, G, hd], slots i64, tables i32 [B, W], lens i32 [B] or None, cu_q, cu_k i32 [B + 1] or None,
 //                 workspace or None, heads, kv heads, head dim, longest query, window, scale, cap, e4m3 cache)
 // decode: lens and a workspace; prompt: cu_q and cu_k.  An error of the cache write comes back as its negative code.
 PyObject* py_paged_attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
@@ -140,7 +148,7 @@ PyObject* py_paged_attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     if (!L.ready || n_args != 20) Py_RETURN_NONE;
     bool prompt, e4m3;
     if (!number(*a++, prompt)) Py_RETURN_NONE;
-    const at::Tensor *q = plain(a[0]), *k = plain(a[1]), *v = plain(a[2]), *kc = plain(a[3]), *vc = plain(a[4]), *slots = plain(a[5]), *bt = plain(a[6]);
+    const at::Tensor *q = plain(a[0]), *k = rows(a[1]), *v = rows(a[2]), *kc = plain(a[3]), *vc = plain(a[4]), *slots = plain(a[5]), *bt = plain(a[6]);
     if (!q || !k || !v || !kc || !vc || !slots || !bt) Py_RETURN_NONE;
     const at::Tensor *lens = prompt || a[7] == Py_None ? nullptr : plain(a[7]), *cu_q = prompt ? plain(a[8]) : nullptr, *cu_k = prompt ? plain(a[9]) : nullptr, *ws = prompt || a[10] == Py_None ? nullptr : plain(a[10]);
     if (prompt ? (!cu_q || !cu_k) : (!lens || !ws)) Py_RETURN_NONE;
@@ -168,7 +176,7 @@ PyObject* py_paged_attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     {
         Unlocked u;
         L.cache(k->data_ptr(), v->data_ptr(), kc->data_ptr(), vc->data_ptr(), static_cast<const int64_t*>(slots->data_ptr()), (int32_t)k->size(0), (int32_t)G, (int32_t)hd, (int32_t)bs,
-                k->size(1) * k->size(2), v->size(1) * v->size(2), type, cache_type, B200_KV_FLASH, st);
+                row_stride(*k), row_stride(*v), type, cache_type, B200_KV_FLASH, st);
         write_error = L.last_error();
         const auto* tables = static_cast<const uint32_t*>(bt->data_ptr());
         if (write_error) {

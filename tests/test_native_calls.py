@@ -180,12 +180,55 @@ def test_paged_attention(through_python, prompt, fp8, strided):
     ref = call(through_python)
     for _ in range(2):
         assert all(torch.equal(a, b) for a, b in zip(call(lambda f: f()), ref))
+    taken = _lib.calls().paged_attention(prompt, q, k, v, *cache, meta.slot_mapping, meta.block_tables, meta.context_lens, meta.cu_seqlens_q, meta.cu_seqlens_k, op._ws, H, G_, hd, T, 0, hd ** -0.5,
+                                         0.0, fp8)
+    assert torch.equal(taken, ref[0])                     # (K and V as parts of a fused projection as well)
+    assert _lib.calls().paged_attention(prompt, q, k.transpose(0, 1), v.transpose(0, 1), *cache, meta.slot_mapping, meta.block_tables, meta.context_lens, meta.cu_seqlens_q, meta.cu_seqlens_k,
+                                        op._ws, H, G_, hd, T, 0, hd ** -0.5, 0.0, fp8) is None
     if not prompt:
         with pytest.raises(pkg.BackendError):
             op.forward(q, k, v, None, cache[0], cache[1], pkg.InputMetadata(False, meta.slot_mapping, meta.block_tables, cu_seqlens_q=i32([0, T]), cu_seqlens_k=i32([0, T])))
-    with pytest.raises(pkg.BackendError):                 # 80 wide heads: refused by the library, natively too
-        odd = pkg.PagedAttention(H, 72, 1.0, G_)
+    odd = pkg.PagedAttention(H, 72, 1.0, G_)              # a cache of another type than the model's: left to Python, which refuses it
+    with pytest.raises(pkg.BackendError, match="cache dtype"):
         odd.forward(mk(T, H, 72), mk(T, G_, 72), mk(T, G_, 72), None, torch.zeros(nb, 64, G_, 72, dtype=torch.float32, device="cuda"), torch.zeros(nb, 64, G_, 72, dtype=torch.float32, device="cuda"), meta)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prompt", [False, True])
+def test_refusals_of_the_library(through_python, prompt):
+    """what passes the native checks and is refused by the library comes back as its error, in the words of the way through Python"""
+    T, H, G_, nb, native = 2, 4, 2, 4, _lib.calls()
+    i32 = lambda a: torch.tensor(a, dtype=torch.int32, device="cuda")
+    mk = lambda *s: torch.zeros(*s, dtype=torch.bfloat16, device="cuda")
+
+    def words(call):
+        with pytest.raises(pkg.BackendError) as e:
+            call()
+        return str(e.value)
+
+    hd = 264                                              # heads of more than 256
+    op = pkg.PagedAttention(H, hd, 1.0, G_)
+    meta = pkg.InputMetadata(prompt, torch.arange(T, device="cuda"), i32([[0]] * T), context_lens=i32([1, 2]), cu_seqlens_q=i32([0, T]), cu_seqlens_k=i32([0, T]), max_seqlen_q=T)
+    call = lambda: op.forward(mk(T, H, hd), mk(T, G_, hd), mk(T, G_, hd), None, mk(nb, 64, G_, hd), mk(nb, 64, G_, hd), meta)
+    ref = through_python(lambda: words(call))             # (makes the workspace)
+    arguments = lambda: (prompt, mk(T, H, hd), mk(T, G_, hd), mk(T, G_, hd), mk(nb, 64, G_, hd), mk(nb, 64, G_, hd), meta.slot_mapping, meta.block_tables, meta.context_lens, meta.cu_seqlens_q,
+                         meta.cu_seqlens_k, op._ws, H, G_, hd, T, 0, 1.0, 0.0, False)
+    assert native.paged_attention(*arguments()) > 0 and words(call) == ref and ref.startswith("PagedAttention.forward: paged_attention")
+
+    def pending():                                        # an error of an unchecked call of this thread is found by the check of the cache write
+        pkg.lib().rms_norm(None, None, None, 1, 4, 0, 0, 0)
+        return call()
+    ref = through_python(lambda: words(pending))
+    assert words(pending) == ref and ref.startswith("reshape_and_cache: rms_norm")
+    pkg.lib().rms_norm(None, None, None, 1, 4, 0, 0, 0)
+    assert native.paged_attention(*arguments()) < 0
+
+    lin = pkg.Linear(mk(8, 64))
+    x = mk(65)[1:]                                        # contiguous, on an odd multiple of two bytes
+    assert native.linear(x, lin.weight, None) > 0 and words(lambda: lin.forward(x)) == through_python(lambda: words(lambda: lin.forward(x)))
+    x, w, ws = torch.zeros(1, 256, device="cuda"), torch.zeros(144 * 8, dtype=torch.uint8, device="cuda"), torch.zeros(1 << 20, dtype=torch.uint8, device="cuda")
+    assert native.qmatmul(x, w, 8, 256, 99, ws) > 0 and b"type" in pkg.lib().b200_last_error_message()
+    assert native.qmatmul(x, w, 8, 256, pkg.GgmlType.Q4_K, ws).shape == (1, 8)
 
 
 @pytest.mark.gpu
