@@ -158,6 +158,16 @@ struct DecodeParams {
     float scale_log2;                 // scale * log2(e)
 };
 
+// The size of a chunk from the device-side context lengths: the host proposes p.chunk_pages (pick_chunk_pages, from the table width); items are whole chunks, so the makespan is rounds x
+// chunk length -- when the proposed size leaves an awkward last round (e.g. 2.16 items per warp = 3 rounds of 16 tiles at ctx 4664 with FP8 KV: 74 us instead of 63), half the size wins.
+// full, half: chunks of all sequences under the two sizes.  Every CTA of the decode kernel and every warp of the merge takes the same decision from the same numbers.
+__device__ __forceinline__ int settled_chunk_pages(int full, int half, int num_kv_heads, int slots, int chunk_pages, int adaptive) {
+    if (chunk_pages <= 1 || !adaptive) return chunk_pages;
+    const int64_t r0 = ((uint32_t)full * (uint32_t)num_kv_heads + slots - 1) / (uint32_t)slots, r1 = ((uint32_t)half * (uint32_t)num_kv_heads + slots - 1) / (uint32_t)slots;
+    // cost in tiles: rounds x (tiles per chunk + ~1 tile of per-item overhead: claim, Q fragments, partial write, merge)
+    return r1 * (chunk_pages + 1) < r0 * (2 * chunk_pages + 1) ? chunk_pages / 2 : chunk_pages;
+}
+
 // One work item = (sequence b, kv head h, chunk c of <= chunk_pages pages), owned by ONE warp.
 // Header words in shared memory: {valid, b, h, c, ctx, ntiles}.
 //
@@ -203,10 +213,6 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_
     }
     pdl_wait();            // context_lens / q / KV written by the previous kernels
     pdl_trigger();
-    // Chunk size from the DEVICE-side context lengths: the host proposes p.chunk_pages (pick_chunk_pages, from the table width);
-    // items are whole chunks, so the makespan is rounds x chunk length -- when the proposed size leaves an awkward last round (e.g. 2.16
-    // items per warp = 3 rounds of 16 tiles at ctx 4664 with FP8 KV: 74 us instead of 63), half the size wins.  Every CTA takes the same
-    // decision from the same numbers; CTA 0 publishes it in the workspace header for the merge kernel.
     int* prefix_half = reinterpret_cast<int*>(smem + PL::kHalf);           // chunk prefix for the halved chunk size
     int* decision = reinterpret_cast<int*>(smem + PL::kMail + 96);
     {
@@ -221,16 +227,7 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_
     if (threadIdx.x == 0) {
         prefix[0] = prefix_half[0] = 0;
         for (int b = 0; b < p.num_seqs; ++b) { prefix[b + 1] += prefix[b]; prefix_half[b + 1] += prefix_half[b]; }
-        int cp = p.chunk_pages;
-        if (p.chunk_pages > 1 && p.adaptive_chunks) {
-            const int64_t slots = (int64_t)gridDim.x * PL::kWarps;
-            const int64_t r0 = ((int64_t)prefix[p.num_seqs] * p.num_kv_heads + slots - 1) / slots;
-            const int64_t r1 = ((int64_t)prefix_half[p.num_seqs] * p.num_kv_heads + slots - 1) / slots;
-            // cost in tiles: rounds x (tiles per chunk + ~1 tile of per-item overhead: claim, Q fragments, partial write, merge)
-            if (r1 * (p.chunk_pages + 1) < r0 * (2 * p.chunk_pages + 1)) cp = p.chunk_pages / 2;
-        }
-        decision[0] = cp;
-        if (blockIdx.x == 0) p.counter[4] = (unsigned int)cp;
+        decision[0] = settled_chunk_pages(prefix[p.num_seqs], prefix_half[p.num_seqs], p.num_kv_heads, (int)gridDim.x * PL::kWarps, p.chunk_pages, p.adaptive_chunks);
     }
     __syncthreads();
     const int chunk_pages = decision[0];
@@ -536,52 +533,60 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_
     }
 }
 
-// Merges the chunk partials of one (sequence, head), four dims a lane: by a warp, or (kSplit 4) by a CTA whose warps take every fourth chunk each, if there may be more than kSplitChunks.
-// The kernel is latency: launched beside the decode kernel, it has the context length before that kernel ends (which lets its dependents start only after it has waited for what came
-// before), and when it has ended asks at once for the chunk size and for the partials of all chunks that there are under the smaller of the two sizes; what the larger size leaves unwritten
-// is not looked at.  A lane holds the maximum and the sum of one chunk, so that the weights cost one exponential a lane.
-// [us the whole call, a thread per dim with everything after the wait / a warp for any number of chunks, asking first for the chunks of the larger size / now: 32 sequences of about 4000
-// keys 93.7 / 90.1 / 90; one of 700 9.0 / 8.8 / 8.2; four of 700 under a table of 128 blocks 10.8 / 11.3 / 10.6; one of 8000 with 4 kv heads 16.8 / 18.7 / 10.4, of 30000 23.6 / 24.2 / 17.4.]
+// Merges the chunk partials of one (sequence, head), four dims a lane: by a warp, or (kSplit 4) by a CTA whose warps take every fourth chunk each, if there are more than kSplitChunks.
+// The kernel is latency: launched beside the decode kernel, it has the context lengths before that kernel ends (which lets its dependents start only after it has waited for what came
+// before), settles the chunk size for itself from them and asks for everything at once when that kernel has ended.  A lane holds the maximum and the sum of one chunk, so that the weights
+// cost one exponential a lane.
+// [The chunk size read from where the decode kernel puts it: the chunks that a halved size adds come a round trip later; asked for on suspicion, those that were never written come from DRAM,
+// a decode step of 4 rows 295.8 -> 298.  us the whole call, a thread per dim with everything after the wait / a warp for any number of chunks, reading the size / now: 32 sequences of about
+// 4000 keys 93.7 / 90.1 / 90; one of 700 8.8 / 8.4 / 8.1; four of 700 under a table of 128 blocks 10.8 / 11.3 / 10.8; one of 8000 with 4 kv heads 16.8 / 18.8 / 10.7, of 30000 23.7 / 24.2
+// / 17.9.  Decode steps of 1 to 6 rows under such a table: within 0.5 % of the second.]
 // kSplitChunks: a warp's lanes hold 32.  [Four warps from 16 on: 8 sequences of 4000 keys, 32 chunks each, 19.2 -> 20.2 with an 8-bit cache, one of 1400, 22 chunks, 9.1 -> 8.4; from 32 on:
 // one of 3000, 47 chunks, 11.0 -> 8.9.]
 constexpr int kSplitChunks = 32;
 template <typename T, typename TOut, bool kK4, int kSplit>
 __global__ void __launch_bounds__(128)
-paged_attn_merge_kernel(TOut* __restrict__ out, const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                        const uint32_t* __restrict__ context_lens, unsigned int* __restrict__ counter, int num_heads,
-                        int num_kv_heads, int group, int max_chunks, int chunk_pages, int min_pages) {
+paged_attn_merge_kernel(TOut* __restrict__ out, const DecodeParams p, int group, int slots) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, b = blockIdx.y;
-    const int head = kSplit > 1 ? (int)blockIdx.x : (int)blockIdx.x * 4 + warp;
-    const int h = min(head, num_heads - 1) / group, r = min(head, num_heads - 1) - h * group;
-    const int ctx = (int)context_lens[b];
-    const int most = min((ctx + min_pages * kPage - 1) / (min_pages * kPage), max_chunks), fewest = (ctx + chunk_pages * kPage - 1) / (chunk_pages * kPage);
-    const int part = kSplit > 1 ? warp : 0, shift = kSplit > 1 && most > kSplitChunks ? 2 : 0, parts = 1 << shift;
+    const int ctx = (int)p.context_lens[b];
+    int pages = p.chunk_pages;
+    if (p.min_pages != p.chunk_pages) {
+        unsigned n0 = 0, n1 = 0;
+        for (int i = lane; i < p.num_seqs; i += 32) {
+            const unsigned c = ((int)p.context_lens[i] + kPage - 1) / kPage;
+            n0 += (c + p.chunk_pages - 1) / (unsigned)p.chunk_pages; n1 += (c + p.min_pages - 1) / (unsigned)p.min_pages;
+        }
+        pages = settled_chunk_pages((int)__reduce_add_sync(0xffffffffu, n0), (int)__reduce_add_sync(0xffffffffu, n1), p.num_kv_heads, slots, p.chunk_pages, 1);
+    }
+    const int total = (int)(((unsigned)(ctx + kPage - 1) / kPage + pages - 1) / (unsigned)pages);
+    // kSplit: a CTA for each head, of which every fourth does four heads and the others leave at once where the chunks are few (they would take the registers that the next kernel starts in)
     static_assert(kSplit == 1 || kSplit == 4, "parts");
-    auto own = [&](int chunks) { return (chunks - part + parts - 1) >> shift; };         // of that many, this warp's: part, part + parts, ...
-    const int64_t first = (((int64_t)b * num_kv_heads + h) * max_chunks + part) * group + r, pitch = (int64_t)group * parts;
-    const float2* const mls = reinterpret_cast<const float2*>(part_ml) + first;
-    const float4* const os = reinterpret_cast<const float4*>(part_o) + first * (kHeadDim / 4) + lane;
+    const bool split = kSplit > 1 && total > kSplitChunks;
+    if (kSplit > 1 && !split && (blockIdx.x & 3)) return;
+    const int head = split ? (int)blockIdx.x : (kSplit > 1 ? (int)blockIdx.x : (int)blockIdx.x * 4) + warp;
+    const int h = min(head, p.num_heads - 1) / group, r = min(head, p.num_heads - 1) - h * group;
+    const int part = split ? warp : 0, shift = split ? 2 : 0, parts = 1 << shift;
+    const int nchunks = (total - part + parts - 1) >> shift;                             // this warp's: part, part + parts, ...
+    const int64_t first = (((int64_t)b * p.num_kv_heads + h) * p.max_chunks + part) * group + r, pitch = (int64_t)group * parts;
+    const float2* const mls = reinterpret_cast<const float2*>(p.part_ml) + first;
+    const float4* const os = reinterpret_cast<const float4*>(p.part_o) + first * (kHeadDim / 4) + lane;
     const int64_t o_pitch = pitch * (kHeadDim / 4);
     pdl_wait();
     pdl_trigger();
-    if (head >= num_heads || part >= parts) return;
-    const int settled = (int)*reinterpret_cast<volatile unsigned int*>(counter + 4);    // the chunk size the decode kernel settled on
+    if (head >= p.num_heads) return;
     constexpr int kU = 8;                                                                // partials in flight at a time
-    const int ahead = own(most);
     const float2 none = make_float2(-INFINITY, 0.f);
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float2 ml = lane < ahead ? mls[(int64_t)lane * pitch] : none;
+    float2 ml = lane < nchunks ? mls[(int64_t)lane * pitch] : none;
     float4 o[kU];
 #pragma unroll
-    for (int i = 0; i < kU; ++i) o[i] = i < ahead ? os[i * o_pitch] : zero;
-    const int nchunks = own(settled == chunk_pages ? fewest : most);
-    if (blockIdx.x == 0 && b == 0 && threadIdx.x == 0) *counter = 0u;                   // leave the work queue ready for the next launch
+    for (int i = 0; i < kU; ++i) o[i] = i < nchunks ? os[i * o_pitch] : zero;
+    if (blockIdx.x == 0 && b == 0 && threadIdx.x == 0) *p.counter = 0u;                 // leave the work queue ready for the next launch
     float M = -INFINITY, L = 0.f;
     float4 acc = zero;
     for (int s0 = 0; s0 < nchunks; s0 += 32) {
         const int n = min(32, nchunks - s0);
         if (s0 > 0) ml = lane < n ? mls[(int64_t)(s0 + lane) * pitch] : none;
-        else if (lane >= n) ml = none;
         const float bm = fmaxf(M, warp_max(ml.x));
         const float corr = bm == -INFINITY ? 1.f : exp2f(M - bm);                        // (first chunks: exp2(-inf) = 0 on zero accumulators)
         const float w = bm == -INFINITY ? 0.f : exp2f(ml.x - bm);
@@ -600,7 +605,7 @@ paged_attn_merge_kernel(TOut* __restrict__ out, const float* __restrict__ part_o
             }
         }
     }
-    if (kSplit > 1 && parts > 1) {
+    if (split) {
         __shared__ float4 accs[kSplit][32];
         __shared__ float2 sums[kSplit];
         accs[warp][lane] = acc;
@@ -621,7 +626,7 @@ paged_attn_merge_kernel(TOut* __restrict__ out, const float* __restrict__ part_o
     TOut res[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) res[kK4 ? (int)k4_index(e) : e] = from_f32<TOut>(to_f32(from_f32<T>(ctx > 0 && L > 0.f ? inv[e] / L : 0.f)));
-    TOut* const dst = out + ((int64_t)b * num_heads + head) * kHeadDim + lane * 4;
+    TOut* const dst = out + ((int64_t)b * p.num_heads + head) * kHeadDim + lane * 4;
     if (reinterpret_cast<uintptr_t>(out) & (4 * sizeof(TOut) - 1)) {                     // (an output that does not start on four entries)
         for (int e = 0; e < 4; ++e) dst[e] = res[e];
     } else if constexpr (sizeof(TOut) == 2) {
@@ -690,8 +695,7 @@ void launch(const DecodeArgs& a, const CUtensorMap& kmap, const CUtensorMap& vma
     auto merge = [&](auto split) {
         constexpr int kSplit = decltype(split)::value;
         launch_pdl(paged_attn_merge_kernel<T, TOut, kK4, kSplit>, dim3(kSplit > 1 ? a.num_heads : (a.num_heads + 3) / 4, a.num_seqs), dim3(128), 0, st,
-                   static_cast<TOut*>(a.out), (const float*)p.part_o, (const float*)p.part_ml, a.context_lens, p.counter, (int)a.num_heads,
-                   (int)a.num_kv_heads, (int)kGroup, (int)p.max_chunks, (int)p.chunk_pages, (int)p.min_pages);
+                   static_cast<TOut*>(a.out), p, (int)kGroup, grid * PL::kWarps);
     };
     if (p.max_chunks > kSplitChunks) merge(std::integral_constant<int, 4>{});
     else merge(std::integral_constant<int, 1>{});
@@ -755,8 +759,8 @@ void paged_attention_decode_tma(const DecodeArgs& a, cudaStream_t st) {
         return;
     }
     if ((uintptr_t)a.workspace & 3) { set_error(kErrBadArg, "paged_attention_decode: workspace must start on 4 bytes"); return; }
-    // layout: [counter] [partial O] [partial (m, l)].  The merge reads partial O sixteen bytes at a time, so it starts on the last such boundary that leaves the counter's five words
-    // 244 to 256 bytes, wherever the caller's workspace starts.
+    // layout: [counter] [partial O] [partial (m, l)].  The merge reads partial O sixteen bytes at a time, so it starts on the last such boundary that leaves the counter 244 to 256 bytes,
+    // wherever the caller's workspace starts.
     p.counter = static_cast<unsigned int*>(a.workspace);
     p.part_o = reinterpret_cast<float*>(((uintptr_t)a.workspace + 256) & ~(uintptr_t)15);
     p.part_ml = p.part_o + n_part * kHeadDim;

@@ -858,13 +858,22 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
                     if (lane == 0) mbar_arrive(d_empty(db));
                 }
                 if constexpr (kMB == 32 && !kGrouped) {
-                    if (ti.count == 1) {                              // one row: nothing to lay side by side (0.05 to 0.2 us a product)
-                        float* const y1 = ybase + n_idx;
+                    if (ti.count <= 2) {                              // one row or two: nothing to lay side by side (0.05 to 0.2 us a product)
+                        float* const o0 = ybase + n_idx;
+                        float* const o1 = o0 + p.ldy;
+                        const bool two = ti.count == 2;
                         if (n_idx < n_rows) {
                             if (store) {
-                                *y1 = __uint_as_float(acc[0]);
-                                for (int z = 1; z <= zero_slabs; ++z) y1[(int64_t)z * p.slab_stride] = 0.f;
-                            } else asm volatile("red.global.add.f32 [%0], %1;" ::"l"(y1), "f"(__uint_as_float(acc[0])) : "memory");
+                                *o0 = __uint_as_float(acc[0]);
+                                if (two) *o1 = __uint_as_float(acc[1]);
+                                for (int z = 1; z <= zero_slabs; ++z) {
+                                    o0[(int64_t)z * p.slab_stride] = 0.f;
+                                    if (two) o1[(int64_t)z * p.slab_stride] = 0.f;
+                                }
+                            } else {
+                                asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o0), "f"(__uint_as_float(acc[0])) : "memory");
+                                if (two) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(o1), "f"(__uint_as_float(acc[1])) : "memory");
+                            }
                         }
                         break;
                     }

@@ -82,7 +82,7 @@ def test_workspace_may_start_on_any_word(shift):
 
 @pytest.mark.parametrize("lens,width", [([700, 100, 64], 128), ([1, 700, 2100], 128), ([3000], 47), ([4200, 64, 2048, 2049], 66)])
 def test_merge_looks_at_written_partials_only(lens, width):
-    """the partials of chunks that the larger chunk size leaves out are asked for and not looked at; tables wider than the contexts, few and many chunks in one launch"""
+    """partials that the chunk size which decode kernel and merge settle for leaves out are not looked at; tables wider than the contexts, few and many chunks in one launch"""
     heads, kv_heads = 8, 2
     gen = torch.Generator(device="cuda").manual_seed(width)
     mk = lambda *s: torch.randn(*s, generator=gen, device="cuda").bfloat16()
