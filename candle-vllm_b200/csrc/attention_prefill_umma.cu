@@ -17,8 +17,9 @@
 // O_i += P_i V of step j - 1 is complete, because a commit covers every MMA issued before it.
 //
 // Bound: exp2 (16 per clock and SM) and the tensor pipe need 1024 clocks each for a 128 x 128 tile; the counters say 42 % of either, and 32 % of the issue slots (4096 tokens).  What
-// takes the time is a tile's chain -- scores, maximum, exponentials, P, rescaled O -- with two tiles in flight per SM, and power in a loop.
-// us, mma.sync kernel / this one (B200, bf16, 32 heads / 8 kv heads): 8192 tokens 2290 / 603, three prompts of 280 to 700 tokens on cached prefixes 238 / 82, 300 tokens on 4000
+// takes the time is a tile's chain -- scores, maximum, exponentials, P, rescaled O -- with two tiles in flight per SM, and in a loop power (8192 tokens: 536 us at
+// 1965 MHz after idling, 607 at 1728 MHz, as many clocks).
+// us, mma.sync kernel / this one (B200, bf16, 32 heads / 8 kv heads): 8192 tokens 2290 / 600, three prompts of 280 to 700 tokens on cached prefixes 238 / 79, 300 tokens on 4000
 // 167 / 82, 32 single tokens on 1000 164 / 53, one on 700 26 / 18.
 #include <cuda.h>
 
@@ -175,7 +176,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
     const uint32_t sb = smem_u32(smem);
     const int tp = 128 / p.hp;                                       // tokens per M tile; a CTA has two
 
-    // which (sequence, tile of 2 tp tokens)?  Tiles are numbered sequence by sequence and dealt out from the last: the rows with most keys start first
+    // which (sequence, tile of 2 tp tokens)?  Tiles are numbered sequence by sequence and dealt out from the last: of each sequence, the rows with most keys start first
     int seq = -1, tile = 0;
     {
         const int want = p.tiles - 1 - (int)blockIdx.y;
