@@ -19,8 +19,11 @@
 // Bound: exp2 (16 per clock and SM) and the tensor pipe need 1024 clocks each for a 128 x 128 tile; the counters say 42 % of either, and 32 % of the issue slots (4096 tokens).  What
 // takes the time is a tile's chain -- scores, maximum, exponentials, P, rescaled O -- with two tiles in flight per SM, and in a loop power (8192 tokens: 536 us at
 // 1965 MHz after idling, 607 at 1728 MHz, as many clocks).
-// us, mma.sync kernel / this one (B200, bf16, 32 heads / 8 kv heads): 8192 tokens 2290 / 600, three prompts of 280 to 700 tokens on cached prefixes 238 / 79, 300 tokens on 4000
-// 167 / 82, 32 single tokens on 1000 164 / 53, one on 700 26 / 18.
+// A step of 128 keys takes 3900 clocks where 16 CTAs run and 4700 to 5000 where all SMs do (stamped: per tile 1300 waiting for its products, 100 scores, 250 to 350 maximum, 1300
+// exponentials, 400 to 550 O, 85 stores of P).  Level or slower, all measured: rows shared by two warps, O rescaled by warps of its own, O += P V started with 96 of the 128 keys,
+// one issuing warp per tile (94 us for 76), scores read from TMEM a second time in place of 128 registers (77), persistent CTAs that fetch the next tile's queries ahead.
+// us, mma.sync kernel / this one (B200, bf16, 32 heads / 8 kv heads): 8192 tokens 2290 / 577, three prompts of 280 to 700 tokens on cached prefixes 238 / 77, 100 tokens on 4000
+// 76 / 31 (without / with clusters that share a tile's keys).
 #include <cuda.h>
 
 #include <type_traits>
@@ -36,16 +39,21 @@ using namespace tc;
 
 constexpr int kHd = 128, kPg = 64, kKt = 128;           // head size, tokens per page, keys per tile
 constexpr int kThreadsU = 12 * 32;                        // two softmax warpgroups, one for TMA and MMA (two of its warps idle)
-// registers a thread after the split: 2 x 128 x 216 + 128 x 72 = 64512 = the 384 x 168 of the launch
-constexpr int kRegsSoftmax = 216, kRegsOther = 72;
+// registers a thread after the split: 2 x 128 x 208 + 128 x 88 = 64512 = the 384 x 168 of the launch.  (216 and 72 spilled 48 bytes in the TMA and MMA warps, and with next to no L1
+// a spilled word comes from L2: 100 tokens on 4000 76.3 / 75.8 us, four prompts of 1400 to 2000 tokens 145 / 144.)
+constexpr int kRegsSoftmax = 208, kRegsOther = 88;
 static_assert(256 * kRegsSoftmax + 128 * kRegsOther <= kThreadsU * 168, "register split");
 constexpr int kTileBytes = 128 * kHd * 2;               // a Q, K or V tile: two halves of 64 dims, 128 rows of 128 bytes each
 constexpr int kRing = 5;
 constexpr int kSmQ = 0, kSmKv = 2 * kTileBytes, kSmBar = kSmKv + kRing * kTileBytes;
 constexpr int kNumBars = 1 + 2 * kRing + 8;             // q_full, kv_full[], kv_empty[], s_full[2], p_ready[2], o_full[2], scan_go, v_clean
 constexpr int kSmFlag = kSmBar + kNumBars * 8, kSmTmem = kSmFlag + 4, kSmDirty = kSmTmem + 4, kSmOInit = kSmDirty + 8;
-constexpr int kSmemU = kSmOInit + 8;
+constexpr int kSmPlace = kSmOInit + 8;                    // where the CTA's tile lies: a Place
+constexpr int kSmemU = kSmPlace + 32;
 static_assert(kSmemU <= 232448, "shared memory");
+// a part's results, where Q, K and V were: O f32 [256][128], 16-byte pieces of a row exchanged by its number, then (maximum, sum) of each row
+constexpr int kSmO = 0, kSmMl = 256 * kHd * 4;
+constexpr int kMaxParts = 8, kPartTiles = 2;              // CTAs that share a tile at most; key tiles that a part has at least
 
 struct UmmaPrefillParams {
     void* out;
@@ -53,7 +61,7 @@ struct UmmaPrefillParams {
     const uint32_t* block_tables; const uint32_t* cu_q; const uint32_t* cu_k;
     int num_seqs, num_heads, num_kv_heads, max_blocks, window, chunk;
     int hp;                          // heads per tile (power of two, divides the heads of a kv head)
-    int tiles;                       // grid.y: upper bound of the token tiles over all sequences
+    int parts;                       // CTAs of a cluster
     float scale_log2;                // > 0
     const float* sink;               // [H] or null
     uint32_t* report;                // where a wait that was given up is reported
@@ -167,7 +175,32 @@ __device__ __forceinline__ void add_nonfinite(const T* values, const uint32_t* t
 // 561 / 603.]
 __device__ __forceinline__ int two_part_keys(int klen) { return klen > 2048 ? kKt : kKt / 2; }
 
-template <typename T>
+// The `work`-th (tile, group of heads), the groups of a tile side by side, tiles numbered sequence by sequence from its last one: of each sequence, the rows with most keys start
+// first.  By one warp, a lane per sequence: an SM's L1 is what 227 KB of shared memory leave of it, so that whatever is read twice comes from L2 twice.
+// [Dealt out by keys over all sequences, the longest first, by CTAs of their own or by persistent ones that fetch the next tile's queries ahead: level at three prompts of 280 to
+// 701 tokens on prefixes (78 us either way), slower for four prompts of 1400 to 2000 tokens (151 and 161 against 144).]
+struct Place { int seq, q_begin, qlen, klen, tile; };                // seq = -1: no such tile
+__device__ __forceinline__ Place tile_place(const UmmaPrefillParams& p, int toks, int want) {
+    const int lane = threadIdx.x & 31;
+    for (int s0 = 0; s0 < p.num_seqs; s0 += 32) {
+        const int s = min(s0 + lane, p.num_seqs - 1), begin = (int)p.cu_q[s], qlen = (int)p.cu_q[s + 1] - begin, klen = (int)(p.cu_k[s + 1] - p.cu_k[s]);
+        const int nt = s0 + lane < p.num_seqs ? (qlen + toks - 1) / toks : 0;
+        int upto = nt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += u; }
+        const uint32_t hit = __ballot_sync(0xffffffffu, want >= upto - nt && want < upto);
+        if (hit) {
+            const int l = __ffs(hit) - 1;
+            return Place{s0 + l, __shfl_sync(0xffffffffu, begin, l), __shfl_sync(0xffffffffu, qlen, l), __shfl_sync(0xffffffffu, klen, l), __shfl_sync(0xffffffffu, upto, l) - 1 - want};
+        }
+        want -= __shfl_sync(0xffffffffu, upto, 31);
+    }
+    return Place{-1, 0, 0, 0, 0};
+}
+
+// kSplit: the CTAs of a cluster share a tile's keys.  Each leaves O, the maxima and the sums of its part in its shared memory, and takes the merge of a share of the rows from all of
+// them.  A part has kPartTiles key tiles at least: where a tile has fewer, the last CTAs have nothing to do.
+template <typename T, bool kSplit>
 __global__ void __launch_bounds__(kThreadsU, 1)
 paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                                const UmmaPrefillParams p) {
@@ -175,39 +208,6 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t sb = smem_u32(smem);
     const int tp = 128 / p.hp;                                       // tokens per M tile; a CTA has two
-
-    // which (sequence, tile of 2 tp tokens)?  Tiles are numbered sequence by sequence and dealt out from the last: of each sequence, the rows with most keys start first
-    int seq = -1, tile = 0;
-    {
-        const int want = p.tiles - 1 - (int)blockIdx.y;
-        int acc = 0;
-        for (int s = 0; s < p.num_seqs; ++s) {
-            const int nt = ((int)(p.cu_q[s + 1] - p.cu_q[s]) + 2 * tp - 1) / (2 * tp);
-            if (want < acc + nt) { seq = s; tile = want - acc; break; }
-            acc += nt;
-        }
-    }
-    if (seq < 0) return;
-    const int head0 = blockIdx.x * p.hp, kvh = head0 / (p.num_heads / p.num_kv_heads);
-    const int q_begin = (int)p.cu_q[seq], qlen = (int)p.cu_q[seq + 1] - q_begin, klen = (int)(p.cu_k[seq + 1] - p.cu_k[seq]);
-    const int q0 = tile * 2 * tp, pos0 = klen - qlen + q0;           // first token of the CTA and its position
-    int first_key = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
-    if (p.chunk > 0) first_key = max(first_key, (pos0 / p.chunk) * p.chunk);
-    const int kt0 = first_key & ~(kKt - 1), page_lo = first_key / kPg, page_end = (klen - 1) / kPg;
-    // key tiles of the two M tiles (none when the tile has no token)
-    int nk[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int toks = min(tp, qlen - q0 - i * tp);
-        nk[i] = toks > 0 ? max((pos0 + i * tp + toks - 1 - kt0) / kKt + 1, 1) : 0;      // (at least one: rows before a context that is too short see nothing and are written as 0)
-    }
-    const int n = max(nk[0], nk[1]), two_keys = two_part_keys(klen);
-    // tiles in which a row of the CTA has hidden keys: past the first row's position, or before the last row's first key
-    const int pos_last = pos0 + min(2 * tp, qlen - q0) - 1;
-    int last_lo = p.window > 0 ? max(0, pos_last - p.window + 1) : 0;
-    if (p.chunk > 0) last_lo = max(last_lo, (pos_last / p.chunk) * p.chunk);
-    auto hides = [&](int j) { return kt0 + j * kKt + kKt - 1 > pos0 || kt0 + j * kKt < last_lo; };
-
     const uint32_t bars = sb + kSmBar;
     const uint32_t q_full = bars;
     auto kv_full = [&](int s) { return bars + (1 + s) * 8; };
@@ -220,6 +220,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
     volatile uint32_t* o_init = reinterpret_cast<volatile uint32_t*>(smem + kSmOInit);        // [2]: O_i holds something before its first product
     volatile uint32_t* flag = reinterpret_cast<volatile uint32_t*>(smem + kSmFlag);
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + kSmTmem);
+    volatile int* place = reinterpret_cast<volatile int*>(smem + kSmPlace);
     const GiveUp give_up{flag, p.report, kWaitPromptAttention, kWaitLimitNs};
     if (threadIdx.x == 0) {
         *flag = 0u;
@@ -235,10 +236,50 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "r"(512));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
+    // Lengths, tables and the cache may come from the kernel before.  (No early trigger for the kernel behind: its CTAs, waiting on the SMs, cost 1 to 1.5 us at 1000 to 2000 tokens.)
+    pdl_wait();
+    if (warp == 8) {
+        if (lane < 3) asm volatile("prefetch.tensormap [%0];" ::"l"(lane == 0 ? &qmap : lane == 1 ? &kmap : &vmap) : "memory");
+        const Place w = tile_place(p, 2 * tp, (int)blockIdx.y);
+        if (lane == 0) { place[0] = w.seq; place[1] = w.q_begin; place[2] = w.qlen; place[3] = w.klen; place[4] = w.tile; }
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    const int seq = place[0], q_begin = place[1], qlen = place[2], klen = place[3], tile = place[4], group = kSplit ? (int)blockIdx.x / p.parts : (int)blockIdx.x, rank = kSplit ? (int)blockIdx.x % p.parts : 0;
+    auto leave = [&] { if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512)); };
+    if (seq < 0) { leave(); return; }
+    const int head0 = group * p.hp, kvh = head0 / (p.num_heads / p.num_kv_heads);
+    const int q0 = tile * 2 * tp, pos0 = klen - qlen + q0;           // first token of the CTA and its position
+    int first_key = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;
+    if (p.chunk > 0) first_key = max(first_key, (pos0 / p.chunk) * p.chunk);
+    int kt0 = first_key & ~(kKt - 1);
+    const int page_lo = first_key / kPg, page_end = (klen - 1) / kPg;
+    // key tiles of the two M tiles (none when the tile has no token)
+    int nk[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int toks = min(tp, qlen - q0 - i * tp);
+        nk[i] = toks > 0 ? max((pos0 + i * tp + toks - 1 - kt0) / kKt + 1, 1) : 0;      // (at least one: rows before a context that is too short see nothing and are written as 0)
+    }
+    int n = max(nk[0], nk[1]), parts = 1;
+    if (kSplit) {                                                    // this CTA's key tiles
+        parts = min(p.parts, max(n / kPartTiles, 1));
+        if (rank >= parts) { leave(); return; }
+        const int from = rank * n / parts, to = (rank + 1) * n / parts;
+        kt0 += from * kKt;
+        n = to - from;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) nk[i] = min(max(nk[i] - from, 0), n);
+    }
+    const int two_keys = rank == 0 ? two_part_keys(klen) : 0;
+    // tiles in which a row of the CTA has hidden keys: past the first row's position, or before the last row's first key
+    const int pos_last = pos0 + min(2 * tp, qlen - q0) - 1;
+    int last_lo = p.window > 0 ? max(0, pos_last - p.window + 1) : 0;
+    if (p.chunk > 0) last_lo = max(last_lo, (pos_last / p.chunk) * p.chunk);
+    auto hides = [&](int j) { return kt0 + j * kKt + kKt - 1 > pos0 || kt0 + j * kKt < last_lo; };
+
     int issued = 0;                                                  // key and value tiles that warp 8 has sent for
 
     if (warp >= 8) {
@@ -401,6 +442,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
             __syncwarp();
         }
     }
+    if (kSplit && parts > 1) { __syncwarp(); cluster_sync(); cluster_sync(); }      // (with the softmax warps)
     } else {
         // ============================================ SOFTMAX ===============================================================
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
@@ -416,11 +458,11 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         int scans = 0;
         int w_max_lo = p.window > 0 ? max(0, klen - qlen + w_last - p.window + 1) : 0;
         if (p.chunk > 0) w_max_lo = max(w_max_lo, ((klen - qlen + w_last) / p.chunk) * p.chunk);
-        const float sink = p.sink ? p.sink[head] * 1.4426950408889634f : -INFINITY;
+        const float sink = p.sink && rank == 0 ? p.sink[head] * 1.4426950408889634f : -INFINITY;
         float m = sink;                                                             // what the row's P are scaled by (log2 units)
         float2 l2 = make_float2(sink != -INFINITY ? 1.f : 0.f, 0.f);
         bool ok = true;
-        const int nki = nk[i];
+        const int nki = i ? nk[1] : nk[0];
         // a tile without hidden keys needs no mask and no look at its values: a body of its own, so that the rare paths stay out of the hot one
         auto step = [&](int j, auto hiding, auto two_parts) -> bool {
             constexpr bool kHides = decltype(hiding)::value, kTwo = decltype(two_parts)::value;
@@ -509,26 +551,100 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
         };
         if (nki > 0) ok = step(0, std::true_type{}, std::true_type{});
         for (int j = 1; j < nki && ok; ++j) ok = hides(j) ? step(j, std::true_type{}, std::false_type{}) : step(j, std::false_type{}, std::false_type{});
-        if (nki > 0 && ok && mbar_wait_or_flag(o_full(i), 0, give_up)) {
+        if (kSplit && parts > 1) {
+            // the last products of both tiles are over, so that nothing reads Q, K and V any more: O, maximum and sum go there
+            for (int k = 0; k < 2; ++k) ok = ok && (nk[k] == 0 || mbar_wait_or_flag(o_full(k), 0, give_up));
+            tc_fence_after();
+            const int r = i * 128 + row;
+            if (nki > 0 && ok) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t o[32];
+                    ld32(o_t + c * 32, o);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        *reinterpret_cast<uint4*>(smem + kSmO + r * (kHd * 4) + (((c * 8 + e) ^ lane) << 4)) = make_uint4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
+                }
+            }
+            *reinterpret_cast<float2*>(smem + kSmMl + r * 8) = nki > 0 ? make_float2(m, l2.x + l2.y) : make_float2(-INFINITY, 0.f);
+            __syncwarp();
+            cluster_sync();
+            // rows [first, last) of the 256, four at a time by a warp; a lane has four entries of each, and (maximum, sum) of one row in one part
+            const int first = rank * 256 / parts, last = (rank + 1) * 256 / parts;
+            for (int r0 = first + warp * 4; r0 < last; r0 += 32) {
+                const int mr = min(r0 + (lane >> 3), last - 1), mq = lane & 7;
+                float2 ml = make_float2(-INFINITY, 0.f);
+                if (mq < parts) {
+                    const uint32_t at = cluster_map(sb + kSmMl + mr * 8, mq);
+                    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(ml.x), "=f"(ml.y) : "r"(at));
+                }
+                float mm = ml.x;
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
+                const bool none = ml.x == -INFINITY && ml.y == 0.f;                  // no visible key in this part, or no such tile: its O is not looked at
+                const float w = none ? 0.f : ex2(ml.x == -INFINITY && mm == -INFINITY ? 0.f : ml.x - mm);
+                float l = none ? 0.f : w * ml.y;
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+                const uint32_t empty = __ballot_sync(0xffffffffu, none);
+                float4 acc[4];
+#pragma unroll
+                for (int g = 0; g < 4; ++g) acc[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+                for (int q = 0; q < parts; ++q) {
+                    const uint32_t base = cluster_map(sb + kSmO, q);
+                    float4 v[4];
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        const int rr = min(r0 + g, last - 1);
+                        v[g] = (empty >> (8 * g + q)) & 1u ? make_float4(0.f, 0.f, 0.f, 0.f) : ld_cluster_f32x4(base + rr * (kHd * 4) + ((lane ^ (rr & 31)) << 4));
+                    }
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        const float wq = __shfl_sync(0xffffffffu, w, 8 * g + q);
+                        acc[g].x = fmaf(wq, v[g].x, acc[g].x); acc[g].y = fmaf(wq, v[g].y, acc[g].y);
+                        acc[g].z = fmaf(wq, v[g].z, acc[g].z); acc[g].w = fmaf(wq, v[g].w, acc[g].w);
+                    }
+                }
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    const float lg = __shfl_sync(0xffffffffu, l, 8 * g), inv = lg > 0.f ? 1.f / lg : 0.f;
+                    const int rr = r0 + g, tk = q0 + (rr >> 7) * tp + (rr & 127) / p.hp;
+                    if (rr < last && tk < qlen && ok)
+                        *reinterpret_cast<uint2*>(static_cast<T*>(p.out) + ((int64_t)(q_begin + tk) * p.num_heads + head0 + (rr & 127) % p.hp) * kHd + lane * 4) =
+                            make_uint2(pack2<T>(acc[g].x * inv, acc[g].y * inv), pack2<T>(acc[g].z * inv, acc[g].w * inv));
+                }
+            }
+            __syncwarp();
+            cluster_sync();                                                         // nobody reads this CTA's part any more
+        } else if (nki > 0 && ok && mbar_wait_or_flag(o_full(i), 0, give_up)) {
             tc_fence_after();
             const float l = l2.x + l2.y, inv = l > 0.f ? 1.f / l : 0.f;
-            T* dst = static_cast<T*>(p.out) + ((int64_t)(q_begin + tok) * p.num_heads + head) * kHd;
+            // rows as they leave: through the query tile, which has been read for the last time, so that a store of a warp covers two rows and not a piece of 32
+            uint8_t* const mine = smem + kSmQ + i * kTileBytes + (warp & 3) * (kTileBytes / 4);
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 uint32_t o[32];
                 ld32(o_t + c * 32, o);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (tok < qlen) {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        uint4 w;
-                        w.x = pack2<T>(__uint_as_float(o[8 * e]) * inv, __uint_as_float(o[8 * e + 1]) * inv);
-                        w.y = pack2<T>(__uint_as_float(o[8 * e + 2]) * inv, __uint_as_float(o[8 * e + 3]) * inv);
-                        w.z = pack2<T>(__uint_as_float(o[8 * e + 4]) * inv, __uint_as_float(o[8 * e + 5]) * inv);
-                        w.w = pack2<T>(__uint_as_float(o[8 * e + 6]) * inv, __uint_as_float(o[8 * e + 7]) * inv);
-                        *reinterpret_cast<uint4*>(dst + c * 32 + e * 8) = w;
-                    }
+                for (int e = 0; e < 4; ++e) {
+                    uint4 w;
+                    w.x = pack2<T>(__uint_as_float(o[8 * e]) * inv, __uint_as_float(o[8 * e + 1]) * inv);
+                    w.y = pack2<T>(__uint_as_float(o[8 * e + 2]) * inv, __uint_as_float(o[8 * e + 3]) * inv);
+                    w.z = pack2<T>(__uint_as_float(o[8 * e + 4]) * inv, __uint_as_float(o[8 * e + 5]) * inv);
+                    w.w = pack2<T>(__uint_as_float(o[8 * e + 6]) * inv, __uint_as_float(o[8 * e + 7]) * inv);
+                    *reinterpret_cast<uint4*>(mine + lane * (kHd * 2) + (((c * 4 + e) ^ (lane & 15)) << 4)) = w;
                 }
+            }
+            __syncwarp();
+#pragma unroll 4
+            for (int r = lane >> 4; r < 32; r += 2) {
+                const int rr = (warp & 3) * 32 + r, tk = q0 + i * tp + rr / p.hp;
+                if (tk < qlen)
+                    *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + ((int64_t)(q_begin + tk) * p.num_heads + head0 + rr % p.hp) * kHd + (lane & 15) * 8) =
+                        *reinterpret_cast<const uint4*>(mine + r * (kHd * 2) + (((lane & 15) ^ (r & 15)) << 4));
             }
         }
     }
@@ -585,15 +701,32 @@ bool paged_attention_prefill_umma(void* out, const void* q, const void* kc, cons
         const cuuint32_t box[4] = {64, 1, (cuuint32_t)kPg, 1};
         if (!make_map(&km, kc, 4, dims, strides, box, bf16) || !make_map(&vm, vc, 4, dims, strides, box, bf16)) return false;
     }
-    const UmmaPrefillParams p{out, vc, block_tables, cu_q, cu_k, num_seqs, num_heads, num_kv_heads, max_blocks, window, chunk, hp, tiles, scale * 1.4426950408889634f, sink, wait_report_word()};
-    const dim3 grid(num_heads / hp, tiles);
-    if (bf16) {
-        ensure_dynamic_smem(reinterpret_cast<const void*>(paged_attn_prefill_umma_kernel<__nv_bfloat16>), kSmemU);
-        paged_attn_prefill_umma_kernel<__nv_bfloat16><<<grid, kThreadsU, kSmemU, st>>>(qm, km, vm, p);
-    } else {
-        ensure_dynamic_smem(reinterpret_cast<const void*>(paged_attn_prefill_umma_kernel<__half>), kSmemU);
-        paged_attn_prefill_umma_kernel<__half><<<grid, kThreadsU, kSmemU, st>>>(qm, km, vm, p);
-    }
+    UmmaPrefillParams p{out, vc, block_tables, cu_q, cu_k, num_seqs, num_heads, num_kv_heads, max_blocks, window, chunk, hp, 1, scale * 1.4426950408889634f, sink, wait_report_word()};
+    // Few tiles: clusters share their keys, as many CTAs a tile as run at the same time.  (About this many tiles there are, sequences of equal length supposed: the lengths are on the
+    // device, and a tile takes fewer CTAs where it has few keys.)  The table's width bounds what a tile can have.
+    // [us without / with, graph: 100 tokens on 4000 75 / 33 (8 CTAs a tile), 512 on 4000 84 / 60 (2), four of 60 on 1000 29 / 25 (4), 700 on 300 with 8 heads 27 / 25 (5).  More CTAs
+    // than run at the same time cost more than they give: 1000 tokens 27 / 45, three prompts of 280 to 701 tokens on prefixes 78 / 136.]
+    const int groups = num_heads / hp;
+    const int64_t ctas = (int64_t)num_seqs * ceil_div(ceil_div(total_q, num_seqs), 2 * tp) * groups;
+    const void* split = bf16 ? reinterpret_cast<const void*>(paged_attn_prefill_umma_kernel<__nv_bfloat16, true>) : reinterpret_cast<const void*>(paged_attn_prefill_umma_kernel<__half, true>);
+    int most = (int)min((int64_t)kMaxParts, (int64_t)max_blocks * kPg / (kPartTiles * kKt));
+    if (ctas * 2 > sm_count()) most = 1;
+    for (int c = most; c > 1 && p.parts == 1; --c)
+        if (max_active_clusters(split, kThreadsU, kSmemU, c) >= ctas) p.parts = c;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(groups * p.parts), (unsigned)tiles); cfg.blockDim = dim3(kThreadsU); cfg.dynamicSmemBytes = kSmemU; cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)p.parts; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = p.parts > 1 ? 2 : 1;
+    auto launch = [&](auto kern) {
+        ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kSmemU);
+        cudaLaunchKernelEx(&cfg, kern, qm, km, vm, p);
+    };
+    if (bf16) { if (p.parts > 1) launch(paged_attn_prefill_umma_kernel<__nv_bfloat16, true>); else launch(paged_attn_prefill_umma_kernel<__nv_bfloat16, false>); }
+    else { if (p.parts > 1) launch(paged_attn_prefill_umma_kernel<__half, true>); else launch(paged_attn_prefill_umma_kernel<__half, false>); }
     count_launch();
     check_launch("paged_attention_prefill");
     return true;
