@@ -77,36 +77,6 @@ __device__ __forceinline__ void tma_4d(uint32_t dst, const CUtensorMap* map, uin
                  "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                  : "memory");
 }
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// MN-major operand, 128-byte swizzle: 64 entries of a row are contiguous, the next 64 lie `lead` bytes further, 8-row groups 1024 bytes apart
-__device__ __forceinline__ uint64_t make_mn_desc(uint32_t saddr, uint32_t lead) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);
-    d |= (uint64_t)(lead >> 4) << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
-__device__ __forceinline__ void ld32(uint32_t taddr, uint32_t* v) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,"
-        "%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
-          "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
-          "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]),
-          "=r"(v[31])
-        : "r"(taddr)
-        : "memory");
-}
 __device__ __forceinline__ void st8(uint32_t taddr, const uint32_t (&v)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]),
                  "r"(v[6]), "r"(v[7])
@@ -335,7 +305,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
 #pragma unroll
                 for (int ks = 0; ks < 8; ++ks) {
                     const uint64_t o = (uint64_t)(((ks >> 2) * (kTileBytes / 2) + (ks & 3) * 32) >> 4);
-                    mma_ss(tmem + i * 128, a + o, b + o, idesc_s, ks > 0 ? 1u : 0u);
+                    tc_mma_ss(tmem + i * 128, a + o, b + o, idesc_s, ks > 0 ? 1u : 0u);
                 }
                 tc_commit(s_full(i));
             }
@@ -470,7 +440,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
             tc_fence_after();
             uint32_t s[128];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) ld32(s_t + c * 32, s + c * 32);
+            for (int c = 0; c < 4; ++c) tc_ld32p(s_t + c * 32, s + c * 32);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             const int k0 = kt0 + j * kKt;
             if (kHides && (k0 + kKt - 1 > w_min_pos || k0 < w_max_lo)) {
@@ -560,7 +530,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     uint32_t o[32];
-                    ld32(o_t + c * 32, o);
+                    tc_ld32p(o_t + c * 32, o);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                     for (int e = 0; e < 8; ++e)
@@ -626,7 +596,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 uint32_t o[32];
-                ld32(o_t + c * 32, o);
+                tc_ld32p(o_t + c * 32, o);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {

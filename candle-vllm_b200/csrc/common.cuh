@@ -25,7 +25,7 @@ void ensure_dynamic_smem(const void* kernel, int bytes);
 int max_active_clusters(const void* kernel, int threads, int smem, int size);
 
 // device address of a host-mapped word in which a kernel that gave up a wait sets its bit (null if it cannot be had); b200_last_error reads and clears it
-enum WaitReport : uint32_t { kWaitPromptAttention = 1, kWaitPairGemm = 2, kWaitCheck = 4 };
+enum WaitReport : uint32_t { kWaitPromptAttention = 1, kWaitPairGemm = 2, kWaitCheck = 4, kWaitLatentDecode = 8 };
 uint32_t* wait_report_word();
 
 #define B200_REQUIRE(cond, code, ...)                  \

@@ -140,8 +140,8 @@ int b200_last_error(void) {
     if (word && *static_cast<volatile uint32_t*>(word)) {
         const uint32_t w = __atomic_exchange_n(word, 0u, __ATOMIC_ACQ_REL);
         if (w) {
-            b200::set_error(b200::kErrCuda, "a kernel of an earlier call gave up a wait and left its output unwritten:%s%s%s", w & b200::kWaitPromptAttention ? " prompt attention" : "",
-                            w & b200::kWaitPairGemm ? " two-SM GEMM" : "", w & b200::kWaitCheck ? " wait limit check" : "");
+            b200::set_error(b200::kErrCuda, "a kernel of an earlier call gave up a wait and left its output unwritten:%s%s%s%s", w & b200::kWaitPromptAttention ? " prompt attention" : "",
+                            w & b200::kWaitPairGemm ? " two-SM GEMM" : "", w & b200::kWaitLatentDecode ? " latent decode" : "", w & b200::kWaitCheck ? " wait limit check" : "");
             e = b200::t_err;
         }
     }

@@ -7,19 +7,22 @@
 // the latent space: score(t) = (q_abs . ckv_t + q_pe . kpe_t) * sm_scale, out = sum_t softmax(score)_t ckv_t  -> [T, H, 512].
 // Every head of a sequence reads the SAME 1152 bytes per token: the op is MQA with a 576-wide key and a 512-wide value.
 //
-// Decode kernel (tensor cores, flash-decoding split over the context): a CTA of 4 warps owns (sequence, chunk of 256 tokens or more,
-// group of 16 heads).  32-token latent tiles land by TMA (nine {64 dims, 32 tokens} boxes, 128-byte swizzle, 3 stages of 36 KB); the
-// 16 heads are the M rows of mma.sync m16n8k16.  Per tile: warp w computes S for tokens [8w, 8w+8) over all 576 dims (Q fragments in
-// registers), the warps agree on the running row maxima through shared memory, P goes to shared memory as 16-bit,
-// and warp w accumulates O for latent dims [128w, 128w+128) over all 32 tokens.  Partials (m, l, O) per chunk are folded by a merge
-// kernel.  Bytes dominate at 16 heads per rank (TP 8): 30 flop / byte; with all 128 heads on one GPU the same tiles serve 8 head groups
-// from L2.
+// Decode kernels (tensor cores, flash-decoding split over the context, partials (m, l, O) per chunk folded by a merge kernel):
+// * mla_decode_umma_kernel, more than 8 heads: tcgen05, the latent tile is the 128-row operand and the heads are the columns (below).
+// * mla_decode_kernel: windows, many sequences, few heads, one page: a CTA of 4 warps owns (sequence, chunk of 256 tokens or more,
+//   group of 16 heads).  32-token latent tiles land by TMA (nine {64 dims, 32 tokens} boxes, 128-byte swizzle, 3 stages of 36 KB); the
+//   16 heads are the M rows of mma.sync m16n8k16.  Per tile: warp w computes S for tokens [8w, 8w+8) over all 576 dims (Q fragments in
+//   registers), the warps agree on the running row maxima through shared memory, P goes to shared memory as 16-bit,
+//   and warp w accumulates O for latent dims [128w, 128w+128) over all 32 tokens.
+// us, the second / the first (B200, bf16, cache write and merge included, 32 sequences of 2900 to 4096 keys): 16 heads 40.0 / 35.6, 32 heads 59 / 40, 128 heads 265 / 81; one sequence of 1000
+// keys, 16 heads 18.0 / 13.6.
 // Prefill (causal, chunked) runs a shape-generic kernel: one CTA per (query row, head).
 #include <cuda.h>
 
 #include <type_traits>
 
 #include "attention.cuh"
+#include "tc_common.cuh"
 
 namespace b200 {
 
@@ -36,23 +39,8 @@ constexpr int kSmStage = 0, kSmP = kSmStage + kMlaStages * kStageB, kSmMax = kSm
 static_assert(2 * (kSmBar + 64 + 1024) <= 233472, "two CTAs per SM");
 constexpr int kMlaSmem = kSmBar + 64;
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count)); }
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "WAIT_LOOP:\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n"
-        "@p bra WAIT_DONE;\n"
-        "bra WAIT_LOOP;\n"
-        "WAIT_DONE:\n"
-        "}\n" ::"r"(bar), "r"(parity)
-        : "memory");
-}
+using namespace tc;
+
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst), "l"(map),
                  "r"(bar), "r"(c0), "r"(c1), "r"(c2)
@@ -106,6 +94,7 @@ struct MlaParams {
     float scale_log2;
     int window;                                // > 0: a row sees only the last `window` keys of its context
     int num_seqs, places;                      // places: CTAs that run at the same time
+    uint32_t* report;                          // where a wait that was given up is reported
 };
 
 // Tokens per chunk of a launch, from the sum and the longest of its contexts (`places` CTAs run at the same time): kChunkTok, what the workspace is sized for, or longer,
@@ -296,14 +285,376 @@ mla_decode_kernel(const __grid_constant__ CUtensorMap cmap, const __grid_constan
     }
 }
 
+// ---- the same on tcgen05: up to 128 sequences without a window -----------------------------------------------------------------------------
+// The latent tile is the 128-row operand and the heads are the columns, so that 16 heads do not leave 7/8 of the products to padding and 64 heads read a tile once:
+//   S^T [128 tokens, N heads] = tile [tokens, 576] Q^T [576, N]     (both K-major in shared memory, as TMA leaves them)
+//   O^T [512, N] += latents^T [512, 128 tokens] P^T [128, N]         (the same tile read MN-major, four blocks of 128 rows; P as [token][head] rows of 128 bytes, MN-major too)
+// N = 16, 32 or 64 heads of a CTA.  One CTA per SM:
+//   warps 0-3 (64 heads: 0-7, two to a token)  thread = token: its scores from TMEM, the heads' maxima over the 128 tokens by halving exchanges and shared memory, P
+//   four warps  O is rescaled where a maximum has grown, beside the weights
+//   one warp    TMA: Q, then tiles of 128 tokens (two pages): four pairs of {64 entries, 128 tokens} boxes in a ring of 4 to 6 pairs, the rotated part where P of the tile before was
+//   one warp    MMA
+// TMEM: S in columns [0, 64), O block b in [64 + b N, ..).
+// Bound: bytes at 16 heads (a tile is 144 KB, 6600 clocks of an SM's share of HBM; 5300 with its products and softmax where not all SMs read, stamped: scores 2300 behind the pairs' arrival,
+// softmax 1200, O 1400); at 64 heads and more the chain of a tile, 7000 to 8000 clocks, since the ring holds one tile.  [O rescaled by the softmax warps, descriptors made anew for
+// every product: 91 us at 128 heads; one softmax warp per 32 tokens there: 88; 81 so.]
+constexpr int kUt = 128, kUPairB = 2 * kUt * 128, kUSubB = kUt * 128;
+template <int kN> struct UCfg {
+    static constexpr int kHalves = kN == 64 ? 2 : 1, kCols = kN / kHalves;           // warps that share a token's heads
+    static constexpr int kWarpO = 4 * kHalves, kWarpT = kWarpO + 4, kWarpM = kWarpT + 1, kThreads = (kWarpM + 1) * 32;
+    static constexpr int kPairs = kN == 16 ? 6 : kN == 32 ? 5 : 4;
+    static constexpr int kQ = kPairs * kUPairB, kP = kQ + 9 * kN * 128, kBar = kP + kUSubB, kNumBars = 2 * kPairs + 5;
+    static constexpr int kRed = kBar + (kNumBars * 8 + 15) / 16 * 16, kMax = kRed + 4 * kN * 4, kCorr = kMax + kN * 4, kFlag = kCorr + kN * 4, kTmem = kFlag + 4, kSmem = kTmem + 4;
+    static_assert(kSmem <= 232448, "shared memory");
+};
+// Tokens per chunk: whole pages, kChunkTok at least (what the workspace is sized for).  Fewer (sequence, head group) pairs than SMs: one round, half a chunk of padding per pair
+// counted in; otherwise the even share of an SM, above which only contexts longer than that are cut.
+__host__ __device__ inline int mla_wide_chunk_rule(int64_t tokens, int num_seqs, int head_groups, int places) {
+    const int64_t work = tokens * head_groups, pairs = (int64_t)num_seqs * head_groups, whole = pairs <= places ? places - pairs / 2 : places;
+    const int64_t want = (work + whole - 1) / whole;
+    return want <= kChunkTok ? kChunkTok : (int)((want + kPg - 1) / kPg * kPg);
+}
+// v[0..kN) of each lane -> v[0] over the 32 lanes: kN = 32: lane h has head h; kN = 16: lanes 2 h and 2 h + 1 have it
+template <int kN, int kHave = kN, int kOff = 16, typename Op> __device__ __forceinline__ void across_lanes(float (&v)[kN], Op op) {
+    if constexpr (kHave > 1) {
+        const bool up = (threadIdx.x & kOff) != 0;
+#pragma unroll
+        for (int i = 0; i < kHave / 2; ++i) {
+            const float give = up ? v[i] : v[i + kHave / 2], keep = up ? v[i + kHave / 2] : v[i];
+            v[i] = op(keep, __shfl_xor_sync(0xffffffffu, give, kOff));
+        }
+    } else {
+        v[0] = op(v[0], __shfl_xor_sync(0xffffffffu, v[0], kOff));
+    }
+    if constexpr (kOff > 1) across_lanes<kN, (kHave > 1 ? kHave / 2 : 1), kOff / 2>(v, op);
+}
+template <int kCols> __device__ __forceinline__ void tmem_columns(uint32_t taddr, uint32_t* v) {
+#pragma unroll
+    for (int c = 0; c < kCols; c += 16) {
+        if constexpr (kCols % 32 == 0) { if (c % 32 == 0) tc_ld32p(taddr + c, v + c); }
+        else tc_ld16(taddr + c, *reinterpret_cast<uint32_t(*)[16]>(v + c));
+    }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+template <typename T, int kN>
+__global__ void __launch_bounds__(UCfg<kN>::kThreads, 1)
+mla_decode_umma_kernel(const __grid_constant__ CUtensorMap cmap, const __grid_constant__ CUtensorMap pmap, const __grid_constant__ CUtensorMap qmap,
+                       const __grid_constant__ CUtensorMap qpmap, const MlaParams p) {
+    using C = UCfg<kN>;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t sb = smem_u32(smem), bars = sb + C::kBar;
+    auto full = [&](int s) { return bars + s * 8; };
+    auto empty = [&](int s) { return bars + (C::kPairs + s) * 8; };
+    const uint32_t q_full = bars + 2 * C::kPairs * 8, rot_full = q_full + 8, s_full = rot_full + 8, p_full = s_full + 8, pv_done = p_full + 8;
+    volatile uint32_t* flag = reinterpret_cast<volatile uint32_t*>(smem + C::kFlag);
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + C::kTmem);
+    const GiveUp give_up{flag, p.report, kWaitLatentDecode, kWaitLimitNs};
+    if (threadIdx.x == 0) {
+        *flag = 0u;
+        for (int i = 0; i < C::kPairs; ++i) { mbar_init(full(i), 1); mbar_init(empty(i), 1); }
+        mbar_init(q_full, 1); mbar_init(rot_full, 1); mbar_init(s_full, 1); mbar_init(p_full, C::kWarpT); mbar_init(pv_done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == C::kWarpT && lane < 4) asm volatile("prefetch.tensormap [%0];" ::"l"(lane == 0 ? &cmap : lane == 1 ? &pmap : lane == 2 ? &qmap : &qpmap) : "memory");
+    pdl_wait();
+    pdl_trigger();
+    // which (sequence, chunk, head group)?  Every warp for itself, lane l has sequences 4 l .. 4 l + 3; the groups of a chunk side by side
+    const int groups = (p.num_heads + kN - 1) / kN, group = (int)blockIdx.x % groups;
+    int seq, chunk, ctx, chunk_tok;
+    {
+        int len[4], own = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { len[i] = 4 * lane + i < p.num_seqs ? (int)p.context_lens[4 * lane + i] : 0; own += len[i]; }
+        chunk_tok = mla_wide_chunk_rule(__reduce_add_sync(0xffffffffu, own), p.num_seqs, groups, p.places);
+        own = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) own += (len[i] + chunk_tok - 1) / chunk_tok;
+        int upto = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += u; }
+        int item = (int)blockIdx.x / groups;
+        const uint32_t hit = __ballot_sync(0xffffffffu, item < upto);
+        if (!hit) return;                                             // past the last chunk: the whole CTA
+        const int l = __ffs(hit) - 1;
+        item -= __shfl_sync(0xffffffffu, upto - own, l);
+        seq = 4 * l; ctx = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int c = __shfl_sync(0xffffffffu, len[i], l), n = (c + chunk_tok - 1) / chunk_tok;
+            if (ctx == 0 && item >= 0) { if (item < n) { ctx = c; seq = 4 * l + i; chunk = item; item = -1; } else item -= n; }
+        }
+    }
+    const int tok_begin = chunk * chunk_tok, ntok = min(chunk_tok, ctx - tok_begin), nt = (ntok + kUt - 1) / kUt, head0 = group * kN;
+    if (warp == C::kWarpM) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "r"(512));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    int issued = 0, rots = 0;                                        // pairs and rotated parts that the TMA warp has sent for
+
+    if (warp == C::kWarpT) {
+        // ============================================ TMA ===================================================================
+        const bool leader = elect_one();
+        const uint32_t* table = p.block_tables + (int64_t)seq * p.max_blocks;
+        if (leader) {
+            mbar_expect_tx(q_full, 9 * kN * 128);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) tma_load_3d(sb + C::kQ + j * kN * 128, &qmap, q_full, j * 64, head0, seq);
+            tma_load_3d(sb + C::kQ + 8 * kN * 128, &qpmap, q_full, 0, head0, seq);
+        }
+        __syncwarp();
+        const int pages = (ntok + kPg - 1) / kPg, page0 = tok_begin / kPg;
+        int b0 = (int)table[page0], b1 = pages > 1 ? (int)table[page0 + 1] : 0;
+        bool ok = true;
+        int it = 0;
+        for (int t = 0; t < nt && ok; ++t) {
+            const int here = min(pages - 2 * t, 2), blk0 = b0, blk1 = b1;
+            if (2 * t + 2 < pages) b0 = (int)table[page0 + 2 * t + 2];
+            if (2 * t + 3 < pages) b1 = (int)table[page0 + 2 * t + 3];
+            for (int b = 0; b < 4 && ok; ++b, ++it) {
+                const int slot = it % C::kPairs;
+                ok = mbar_wait_or_flag(empty(slot), ((it / C::kPairs) & 1) ^ 1, give_up);
+                if (ok && leader) {
+                    const uint32_t dst = sb + slot * kUPairB;
+                    mbar_expect_tx(full(slot), here * 2 * (kUSubB / 2));
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        tma_load_3d(dst + h * kUSubB, &cmap, full(slot), (2 * b + h) * 64, 0, blk0);
+                        if (here > 1) tma_load_3d(dst + h * kUSubB + kUSubB / 2, &cmap, full(slot), (2 * b + h) * 64, 0, blk1);
+                    }
+                }
+                if (ok) issued = it + 1;
+                __syncwarp();
+            }
+            ok = ok && (t == 0 || mbar_wait_or_flag(pv_done, (t - 1) & 1, give_up));
+            if (ok && leader) {
+                mbar_expect_tx(rot_full, here * (kUSubB / 2));
+                tma_load_3d(sb + C::kP, &pmap, rot_full, 0, 0, blk0);
+                if (here > 1) tma_load_3d(sb + C::kP + kUSubB / 2, &pmap, rot_full, 0, 0, blk1);
+            }
+            if (ok) rots = t + 1;
+            __syncwarp();
+        }
+    } else if (warp == C::kWarpM) {
+        // ============================================ MMA ===================================================================
+        // what lies between two products has to be short: addresses are the same for the whole warp and the compiler is told so, descriptors differ in their low words alone
+        const bool leader = elect_one();
+        const uint32_t fmt = std::is_same<T, __nv_bfloat16>::value ? 1u : 0u;
+        const uint32_t idesc_s = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(kN >> 3) << 17) | (8u << 24);         // M 128, N heads, both K-major
+        const uint32_t idesc_o = idesc_s | (1u << 15) | (1u << 16);                                                          // both MN-major
+        const uint32_t ub = __shfl_sync(0xffffffffu, sb, 0), tm = __shfl_sync(0xffffffffu, tmem, 0), tiles = __shfl_sync(0xffffffffu, nt, 0);
+        const uint64_t tile_k = make_b_desc(ub), query = make_b_desc(ub + C::kQ), rot = make_b_desc(ub + C::kP), tile_mn = make_mn_desc(ub, kUSubB), weights = make_mn_desc(ub + C::kP, kUSubB);
+        auto plus = [](uint64_t d, uint32_t bytes) { return (d & 0xffffffff00000000ull) | (uint32_t)((uint32_t)d + (bytes >> 4)); };
+        bool ok = mbar_wait_or_flag(q_full, 0, give_up);
+        int first = 0;                                               // slot of the tile's first pair, and its phase
+        uint32_t phase = 0;
+        for (int t = 0; t < (int)tiles && ok; ++t) {
+            int slot = first;
+            uint32_t ph = phase;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                ok = ok && mbar_wait_or_flag(full(slot), ph, give_up);
+                tc_fence_after();
+                if (ok && leader) {
+                    const uint64_t a = plus(tile_k, slot * kUPairB);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        tc_mma_ss(tm, plus(a, (k >> 2) * kUSubB + (k & 3) * 32), plus(query, (2 * b + (k >> 2)) * kN * 128 + (k & 3) * 32), idesc_s, b > 0 || k > 0 ? 1u : 0u);
+                }
+                __syncwarp();
+                if (++slot == C::kPairs) { slot = 0; ph ^= 1u; }
+            }
+            ok = ok && mbar_wait_or_flag(rot_full, t & 1, give_up);
+            tc_fence_after();
+            if (ok && leader) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) tc_mma_ss(tm, plus(rot, k * 32), plus(query, 8 * kN * 128 + k * 32), idesc_s, 1u);
+                tc_commit(s_full);
+            }
+            __syncwarp();
+            ok = ok && mbar_wait_or_flag(p_full, t & 1, give_up);
+            tc_fence_after();
+            const uint32_t add = t > 0 ? 1u : 0u;
+            int at = first;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                if (ok && leader) {
+                    const uint64_t a = plus(tile_mn, at * kUPairB);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) tc_mma_ss(tm + 64 + b * kN, plus(a, k * 16 * 128), plus(weights, k * 16 * 128), idesc_o, k > 0 ? 1u : add);
+                    tc_commit(empty(at));
+                    if (b == 3) tc_commit(pv_done);
+                }
+                __syncwarp();
+                if (++at == C::kPairs) at = 0;
+            }
+            first = slot;
+            phase = ph;
+        }
+    } else if (warp >= C::kWarpO) {
+        // ============================================ O =====================================================================
+        // (wait given up or not: these warps meet the softmax warps once in every tile)
+        const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
+        const float* const corrs = reinterpret_cast<const float*>(smem + C::kCorr);
+        for (int t = 0; t < nt; ++t) {
+            asm volatile("bar.sync 2, %0;" ::"n"(128 * C::kHalves + 128) : "memory");           // corrs are there, and S: its barrier covers the products of the tiles before
+            tc_fence_after();
+            if (t > 0) {
+                bool moved = false;
+#pragma unroll
+                for (int c = lane; c < kN; c += 32) moved = moved || corrs[c] != 1.f;
+                if (__any_sync(0xffffffffu, moved)) {
+                    constexpr int kAt = kN == 16 ? 16 : 32;
+#pragma unroll 1
+                    for (int b = 0; b < 4 * kN; b += kAt) {
+                        const float* const f = corrs + b % kN;
+                        uint32_t o[kAt];
+                        tmem_columns<kAt>(tmem + lane_addr + 64 + b, o);
+#pragma unroll
+                        for (int c = 0; c < kAt; c += 4) {
+                            const float4 f4 = *reinterpret_cast<const float4*>(f + c);
+                            o[c] = __float_as_uint(__uint_as_float(o[c]) * f4.x); o[c + 1] = __float_as_uint(__uint_as_float(o[c + 1]) * f4.y);
+                            o[c + 2] = __float_as_uint(__uint_as_float(o[c + 2]) * f4.z); o[c + 3] = __float_as_uint(__uint_as_float(o[c + 3]) * f4.w);
+                        }
+#pragma unroll
+                        for (int c = 0; c < kAt; c += 16) tc_st16(tmem + lane_addr + 64 + b + c, *reinterpret_cast<uint32_t(*)[16]>(o + c));
+                    }
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_full);
+        }
+    } else {
+        // ============================================ SOFTMAX ===============================================================
+        // (a wait that was given up does not end the loop: the four warps meet at a barrier in every tile)
+        constexpr int kC = C::kCols;
+        const int quad = warp & 3, half = warp >> 2, row = quad * 32 + lane;          // token of the tile, TMEM lane; the half of the heads
+        const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
+        float* const red = reinterpret_cast<float*>(smem + C::kRed);
+        float* const top = reinterpret_cast<float*>(smem + C::kMax);
+        float* const corrs = reinterpret_cast<float*>(smem + C::kCorr);
+        auto meet = [] { asm volatile("bar.sync 1, %0;" ::"n"(128 * C::kHalves) : "memory"); };
+        // this lane's results of across_lanes -> [warp][head]
+        auto leave = [&](const float (&v)[kC]) {
+            if constexpr (kC == 32) red[quad * kN + half * kC + lane] = v[0];
+            else if ((lane & 1) == 0) red[quad * kN + (lane >> 1)] = v[0];
+        };
+        float l[kC], m_run = -INFINITY;                              // sums of this thread's tokens; the maximum of head `threadIdx.x`
+#pragma unroll
+        for (int h = 0; h < kC; ++h) l[h] = 0.f;
+        bool ok = true;
+        for (int t = 0; t < nt; ++t) {
+            ok = ok && mbar_wait_or_flag(s_full, t & 1, give_up);
+            tc_fence_after();
+            const int valid = ntok - t * kUt;
+            float s[kC];
+            tmem_columns<kC>(tmem + lane_addr + half * kC, reinterpret_cast<uint32_t*>(s));
+#pragma unroll
+            for (int h = 0; h < kC; ++h) s[h] = row < valid ? s[h] * p.scale_log2 : -INFINITY;
+            {
+                float v[kC];
+#pragma unroll
+                for (int h = 0; h < kC; ++h) v[h] = s[h];
+                across_lanes<kC>(v, [](float a, float b) { return fmaxf(a, b); });
+                leave(v);
+            }
+            meet();
+            if (threadIdx.x < kN) {                                  // (a tile has a token, so that the new maximum is finite)
+                const int h = threadIdx.x;
+                const float mn = fmaxf(m_run, fmaxf(fmaxf(red[h], red[kN + h]), fmaxf(red[2 * kN + h], red[3 * kN + h])));
+                top[h] = mn;
+                corrs[h] = fast_exp2(m_run - mn);
+                m_run = mn;
+            }
+            tc_fence_before();
+            asm volatile("bar.sync 2, %0;" ::"n"(128 * C::kHalves + 128) : "memory");           // with the warps that have O
+            uint8_t* const prow = smem + C::kP + row * 128;           // S has been computed: the rotated part is not needed any more
+#pragma unroll
+            for (int c = 0; c < kC / 8; ++c) {
+                uint32_t pk[4];
+#pragma unroll
+                for (int e = 0; e < 8; e += 4) {
+                    const float4 m4 = *reinterpret_cast<const float4*>(top + half * kC + c * 8 + e), c4 = *reinterpret_cast<const float4*>(corrs + half * kC + c * 8 + e);
+                    float* const sv = s + c * 8 + e;
+                    float* const lv = l + c * 8 + e;
+                    const float x0 = fast_exp2(sv[0] - m4.x), x1 = fast_exp2(sv[1] - m4.y), x2 = fast_exp2(sv[2] - m4.z), x3 = fast_exp2(sv[3] - m4.w);
+                    lv[0] = fmaf(lv[0], c4.x, x0); lv[1] = fmaf(lv[1], c4.y, x1); lv[2] = fmaf(lv[2], c4.z, x2); lv[3] = fmaf(lv[3], c4.w, x3);
+                    pk[e >> 1] = pack2<T>(x0, x1);
+                    pk[(e >> 1) + 1] = pack2<T>(x2, x3);
+                }
+                *reinterpret_cast<uint4*>(prow + (((half * (kC / 8) + c) ^ (row & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            }
+            // latents past the context may hold anything: zeroed, their weight is 0 but 0 * NaN would poison O
+            if (row >= valid) {
+#pragma unroll 1
+                for (int b = half; b < 8; b += C::kHalves) {
+                    uint4* const at = reinterpret_cast<uint4*>(smem + ((4 * t + (b >> 1)) % C::kPairs) * kUPairB + (b & 1) * kUSubB + row * 128);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) at[(e + row) & 7] = make_uint4(0, 0, 0, 0);                  // (neighbouring rows: other banks)
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_full);
+        }
+        across_lanes<kC>(l, [](float a, float b) { return a + b; });
+        leave(l);
+        meet();
+        ok = ok && mbar_wait_or_flag(pv_done, (nt - 1) & 1, give_up);
+        tc_fence_after();
+        const int heads = min(kN, p.num_heads - head0);
+        if (ok && threadIdx.x < heads) {
+            const int h = threadIdx.x;
+            const int64_t slot = ((int64_t)seq * p.num_heads + head0 + h) * p.max_chunks + chunk;
+            p.part_ml[slot * 2] = m_run;
+            p.part_ml[slot * 2 + 1] = (red[h] + red[kN + h]) + (red[2 * kN + h] + red[3 * kN + h]);
+        }
+#pragma unroll 1
+        for (int b = half; b < 4; b += C::kHalves)
+#pragma unroll 1
+            for (int c = 0; c < kN; c += 16) {
+                uint32_t o[16];
+                tmem_columns<16>(tmem + lane_addr + 64 + b * kN + c, o);
+                float* dst = p.part_o + (((int64_t)seq * p.num_heads + head0 + c) * p.max_chunks + chunk) * kLat + b * 128 + row;
+#pragma unroll
+                for (int e = 0; e < 16; ++e)
+                    if (ok && c + e < heads) dst[(int64_t)e * p.max_chunks * kLat] = __uint_as_float(o[e]);
+            }
+    }
+    tc_fence_before();
+    __syncthreads();
+    // nothing may be in flight into this CTA's shared memory when it leaves: every copy is awaited by its reader, unless a wait was given up
+    if (warp == C::kWarpT && *flag) { drain_loads(q_full, 1, 1); drain_loads(full(0), C::kPairs, issued); drain_loads(rot_full, 1, rots); }
+    if (warp == C::kWarpM) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(128)
 mla_merge_kernel(T* __restrict__ out, const float* __restrict__ part_o, const float* __restrict__ part_ml, const uint32_t* __restrict__ context_lens,
-                 int num_heads, int max_chunks, const float* __restrict__ sink, int window, int num_seqs, int places) {
+                 int num_heads, int max_chunks, const float* __restrict__ sink, int window, int num_seqs, int places, int wide) {
     const int head = blockIdx.x, seq = blockIdx.y;
     // before the decode kernel ends: it lets its dependents start only after it has waited for what came before, the context lengths among it
     const int ctx = (int)context_lens[seq];
-    const int chunk_tok = mla_chunk_tokens(context_lens, num_seqs, (num_heads + kHg - 1) / kHg, window, places);
+    int chunk_tok;
+    if (wide) {                                                       // heads per CTA of the tcgen05 kernel
+        const int lane = threadIdx.x & 31;
+        int own = 0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) own += lane + 32 * i < num_seqs ? (int)context_lens[lane + 32 * i] : 0;
+        chunk_tok = mla_wide_chunk_rule(__reduce_add_sync(0xffffffffu, own), num_seqs, (num_heads + wide - 1) / wide, places);
+    } else chunk_tok = mla_chunk_tokens(context_lens, num_seqs, (num_heads + kHg - 1) / kHg, window, places);
     const int nchunks = (ctx - (mla_first_key(ctx, window) & ~(kTl - 1)) + chunk_tok - 1) / chunk_tok;
     const int64_t base = ((int64_t)seq * num_heads + head) * max_chunks;
     // a softmax sink (one learned score per head, no key, no value) joins the maximum and the denominator here; the partial maxima are in
@@ -411,12 +762,12 @@ EncodeTiledFn encode_fn() {
     }
     return fn;
 }
-bool make_lat_map(CUtensorMap* map, const void* cache, int64_t num_blocks, int width, int dtype) {
+bool make_lat_map(CUtensorMap* map, const void* cache, int64_t num_blocks, int width, int dtype, int rows = kPg, int box_rows = kTl) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return false;
-    const cuuint64_t dims[3] = {(cuuint64_t)width, (cuuint64_t)kPg, (cuuint64_t)num_blocks};
-    const cuuint64_t strides[2] = {(cuuint64_t)width * 2, (cuuint64_t)kPg * width * 2};
-    const cuuint32_t box[3] = {64, (cuuint32_t)kTl, 1};
+    const cuuint64_t dims[3] = {(cuuint64_t)width, (cuuint64_t)rows, (cuuint64_t)num_blocks};
+    const cuuint64_t strides[2] = {(cuuint64_t)width * 2, (cuuint64_t)rows * width * 2};
+    const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     return enc(map, dtype == B200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(cache), dims, strides,
                box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -496,24 +847,50 @@ void mla_paged_attention_window(void* out, const void* q_absorbed, const void* q
     const size_t need = mla_paged_decode_workspace_bytes(num_seqs, num_heads, max_blocks_per_seq, block_size);
     if (decode && kv_lora_rank == kLat && qk_rope_head_dim == kRope && block_size == kPg && num_blocks > 0 && workspace && workspace_bytes >= need &&
         num_seqs <= 65535 && (((uintptr_t)q_absorbed | (uintptr_t)q_pe | (uintptr_t)ckv_cache | (uintptr_t)kpe_cache) & 15) == 0) {
+        const int max_chunks = (int)(((size_t)max_blocks_per_seq * block_size + kChunkTok - 1) / kChunkTok);
+        MlaParams p{q_absorbed, q_pe, block_tables, context_lens, static_cast<float*>(workspace),
+                    static_cast<float*>(workspace) + (size_t)num_seqs * num_heads * max_chunks * kLat, num_heads, max_blocks_per_seq, max_chunks,
+                    sm_scale * 1.4426950408889634f, window > 0 ? window : 0, num_seqs, 2 * sm_count(), wait_report_word()};
+        const bool bf16 = dtype == B200_BF16;
+        auto merge = [&](int wide) {
+            if (bf16) launch_pdl(mla_merge_kernel<__nv_bfloat16>, dim3(num_heads, num_seqs), dim3(128), 0, st, (__nv_bfloat16*)out, p.part_o, p.part_ml, context_lens, num_heads, max_chunks, sink, p.window, num_seqs, p.places, wide);
+            else launch_pdl(mla_merge_kernel<__half>, dim3(num_heads, num_seqs), dim3(128), 0, st, (__half*)out, p.part_o, p.part_ml, context_lens, num_heads, max_chunks, sink, p.window, num_seqs, p.places, wide);
+            count_launch(2);
+            check_launch("mla_paged_attention");
+        };
+        // The tcgen05 kernel: a window and more sequences than a warp adds up are the other one's, and so are up to 8 heads, whose products it has no use for (4 heads, 100 sequences of
+        // 2000 keys: 46 us mma.sync / 50 tcgen05; 8: 48 / 50; 12: 52 / 52; 16: 56 / 53; 64: 207 / 78), and contexts of one page (16 heads: 8.9 / 9.4; of two 11.3 / 9.2).
+        if (num_heads > 8 && max_blocks_per_seq > 1 && num_seqs <= 128 && window <= 0) {
+            const int wide = num_heads <= 16 ? 16 : num_heads <= 32 ? 32 : 64;
+            CUtensorMap cm, pm, qm, qpm;
+            if (make_lat_map(&cm, ckv_cache, num_blocks, kLat, dtype, kPg, kPg) && make_lat_map(&pm, kpe_cache, num_blocks, kRope, dtype, kPg, kPg) &&
+                make_lat_map(&qm, q_absorbed, num_seqs, kLat, dtype, num_heads, wide) && make_lat_map(&qpm, q_pe, num_seqs, kRope, dtype, num_heads, wide)) {
+                p.places = sm_count();
+                // chunks there can be: by the table's width, and by the rule, whatever the lengths (a chunk that is not its context's last one is an SM's share at least)
+                const int64_t pairs = (int64_t)num_seqs * ceil_div(num_heads, wide), by_rule = p.places + (pairs <= p.places ? (pairs + 1) / 2 : pairs);
+                const dim3 grid((unsigned)(pairs * max_chunks < by_rule ? pairs * max_chunks : by_rule));
+                auto go = [&](auto kern, int smem, int threads) {
+                    ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
+                    launch_pdl(kern, grid, dim3((unsigned)threads), (size_t)smem, st, cm, pm, qm, qpm, p);
+                };
+                if (wide == 16) { if (bf16) go(mla_decode_umma_kernel<__nv_bfloat16, 16>, UCfg<16>::kSmem, UCfg<16>::kThreads); else go(mla_decode_umma_kernel<__half, 16>, UCfg<16>::kSmem, UCfg<16>::kThreads); }
+                else if (wide == 32) { if (bf16) go(mla_decode_umma_kernel<__nv_bfloat16, 32>, UCfg<32>::kSmem, UCfg<32>::kThreads); else go(mla_decode_umma_kernel<__half, 32>, UCfg<32>::kSmem, UCfg<32>::kThreads); }
+                else { if (bf16) go(mla_decode_umma_kernel<__nv_bfloat16, 64>, UCfg<64>::kSmem, UCfg<64>::kThreads); else go(mla_decode_umma_kernel<__half, 64>, UCfg<64>::kSmem, UCfg<64>::kThreads); }
+                merge(wide);
+                return;
+            }
+        }
         CUtensorMap cm, pm;
         if (make_lat_map(&cm, ckv_cache, num_blocks, kLat, dtype) && make_lat_map(&pm, kpe_cache, num_blocks, kRope, dtype)) {
-            const int max_chunks = (int)(((size_t)max_blocks_per_seq * block_size + kChunkTok - 1) / kChunkTok);
-            MlaParams p{q_absorbed, q_pe, block_tables, context_lens, static_cast<float*>(workspace),
-                        static_cast<float*>(workspace) + (size_t)num_seqs * num_heads * max_chunks * kLat, num_heads, max_blocks_per_seq, max_chunks,
-                        sm_scale * 1.4426950408889634f, window > 0 ? window : 0, num_seqs, 2 * sm_count()};
             const dim3 grid(max_chunks, num_seqs, ceil_div(num_heads, kHg));
-            if (dtype == B200_BF16) {
+            if (bf16) {
                 ensure_dynamic_smem(reinterpret_cast<const void*>(mla_decode_kernel<__nv_bfloat16>), kMlaSmem);
                 launch_pdl(mla_decode_kernel<__nv_bfloat16>, grid, dim3(128), kMlaSmem, st, cm, pm, p);
-                launch_pdl(mla_merge_kernel<__nv_bfloat16>, dim3(num_heads, num_seqs), dim3(128), 0, st, (__nv_bfloat16*)out, p.part_o, p.part_ml, context_lens, num_heads, max_chunks, sink, p.window, num_seqs, p.places);
             } else {
                 ensure_dynamic_smem(reinterpret_cast<const void*>(mla_decode_kernel<__half>), kMlaSmem);
                 launch_pdl(mla_decode_kernel<__half>, grid, dim3(128), kMlaSmem, st, cm, pm, p);
-                launch_pdl(mla_merge_kernel<__half>, dim3(num_heads, num_seqs), dim3(128), 0, st, (__half*)out, p.part_o, p.part_ml, context_lens, num_heads, max_chunks, sink, p.window, num_seqs, p.places);
             }
-            count_launch(2);
-            check_launch("mla_paged_attention");
+            merge(0);
             return;
         }
     }
