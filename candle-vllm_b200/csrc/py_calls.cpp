@@ -4,7 +4,8 @@
 // dozen arguments, the error check.  Here a call whose arguments are plain -- torch tensors of the exact class, on the current device, contiguous, of the types the kernel takes -- is
 // checked, allocated for and launched natively.  Anything else returns None and the caller goes the way through Python: nothing is accepted here that is refused there.  So do the calls
 // that find no workspace or too small a one, an operator's first and those that grow it.
-// [Host time, us a call, Python -> here: Linear.forward 12.8 -> 4.2, QMatMul.forward 16.6 -> 7.4, silu_mul 10.2 -> 4.2, PagedAttention.forward (decode, with its cache write) 25.2 -> 9.7; a
+// [Host time, us a call, Python -> here: Linear.forward 12.8 -> 4.2, QMatMul.forward 16.6 -> 7.4, silu_mul 10.2 -> 4.2, PagedAttention.forward (decode, with its cache write) 25.2 -> 9.7,
+// latent decode with its cache write 26 -> less than the GPU's 13.8 (one sequence of 1000 keys); a
 // call that is left to Python 0.3 more than without the look.]
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -29,6 +30,9 @@ struct Library {
     decltype(&paged_attention_decode) decode = nullptr;
     decltype(&paged_attention_decode_workspace_bytes) decode_bytes = nullptr;
     decltype(&paged_attention_prefill) prefill = nullptr;
+    decltype(&concat_and_cache_mla) latent_cache = nullptr;
+    decltype(&mla_paged_attention) latent = nullptr;
+    decltype(&mla_paged_decode_workspace_bytes) latent_bytes = nullptr;
     decltype(&b200_last_error) last_error = nullptr;
     decltype(&b200_device_cc) cc = nullptr;
     bool ready = false;
@@ -192,6 +196,55 @@ PyObject* py_paged_attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     END_HANDLE_TH_ERRORS
 }
 
+// latent_cache(ckv [T, R], k_pe [T, P], their caches [blocks, bs, 1, R] and [.., P], slots i64 [T]) -> 0 or the error's code
+PyObject* py_latent_cache(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    HANDLE_TH_ERRORS
+    if (!L.ready || n_args != 5) Py_RETURN_NONE;
+    const at::Tensor *c = plain(a[0]), *r = plain(a[1]), *cc = plain(a[2]), *rc = plain(a[3]), *slots = plain(a[4]);
+    if (!c || !r || !cc || !rc || !slots || c->dim() != 2 || r->dim() != 2 || cc->dim() != 4 || rc->dim() != 4) Py_RETURN_NONE;
+    const int type = type16(*c), dev = c->get_device();
+    if (type < 0 || cc->scalar_type() != c->scalar_type() || r->scalar_type() != c->scalar_type() || rc->scalar_type() != c->scalar_type() || slots->scalar_type() != at::kLong) Py_RETURN_NONE;
+    const int64_t T = c->size(0), R = c->size(1), P = r->size(1);
+    if (!fits(T) || !fits(R) || !fits(P) || r->size(0) != T || slots->numel() != T || cc->size(3) != R || rc->size(3) != P || cc->size(2) != 1 || rc->size(2) != 1) Py_RETURN_NONE;
+    for (const at::Tensor* t : {r, cc, rc, slots}) if (!here(*t, dev)) Py_RETURN_NONE;
+    if (dev != c10::cuda::current_device() || L.cc() < 100) Py_RETURN_NONE;
+    const int64_t st = reinterpret_cast<int64_t>(c10::cuda::getCurrentCUDAStream(dev).stream());
+    {
+        Unlocked u;
+        L.latent_cache(c->data_ptr(), r->data_ptr(), cc->data_ptr(), rc->data_ptr(), static_cast<const int64_t*>(slots->data_ptr()), (int32_t)T, (int32_t)R, (int32_t)P, type, st);
+    }
+    return PyLong_FromLong(L.last_error());
+    END_HANDLE_TH_ERRORS
+}
+
+// latent_decode(q [B, H, R], q_pe [B, H, P], caches, tables i32 [B, W], lens i32 [B], scale): one row per sequence
+PyObject* py_latent_decode(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    HANDLE_TH_ERRORS
+    if (!L.ready || n_args != 7) Py_RETURN_NONE;
+    const at::Tensor *q = plain(a[0]), *qp = plain(a[1]), *cc = plain(a[2]), *rc = plain(a[3]), *bt = plain(a[4]), *lens = plain(a[5]);
+    double scale;
+    if (!q || !qp || !cc || !rc || !bt || !lens || q->dim() != 3 || qp->dim() != 3 || cc->dim() != 4 || rc->dim() != 4 || bt->dim() != 2 || !number(a[6], scale)) Py_RETURN_NONE;
+    const int type = type16(*q), dev = q->get_device();
+    if (type < 0 || qp->scalar_type() != q->scalar_type() || cc->scalar_type() != q->scalar_type() || rc->scalar_type() != q->scalar_type()) Py_RETURN_NONE;
+    const int64_t B = q->size(0), H = q->size(1), R = q->size(2), P = qp->size(2), W = bt->size(1), nb = cc->size(0), bs = cc->size(1);
+    if (!fits(B) || !fits(H) || !fits(R) || !fits(P) || !fits(W) || !fits(nb) || !fits(bs) || qp->size(0) != B || qp->size(1) != H || bt->size(0) != B || lens->numel() != B) Py_RETURN_NONE;
+    if (cc->size(2) != 1 || rc->size(2) != 1 || cc->size(3) != R || rc->size(3) != P || rc->size(0) != nb || rc->size(1) != bs) Py_RETURN_NONE;
+    if (bt->scalar_type() != at::kInt || lens->scalar_type() != at::kInt) Py_RETURN_NONE;
+    for (const at::Tensor* t : {qp, cc, rc, bt, lens}) if (!here(*t, dev)) Py_RETURN_NONE;
+    if (dev != c10::cuda::current_device() || L.cc() < 100) Py_RETURN_NONE;
+    const size_t need = L.latent_bytes((int32_t)B, (int32_t)H, (int32_t)W, (int32_t)bs);
+    if (need > (size_t)INT64_MAX) Py_RETURN_NONE;
+    at::Tensor out = fresh(q->sizes(), *q, q->scalar_type()), ws = fresh({(int64_t)need}, *q, at::kByte);
+    const int64_t st = reinterpret_cast<int64_t>(c10::cuda::getCurrentCUDAStream(dev).stream());
+    {
+        Unlocked u;
+        L.latent(out.data_ptr(), q->data_ptr(), qp->data_ptr(), cc->data_ptr(), rc->data_ptr(), static_cast<const uint32_t*>(bt->data_ptr()), static_cast<const uint32_t*>(lens->data_ptr()),
+                 nullptr, (int32_t)B, (int32_t)B, (int32_t)H, (int32_t)R, (int32_t)P, (int32_t)bs, (int32_t)W, nb, (float)scale, type, ws.data_ptr(), need, st);
+    }
+    return result(std::move(out));
+    END_HANDLE_TH_ERRORS
+}
+
 // bind(path of the library that is loaded)
 PyObject* py_bind(PyObject*, PyObject* path) {
     const char* p = PyUnicode_AsUTF8(path);
@@ -202,6 +255,7 @@ PyObject* py_bind(PyObject*, PyObject* path) {
     auto find = [&](auto& f, const char* name) { f = reinterpret_cast<std::remove_reference_t<decltype(f)>>(dlsym(h, name)); ok = ok && f; };
     find(L.linear, "linear_16bit"); find(L.qmatmul, "qmatmul_f32"); find(L.qmatmul_bytes, "qmatmul_workspace_bytes"); find(L.silu, "silu_mul"); find(L.cache, "reshape_and_cache");
     find(L.decode, "paged_attention_decode"); find(L.decode_bytes, "paged_attention_decode_workspace_bytes"); find(L.prefill, "paged_attention_prefill");
+    find(L.latent_cache, "concat_and_cache_mla"); find(L.latent, "mla_paged_attention"); find(L.latent_bytes, "mla_paged_decode_workspace_bytes");
     find(L.last_error, "b200_last_error"); find(L.cc, "b200_device_cc");
     if (!ok) { PyErr_Format(PyExc_ImportError, "%s lacks a function", p); return nullptr; }
     L.ready = true;
@@ -213,6 +267,8 @@ PyMethodDef kMethods[] = {{"bind", py_bind, METH_O, nullptr},
                           {"qmatmul", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_qmatmul)), METH_FASTCALL, nullptr},
                           {"silu_mul", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_silu_mul)), METH_FASTCALL, nullptr},
                           {"paged_attention", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_paged_attention)), METH_FASTCALL, nullptr},
+                          {"latent_cache", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_latent_cache)), METH_FASTCALL, nullptr},
+                          {"latent_decode", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(py_latent_decode)), METH_FASTCALL, nullptr},
                           {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_calls", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 

@@ -6,12 +6,17 @@ from typing import Optional
 
 import torch
 
-from ._lib import BackendError, check, require_device, typed
+from ._lib import BackendError, calls, check, fail, require_device, typed
 from .backend import _F, _I, _L, _P, _Z, _at, _cuda, _dt, _guard, _raw_stream
 
 
 def concat_and_cache_mla(ckv: torch.Tensor, k_pe: torch.Tensor, ckv_cache: torch.Tensor, kpe_cache: torch.Tensor, slot_mapping: torch.Tensor) -> None:
     """ckv [T, R], k_pe [T, P] -> caches [nb, bs, 1, R] / [nb, bs, 1, P] at slot_mapping (i64; negative = pad)."""
+    native = calls()
+    if native:
+        r = native.latent_cache(ckv, k_pe, ckv_cache, kpe_cache, slot_mapping)
+        if r is not None:
+            return fail("concat_and_cache_mla", r) if r else None
     for t, n in ((ckv, "ckv"), (k_pe, "k_pe"), (ckv_cache, "ckv_cache"), (kpe_cache, "kpe_cache"), (slot_mapping, "slot_mapping")):
         _cuda(t, n)
     require_device()
@@ -50,6 +55,11 @@ def _mla(q_absorbed, q_pe, ckv_cache, kpe_cache, block_tables, context_lens, cu_
 
 def mla_paged_decode(q_absorbed, q_pe, ckv_cache, kpe_cache, block_tables, context_lens, sm_scale: float) -> torch.Tensor:
     """attention_rs::mla::mla_paged_decode (mla_attention.rs:541-550): one query row per sequence -> [B, H, kv_lora_rank]."""
+    native = calls()
+    if native:
+        r = native.latent_decode(q_absorbed, q_pe, ckv_cache, kpe_cache, block_tables, context_lens, sm_scale)
+        if r is not None:
+            return r if r.__class__ is not int else fail("mla_paged_attention", r)
     return _mla(q_absorbed, q_pe, ckv_cache, kpe_cache, block_tables, context_lens, None, sm_scale)
 
 
