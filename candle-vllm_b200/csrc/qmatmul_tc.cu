@@ -30,6 +30,7 @@
 #include <cuda.h>
 
 #include <cstdlib>
+#include <type_traits>
 
 #include "qmatmul.cuh"
 #include "tc_common.cuh"
@@ -54,7 +55,9 @@ struct Cfg {
     static constexpr int kDBufs = kMB <= 64 ? 2 : 1;
     static constexpr int kBlk = kType == B200_GGML_Q4_K ? 144 : (is_4bit_rows(kType) ? 128 : (kType == kTypeF8 ? 256 : 240));
     static constexpr int kWBytes = kTileN * kBlk;                  // raw weights of one unit (18 KB / 30 KB)
-    static constexpr int kXSlices = kMB == 256 ? 1 : 4;            // 64-wide slices of the activations per stage: a whole unit, or a quarter of it at 256 rows
+    // 64-wide slices of the activations per stage: a whole unit, or a quarter of it at 256 rows, of which up to 128 rows leave room for a second one (with half a stage empty half as
+    // many bytes were on their way)
+    static constexpr int kXSlices = kMB == 256 ? 1 : 4;
     static constexpr int kXBytes = kXSlices * kMB * kXSubBytes;    // slices of [kMB][64] fp16 (16 / 32 / 64 / 32 KB)
     // Two rings.  Raw weight bytes are dead as soon as the dequant warps have pulled them into registers, so the
     // W ring is deep and recycles fast (more HBM reads in flight); the activation slices live until their MMAs
@@ -117,6 +120,12 @@ __device__ __forceinline__ int seg_of_tile(const GemmParams& p, int tile) { retu
 // first tile of segment sg (constant indices only: dynamic indexing would spill the parameter struct to local memory)
 __device__ __forceinline__ int seg_first_tile(const GemmParams& p, int sg) { return sg == 0 ? 0 : (sg == 1 ? p.tile_end[0] : p.tile_end[1]); }
 __device__ __forceinline__ int seg_rows(const GemmParams& p, int sg) { return sg == 0 ? p.n[0] : (sg == 1 ? p.n[1] : p.n[2]); }
+// Rows of a TMA box of activations.  One box where all rows of a tile are loaded anyway (rows past the last one are zeros and cost nothing): a box costs the producer 60 clocks and more,
+// and with boxes of 32 rows a unit of 224 rows was 28 of them, as long as its products.  Routed rows: what a chunk has, in boxes of 64 and one of 32.
+// [us, boxes of 32 / so: MLP of 4096 x 14336, Q4_K, 66 rows 77 / 59, 128 rows 84 / 70, 400 rows 199 / 178, 2000 rows 919 / 850; Q6_K, 203 rows 115 / 108; routed experts, 1000 tokens of 32: 115 / 110]
+constexpr int x_box_rows(int mb, int tile_rows) { return mb == 256 ? tile_rows : mb; }
+// 256 rows: slices that share a stage
+__device__ __forceinline__ int slices_per_stage(int tile_rows) { return tile_rows <= 128 ? 2 : 1; }
 // what a tile id means
 struct Tile {
     int sg, n0;          // segment, first weight row within the segment's matrix
@@ -633,23 +642,42 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         const bool leader = elect_one();
         uint64_t pol_x;
         asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_x));
-        int it = 0;
+        int it = 0, xs = 0;                                // (256 rows: stage and its phase)
+        uint32_t xph = 0;
         int sb = (int)sb0, xtile = (int)tile0;
         Tile ti = u0 < u1 ? tile_of<kMB, kGrouped>(p, xtile) : Tile{};
         for (uint32_t u = u0; u < u1; ++u, ++it) {
-            const int nb = kMB == 32 || (kMB == 64 && !kGrouped) ? kMB / 32 : (ti.count + 31) >> 5;                 // only the 32-row groups that hold rows of this tile
-#pragma unroll
-            for (int q0 = 0; q0 < 4; q0 += C::kXSlices) {
-                const int xi = it * (4 / C::kXSlices) + q0 / C::kXSlices, s = xi % kX;
-                mbar_wait(x_empty(s), ((xi / kX) & 1) ^ 1);
+            if constexpr (kMB == 256) {
+                const int per = slices_per_stage(p.mrows), slice = p.mrows * kXSubBytes;
+                for (int q0 = 0; q0 < 4; q0 += per) {
+                    mbar_wait(x_empty(xs), xph ^ 1);
+                    if (leader) {
+                        mbar_expect_tx(x_full(xs), (uint32_t)(per * slice));
+                        const uint32_t dst = smem_base + C::kXOff + xs * C::kXBytes;
+                        tma_load_2d(dst, &xmap, x_full(xs), sb * kSB + q0 * 64, ti.xrow, pol_x);
+                        if (per == 2) tma_load_2d(dst + slice, &xmap, x_full(xs), sb * kSB + q0 * 64 + 64, ti.xrow, pol_x);
+                    }
+                    __syncwarp();
+                    if (++xs == kX) { xs = 0; xph ^= 1; }
+                }
+            } else {
+                const int nb = kGrouped && kMB > 32 ? (ti.count + 31) >> 5 : kMB / 32, s = it % kX;       // only the 32-row groups that hold rows of this tile
+                mbar_wait(x_empty(s), ((it / kX) & 1) ^ 1);
                 if (leader) {
-                    mbar_expect_tx(x_full(s), (uint32_t)(nb * C::kXSlices) * (32 * kXSubBytes));
+                    mbar_expect_tx(x_full(s), (uint32_t)(nb * 4) * (32 * kXSubBytes));
                     const uint32_t dst = smem_base + C::kXOff + s * C::kXBytes;
 #pragma unroll
-                    for (int q = 0; q < C::kXSlices; ++q)
+                    for (int q = 0; q < 4; ++q) {
+                        const uint32_t at = dst + q * kMB * kXSubBytes;
+                        const int col = sb * kSB + q * 64;
+                        if constexpr (!kGrouped || kMB == 32) tma_load_2d(at, &xmap, x_full(s), col, ti.xrow, pol_x);
+                        else {                             // wmap2 has boxes of 64 rows (a grouped launch has two weight matrices at most)
 #pragma unroll
-                        for (int b = 0; b < kMB / 32; ++b)
-                            if (b < nb) tma_load_2d(dst + q * kMB * kXSubBytes + b * (32 * kXSubBytes), &xmap, x_full(s), sb * kSB + (q0 + q) * 64, ti.xrow + b * 32, pol_x);
+                            for (int b = 0; b < kMB / 64; ++b)
+                                if (2 * b + 1 < nb) tma_load_2d(at + b * (64 * kXSubBytes), &wmap2, x_full(s), col, ti.xrow + b * 64, pol_x);
+                            if (nb & 1) tma_load_2d(at + (nb - 1) * (32 * kXSubBytes), &xmap, x_full(s), col, ti.xrow + (nb - 1) * 32, pol_x);
+                        }
+                    }
                 }
                 __syncwarp();
             }
@@ -660,8 +688,8 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
         // The whole warp runs the (warp-uniform) loop so descriptors / TMEM addresses live in uniform registers;
         // one elected lane issues.  (With a single-lane loop every tcgen05.mma cost ~110 cycles of R2UR traffic.)
         const bool leader = elect_one();
-        int it = 0, seg = 0, ab = 0;
-        uint32_t aph = 0;
+        int it = 0, seg = 0, ab = 0, xs256 = 0;
+        uint32_t aph = 0, xph256 = 0;
         uint32_t tile = tile0;
         for (uint32_t u = u0; u < u1; ++tile) {
             const uint32_t tile_end = (tile + 1) * nsb;
@@ -677,26 +705,32 @@ qmatmul_tc_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_consta
             bool first = true;
             for (; u < seg_end; ++u, ++it) {
                 const uint32_t a_t = tmem + kColA + ab * 128;
-#pragma unroll
-                for (int q0 = 0; q0 < 4; q0 += C::kXSlices) {
-                    const int xi = it * (4 / C::kXSlices) + q0 / C::kXSlices, xs = xi % kX;
-                    mbar_wait(x_full(xs), (xi / kX) & 1);             // activations landed (TMA)
+                // k-step ks of the unit: 64-wide slice ks / 4, 32 bytes per k-step inside its 128-byte swizzled rows; kPer slices of `slice` bytes in a stage
+                auto products = [&](auto slices, int q0, int xs, uint32_t ph, uint32_t slice) {
+                    constexpr int kPer = decltype(slices)::value;
+                    mbar_wait(x_full(xs), ph);                        // activations landed (TMA)
                     if (q0 == 0) mbar_wait(a_ready(ab), aph);         // dequantised A tile is in TMEM
                     tc_fence_after();
                     const uint64_t bd0 = make_b_desc(smem_base + C::kXOff + xs * C::kXBytes);
                     if (leader) {
 #pragma unroll
-                        for (int kq = 0; kq < 4 * C::kXSlices; ++kq) {
-                            // k-step ks of the unit: 64-wide slice (ks / 4), 32 bytes per k-step inside its 128-byte swizzled rows
-                            const int ks = q0 * 4 + kq;
-                            const uint64_t bd = bd0 + (uint64_t)((((kq >> 2) * kMB * kXSubBytes) + (kq & 3) * 32) >> 4);
-                            tc_mma_ts(d_t, a_t + ks * 8, bd, idesc, (first && ks == 0) ? 0u : 1u);
-                        }
-                        tc_commit(x_empty(xs));           // activation slice reusable once these MMAs retire
-                        if (q0 + C::kXSlices == 4) tc_commit(a_free(ab));            // and so is the A buffer
+                        for (int kq = 0; kq < 4 * kPer; ++kq)
+                            tc_mma_ts(d_t, a_t + (q0 * 4 + kq) * 8, bd0 + (uint64_t)(((kq >> 2) * slice + (kq & 3) * 32) >> 4), idesc, (first && q0 == 0 && kq == 0) ? 0u : 1u);
+                        tc_commit(x_empty(xs));                       // activation slices reusable once these MMAs retire
+                        if (q0 + kPer == 4) tc_commit(a_free(ab));    // and so is the A buffer
                     }
                     __syncwarp();
-                }
+                };
+                if constexpr (kMB == 256) {
+                    auto turn = [&] { if (++xs256 == kX) { xs256 = 0; xph256 ^= 1; } };
+                    if (slices_per_stage(p.mrows) == 2) {
+#pragma unroll
+                        for (int q0 = 0; q0 < 4; q0 += 2) { products(std::integral_constant<int, 2>{}, q0, xs256, xph256, (uint32_t)(p.mrows * kXSubBytes)); turn(); }
+                    } else {
+#pragma unroll
+                        for (int q0 = 0; q0 < 4; ++q0) { products(std::integral_constant<int, 1>{}, q0, xs256, xph256, 0u); turn(); }
+                    }
+                } else products(std::integral_constant<int, 4>{}, 0, it % kX, (uint32_t)(it / kX) & 1u, kMB * kXSubBytes);
                 first = false;
                 if (++ab == kGroups) { ab = 0; aph ^= 1; }
             }
@@ -1183,7 +1217,7 @@ int qmatmul_tc_multi(const void* x_f16, int nseg, const void* const* w, float* c
     {
         const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
         const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-        const cuuint32_t box[2] = {64, 32};
+        const cuuint32_t box[2] = {64, (cuuint32_t)x_box_rows(mb, tile_rows(m))};
         const cuuint32_t es[2] = {1, 1};
         CUresult r = enc(&xm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x_f16), dims, strides, box, es,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1255,7 +1289,7 @@ static void wq16_launch(int kind, const void* x_f16, const void* w, const void* 
     {
         const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
         const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-        const cuuint32_t box[2] = {64, 32};
+        const cuuint32_t box[2] = {64, (cuuint32_t)x_box_rows(mb, mb)};
         const cuuint32_t es[2] = {1, 1};
         CUresult r = enc(&xm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x_f16), dims, strides, box, es,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1324,7 +1358,7 @@ void marlin_tc_f32_multi(const void* x_f16_k4, int nseg, const void* const* w, c
     {
         const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)m};
         const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-        const cuuint32_t box[2] = {64, 32};
+        const cuuint32_t box[2] = {64, (cuuint32_t)x_box_rows(mb, mb)};
         const cuuint32_t es[2] = {1, 1};
         CUresult r = enc(&xm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x_f16_k4), dims, strides, box, es,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1379,10 +1413,10 @@ bool qmatmul_tc_moe_supported(int n, int k, int ggml_type) {
     return false;
 }
 
-static bool moe_x_map(CUtensorMap* xm, const void* xs, int rows, int k, const char* who) {
+static bool moe_x_map(CUtensorMap* xm, const void* xs, int rows, int k, int box_rows, const char* who) {
     const cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)k * 2};
-    const cuuint32_t box[2] = {64, 32};
+    const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
     const cuuint32_t es[2] = {1, 1};
     const CUresult r = encode_fn()(xm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(xs), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1403,7 +1437,7 @@ void qmatmul_tc_moe_fp8(const void* xs_f16, int xs_rows, const void* w, const fl
     count_launch();
     CUtensorMap wm[kMaxSeg], xm;
     for (int i = 0; i < kMaxSeg; ++i) if (!make_w_map(&wm[i], w, num_experts * n, nsb, kTypeF8)) return;
-    if (!moe_x_map(&xm, xs_f16, xs_rows, k, "moe_gemm_fp8")) return;
+    if (!moe_x_map(&xm, xs_f16, xs_rows, k, 32, "moe_gemm_fp8")) return;
     if ((int64_t)max_chunks * tiles * nsb * sm_count() >= (int64_t)1 << 31) { set_error(kErrUnsupported, "moe_gemm_fp8: %d items x %d super-blocks exceed the 32-bit unit range", max_chunks * tiles, nsb); return; }
     GemmParams p{};
     for (int i = 0; i < kMaxSeg; ++i) { p.y[i] = y; p.n[i] = n; p.tile_end[i] = 0x7fffffff; p.scales_seg[i] = scale; p.zp_seg[i] = nullptr; }
@@ -1427,7 +1461,8 @@ void qmatmul_tc_moe(const void* xs_f16_k4, int xs_rows, int nseg, const void* co
         if (!make_w_map(&wm[i], w[j], num_experts * n, nsb, ggml_type)) return;      // experts stacked along the rows
         p.y[i] = y[j]; p.n[i] = n; p.tile_end[i] = i < nseg ? (i + 1) * tiles : 0x7fffffff;
     }
-    if (!moe_x_map(&xm, xs_f16_k4, xs_rows, k, "moe_gemm")) return;
+    if (nseg > 2) { set_error(kErrBadArg, "moe_gemm: %d segments (max 2)", nseg); return; }
+    if (!moe_x_map(&xm, xs_f16_k4, xs_rows, k, 32, "moe_gemm") || !moe_x_map(&wm[2], xs_f16_k4, xs_rows, k, 64, "moe_gemm")) return;
     if ((int64_t)max_chunks * nseg * tiles * nsb * sm_count() >= (int64_t)1 << 31) { set_error(kErrUnsupported, "moe_gemm: %d items x %d super-blocks exceed the 32-bit unit range", max_chunks * nseg * tiles, nsb); return; }
     p.ldy = ldy; p.m = chunk_rows; p.nsb = nsb; p.n_tiles = nseg * tiles; p.m_tiles = 1; p.mrows = chunk_rows; p.accumulate = 0; p.whole_tiles = 1;
     p.chunks = chunks; p.num_chunks = num_chunks; p.row_map = row_map; p.row_scale = row_scale;
