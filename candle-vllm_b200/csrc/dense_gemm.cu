@@ -18,6 +18,8 @@
 // Tiles are walked n-major within a band of m-tiles so that CTAs running together share the W tile (L2).
 #include <cuda.h>
 
+#include <algorithm>
+
 #include "qmatmul.cuh"
 #include "tc_common.cuh"
 
@@ -37,20 +39,12 @@ struct DCfg {
     static constexpr int kStages = (200 * 1024) / kStageBytes > 8 ? 8 : (200 * 1024) / kStageBytes;
     static constexpr int kBars = kStages * kStageBytes;              // full[kStages] empty[kStages] tmem_full[2] tmem_empty[2]
     static constexpr int kTmemSlot = kBars + (2 * kStages + 4) * 8;
-    static constexpr int kTotal = kTmemSlot + 16;
+    static constexpr int kBias = kTmemSlot + 16;                     // cluster instances: bias of this CTA's columns, f32
+    static constexpr int kTotal = kBias + kBN * 4;
     static constexpr int kTmemCols = 2 * kBN < 32 ? 32 : 2 * kBN;    // power of two >= 32: 64, 128, 512
     static_assert(kTotal <= 232448, "shared memory");
 };
 
-__device__ __forceinline__ void tc_mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,"
@@ -61,6 +55,10 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
           "=r"(v[31])
         : "r"(taddr)
         : "memory");
+}
+
+__device__ __forceinline__ void st_cluster_f32x4(uint32_t addr, const uint32_t* v) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
 }
 
 struct DenseParams {
@@ -118,6 +116,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
     auto tmem_empty = [&](int b) { return bars + (2 * kS + 2 + b) * 8; };
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + C::kTmemSlot);
 
+    if (warp == 0 && lane < 2) asm volatile("prefetch.tensormap [%0];" ::"l"(lane ? &bmap : &amap) : "memory");
     if (threadIdx.x == 0) {
         for (int s = 0; s < kS; ++s) { mbar_init(full(s), 1); mbar_init(empty(s), 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(tmem_full(b), 1); mbar_init(tmem_empty(b), 4); }
@@ -148,6 +147,11 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
             kb0 = nkb_all * z / p.ksplit; kb1 = nkb_all * (z + 1) / p.ksplit;
         }
     };
+    // clusters: the sums' way.  Up to 64 rows (32 or 64 columns a tile) every CTA leaves its sums where they are and reads its share of the others'; with more rows it sends each CTA its
+    // share, since a load from another SM takes a microsecond and a store nothing  [100 rows, 4 CTAs a tile, tile of 128 columns: 5.9 us from the last product on read, 5.1 sent; 32 rows:
+    // 2.9 read, 3.3 sent]
+    const bool few_rows = kBN == 32 || (kBN == 64 && p.swap);
+    auto lo_group = [&](int q) { return kBN / 8 * q / p.csplit; };       // clusters: first group of eight columns that CTA q adds up
     auto tile_coords = [&](int t, int& ta, int& tb) {
         if (p.ksplit > 1) { ta = t / p.ksplit; tb = 0; return; }
         if (p.tile_group && p.swap) { tb = t / p.tiles_a; ta = t - tb * p.tiles_a; return; }
@@ -239,20 +243,60 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
             tile_coords(t, ta, tb);
             if (p.tile_group && p.tile_group[p.swap ? tb : ta] < 0) continue;
             const int ab = tcount & 1;
+            const int crank = kCluster ? (int)blockIdx.x % p.csplit : 0;
+            unsigned long long ends = 0;                        // first group past CTA q's, a byte each
+            if constexpr (kCluster) {
+                for (int q = 0; q < p.csplit; ++q) ends |= (unsigned long long)lo_group(q + 1) << (8 * q);
+                pdl_wait();
+                if (!few_rows && bias) {
+                    const int j0 = tb * kBN + lo_group(crank) * 8, cols = (lo_group(crank + 1) - lo_group(crank)) * 8;
+                    for (int j = threadIdx.x - 64; j < cols; j += 128) reinterpret_cast<float*>(smem + C::kBias)[j] = j0 + j < p.n ? to_f32(bias[j0 + j]) : 0.f;
+                }
+            }
             mbar_wait(tmem_full(ab), (tcount >> 1) & 1);
             tc_fence_after();
-            if (!waited) { pdl_wait(); waited = true; }
+            if (!kCluster && !waited) { pdl_wait(); waited = true; }
             if constexpr (kCluster) {
-                // partial sums -> [4 columns][128 rows][4] over the drained ring (every load of this CTA has been consumed)
-                float4* part = reinterpret_cast<float4*>(smem);
+                if (few_rows) {
+                    // partial sums -> [4 columns][128 rows][4] over the drained ring (every load of this CTA has been consumed)
+                    float4* part = reinterpret_cast<float4*>(smem);
+#pragma unroll 1
+                    for (int c0 = 0; c0 < kBN; c0 += 32) {
+                        uint32_t acc[32];
+                        tc_ld32(tmem + ab * kBN + lane_addr + c0, acc);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            part[(c0 / 4 + i) * kBM + r] = make_float4(__uint_as_float(acc[4 * i]), __uint_as_float(acc[4 * i + 1]), __uint_as_float(acc[4 * i + 2]), __uint_as_float(acc[4 * i + 3]));
+                    }
+                    continue;                                   // the only tile of this CTA
+                }
+                // This CTA adds up the columns [lo(rank), lo(rank + 1)) of the tile, in groups of eight; every CTA puts its sums of them there, as [part][group][two of 4 columns][128 rows][4],
+                // over the ring, which is drained in all of them once all have come to the first barrier.
+                __syncwarp();
+                cluster_sync();
+                const bool row_counts = ta * kBM + r < p.m;
+                int to = 0, from = 0, end = (int)(ends & 255u);
 #pragma unroll 1
                 for (int c0 = 0; c0 < kBN; c0 += 32) {
                     uint32_t acc[32];
                     tc_ld32(tmem + ab * kBN + lane_addr + c0, acc);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        part[(c0 / 4 + i) * kBM + r] = make_float4(__uint_as_float(acc[4 * i]), __uint_as_float(acc[4 * i + 1]), __uint_as_float(acc[4 * i + 2]), __uint_as_float(acc[4 * i + 3]));
+                    for (int g = 0; g < 4; ++g) {
+                        const int b = c0 / 8 + g;
+                        if (b == end) { from = end; end = (int)(ends >> (8 * ++to)) & 255; }
+                        const uint32_t own = (uint32_t)(((crank * (end - from) + b - from) * 2) * kBM + r) * 16;
+                        if (!row_counts) continue;
+                        if (to == crank) {
+                            *reinterpret_cast<uint4*>(smem + own) = make_uint4(acc[8 * g], acc[8 * g + 1], acc[8 * g + 2], acc[8 * g + 3]);
+                            *reinterpret_cast<uint4*>(smem + own + kBM * 16) = make_uint4(acc[8 * g + 4], acc[8 * g + 5], acc[8 * g + 6], acc[8 * g + 7]);
+                        } else {
+                            const uint32_t at = cluster_map(smem_base + own, (uint32_t)to);
+                            st_cluster_f32x4(at, acc + 8 * g);
+                            st_cluster_f32x4(at + kBM * 16, acc + 8 * g + 4);
+                        }
+                    }
                 }
                 continue;                                       // the only tile of this CTA
             }
@@ -308,33 +352,27 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
     }
 
     if constexpr (kCluster) {
+        const int crank = (int)blockIdx.x % p.csplit, from = lo_group(crank), groups = lo_group(crank + 1) - from;
+        int ta, tb;
+        tile_coords((int)blockIdx.x / p.csplit, ta, tb);
+        const int r = (warp & 3) * 32 + lane, ia = ta * kBM + r;
+        const TOut* bias = static_cast<const TOut*>(p.bias);
+        const float bias_row = warp >= 2 && p.swap && bias && ia < p.n ? to_f32(bias[ia]) : 0.f;
         __syncwarp();
-        cluster_sync();                                                   // every CTA's sums are written
+        if (warp < 2 && !few_rows) cluster_sync();                        // (the first barrier: the epilogue warps have passed it)
+        cluster_sync();                                                   // every CTA's sums are here, or where they were made
         if (warp >= 2) {
-            const int crank = (int)blockIdx.x % p.csplit;
-            int ta, tb;
-            tile_coords((int)blockIdx.x / p.csplit, ta, tb);
-            const int r = (warp & 3) * 32 + lane, ia = ta * kBM + r;
-            const TOut* bias = static_cast<const TOut*>(p.bias);
-            // eight columns at a time, two CTAs' loads in flight together
-            for (int b = kBN / 8 * crank / p.csplit; b < kBN / 8 * (crank + 1) / p.csplit; ++b) {
-                float v[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = 0.f;
-#pragma unroll 4
-                for (int q = 0; q < p.csplit; ++q) {
-                    const uint32_t at = cluster_map(smem_base + (uint32_t)(b * 2 * kBM + r) * 16, (uint32_t)q);
-                    const float4 f = ld_cluster_f32x4(at), g = ld_cluster_f32x4(at + kBM * 16);
-                    v[0] += f.x; v[1] += f.y; v[2] += f.z; v[3] += f.w; v[4] += g.x; v[5] += g.y; v[6] += g.z; v[7] += g.w;
-                }
+            const float* const held = reinterpret_cast<const float*>(smem + C::kBias);
+            // the sums of eight columns
+            auto store = [&](int b, float (&v)[8]) {
                 const int jb = tb * kBN + b * 8;
                 if (!p.swap) {
-                    if (ia >= p.m) continue;
+                    if (ia >= p.m) return;
                     TOut* dst = static_cast<TOut*>(p.y) + (int64_t)ia * p.ldy + jb;
                     TOut o[8];
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
-                        if (bias && jb + i < p.n) v[i] += to_f32(bias[jb + i]);
+                        if (bias) v[i] += held[(b - from) * 8 + i];
                         o[i] = from_f32<TOut>(v[i]);
                     }
                     if (sizeof(TOut) == 2 && jb + 8 <= p.n && (((uintptr_t)dst) & 15) == 0) *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(o);
@@ -342,15 +380,33 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
                         for (int i = 0; i < 8; ++i)
                             if (jb + i < p.n) dst[i] = o[i];
                 } else if (ia < p.n) {
-                    const float bv = bias ? to_f32(bias[ia]) : 0.f;
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
-                        if (jb + i < p.m) static_cast<TOut*>(p.y)[(int64_t)(jb + i) * p.ldy + ia] = from_f32<TOut>(v[i] + bv);
+                        if (jb + i < p.m) static_cast<TOut*>(p.y)[(int64_t)(jb + i) * p.ldy + ia] = from_f32<TOut>(v[i] + bias_row);
                 }
+            };
+#pragma unroll 2
+            for (int g = 0; g < groups; ++g) {
+                float v[8] = {};
+#pragma unroll 4
+                for (int q = 0; q < p.csplit; ++q) {
+                    float4 x, y;
+                    if (few_rows) {
+                        const uint32_t at = cluster_map(smem_base + (uint32_t)((from + g) * 2 * kBM + r) * 16, (uint32_t)q);
+                        x = ld_cluster_f32x4(at); y = ld_cluster_f32x4(at + kBM * 16);
+                    } else {
+                        const float4* const f = reinterpret_cast<const float4*>(smem) + ((q * groups + g) * 2) * kBM + r;
+                        x = f[0]; y = f[kBM];
+                    }
+                    v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w; v[4] += y.x; v[5] += y.y; v[6] += y.z; v[7] += y.w;
+                }
+                store(from + g, v);
             }
         }
-        __syncwarp();
-        cluster_sync();                                                   // nobody leaves while its shared memory is read
+        if (few_rows) {
+            __syncwarp();
+            cluster_sync();                                               // nobody leaves while its shared memory is read
+        }
     }
     tc_fence_before();
     __syncthreads();
@@ -597,12 +653,16 @@ void launch_out(const CUtensorMap& am, const CUtensorMap& bm, const DenseParams&
     else launch_dense<kBN, __half>(am, bm, p, st);
 }
 
-// CTAs that share a tile over k while there are fewer tiles than SMs: as many as keep every tile's cluster in the first round, at least four k blocks each.  [100 x 4096 x
-// 4096 as 16 clusters of 8: 26 us, a second round for the last one; as 64 single tiles 15.]
+// s CTAs can share each tile over k: all clusters in the first round, at least four k blocks each.  [100 x 4096 x 4096 as 16 clusters of 8: 26 us, a second round for the last one; as 64
+// single tiles 15.]
+bool cluster_fits(int64_t tiles, int nkb, int s) {
+    return tiles * s <= sm_count() && s <= nkb / 4 &&
+           tiles <= max_active_clusters(reinterpret_cast<const void*>(dense_gemm_kernel<128, __nv_bfloat16, true>), kGemmThreads, DCfg<128>::kTotal, s);
+}
+// Up to 64 rows: a weight stream, over as many CTAs as can be had.
 int cluster_split(int64_t tiles, int nkb) {
     for (int s = 8; s > 1; --s)
-        if (tiles * s <= sm_count() && s <= nkb / 4 &&
-            tiles <= max_active_clusters(reinterpret_cast<const void*>(dense_gemm_kernel<128, __nv_bfloat16, true>), kGemmThreads, DCfg<128>::kTotal, s)) return s;
+        if (cluster_fits(tiles, nkb, s)) return s;
     return 1;
 }
 
@@ -641,20 +701,29 @@ bool dense_gemm_16(const void* x, const void* w, const void* bias, void* y, int 
         if (!make_map(&am, w, n, k, ldw, kBM, bf16) || !make_map(&bm, x, m, k, ldx, bn, bf16)) return false;
         if (bn == 32) launch_out<32>(am, bm, p, st); else launch_out<64>(am, bm, p, st);
     } else {
-        // The tile and the split that are done first by this count (clocks): rounds of CTAs (pairs) times (k blocks times the longer of the MMA, 2 BN a block, and
-        // the operands at 64 bytes a clock, plus fixed cost); a shared tile also pays for the sums' way through shared memory.
-        const int64_t nkb = (k + kBK - 1) / kBK;
+        // The tile and the split that are done first by this count (clocks): rounds of CTAs times k blocks, a block's clocks growing with the CTAs that share L2, or the weights' way from
+        // HBM where that is longer; a shared tile pays for the sums' way to the CTAs that add them up.  [Fitted to every (tile, split) at 65 to 1000 rows of six weights.  us, largest split /
+        // so: 100 x 4096 x 4096 13.5 / 12.3, 200 x 4096 x 4096 17.6 / 14.1, 400 x 4096 x 4096 24.9 / 17.1, 100 x 14336 x 4096 32.1 / 25.0, 300 x 6144 x 4096 26 / 19.1, 400 x 2048 x 2048
+        // 13.1 / 8.6; it is within 4 % of the best one everywhere there.]
+        const int64_t nkb = (k + kBK - 1) / kBK, sms = sm_count(), weights = (int64_t)n * k * 2;
         int bn = 256, split = 1;
         int64_t best = INT64_MAX;
         for (int b : {256, 128, 64}) {
             const int64_t tiles = (int64_t)((m + kBM - 1) / kBM) * ((n + b - 1) / b);
-            const int s = accumulate ? 1 : cluster_split(tiles, (int)nkb);
-            const int64_t rounds = (tiles * s + sm_count() - 1) / sm_count(), block = 2 * b > (128 + b) * 2 ? 2 * b : (128 + b) * 2;
-            const int64_t clocks = rounds * ((nkb + s - 1) / s * block + 1500) + (s > 1 ? 2000 + 16 * b : 0);
-            if (clocks < best) { best = clocks; bn = b; split = s; }
+            for (int s = 1; s <= (accumulate ? 1 : 8); ++s) {
+                // (more than two to a cluster: two SMs in sixteen left free, since with clusters on nearly all of them some wait for a place -- 300 x 1024 x 4096 as 48 clusters of 3 11.2 to
+                // 12.8 us, 24 of 5 10.7)
+                if (s > 1 && (tiles * s > sms * (s > 2 ? 14 : 16) / 16 || !cluster_fits(tiles, (int)nkb, s))) continue;
+                const int64_t ctas = tiles * s < sms ? tiles * s : sms, rounds = (tiles * s + sms - 1) / sms;
+                const int64_t block = b == 256 ? 620 + ctas * 12 / 5 : (b == 128 ? 400 + ctas * 9 / 20 : 350), work = rounds * ((nkb + s - 1) / s) * block;
+                const int64_t stream = weights / std::min<int64_t>(b == 64 ? 2400 : 2650, ctas * 22);
+                const int64_t clocks = (work > stream ? work : stream) + (s > 1 ? 2700 + 60 * b : 0);
+                if (clocks < best) { best = clocks; bn = b; split = s; }
+            }
         }
-        const int64_t pair_tiles = (int64_t)((m + 255) / 256) * ((n + 255) / 256), pairs = sm_count() / 2;
-        if (!accumulate && (pair_tiles + pairs - 1) / pairs * (nkb * 512 + 2000) <= best) {
+        const int64_t pair_tiles = (int64_t)((m + 255) / 256) * ((n + 255) / 256), pairs = sms / 2, active = pair_tiles < pairs ? pair_tiles : pairs;
+        const int64_t pair_work = (pair_tiles + pairs - 1) / pairs * nkb * (590 + active * 7 / 5), pair_stream = weights / std::min<int64_t>(2650, active * 44) + 2000;
+        if (!accumulate && (pair_work > pair_stream ? pair_work : pair_stream) <= best) {
             p.swap = 0; p.tiles_a = (m + 255) / 256; p.tiles_b = (n + 255) / 256; p.report = wait_report_word();
             if (!make_map(&am, x, m, k, ldx, kBM, bf16) || !make_map(&bm, w, n, k, ldw, kBM, bf16)) return false;
             if (out_dtype == B200_F32) launch_pair<float>(am, bm, p, st);
