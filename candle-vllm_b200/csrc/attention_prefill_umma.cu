@@ -54,6 +54,10 @@ static_assert(kSmemU <= 232448, "shared memory");
 // a part's results, where Q, K and V were: O f32 [256][128], 16-byte pieces of a row exchanged by its number, then (maximum, sum) of each row
 constexpr int kSmO = 0, kSmMl = 256 * kHd * 4;
 constexpr int kMaxParts = 8, kPartTiles = 2;              // CTAs that share a tile at most; key tiles that a part has at least
+// Key tiles that sharing takes off a CTA, at least: the merge costs what three of them take.  [31 tokens with 32 heads on 594 / 700 / 1000 (5, 6 and 9 key tiles), us: shared by 2, 3
+// and 4 CTAs 20.3 / 18.0 / 19.5, unshared 18.0 / 20.2 / 26.7; eight such prompts on 820 / 900, two CTAs at most a tile: 23.5 unshared / 24.4 shared, 24.9 unshared]
+constexpr int kPartSaves = 4;
+__host__ __device__ constexpr bool parts_pay(int n, int parts) { return n - (n + parts - 1) / parts >= kPartSaves; }
 
 struct UmmaPrefillParams {
     void* out;
@@ -236,6 +240,7 @@ paged_attn_prefill_umma_kernel(const __grid_constant__ CUtensorMap qmap, const _
     int n = max(nk[0], nk[1]), parts = 1;
     if (kSplit) {                                                    // this CTA's key tiles
         parts = min(p.parts, max(n / kPartTiles, 1));
+        if (!parts_pay(n, parts)) parts = 1;
         if (rank >= parts) { leave(); return; }
         const int from = rank * n / parts, to = (rank + 1) * n / parts;
         kt0 += from * kKt;
@@ -674,14 +679,15 @@ bool paged_attention_prefill_umma(void* out, const void* q, const void* kc, cons
     UmmaPrefillParams p{out, vc, block_tables, cu_q, cu_k, num_seqs, num_heads, num_kv_heads, max_blocks, window, chunk, hp, 1, scale * 1.4426950408889634f, sink, wait_report_word()};
     // Few tiles: clusters share their keys, as many CTAs a tile as run at the same time.  (About this many tiles there are, sequences of equal length supposed: the lengths are on the
     // device, and a tile takes fewer CTAs where it has few keys.)  The table's width bounds what a tile can have.
-    // [us without / with, graph: 100 tokens on 4000 75 / 33 (8 CTAs a tile), 512 on 4000 84 / 60 (2), four of 60 on 1000 29 / 25 (4), 700 on 300 with 8 heads 27 / 25 (5).  More CTAs
+    // [us without / with, graph: 100 tokens on 4000 75 / 33 (8 CTAs a tile), 512 on 4000 84 / 60 (2), four of 60 on 1000 29 / 25 (4), 700 on 300 with 8 heads 27 / 24 (4).  More CTAs
     // than run at the same time cost more than they give: 1000 tokens 27 / 45, three prompts of 280 to 701 tokens on prefixes 78 / 136.]
     const int groups = num_heads / hp;
     const int64_t ctas = (int64_t)num_seqs * ceil_div(ceil_div(total_q, num_seqs), 2 * tp) * groups;
     const void* split = bf16 ? reinterpret_cast<const void*>(paged_attn_prefill_umma_kernel<__nv_bfloat16, true>) : reinterpret_cast<const void*>(paged_attn_prefill_umma_kernel<__half, true>);
-    int most = (int)min((int64_t)kMaxParts, (int64_t)max_blocks * kPg / (kPartTiles * kKt));
+    const int key_tiles = min(ceil_div((int64_t)max_blocks * kPg, kKt), kMaxParts * kPartTiles);
+    int most = key_tiles / kPartTiles;
     if (ctas * 2 > sm_count()) most = 1;
-    for (int c = most; c > 1 && p.parts == 1; --c)
+    for (int c = most; c > 1 && p.parts == 1 && parts_pay(key_tiles, c); --c)
         if (max_active_clusters(split, kThreadsU, kSmemU, c) >= ctas) p.parts = c;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)(groups * p.parts), (unsigned)tiles); cfg.blockDim = dim3(kThreadsU); cfg.dynamicSmemBytes = kSmemU; cfg.stream = st;

@@ -15,13 +15,13 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("H,kvh,qlens,cached,window,loud", [
     (8, 2, [5], [8100], None, 1.0),                    # eight parts of eight key tiles
-    (8, 2, [1, 1], [383, 511], None, 1.0),             # three and four key tiles: one part and two
+    (8, 2, [1, 1], [639, 767], None, 1.0),             # five and six key tiles: one part and three
     (32, 8, [100], [1950], None, 1.0),                 # 17 key tiles, the second M tile one token short of a third of its rows
     (4, 4, [250], [900], None, 6.0),                   # one head per tile: the first M tile's last row sees two key tiles less than the second one's; loud scores
-    (4, 4, [256], [0], None, 1.0),                     # no prefix: the second part is hidden from the first M tile
+    (4, 4, [256], [0], None, 1.0),                     # no prefix, two key tiles: not shared
     (8, 2, [64, 3, 40], [2000, 60, 700], None, 1.0),   # tiles of many keys and of few in one launch
     (8, 2, [60], [4000], 700, 1.0),                    # a window: its first key inside a page, six key tiles
-    (8, 2, [64], [4000], 130, 1.0),                    # two or three key tiles, most keys of each hidden from some row
+    (8, 2, [64], [4000], 130, 1.0),                    # two or three key tiles, not shared in a launch of clusters
 ])
 def test_parts_of_a_tile(dtype, H, kvh, qlens, cached, window, loud):
     g = torch.Generator(device=DEV)
