@@ -99,13 +99,17 @@ __device__ __forceinline__ void store_row16(TOut* dst, const uint32_t* acc, cons
     }
 }
 
-// kCluster: tiles shared over k by clusters, in instances of their own: with the branch at run time, or its values in common variables, the others were slower [decode step
+// Tiles shared over k by clusters: kRead up to 64 rows, where every CTA leaves its sums where they are and reads its share of the others'; kSent with more rows, where it sends each CTA its
+// share, since a load from another SM takes a microsecond and a store nothing  [100 rows, 4 CTAs a tile, tile of 128 columns: 5.9 us from the last product on read, 5.1 sent; 32 rows:
+// 2.9 read, 3.3 sent].  In instances of their own: with the branch at run time, or its values in common variables, the others were slower [64 x 6144 x 4096 15.0 / 15.2; decode step
 // with 16-bit weights, 8 layers of 8B sizes, 2 / 9 / 32 rows, us a layer: 120.2 / 124.2 / 136.4, before the cluster split 119.4 / 123.0 / 135.4]
-template <int kBN, typename TOut, bool kCluster>
+enum Share { kAlone, kRead, kSent };
+template <int kBN, typename TOut, Share kShare>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constant__ CUtensorMap bmap, const DenseParams p) {
     using C = DCfg<kBN>;
     constexpr int kS = C::kStages;
+    constexpr bool kCluster = kShare != kAlone, kFewRows = kShare == kRead;
     extern __shared__ __align__(1024) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t smem_base = smem_u32(smem);
@@ -147,10 +151,6 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
             kb0 = nkb_all * z / p.ksplit; kb1 = nkb_all * (z + 1) / p.ksplit;
         }
     };
-    // clusters: the sums' way.  Up to 64 rows (32 or 64 columns a tile) every CTA leaves its sums where they are and reads its share of the others'; with more rows it sends each CTA its
-    // share, since a load from another SM takes a microsecond and a store nothing  [100 rows, 4 CTAs a tile, tile of 128 columns: 5.9 us from the last product on read, 5.1 sent; 32 rows:
-    // 2.9 read, 3.3 sent]
-    const bool few_rows = kBN == 32 || (kBN == 64 && p.swap);
     auto lo_group = [&](int q) { return kBN / 8 * q / p.csplit; };       // clusters: first group of eight columns that CTA q adds up
     auto tile_coords = [&](int t, int& ta, int& tb) {
         if (p.ksplit > 1) { ta = t / p.ksplit; tb = 0; return; }
@@ -245,19 +245,20 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
             const int ab = tcount & 1;
             const int crank = kCluster ? (int)blockIdx.x % p.csplit : 0;
             unsigned long long ends = 0;                        // first group past CTA q's, a byte each
-            if constexpr (kCluster) {
+            if (kCluster && !kFewRows) {
                 for (int q = 0; q < p.csplit; ++q) ends |= (unsigned long long)lo_group(q + 1) << (8 * q);
                 pdl_wait();
-                if (!few_rows && bias) {
+                waited = true;
+                if (bias) {
                     const int j0 = tb * kBN + lo_group(crank) * 8, cols = (lo_group(crank + 1) - lo_group(crank)) * 8;
                     for (int j = threadIdx.x - 64; j < cols; j += 128) reinterpret_cast<float*>(smem + C::kBias)[j] = j0 + j < p.n ? to_f32(bias[j0 + j]) : 0.f;
                 }
             }
             mbar_wait(tmem_full(ab), (tcount >> 1) & 1);
             tc_fence_after();
-            if (!kCluster && !waited) { pdl_wait(); waited = true; }
+            if (!waited) { pdl_wait(); waited = true; }
             if constexpr (kCluster) {
-                if (few_rows) {
+                if (kFewRows) {
                     // partial sums -> [4 columns][128 rows][4] over the drained ring (every load of this CTA has been consumed)
                     float4* part = reinterpret_cast<float4*>(smem);
 #pragma unroll 1
@@ -359,7 +360,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
         const TOut* bias = static_cast<const TOut*>(p.bias);
         const float bias_row = warp >= 2 && p.swap && bias && ia < p.n ? to_f32(bias[ia]) : 0.f;
         __syncwarp();
-        if (warp < 2 && !few_rows) cluster_sync();                        // (the first barrier: the epilogue warps have passed it)
+        if (warp < 2 && !kFewRows) cluster_sync();                        // (the first barrier: the epilogue warps have passed it)
         cluster_sync();                                                   // every CTA's sums are here, or where they were made
         if (warp >= 2) {
             const float* const held = reinterpret_cast<const float*>(smem + C::kBias);
@@ -385,13 +386,13 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
                         if (jb + i < p.m) static_cast<TOut*>(p.y)[(int64_t)(jb + i) * p.ldy + ia] = from_f32<TOut>(v[i] + bias_row);
                 }
             };
-#pragma unroll 2
+#pragma unroll(kFewRows ? 1 : 2)
             for (int g = 0; g < groups; ++g) {
                 float v[8] = {};
 #pragma unroll 4
                 for (int q = 0; q < p.csplit; ++q) {
                     float4 x, y;
-                    if (few_rows) {
+                    if (kFewRows) {
                         const uint32_t at = cluster_map(smem_base + (uint32_t)((from + g) * 2 * kBM + r) * 16, (uint32_t)q);
                         x = ld_cluster_f32x4(at); y = ld_cluster_f32x4(at + kBM * 16);
                     } else {
@@ -403,7 +404,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
                 store(from + g, v);
             }
         }
-        if (few_rows) {
+        if (kFewRows) {
             __syncwarp();
             cluster_sync();                                               // nobody leaves while its shared memory is read
         }
@@ -628,7 +629,8 @@ void launch_cluster(K kern, int grid, int cluster, size_t smem, cudaStream_t st,
 
 template <int kBN, typename TOut>
 void launch_dense(const CUtensorMap& am, const CUtensorMap& bm, const DenseParams& p, cudaStream_t st) {
-    auto kern = p.csplit > 1 ? dense_gemm_kernel<kBN, TOut, true> : dense_gemm_kernel<kBN, TOut, false>;
+    constexpr Share kFew = kBN <= 64 ? kRead : kSent, kMore = kBN == 32 ? kRead : kSent;         // (tiles of 32 columns have few rows only, of 128 and 256 never)
+    auto kern = p.csplit <= 1 ? dense_gemm_kernel<kBN, TOut, kAlone> : (p.swap ? dense_gemm_kernel<kBN, TOut, kFew> : dense_gemm_kernel<kBN, TOut, kMore>);
     ensure_dynamic_smem(reinterpret_cast<const void*>(kern), DCfg<kBN>::kTotal);
     const int tiles = p.tiles_a * p.tiles_b * p.ksplit;
     const int grid = tiles < sm_count() ? tiles : sm_count();
@@ -657,7 +659,7 @@ void launch_out(const CUtensorMap& am, const CUtensorMap& bm, const DenseParams&
 // single tiles 15.]
 bool cluster_fits(int64_t tiles, int nkb, int s) {
     return tiles * s <= sm_count() && s <= nkb / 4 &&
-           tiles <= max_active_clusters(reinterpret_cast<const void*>(dense_gemm_kernel<128, __nv_bfloat16, true>), kGemmThreads, DCfg<128>::kTotal, s);
+           tiles <= max_active_clusters(reinterpret_cast<const void*>(dense_gemm_kernel<128, __nv_bfloat16, kSent>), kGemmThreads, DCfg<128>::kTotal, s);
 }
 // Up to 64 rows: a weight stream, over as many CTAs as can be had.
 int cluster_split(int64_t tiles, int nkb) {
@@ -703,7 +705,7 @@ bool dense_gemm_16(const void* x, const void* w, const void* bias, void* y, int 
     } else {
         // The tile and the split that are done first by this count (clocks): rounds of CTAs times k blocks, a block's clocks growing with the CTAs that share L2, or the weights' way from
         // HBM where that is longer; a shared tile pays for the sums' way to the CTAs that add them up.  [Fitted to every (tile, split) at 65 to 1000 rows of six weights.  us, largest split /
-        // so: 100 x 4096 x 4096 13.5 / 12.3, 200 x 4096 x 4096 17.6 / 14.1, 400 x 4096 x 4096 24.9 / 17.1, 100 x 14336 x 4096 32.1 / 25.0, 300 x 6144 x 4096 26 / 19.1, 400 x 2048 x 2048
+        // so: 100 x 4096 x 4096 13.5 / 12.0, 200 x 4096 x 4096 17.6 / 14.1, 400 x 4096 x 4096 24.9 / 17.1, 100 x 14336 x 4096 32.1 / 25.0, 300 x 6144 x 4096 26 / 19.1, 400 x 2048 x 2048
         // 13.1 / 8.6; it is within 4 % of the best one everywhere there.]
         const int64_t nkb = (k + kBK - 1) / kBK, sms = sm_count(), weights = (int64_t)n * k * 2;
         int bn = 256, split = 1;
@@ -711,8 +713,8 @@ bool dense_gemm_16(const void* x, const void* w, const void* bias, void* y, int 
         for (int b : {256, 128, 64}) {
             const int64_t tiles = (int64_t)((m + kBM - 1) / kBM) * ((n + b - 1) / b);
             for (int s = 1; s <= (accumulate ? 1 : 8); ++s) {
-                // (more than two to a cluster: two SMs in sixteen left free, since with clusters on nearly all of them some wait for a place -- 300 x 1024 x 4096 as 48 clusters of 3 11.2 to
-                // 12.8 us, 24 of 5 10.7)
+                // (more than two to a cluster: two SMs in sixteen left free, since with clusters on nearly all of them some wait for a place -- 300 x 1024 x 4096 as 24 clusters of 6 16.5 us,
+                // of 5 10.5)
                 if (s > 1 && (tiles * s > sms * (s > 2 ? 14 : 16) / 16 || !cluster_fits(tiles, (int)nkb, s))) continue;
                 const int64_t ctas = tiles * s < sms ? tiles * s : sms, rounds = (tiles * s + sms - 1) / sms;
                 const int64_t block = b == 256 ? 620 + ctas * 12 / 5 : (b == 128 ? 400 + ctas * 9 / 20 : 350), work = rounds * ((nkb + s - 1) / s) * block;
