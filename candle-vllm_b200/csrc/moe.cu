@@ -28,14 +28,16 @@ namespace {
 
 // ---- routing ------------------------------------------------------------------------------------------------------------------
 // one warp per token; E <= 32 kPer experts, k <= 32.  logits: `splits` partial sums, split_stride apart (1: finished logits).  normalise: the weights are divided by
-// their sum; all are multiplied by `scaling`.  [With 32 slots per lane whatever E, 16 tokens of 128 experts took 8.0 us.]
+// their sum; all are multiplied by `scaling`.  held: the ids go there too (block's own).  A latency chain: the partial sums come in as few batches as registers allow, and a round of
+// the arg-max is two reductions of integers (redux.sync, one instruction each) where a butterfly of (value, id) takes ten shuffles.  [With 32 slots per lane whatever E, 16 tokens of
+// 128 experts took 8.0 us.]
 template <int kPer>
 __device__ __forceinline__ void topk_token(const float* __restrict__ logits, int splits, int64_t split_stride, float* __restrict__ w_out, uint32_t* __restrict__ id_out,
-                                           int t, int E, int k, int normalise, float scaling) {
+                                           uint32_t* held, int t, int E, int k, int normalise, float scaling) {
     const int lane = threadIdx.x & 31;
     float v[kPer];
     float mx = -INFINITY;
-    constexpr int kBatch = kPer <= 8 ? 4 : 1;          // parts of all slots in flight together, added in order
+    constexpr int kBatch = kPer == 1 ? 16 : (kPer <= 4 ? 8 : (kPer == 8 ? 4 : 1));          // parts of all slots in flight together, added in order
 #pragma unroll
     for (int i = 0; i < kPer; ++i) v[i] = 0.f;
     for (int s = 0; s < splits; s += kBatch) {
@@ -43,7 +45,13 @@ __device__ __forceinline__ void topk_token(const float* __restrict__ logits, int
 #pragma unroll
         for (int i = 0; i < kPer; ++i)
 #pragma unroll
-            for (int j = 0; j < kBatch; ++j) b[i][j] = lane + 32 * i < E && s + j < splits ? logits[(s + j) * split_stride + (int64_t)t * E + lane + 32 * i] : 0.f;
+            for (int j = 0; j < kBatch; ++j) {
+                const int e = lane + 32 * i;
+                if constexpr (kPer == 1) {             // [100 tokens of 32 experts 1.9 us, with a condition around each load 2.9; of 128 it is the other way about: 900 tokens 9.1, 3.2]
+                    const float l = logits[min(s + j, splits - 1) * split_stride + (int64_t)t * E + min(e, E - 1)];
+                    b[i][j] = s + j < splits ? l : 0.f;
+                } else b[i][j] = e < E && s + j < splits ? logits[(s + j) * split_stride + (int64_t)t * E + e] : 0.f;
+            }
 #pragma unroll
         for (int i = 0; i < kPer; ++i)
 #pragma unroll
@@ -60,26 +68,31 @@ __device__ __forceinline__ void topk_token(const float* __restrict__ logits, int
     for (int i = 0; i < kPer; ++i) { v[i] = lane + 32 * i < E ? __expf(v[i] - mx) : 0.f; sum += v[i]; }
     sum = warp_sum(sum);
     const float inv = 1.f / sum;
-    float mine = 0.f, total = 0.f;                     // lane j keeps the weight of round j
+    // What a probability is ordered by: its bits, as it is at least 0, over an entry that has won (1) and NaN (0: it never wins).
+    uint32_t key[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) key[i] = lane + 32 * i < E && v[i] >= 0.f ? __float_as_uint(v[i]) + 2u : 0u;
+    float mine = 0.f, total = 0.f;                     // lane j keeps the weight and the expert of round j
+    uint32_t chosen = 0;
     for (int j = 0; j < k; ++j) {                      // k rounds of arg-max; ties -> the smallest expert id
-        float best = -1.f;
-        int bi = 0x7fffffff;
+        uint32_t top = key[0], at = 0x7fffffffu;
 #pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-            const int e = lane + 32 * i;
-            if (e < E && (v[i] > best || (v[i] == best && e < bi))) { best = v[i]; bi = e; }
-        }
+        for (int i = 1; i < kPer; ++i) top = max(top, key[i]);
+        top = __reduce_max_sync(0xffffffffu, top);
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-        }
-        if (lane == j) { mine = best * inv; id_out[(int64_t)t * k + j] = (uint32_t)bi; }
-        total += best * inv;
+        for (int i = kPer - 1; i >= 0; --i)
+            if (key[i] == top && top) at = lane + 32 * i;
+        at = __reduce_min_sync(0xffffffffu, at);
+        const float weight = (top >= 2 ? __uint_as_float(top - 2u) : -1.f) * inv;
+        if (lane == j) { mine = weight; chosen = at; }
+        total += weight;
 #pragma unroll
         for (int i = 0; i < kPer; ++i)
-            if (lane + 32 * i == bi) v[i] = -1.f;      // remove the winner (probabilities are >= 0)
+            if (lane + 32 * i == (int)at) key[i] = 1u;
+    }
+    if (lane < k) {
+        id_out[(int64_t)t * k + lane] = chosen;
+        if (held) held[t * k + lane] = chosen;
     }
     if (lane < k) w_out[(int64_t)t * k + lane] = (normalise ? mine / total : mine) * scaling;
 }
@@ -90,7 +103,7 @@ topk_softmax_kernel(const float* __restrict__ logits, int splits, int64_t split_
     pdl_wait();
     pdl_trigger();
     const int t = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (t < tokens) topk_token<kPer>(logits, splits, split_stride, w_out, id_out, t, E, k, normalise, scaling);
+    if (t < tokens) topk_token<kPer>(logits, splits, split_stride, w_out, id_out, nullptr, t, E, k, normalise, scaling);
 }
 void topk_launch(const float* logits, int splits, int64_t split_stride, float* w, uint32_t* ids, int tokens, int E, int k, int normalise, float scaling, cudaStream_t st) {
     auto kern = E <= 32 ? topk_softmax_kernel<1> : E <= 128 ? topk_softmax_kernel<4> : E <= 256 ? topk_softmax_kernel<8> : topk_softmax_kernel<32>;
@@ -146,6 +159,60 @@ moe_router_kernel(const float* __restrict__ x, const float* __restrict__ gate, f
             if (t0 + tr * 4 + i < tokens && e0 + er * 4 + j < E) o[(int64_t)(t0 + tr * 4 + i) * E + e0 + er * 4 + j] = acc[i][j];
 }
 
+// The same for up to kRows = 16 or 32 tokens, where only the time until the loads arrive and the chain of steps count: 128 of k at a time in one batch of loads, the next batch in
+// registers, k along the rows of both tiles (no transposing stores, conflict-free 16-byte loads), thread = kRows / 16 x 4.  Each sum runs over k in the same order as above.
+// [16 tokens of 128 experts, H 2048: 4.5 us before, 2.9 so.  With more tokens this layout is level (64 rows, 900 tokens: 21.2 against 22.2 us, 100 of 32 experts: 4.9 against 4.5).]
+constexpr int kRfK = 128, kRfLd = kRfK + 4;
+template <int kRows>
+__global__ void __launch_bounds__(128)
+moe_router_few_kernel(const float* __restrict__ x, const float* __restrict__ gate, float* __restrict__ part, int tokens, int E, int H, int steps_per) {
+    __shared__ __align__(16) float xs[kRows * kRfLd], gs[kRtE * kRfLd];
+    constexpr int kR = kRows / 16;
+    const int e0 = blockIdx.y * kRtE, k0 = blockIdx.z * steps_per * kRtK, k1 = min(k0 + steps_per * kRtK, H);
+    const int tid = threadIdx.x, tr = tid >> 3, er = tid & 7;          // 16 x 8 threads: rows tr + 16 i, experts er + 8 j
+    const int lr = tid >> 5, lc = (tid & 31) * 4;                      // loads: a row a warp
+    pdl_wait();
+    pdl_trigger();
+    float4 xv[kRows / 4], gv[kRtE / 4];
+    auto fetch = [&](int k) {
+        const bool in = k + lc < k1;
+#pragma unroll
+        for (int i = 0; i < kRtE / 4; ++i) { const int e = e0 + lr + 4 * i; gv[i] = in && e < E ? *reinterpret_cast<const float4*>(gate + (int64_t)e * H + k + lc) : make_float4(0.f, 0.f, 0.f, 0.f); }
+#pragma unroll
+        for (int i = 0; i < kRows / 4; ++i) { const int r = lr + 4 * i; xv[i] = in && r < tokens ? *reinterpret_cast<const float4*>(x + (int64_t)r * H + k + lc) : make_float4(0.f, 0.f, 0.f, 0.f); }
+    };
+    float acc[kR][4] = {};
+    if (k0 < k1) fetch(k0);
+    for (int k = k0; k < k1; k += kRfK) {
+#pragma unroll
+        for (int i = 0; i < kRtE / 4; ++i) *reinterpret_cast<float4*>(gs + (lr + 4 * i) * kRfLd + lc) = gv[i];
+#pragma unroll
+        for (int i = 0; i < kRows / 4; ++i) *reinterpret_cast<float4*>(xs + (lr + 4 * i) * kRfLd + lc) = xv[i];
+        __syncthreads();
+        if (k + kRfK < k1) fetch(k + kRfK);
+        const int n = min(kRfK, k1 - k);                               // a multiple of kRtK
+#pragma unroll 8
+        for (int c = 0; c < n; c += 4) {
+            float4 a[kR], b[4];
+#pragma unroll
+            for (int i = 0; i < kR; ++i) a[i] = *reinterpret_cast<const float4*>(xs + (tr + 16 * i) * kRfLd + c);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4*>(gs + (er + 8 * j) * kRfLd + c);
+#pragma unroll
+            for (int i = 0; i < kR; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i].w, b[j].w, fmaf(a[i].z, b[j].z, fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, acc[i][j]))));
+        }
+        __syncthreads();
+    }
+    float* o = part + (int64_t)blockIdx.z * tokens * E;
+#pragma unroll
+    for (int i = 0; i < kR; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (tr + 16 * i < tokens && e0 + er + 8 * j < E) o[(int64_t)(tr + 16 * i) * E + e0 + er + 8 * j] = acc[i][j];
+}
+
 // exclusive prefix sum of one value per thread over a block of 1024; `total` gets the sum.  sums: 33 ints of shared memory
 __device__ __forceinline__ int block_scan_1024(int v, int* sums, int& total) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -167,72 +234,102 @@ __device__ __forceinline__ int block_scan_1024(int v, int* sums, int& total) {
     return sums[warp] + inc - v;
 }
 // chunks of <= rows sorted positions, expert by expert, from the segment [first, first + count) of expert threadIdx.x (block of 1024 = the most experts)
-__device__ __forceinline__ void write_chunks(int e, int first, int count, int rows, MoeChunk* chunks, int* num_chunks, int max_chunks, int* sums) {
-    int total;
+__device__ __forceinline__ void put_chunks(int e, int first, int count, int rows, int at, int total, MoeChunk* chunks, int* num_chunks, int max_chunks) {
     const int nc = (count + rows - 1) / rows;
-    int at = block_scan_1024(nc, sums, total);
     for (int c = 0; c < nc; ++c, ++at)
         if (at < max_chunks) chunks[at] = MoeChunk{e, first + c * rows, min(rows, count - c * rows)};
     if (threadIdx.x == 0) *num_chunks = min(total, max_chunks);
 }
+__device__ __forceinline__ void write_chunks(int e, int first, int count, int rows, MoeChunk* chunks, int* num_chunks, int max_chunks, int* sums) {
+    int total;
+    const int at = block_scan_1024((count + rows - 1) / rows, sums, total);
+    put_chunks(e, first, count, rows, at, total, chunks, num_chunks, max_chunks);
+}
 
 // Stable counting sort of the flattened expert ids, one CTA of 32 warps (experts <= 1024): warp w owns the w-th run of pairs and a histogram of its own; prefix sums over
-// the warps of an expert, then over the experts, give every warp its first position per expert, and a second pass ranks 32 pairs at a time by match.  With chunks it
+// the warps of an expert, then over the experts, give every warp its first position per expert, and a second pass ranks 32 pairs at a time, the lanes
+// with the same expert found by a ballot per bit of its id (match.any takes as many steps as there are different ids: 7200 pairs of 128 experts 11.9 us with it, 8.8 so).  With chunks it
 // also writes the chunk list of the grouped GEMM.  [One thread per expert walking every pair took 124 us for 7200 pairs of 128 experts.]
-// kPer > 0 (few tokens): the top-k of each token comes first, one warp per token, and the ids never leave the SM's caches.
-constexpr int kSortBatch = 8;                                          // ids in flight per lane
+// kPer > 0 (few tokens: 1024 pairs at most): the top-k of each token comes first, one warp per token, the ids stay in shared memory, a warp has one batch of them, and one scan places
+// pairs and chunks.  It is a chain of latencies: [16 tokens of 128 experts, top 8, from the router's last block on, us: 8.2 with ids through memory, butterflies, 32 histograms
+// whatever the pairs and two scans; 5.6 so.  4 of 32 experts 6.0 / 4.5; 1 token 5.3 / 4.1]
 struct TopkArgs { const float* logits; int splits; int64_t split_stride; float* weights; int tokens, k, normalise; float scaling; };
 template <int kPer>
 __global__ void __launch_bounds__(1024)
 moe_sort_kernel(const TopkArgs tk, uint32_t* ids, uint32_t* __restrict__ sorted_expert, uint32_t* __restrict__ sorted_pair, int pairs, int E, MoeChunk* __restrict__ chunks,
                 int* __restrict__ num_chunks, int rows, int max_chunks) {
+    constexpr int kSortBatch = kPer > 0 ? 1 : 8;                       // ids in flight per lane
+    constexpr int kHeld = kPer > 0 ? 1024 : 1;
     extern __shared__ int hist[];                                      // [32][E]
     __shared__ int start[1024], sums[33];
+    __shared__ uint32_t held[kHeld];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < 32 * E; i += 1024) hist[i] = 0;
+    const int per = ((pairs + 31) / 32 + 31) & ~31, p0 = warp * per, p1 = min(pairs, p0 + per), used = (pairs + per - 1) / max(per, 1);       // used: warps that have pairs
+    for (int i = threadIdx.x; i < used * E; i += 1024) hist[i] = 0;
     pdl_wait();
     pdl_trigger();
     if constexpr (kPer > 0)
-        for (int t = warp; t < tk.tokens; t += 32) topk_token<kPer>(tk.logits, tk.splits, tk.split_stride, tk.weights, ids, t, E, tk.k, tk.normalise, tk.scaling);
+        for (int t = warp; t < tk.tokens; t += 32) topk_token<kPer>(tk.logits, tk.splits, tk.split_stride, tk.weights, ids, held, t, E, tk.k, tk.normalise, tk.scaling);
     __syncthreads();
-    const int per = ((pairs + 31) / 32 + 31) & ~31, p0 = warp * per, p1 = min(pairs, p0 + per);
+    auto id_of = [&](int q) { return q < p1 ? (int)min(kPer > 0 ? held[q & (kHeld - 1)] : ids[q], (uint32_t)E - 1) : -1; };
     int* mine = hist + warp * E;
     for (int b = p0; b < p1; b += 32 * kSortBatch) {
         int e[kSortBatch];
 #pragma unroll
-        for (int i = 0; i < kSortBatch; ++i) { const int q = b + 32 * i + lane; e[i] = q < p1 ? (int)min(ids[q], (uint32_t)E - 1) : -1; }
+        for (int i = 0; i < kSortBatch; ++i) e[i] = id_of(b + 32 * i + lane);
 #pragma unroll
         for (int i = 0; i < kSortBatch; ++i) if (e[i] >= 0) atomicAdd(mine + e[i], 1);
     }
     __syncthreads();
-    const int ex = threadIdx.x;
+    const int ex = threadIdx.x, bits = 32 - __clz(E - 1);
     int count = 0;
     if (ex < E)
-        for (int w = 0; w < 32; ++w) { const int c = hist[w * E + ex]; hist[w * E + ex] = count; count += c; }
-    int total;
-    const int first = block_scan_1024(count, sums, total);
+        for (int w = 0; w < used; w += 8) {
+            int c[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) c[i] = w + i < used ? hist[(w + i) * E + ex] : 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (w + i < used) hist[(w + i) * E + ex] = count;
+                count += c[i];
+            }
+        }
+    int total, first, chunk = 0, all_chunks = 0;
+    if constexpr (kPer > 0) {                                          // both sums are at most 1024: one scan
+        const int at = block_scan_1024(count | (count + rows - 1) / rows << 16, sums, total);
+        first = at & 0xffff; chunk = at >> 16; all_chunks = total >> 16;
+    } else first = block_scan_1024(count, sums, total);
     start[ex] = first;
     __syncthreads();
     for (int b = p0; b < p1; b += 32 * kSortBatch) {
         int e[kSortBatch];
 #pragma unroll
-        for (int i = 0; i < kSortBatch; ++i) { const int q = b + 32 * i + lane; e[i] = q < p1 ? (int)min(ids[q], (uint32_t)E - 1) : -1; }
+        for (int i = 0; i < kSortBatch; ++i) e[i] = id_of(b + 32 * i + lane);
+        unsigned same[kSortBatch];
+#pragma unroll
+        for (int i = 0; i < kSortBatch; ++i) same[i] = __ballot_sync(0xffffffffu, e[i] >= 0);
+        for (int bit = 0; bit < bits; ++bit)
+#pragma unroll
+            for (int i = 0; i < kSortBatch; ++i) {
+                const unsigned set = __ballot_sync(0xffffffffu, e[i] >> bit & 1);
+                same[i] &= e[i] >> bit & 1 ? set : ~set;
+            }
 #pragma unroll
         for (int i = 0; i < kSortBatch; ++i) {
-            const unsigned same = __match_any_sync(0xffffffffu, e[i]);
-            const int rank = __popc(same & ((1u << lane) - 1u));
+            const int rank = __popc(same[i] & ((1u << lane) - 1u));
             int base = 0;
             if (e[i] >= 0) base = mine[e[i]] + start[e[i]];
             __syncwarp();
             if (e[i] >= 0) {
-                if (rank == 0) mine[e[i]] += __popc(same);
+                if (rank == 0) mine[e[i]] += __popc(same[i]);
                 if (sorted_expert) sorted_expert[base + rank] = (uint32_t)e[i];
                 sorted_pair[base + rank] = (uint32_t)(b + 32 * i + lane);
             }
             __syncwarp();
         }
     }
-    if (chunks) write_chunks(ex, first, count, rows, chunks, num_chunks, max_chunks, sums);
+    if constexpr (kPer > 0) put_chunks(ex, first, count, rows, chunk, all_chunks, chunks, num_chunks, max_chunks);
+    else if (chunks) write_chunks(ex, first, count, rows, chunks, num_chunks, max_chunks, sums);
 }
 template <int kPer>
 void sort_launch(const TopkArgs& tk, uint32_t* ids, uint32_t* sorted_expert, uint32_t* sorted_pair, int pairs, int E, MoeChunk* chunks, int* num_chunks, int rows, int max_chunks, cudaStream_t st) {
@@ -543,8 +640,8 @@ void moe_block_gguf(const float* x, const float* router, const void* gate, const
     float* g = reinterpret_cast<float*>(ws + p.gu);
     float* u = g + (int64_t)P * inter;
     float* y = reinterpret_cast<float*>(ws + p.y);
-    launch_pdl(moe_router_kernel, dim3(ceil_div(num_tokens, kRtT), ceil_div(num_experts, kRtE), p.splits), dim3(128), 0, st, x, router, logits, (int)num_tokens,
-               (int)num_experts, (int)hidden, p.steps_per);
+    launch_pdl(num_tokens <= 16 ? moe_router_few_kernel<16> : (num_tokens <= 32 ? moe_router_few_kernel<32> : moe_router_kernel),
+               dim3(ceil_div(num_tokens, kRtT), ceil_div(num_experts, kRtE), p.splits), dim3(128), 0, st, x, router, logits, (int)num_tokens, (int)num_experts, (int)hidden, p.steps_per);
     route_launch(TopkArgs{logits, p.splits, (int64_t)num_tokens * num_experts, weights, num_tokens, topk, normalise, scaling}, ids, pair, P, num_experts, chunks, count,
                  p.rows, p.max_chunks, st);
     launch_pdl(moe_gather_kernel, dim3(ceil_div(P, 8)), dim3(256), 0, st, x, (const uint32_t*)pair, xs, P, (int)hidden, 1, (int)topk);
