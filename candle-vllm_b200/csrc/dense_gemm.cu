@@ -717,7 +717,8 @@ bool dense_gemm_16(const void* x, const void* w, const void* bias, void* y, int 
                 // of 5 10.5)
                 if (s > 1 && (tiles * s > sms * (s > 2 ? 14 : 16) / 16 || !cluster_fits(tiles, (int)nkb, s))) continue;
                 const int64_t ctas = tiles * s < sms ? tiles * s : sms, rounds = (tiles * s + sms - 1) / sms;
-                const int64_t block = b == 256 ? 620 + ctas * 12 / 5 : (b == 128 ? 400 + ctas * 9 / 20 : 350), work = rounds * ((nkb + s - 1) / s) * block;
+                // (all SMs together get 8400 bytes a clock from L2: 1122 x 4096 x 14336 in two rounds of 128 columns 136 us, one of 256 114)
+                const int64_t own = b == 256 ? 620 + ctas * 12 / 5 : (b == 128 ? 400 + ctas * 9 / 20 : 350), block = std::max<int64_t>(own, ctas * (128 + b) * 128 / 8400), work = rounds * ((nkb + s - 1) / s) * block;
                 const int64_t stream = weights / std::min<int64_t>(b == 64 ? 2400 : 2650, ctas * 22);
                 const int64_t clocks = (work > stream ? work : stream) + (s > 1 ? 2700 + 60 * b : 0);
                 if (clocks < best) { best = clocks; bn = b; split = s; }
