@@ -22,6 +22,8 @@
 //     and no CTA barrier in the steady state.
 //   * per item the warp writes an fp32 partial (m, l, O) straight from registers; a tiny merge kernel
 //     folds the chunks of each (sequence, head), rounds to bf16 and re-zeroes the queue head.
+//   * few sequences of short contexts wait for latencies, not for memory: there a cluster has all of a
+//     (sequence, kv head) and merges in shared memory, without queue, partials and merge kernel.
 //
 // Semantics: softmax(q k^T * scale) v over the block table, GQA by head grouping
 // (NaiveAttention::forward src/openai/models/mod.rs:1268-1307; call sites
@@ -141,6 +143,13 @@ __device__ __forceinline__ float fast_exp2(float x) {
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
 __device__ __forceinline__ void named_bar_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
@@ -156,6 +165,7 @@ struct DecodeParams {
     int adaptive_chunks;           // 1: the kernel may halve chunk_pages from the device-side context lengths (B200_ATTN_ADAPTIVE=0: off)
     int static_walk;               // queue mode: 0 per-warp tickets, 1 CTA tickets (FP8 cache), 2 static walk (B200_ATTN_STATIC overrides)
     float scale_log2;                 // scale * log2(e)
+    void* out; int out_dtype, ctas;   // kWhole: the result; CTAs of a cluster (1, 2, 4 or 8)
 };
 
 // The size of a chunk from the device-side context lengths: the host proposes p.chunk_pages (pick_chunk_pages, from the table width); items are whole chunks, so the makespan is rounds x
@@ -186,7 +196,9 @@ __device__ __forceinline__ void ldmatrix_x2_trans_b8(uint32_t (&r)[4], uint32_t 
     asm volatile("ldmatrix.sync.aligned.m16n16.x2.trans.shared.b8 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
 
-template <typename T, int kGroup, bool kFp8>
+// kWhole (few sequences of short contexts): a cluster has all of a (sequence, kv head), an equal run of pages a warp, and merges in shared memory: no queue, no partials in memory, no merge
+// kernel, no walk over the sequences.  Every CTA folds its warps' parts and sends each CTA of the cluster the dims that that one finishes.
+template <typename T, int kGroup, bool kFp8, bool kWhole>
 __global__ void __launch_bounds__(Plan<kFp8>::kThreads, 1)
 paged_attn_decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap,
                          const DecodeParams p) {
@@ -213,8 +225,17 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_
     }
     pdl_wait();            // context_lens / q / KV written by the previous kernels
     pdl_trigger();
+    int whole_b = 0, whole_ctx = 0;
     int* prefix_half = reinterpret_cast<int*>(smem + PL::kHalf);           // chunk prefix for the halved chunk size
     int* decision = reinterpret_cast<int*>(smem + PL::kMail + 96);
+    int chunk_pages, total_items = 0;
+    if constexpr (kWhole) {
+        __syncwarp();
+        cluster_arrive();                                       // (the CTAs of the cluster have started: waited for before the first word is sent)
+        whole_b = blockIdx.x / p.ctas / p.num_kv_heads;
+        whole_ctx = min((int)p.context_lens[whole_b], p.max_blocks * kPage);
+        chunk_pages = max((whole_ctx + kPage * p.ctas * PL::kWarps - 1) / (kPage * p.ctas * PL::kWarps), 1);
+    } else {
     {
         const int ct0 = p.chunk_pages * kPage, ct1 = (p.chunk_pages > 1 ? p.chunk_pages / 2 : 1) * kPage;
         for (int b = threadIdx.x; b < p.num_seqs; b += kThreads) {
@@ -230,10 +251,11 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_
         decision[0] = settled_chunk_pages(prefix[p.num_seqs], prefix_half[p.num_seqs], p.num_kv_heads, (int)gridDim.x * PL::kWarps, p.chunk_pages, p.adaptive_chunks);
     }
     __syncthreads();
-    const int chunk_pages = decision[0];
-    const int chunk_tokens = chunk_pages * kPage;
+    chunk_pages = decision[0];
     if (chunk_pages != p.chunk_pages) prefix = prefix_half;
-    const int total_items = prefix[p.num_seqs] * p.num_kv_heads;
+    total_items = prefix[p.num_seqs] * p.num_kv_heads;
+    }
+    const int chunk_tokens = chunk_pages * kPage;
 
     // Claiming the next item of the global queue is split in two so that neither the atomic's round trip (~1 us) nor the block-table
     // load sits in the consumer's instruction stream: claim_begin() issues the atomicAdd, claim_finish() -- one tile later, or at
@@ -249,11 +271,12 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_
     // a CTA = blockIdx + k * grid; uniform batches only; kept for comparison).
     // Mailbox protocol: slot j % 8 holds {j + 1, T}; a reader acknowledges, and warp 0 re-uses a slot only after all kWarps - 1
     // readers of its previous ticket have acknowledged.  Warp 0 never waits for a ticket, readers only for warp 0's own progress.
-    const int qmode = p.static_walk == 2 ? (prefix[p.num_seqs] == p.num_seqs * prefix[1] ? 2 : 0) : p.static_walk;
+    const int qmode = kWhole ? 0 : p.static_walk == 2 ? (prefix[p.num_seqs] == p.num_seqs * prefix[1] ? 2 : 0) : p.static_walk;
     unsigned long long* mail = reinterpret_cast<unsigned long long*>(smem + PL::kMail);
     unsigned int* acks = reinterpret_cast<unsigned int*>(smem + PL::kMail + 64);
     unsigned int n_begun = 0;
     auto claim_begin = [&]() {
+        if constexpr (kWhole) { pending = true; return; }
         // the first ticket of every warp / CTA is its own index: no atomic round trip (~1 us) before the first TMA of the launch
         if (qmode == 2) pend_id = (blockIdx.x + n_begun * gridDim.x) * PL::kWarps + warp;
         else if (n_begun == 0) pend_id = qmode == 1 ? blockIdx.x : blockIdx.x * PL::kWarps + warp;
@@ -272,6 +295,22 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_
         pending = true;
     };
     auto claim_finish = [&](bool& valid, int& h, int& ntiles) -> uint32_t {
+        if constexpr (kWhole) {
+            int* hd = hdr + (n_claimed & 7) * 8;
+            const int c = (int)blockIdx.x % p.ctas * PL::kWarps + warp, ntok = min(chunk_tokens, whole_ctx - c * chunk_tokens);
+            pending = false;
+            valid = n_claimed == 0 && ntok > 0;
+            ++n_claimed;
+            h = 0; ntiles = 0;
+            if (!valid) {
+                if (lane == 0) hd[0] = 0;
+                return 0u;
+            }
+            h = (int)blockIdx.x / p.ctas % p.num_kv_heads;
+            ntiles = (ntok + kTile - 1) / kTile;
+            if (lane == 0) { hd[0] = 1; hd[1] = whole_b; hd[2] = h; hd[3] = c; hd[4] = whole_ctx; hd[5] = ntiles; }
+            return lane < (ntok + kPage - 1) / kPage ? p.block_tables[(int64_t)whole_b * p.max_blocks + c * chunk_pages + lane] : 0u;
+        }
         unsigned int id = __shfl_sync(0xffffffffu, pend_id, 0);
         if (qmode == 1 && n_begun == 1) id = id * PL::kWarps + warp;          // ticket 0 = blockIdx, known to every warp
         else if (qmode == 1) {
@@ -523,12 +562,68 @@ paged_attn_decode_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_
         // ---- fp32 partial of this item straight from registers ----------------------------------------
         l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
         l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
-        if (g < kGroup) {
+        if constexpr (kWhole) {
+            // over the warp's own ring, which is drained: O [group][128], then (m, l) of each row
+            float* const mine = reinterpret_cast<float*>(smem + warp * PL::kWarpBytes);
+            if (g < kGroup) {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) *reinterpret_cast<float2*>(mine + g * kHeadDim + i * 8 + 2 * t) = make_float2(o[i][0], o[i][1]);
+                if (t == 0) *reinterpret_cast<float2*>(mine + kGroup * kHeadDim + g * 2) = make_float2(m_run, l_run);
+            }
+        } else if (g < kGroup) {
             const int64_t slot = (((int64_t)b * p.num_kv_heads + h) * p.max_chunks + c) * kGroup + g;
             float* orow = p.part_o + slot * kHeadDim;
 #pragma unroll
             for (int i = 0; i < 16; ++i) *reinterpret_cast<float2*>(orow + i * 8 + 2 * t) = make_float2(o[i][0], o[i][1]);
             if (t == 0) { p.part_ml[slot * 2] = m_run; p.part_ml[slot * 2 + 1] = l_run; }
+        }
+    }
+    if constexpr (kWhole) {
+        const int rank = (int)blockIdx.x % p.ctas, h = (int)blockIdx.x / p.ctas % p.num_kv_heads, share = kHeadDim / p.ctas;
+        // what the other CTAs send lies where the other form has its prefix sums: O of this CTA's dims [CTA][group][share], (m, l) [CTA][group]
+        const uint32_t land_o = smem_base + PL::kPrefix, land_ml = land_o + kGroup * kHeadDim * 4;
+        auto part_ml = [&](int w, int r) { return *reinterpret_cast<const float2*>(smem + w * PL::kWarpBytes + (kGroup * kHeadDim + r * 2) * 4); };
+        const int used = min(PL::kWarps, max((whole_ctx + chunk_tokens - 1) / chunk_tokens - rank * PL::kWarps, 0));             // warps that have written O
+        __syncthreads();
+        cluster_wait();
+        for (int i = threadIdx.x; i < kGroup * kHeadDim / 4; i += kThreads) {
+            const int r = i / (kHeadDim / 4), d = i % (kHeadDim / 4) * 4, to = d / share;
+            float M = -INFINITY, L = 0.f;
+            for (int w = 0; w < used; ++w) M = fmaxf(M, part_ml(w, r).x);
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int w = 0; w < used; ++w) {
+                const float2 ml = part_ml(w, r);
+                const float4 v = *reinterpret_cast<const float4*>(smem + w * PL::kWarpBytes + (r * kHeadDim + d) * 4);
+                const float e = M == -INFINITY ? 0.f : exp2f(ml.x - M);
+                L += e * ml.y; acc.x += e * v.x; acc.y += e * v.y; acc.z += e * v.z; acc.w += e * v.w;
+            }
+            const uint32_t at = cluster_map(land_o + ((rank * kGroup + r) * share + d - to * share) * 4, (uint32_t)to);
+            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(acc.x), "f"(acc.y), "f"(acc.z), "f"(acc.w) : "memory");
+            if (d == to * share)                                // (the first thread of each CTA's dims sends it the row's maximum and sum)
+                asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(cluster_map(land_ml + (rank * kGroup + r) * 8, (uint32_t)to)), "f"(M), "f"(L) : "memory");
+        }
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        for (int i = threadIdx.x; i < kGroup * share / 4; i += kThreads) {
+            const int r = i / (share / 4), d = i % (share / 4) * 4;
+            const float2* const ml = reinterpret_cast<const float2*>(smem + PL::kPrefix + kGroup * kHeadDim * 4);
+            float M = -INFINITY, L = 0.f;
+            for (int q = 0; q < p.ctas; ++q) M = fmaxf(M, ml[q * kGroup + r].x);
+            float acc[4] = {};
+            for (int q = 0; q < p.ctas; ++q) {
+                const float e = M == -INFINITY ? 0.f : exp2f(ml[q * kGroup + r].x - M);
+                const float4 v = *reinterpret_cast<const float4*>(smem + PL::kPrefix + ((q * kGroup + r) * share + d) * 4);
+                L += e * ml[q * kGroup + r].y; acc[0] += e * v.x; acc[1] += e * v.y; acc[2] += e * v.z; acc[3] += e * v.w;
+            }
+            const int64_t at = ((int64_t)whole_b * p.num_heads + h * kGroup + r) * kHeadDim + rank * share + d;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const T v = from_f32<T>(whole_ctx > 0 && L > 0.f ? acc[e] / L : 0.f);
+                if (p.out_dtype == B200_F16) static_cast<__half*>(p.out)[at + e] = from_f32<__half>(to_f32(v));
+                else if (p.out_dtype == B200_F16_K4) static_cast<__half*>(p.out)[at + k4_index(e)] = from_f32<__half>(to_f32(v));
+                else static_cast<T*>(p.out)[at + e] = v;
+            }
         }
     }
 }
@@ -682,10 +777,49 @@ int pick_chunk_pages(int num_seqs, int kvh, int max_blocks) {
     return chunk;
 }
 
+// CTAs of a cluster for the form with a cluster to a (sequence, kv head), or 0: as many as run at the same time, where no warp has more than four pages.  The contexts are on the
+// device; the table's width bounds them.
+// [us the whole call, queue and merge kernel / so, 32 query and 8 kv heads, 16-bit cache: one sequence of 64 9.0 / 7.2, of 700 9.4 / 7.5, of 8000 13.7 / 12.0; four of 1500 12.4 / 9.8, of
+// 6000 21.9 / 19.1; eight of 700 11.5 / 9.5; 16 of 1500 20.6 / 18.8; 8-bit cache: one of 700 11.4 / 8.5, four of 6000 20.4 / 15.4.  With more pages a warp sequences of like length gain
+// (eight of 6000, 8 pages 36.7 / 32.4), but clusters of short ones leave their SMs idle where the queue would not (lengths down to an eighth of the longest: 16 of 2000, 6 pages 19.4 /
+// 20.0; two of 8000, 6 pages 16.1 / 17.8; 16 of 3000 with an 8-bit cache, 6 pages 20.6 / 21.8); up to four pages nothing was slower.]
+// Clusters on fewer than 64 SMs read memory too slowly for that much: one page a warp, two of an 8-bit cache.  [one sequence, 4 kv heads, 32 CTAs: of 3000 10.4 / 8.3, 4500 (two pages)
+// 10.6 / 10.3, in a graph 10.1 / 10.5, 7400 (three) 11.6 / 12.5; 8-bit: of 7400 (two) 13.8 / 12.1.  64 CTAs, 7400 (three) 13.2 / 12.2]
+template <bool kFp8>
+int whole_ctas(const void* kern, const DecodeArgs& a) {
+    using PL = Plan<kFp8>;
+    const int64_t pairs = (int64_t)a.num_seqs * a.num_kv_heads;
+    for (int c = 8; c >= 1; c >>= 1)
+        if (pairs * c <= sm_count()) {
+            const int pages = pairs * c >= 64 ? 4 : (kFp8 ? 2 : 1);
+            if (a.max_blocks > c * PL::kWarps * pages) return 0;
+            ensure_dynamic_smem(kern, PL::kTotal);
+            if (max_active_clusters(kern, PL::kThreads, PL::kTotal, c) >= pairs) return c;
+        }
+    return 0;
+}
+
 template <typename T, typename TOut, int kGroup, bool kK4, bool kFp8>
 void launch(const DecodeArgs& a, const CUtensorMap& kmap, const CUtensorMap& vmap, const DecodeParams& p, cudaStream_t st) {
     using PL = Plan<kFp8>;
-    auto kern = paged_attn_decode_kernel<T, kGroup, kFp8>;
+    if (const int ctas = whole_ctas<kFp8>(reinterpret_cast<const void*>(paged_attn_decode_kernel<T, kGroup, kFp8, true>), a)) {
+        auto kern = paged_attn_decode_kernel<T, kGroup, kFp8, true>;
+        DecodeParams w = p;
+        w.out = a.out; w.out_dtype = a.out_dtype; w.ctas = ctas;
+        ensure_dynamic_smem(reinterpret_cast<const void*>(kern), PL::kTotal);
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)(a.num_seqs * a.num_kv_heads * ctas)); cfg.blockDim = dim3(PL::kThreads); cfg.dynamicSmemBytes = PL::kTotal; cfg.stream = st;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = (unsigned)ctas; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr; cfg.numAttrs = 2;
+        cudaLaunchKernelEx(&cfg, kern, kmap, vmap, w);
+        count_launch();
+        return;
+    }
+    auto kern = paged_attn_decode_kernel<T, kGroup, kFp8, false>;
     ensure_dynamic_smem(reinterpret_cast<const void*>(kern), PL::kTotal);
     const int64_t max_items = (int64_t)a.num_seqs * a.num_kv_heads * p.max_chunks;
     const int64_t want = (max_items + PL::kWarps - 1) / PL::kWarps;

@@ -1,0 +1,52 @@
+"""Decode attention with a cluster to a (sequence, kv head): clusters of 8, 4, 2 and 1 CTA, contexts of none, of one token and on either side of a page, CTAs and warps without a page,
+tables on either side of what the form takes, 16-bit and e4m3 caches, every result layout.  Reference, inputs and bound as in test_decode_merge_gpu.py (weights and result rounded to the
+16-bit type: 2^-9 / sqrt(3) each in the mean square for bf16); e4m3 is exact in f16, where queries and weights are rounded to 2^-12."""
+import ctypes as C
+
+import pytest
+import torch
+
+import candle_vllm_b200 as pkg
+from tests.test_decode_merge_gpu import _reference
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("fp8", [False, True])
+@pytest.mark.parametrize("heads,kv_heads,lens", [
+    (32, 8, [700]),                              # clusters of 8
+    (8, 8, [64]),                                # one page: one warp of eight CTAs
+    (8, 1, [3072, 1]),                           # the most that 16 CTAs take, 16-bit; a cluster with one page beside it
+    (8, 1, [3073, 6000]),                        # more with a 16-bit cache, not with an 8-bit one
+    (8, 8, [8000]),                              # three pages a warp
+    (32, 8, [1500, 0, 65, 64]),                  # 4; an empty context
+    (16, 8, [63, 700, 129, 1, 2, 640, 700, 3]),  # 2
+    (4, 4, [40] * 30 + [1536]),                  # 1: a warp has four pages
+    (4, 4, [40] * 30 + [1537 + 512]),            # more than the form takes
+])
+def test_clusters(dtype, fp8, heads, kv_heads, lens):
+    gen = torch.Generator(device="cuda").manual_seed(len(lens) + heads)
+    mk = lambda *s: torch.randn(*s, generator=gen, device="cuda").to(dtype)
+    width, blocks, seqs = max(-(-n // 64) for n in lens), 150, len(lens)
+    kc, vc, q = mk(blocks, 64, kv_heads, 128), mk(blocks, 64, kv_heads, 128), mk(seqs, heads, 128)
+    if fp8:
+        kc, vc = kc.to(torch.float8_e4m3fn), vc.to(torch.float8_e4m3fn)
+    tables = torch.randint(0, blocks, (seqs, width), generator=gen, device="cuda", dtype=torch.int32)
+    ctx = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    L = pkg.lib()
+    ws = torch.zeros(int(L.paged_attention_decode_workspace_bytes(*map(C.c_int32, (seqs, heads, 128, width, 64)))), dtype=torch.uint8, device="cuda")
+    p = lambda t: C.c_void_p(t.data_ptr())
+    held = torch.tensor([n > 0 for n in lens], device="cuda")
+    ref = _reference(q, kc.to(dtype), vc.to(dtype), tables, [max(n, 1) for n in lens], heads // kv_heads)[held]
+    code = 2 if dtype == torch.bfloat16 else 1
+    for result in {code, 1, 5}:                  # the model's type, f16, f16 in the order [0, 2, 1, 3] of each four
+        out = torch.full_like(q, 7.0) if result == code else torch.full(q.shape, 7.0, dtype=torch.float16, device="cuda")
+        L.paged_attention_decode(p(out), p(q), p(kc), p(vc), p(tables), p(ctx), *map(C.c_int32, (seqs, heads, kv_heads, 128, 64, width)), C.c_int64(blocks), C.c_float(128 ** -0.5),
+                                 C.c_float(0), *map(C.c_int32, (0, code, 4 if fp8 else code, 0, result)), p(ws), C.c_size_t(ws.numel()), C.c_int64(torch.cuda.current_stream().cuda_stream))
+        assert L.b200_last_error() == 0
+        assert not out[~held].any()
+        y = out[held].double()
+        if result == 5:
+            y = y.unflatten(-1, (32, 4))[..., [0, 2, 1, 3]].flatten(-2)
+        assert float((y - ref).norm() / ref.norm()) < (2.5e-3 if dtype == torch.bfloat16 else 6e-4)
