@@ -152,6 +152,7 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
         }
     };
     auto lo_group = [&](int q) { return kBN / 8 * q / p.csplit; };       // clusters: first group of eight columns that CTA q adds up
+    float bias_row = 0.f;                                                // kRead: the bias of this thread's row, asked for before the products are done
     auto tile_coords = [&](int t, int& ta, int& tb) {
         if (p.ksplit > 1) { ta = t / p.ksplit; tb = 0; return; }
         if (p.tile_group && p.swap) { tb = t / p.tiles_a; ta = t - tb * p.tiles_a; return; }
@@ -245,7 +246,11 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
             const int ab = tcount & 1;
             const int crank = kCluster ? (int)blockIdx.x % p.csplit : 0;
             unsigned long long ends = 0;                        // first group past CTA q's, a byte each
-            if (kCluster && !kFewRows) {
+            if constexpr (kFewRows) {
+                pdl_wait();
+                waited = true;
+                if (bias && ta * kBM + r < p.n) bias_row = to_f32(bias[ta * kBM + r]);
+            } else if constexpr (kCluster) {
                 for (int q = 0; q < p.csplit; ++q) ends |= (unsigned long long)lo_group(q + 1) << (8 * q);
                 pdl_wait();
                 waited = true;
@@ -358,7 +363,6 @@ dense_gemm_kernel(const __grid_constant__ CUtensorMap amap, const __grid_constan
         tile_coords((int)blockIdx.x / p.csplit, ta, tb);
         const int r = (warp & 3) * 32 + lane, ia = ta * kBM + r;
         const TOut* bias = static_cast<const TOut*>(p.bias);
-        const float bias_row = warp >= 2 && p.swap && bias && ia < p.n ? to_f32(bias[ia]) : 0.f;
         __syncwarp();
         if (warp < 2 && !kFewRows) cluster_sync();                        // (the first barrier: the epilogue warps have passed it)
         cluster_sync();                                                   // every CTA's sums are here, or where they were made
