@@ -200,24 +200,24 @@ extern "C" {
 // Which products take the "dequantise once + dense tensor-core GEMM" path: the 16-bit copy of W costs ~4.6 bytes of traffic per weight (0.56 read, 2 written, 2 read back), a
 // row tile of 256 of the dequant-GEMM its conversion, in the instance that rounds a weight once, as the 16-bit copy does.  us, this path / dequant-GEMM:
 //                 1024 x 4096    4096 x 4096    14336 x 4096    4096 x 14336    6144 x 2048    2048 x 6144    (n x k)
-//   Q4_K  512     28.9 / 25.6    66.8 / 28.3    153 / 78        184 / 79        56.3 / 31.6    53.8 / 29.7
-//         1024    35.7 / 25.6    66.8 / 44.0    205 / 155       205 / 145       81.9 / 61.6    70.8 / 42.1
-//         1150    35.8 / 26.1    67.1 / 78.4    216 / 169       210 / 245       79.0 / 57.7    69.7 / 59.7
-//         1536    50.0 / 31.3    91.6 / 81.0    255 / 224       283 / 243       70.7 / 54.7    74.0 / 62.2
-//         2048    52.4 / 34.4    97.1 / 84.8    316 / 307       304 / 261       94.7 / 91.5    80.8 / 73.7
-//   Q6_K  512     25.0 / 21.2    58.3 / 28.6    125 / 78        168 / 86        57.1 / 34.9    58.4 / 32.3
-//         1024    33.8 / 22.7    58.5 / 43.6    186 / 160       182 / 152       79.0 / 64.3    80.1 / 48.9
-//         1150    35.8 / 27.9    58.7 / 78.6    197 / 165       185 / 248       69.4 / 61.1    64.6 / 58.7
-//         1536    49.1 / 31.2    83.5 / 80.6    227 / 244       255 / 251       66.7 / 56.8    70.0 / 62.0
-//         2048    50.3 / 34.5    88.5 / 84.9    319 / 325       316 / 296       105 / 95.8     77.0 / 75.2
-// So Q4_K stays with the dequant-GEMM as far as one call of it goes (a second would convert the weights again; 2300 rows 338 / 342 at 14336 x 4096, 100 / 101 at 4096 x 4096),
-// Q6_K to where wide matrices lose what narrow ones gain; and below that, what takes the dequant-GEMM a second round of tiles that leaves it under three fifths full, while the
-// dense GEMM's tiles of 128 x 256 fit one round, goes the dense way (1025 to 1152 rows of 4096 columns on 148 SMs).  Where the dequant-GEMM has no tensor-core form (Q8_0, Q6_K
-// with k not a multiple of 2048) the dense path starts at kDenseRows.
+//   Q4_K  512     23.6 / 18.1     48.1 / 25.6     145 / 61.1      151 / 64.9      44.9 / 21.7     46.0 / 23.1
+//         1024    26.7 / 20.5     62.7 / 35.5     189 / 124       183 / 118       58.3 / 37.8     51.3 / 33.4
+//         1150    27.3 / 23.5     63.8 / 60.9     192 / 138       198 / 198       57.9 / 38.0     52.9 / 44.9
+//         1536    30.6 / 26.5     84.5 / 63.6     220 / 175       259 / 201       61.6 / 40.0     70.8 / 47.9
+//         2048    34.3 / 29.0     88.8 / 70.3     267 / 235       281 / 233       75.2 / 57.1     75.8 / 56.0
+//   Q6_K  512     21.7 / 18.0     40.3 / 25.6     118 / 62.1      143 / 62.7      39.1 / 25.0     39.7 / 23.5
+//         1024    24.7 / 20.3     54.3 / 34.6     162 / 127       184 / 112       52.3 / 44.3     45.0 / 33.0
+//         1150    25.4 / 23.1     55.7 / 58.8     169 / 141       176 / 190       56.3 / 44.6     47.9 / 43.0
+//         1536    28.7 / 26.0     76.3 / 60.9     196 / 174       237 / 195       56.4 / 41.5     65.1 / 46.6
+//         2048    32.5 / 28.4     80.4 / 70.6     246 / 235       256 / 230       70.9 / 57.6     70.3 / 55.3
+// So both stay with the dequant-GEMM as far as one call of it goes (a second would convert the weights again; Q4_K with 2300 rows 338 / 342 at 14336 x 4096, 100 / 101 at 4096 x 4096),
+// but for Q6_K where it takes a second round of tiles that leaves it under three fifths full, while the dense GEMM's tiles of 128 x 256 fit one round (1025 to 1152 rows of 4096 columns on
+// 148 SMs; Q4_K is level or faster there).  Where the dequant-GEMM has no tensor-core form (Q8_0, Q6_K with k not a multiple of 2048) the dense path starts at kDenseRows.
 static constexpr int kDenseRows = kSingleRoundingRows;
 static bool takes_dense_path(int m, int n, int k, int ggml_type) {
     if (m < kDenseRows) return false;
-    if (!qmatmul_tc_usable(m, n, k, ggml_type) || m > (ggml_type == B200_GGML_Q4_K ? kMaxRows : 1407)) return true;
+    if (!qmatmul_tc_usable(m, n, k, ggml_type) || m > kMaxRows) return true;
+    if (ggml_type == B200_GGML_Q4_K) return false;
     const int64_t sms = sm_count(), tiles = (int64_t)((n + 127) / 128) * ((m + 255) / 256), rounds = (tiles + sms - 1) / sms;
     return rounds > 1 && 5 * tiles < 3 * rounds * sms && (int64_t)((m + 127) / 128) * ((n + 255) / 256) <= sms;
 }

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("t", [pkg.GgmlType.Q4_K, pkg.GgmlType.Q6_K])
-@pytest.mark.parametrize("m", [33, 64, 65, 96, 97, 128, 129, 160, 225, 256, 257, 300, 513, 1000])
+@pytest.mark.parametrize("m", [33, 64, 65, 96, 97, 128, 129, 160, 225, 256, 257, 300, 513, 1000, 1408, 2048, 2049])
 def test_row_tiles(t, m):
     gen = torch.Generator(device=DEV)
     gen.manual_seed(m)
